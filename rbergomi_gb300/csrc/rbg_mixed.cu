@@ -1896,88 +1896,130 @@ __device__ __forceinline__ float mc_payoff_f32(float Ivdt, float IsvdW, float Is
     return fmaxf(ex2_approx(1.4426950408889634f * lnS) - K, 0.0f);
 }
 
+// A block's outputs in FP32: (rho, K, ln K, variance group; -1 past the last).
+// The block converts each output once, into shared memory: the conversions
+// from double run on GB300's FP64 pipe (64 cycles a warp instruction), and
+// every thread doing its own eight outputs' (and eight logarithms) for as few
+// as one path took most of the kernel's time on a large grid.  Held in
+// registers over the path loop from there: 48 x 44 outputs at 2^17 paths 2.86
+// -> 0.77 ms, 21 outputs at 2^22 paths 0.200 -> 0.190 ms.
+struct OutF32 {
+    float rho, K, lnK;
+    int vg;
+};
+
+constexpr int kMaxOutBlocks32 = 4;  // runs of 8 outputs one block of k_payoff_sums_f32 may take
+
+__device__ __forceinline__ void load_outs_f32(const OutDev* __restrict__ outs, int n_out, int o0, int n, OutF32* so)
+{
+    if ((int)threadIdx.x < n) {
+        const int i = o0 + (int)threadIdx.x;
+        const OutDev od = (i < n_out) ? outs[i] : OutDev{0.0, 1.0, -1, 0};
+        so[threadIdx.x] = OutF32{(float)od.rho, (float)od.K, logf((float)od.K), od.vg};
+    }
+    __syncthreads();
+}
+
+// Warp sums of 16 values per lane, in the order of the xor tree 16, 8, 4, 2, 1:
+// each of the first four steps hands half of the values to the partner lane,
+// so 15 exchanges and one last step replace 80.  Returns, on every lane, the
+// sum of value (lane >> 1).
+__device__ __forceinline__ float warp_sums16(float (&v)[16])
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int n = 8, o = 16; n >= 1; n >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const float send = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
 // One block of the FP32 payoff sums: chunk c (paths [256 G c, 256 G (c + 1)))
-// and outputs [o0, o0 + 8).  Shared by the per-request and job-table kernels,
-// so a request's sums do not depend on which of them ran.
+// and nb <= kMaxOutBlocks32 runs of 8 outputs from o0.  Shared by the
+// per-request and job-table kernels, so a request's sums do not depend on
+// which of them ran.
+// The warps' sums are merged in FP64 by one lane per sum, up to 32 sums a
+// warp: an FP64 warp instruction holds its pipe for 64 cycles whatever its
+// active lanes, so a block that takes several runs of outputs pays for that
+// merge once.
 template <bool MC>
 __device__ __forceinline__ void payoff_sums_block(const OutDev* __restrict__ outs, int n_out,
                                                   const float2* __restrict__ ivb, int64_t B, int G,
                                                   double* __restrict__ part, const float* __restrict__ ivq, int c,
-                                                  int o0, double (*red)[kOPB32][2])
+                                                  int o0, int nb)
 {
+    __shared__ OutF32 so[kMaxOutBlocks32 * kOPB32];
+    __shared__ float red[8][2 * kMaxOutBlocks32 * kOPB32];  // [warp][run][sum of x | sum of x^2][output]
+    load_outs_f32(outs, n_out, o0, nb * kOPB32, so);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    float rho[kOPB32], K[kOPB32], lnK[kOPB32];
-    int vg[kOPB32];
-#pragma unroll
-    for (int q = 0; q < kOPB32; ++q) {
-        const int i = o0 + q;
-        const OutDev od = (i < n_out) ? outs[i] : OutDev{0.0, 1.0, -1, 0};
-        rho[q] = (float)od.rho; K[q] = (float)od.K; lnK[q] = logf((float)od.K); vg[q] = od.vg;
-    }
-    // each thread sums its own G paths in FP32 (G <= a few dozen), FP64 from the warp level up
-    float s1[kOPB32], s2[kOPB32];
-#pragma unroll
-    for (int q = 0; q < kOPB32; ++q) { s1[q] = 0.f; s2[q] = 0.f; }
-    for (int sub = 0; sub < G; ++sub) {
-        const int64_t m = ((int64_t)c * G + sub) * 256 + threadIdx.x;
-        if (m >= B) break;
-        int cur = -1;
-        float2 iv = make_float2(0.f, 0.f);
-        float ip = 0.f, srho = 0.f;
-        RtSpot sp{};
+    for (int b = 0; b < nb; ++b) {
+        float rho[kOPB32], K[kOPB32], lnK[kOPB32];
+        int vg[kOPB32];
 #pragma unroll
         for (int q = 0; q < kOPB32; ++q) {
-            if (vg[q] < 0) continue;
-            bool fresh = false;
-            if (vg[q] != cur) {
-                cur = vg[q];
-                iv = ivb[(size_t)cur * B + m];
-                if (MC) ip = ivq[(size_t)cur * B + m];
-                fresh = true;
-            }
-            // the strike-independent terms once per (group, rho): outputs of one
-            // ParamTot tuple share them
-            if (!MC && (fresh || rho[q] != srho)) {
-                sp = rt_spot_f32(iv.x, iv.y, rho[q]);
-                srho = rho[q];
-            }
-            const float x = MC ? mc_payoff_f32(iv.x, iv.y, ip, rho[q], K[q]) : rt_payoff_f32(sp, K[q], lnK[q]);
-            s1[q] += x;
-            s2[q] = fmaf(x, x, s2[q]);
+            const OutF32 od = so[b * kOPB32 + q];
+            rho[q] = od.rho; K[q] = od.K; lnK[q] = od.lnK; vg[q] = od.vg;
         }
-    }
-    // warp tree in FP32 (GB300's FP64 pipe is far too slow for warp-wide
-    // shuffles), one FP64 value per warp and output
+        // each thread sums its own G paths in FP32 (G <= a few dozen), FP64 from the warp level up
+        float s[2 * kOPB32];  // sums of x, then of x^2
 #pragma unroll
-    for (int q = 0; q < kOPB32; ++q) {
-        float a = s1[q], b = s2[q];
+        for (int q = 0; q < 2 * kOPB32; ++q) s[q] = 0.f;
+        for (int sub = 0; sub < G; ++sub) {
+            const int64_t m = ((int64_t)c * G + sub) * 256 + threadIdx.x;
+            if (m >= B) break;
+            int cur = -1;
+            float2 iv = make_float2(0.f, 0.f);
+            float ip = 0.f, srho = 0.f;
+            RtSpot sp{};
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            a += __shfl_xor_sync(0xffffffffu, a, o);
-            b += __shfl_xor_sync(0xffffffffu, b, o);
+            for (int q = 0; q < kOPB32; ++q) {
+                if (vg[q] < 0) continue;
+                bool fresh = false;
+                if (vg[q] != cur) {
+                    cur = vg[q];
+                    iv = ivb[(size_t)cur * B + m];
+                    if (MC) ip = ivq[(size_t)cur * B + m];
+                    fresh = true;
+                }
+                // the strike-independent terms once per (group, rho): outputs of one
+                // ParamTot tuple share them
+                if (!MC && (fresh || rho[q] != srho)) {
+                    sp = rt_spot_f32(iv.x, iv.y, rho[q]);
+                    srho = rho[q];
+                }
+                const float x = MC ? mc_payoff_f32(iv.x, iv.y, ip, rho[q], K[q]) : rt_payoff_f32(sp, K[q], lnK[q]);
+                s[q] += x;
+                s[kOPB32 + q] = fmaf(x, x, s[kOPB32 + q]);
+            }
         }
-        if (lane == 0) { red[w][q][0] = (double)a; red[w][q][1] = (double)b; }
+        // warp tree in FP32 (GB300's FP64 pipe is far too slow for warp-wide shuffles)
+        const float t = warp_sums16(s);
+        if (!(lane & 1)) red[w][2 * kOPB32 * b + (lane >> 1)] = t;
     }
     __syncthreads();
-    if (threadIdx.x < kOPB32 && o0 + (int)threadIdx.x < n_out) {
-        const int q = threadIdx.x;
-        double S = 0, CS = 0, S2 = 0, CS2 = 0;
-        for (int k = 0; k < 8; ++k) {
-            neumaier_add(S, CS, red[k][q][0]);
-            neumaier_add(S2, CS2, red[k][q][1]);
-        }
-        double* pp = part + ((size_t)c * n_out + o0 + q) * 4;
-        pp[0] = S; pp[1] = CS; pp[2] = S2; pp[3] = CS2;
+    // lane (run b, sum z, output q): the 8 warps' values in order, one Neumaier sum
+    const int b = threadIdx.x >> 4, z = (threadIdx.x >> 3) & 1, q = threadIdx.x & 7;
+    if (b < nb && o0 + b * kOPB32 + q < n_out) {
+        double S = 0, C = 0;
+        for (int k = 0; k < 8; ++k) neumaier_add(S, C, (double)red[k][threadIdx.x]);
+        double* pp = part + ((size_t)c * n_out + o0 + b * kOPB32 + q) * 4 + 2 * z;
+        *reinterpret_cast<double2*>(pp) = make_double2(S, C);
     }
 }
 
 template <bool MC>
 __global__ void __launch_bounds__(256) k_payoff_sums_f32(const OutDev* __restrict__ outs, int n_out,
                                                          const float2* __restrict__ ivb, int64_t B, int G,
-                                                         double* __restrict__ part, const float* __restrict__ ivq)
+                                                         double* __restrict__ part, const float* __restrict__ ivq,
+                                                         int nb)
 {
-    __shared__ double red[8][kOPB32][2];
-    payoff_sums_block<MC>(outs, n_out, ivb, B, G, part, ivq, blockIdx.x, blockIdx.y * kOPB32, red);
+    const int o0 = blockIdx.y * nb * kOPB32, left = (n_out - o0 + kOPB32 - 1) / kOPB32;
+    payoff_sums_block<MC>(outs, n_out, ivb, B, G, part, ivq, blockIdx.x, o0, left < nb ? left : nb);
 }
 
 // Job-table form: block b of the launch is block b - jobs[k].block0 of job k
@@ -1985,7 +2027,6 @@ __global__ void __launch_bounds__(256) k_payoff_sums_f32(const OutDev* __restric
 // block = local / nchunks).
 __global__ void __launch_bounds__(256) k_payoff_sums_f32_jobs(const PayoffJob* __restrict__ jobs, int n_jobs)
 {
-    __shared__ double red[8][kOPB32][2];
     int lo = 0, hi = n_jobs - 1;
     while (lo < hi) {  // last job whose first block is <= blockIdx.x
         const int mid = (lo + hi + 1) >> 1;
@@ -1994,15 +2035,19 @@ __global__ void __launch_bounds__(256) k_payoff_sums_f32_jobs(const PayoffJob* _
     const PayoffJob& J = jobs[lo];
     const int local = (int)((int64_t)blockIdx.x - J.block0);
     payoff_sums_block<false>(J.outs, J.n_out, J.ivb, J.B, J.G, J.part, nullptr, local % J.nchunks,
-                             (local / J.nchunks) * kOPB32, red);
+                             (local / J.nchunks) * kOPB32, 1);
 }
 
 void launch_payoff_sums_f32(const OutDev* outs, int n_out, const void* ivb, int64_t B, int G, double* part,
                             int nchunks, cudaStream_t st, const float* ivq)
 {
-    dim3 grid(nchunks, (n_out + kOPB32 - 1) / kOPB32);
-    if (ivq) k_payoff_sums_f32<true><<<grid, 256, 0, st>>>(outs, n_out, (const float2*)ivb, B, G, part, ivq);
-    else k_payoff_sums_f32<false><<<grid, 256, 0, st>>>(outs, n_out, (const float2*)ivb, B, G, part, ivq);
+    // runs of 8 outputs per block: more of them where that still leaves 16 blocks an SM
+    const int64_t runs = (n_out + kOPB32 - 1) / kOPB32;
+    int nb = 1;
+    while (nb < kMaxOutBlocks32 && nchunks * ((runs + nb) / (nb + 1)) >= 16 * (int64_t)device_sms()) ++nb;
+    const dim3 grid(nchunks, (unsigned)((runs + nb - 1) / nb));
+    auto* kern = ivq ? k_payoff_sums_f32<true> : k_payoff_sums_f32<false>;
+    kern<<<grid, 256, 0, st>>>(outs, n_out, (const float2*)ivb, B, G, part, ivq, nb);
     count_launch();
 }
 
