@@ -22,6 +22,7 @@
 #include <tuple>
 #include <vector>
 
+#include "rbg_fp64x.hpp"
 #include "rbg_internal.hpp"
 #include "rbg_mixed.hpp"
 
@@ -144,6 +145,9 @@ struct DevBuf {
 struct TableSet {
     Fp64Tables t{};
     const double* Tvals = nullptr;
+    const X64Vol* xvols = nullptr;  // fixed-point path pass only
+    const X64Group* xgrps = nullptr;
+    const uint64_t* xcomp = nullptr;
 };
 
 struct Ctx {
@@ -151,6 +155,9 @@ struct Ctx {
     cudaStream_t stream = nullptr;
     std::mutex mu;
     DevBuf z, ivb, ivp, part, acc, tabs, res, pay, mixed_ws, cv, sobol, sobol32;
+    // fixed-point FP64 path pass: digits of W1, X, and the Toeplitz panels of the tables in `tabs`
+    DevBuf xdig, xbuf, xpan;
+    bool xpan_ready = false;
     // host images of what `tabs`, `mixed_ws` and `sobol` hold, so that a call
     // with the same tables (a calibration loop, a benchmark) uploads nothing
     std::vector<unsigned char> tabs_img, mixed_img;
@@ -238,8 +245,10 @@ static int fp64_conv_log2(int conv, int N, int* logL)
 }
 
 // logL > 0: also the FP64 FFT convolution's spectra (one per distinct H) and
-// twiddles
-static int upload_tables(Ctx& c, const Plan& plan, cudaStream_t st, TableSet& ts, int logL = 0)
+// twiddles; xt: also the fixed-point path pass's tables, and its Toeplitz
+// panels (built on the device, kept with the tables)
+static int upload_tables(Ctx& c, const Plan& plan, cudaStream_t st, TableSet& ts, int logL = 0,
+                         const X64Tables* xt = nullptr)
 {
     const int nv = (int)plan.vols.size(), ng = (int)plan.vgs.size(), no = (int)plan.outs.size(), N = plan.N;
     std::vector<VolDev> vols(nv);
@@ -264,8 +273,18 @@ static int upload_tables(Ctx& c, const Plan& plan, cudaStream_t st, TableSet& ts
     const size_t L = logL > 0 ? (size_t)1 << logL : 0;
     size_t off_spec = align_up(off_comp + sizeof(double) * plan.comp.size(), 256);
     size_t off_tw = align_up(off_spec + 2 * sizeof(double) * L * nv, 256);
-    size_t total = align_up(off_tw + 2 * sizeof(double) * L, 256);
+    size_t off_xvols = align_up(off_tw + 2 * sizeof(double) * L, 256);
+    size_t off_xgrps = align_up(off_xvols + (xt ? sizeof(X64Vol) * nv : 0), 256);
+    size_t off_xgam = align_up(off_xgrps + (xt ? sizeof(X64Group) * ng : 0), 256);
+    size_t off_xcomp = align_up(off_xgam + (xt ? 8 * (size_t)nv * N : 0), 256);
+    size_t total = align_up(off_xcomp + (xt ? 8 * (size_t)ng * N : 0), 256);
     std::vector<unsigned char> host(total, 0);
+    if (xt) {
+        std::memcpy(host.data() + off_xvols, xt->vols.data(), sizeof(X64Vol) * nv);
+        std::memcpy(host.data() + off_xgrps, xt->grps.data(), sizeof(X64Group) * ng);
+        std::memcpy(host.data() + off_xgam, xt->gam.data(), 8 * xt->gam.size());
+        std::memcpy(host.data() + off_xcomp, xt->comp.data(), 8 * xt->comp.size());
+    }
     if (logL > 0)
         fp64_fft_tables(plan.gamma.data(), nv, N, logL, (double*)(host.data() + off_spec),
                         (double*)(host.data() + off_tw));
@@ -277,6 +296,7 @@ static int upload_tables(Ctx& c, const Plan& plan, cudaStream_t st, TableSet& ts
     std::memcpy(host.data() + off_comp, plan.comp.data(), sizeof(double) * plan.comp.size());
     if (!(c.tabs.p && c.tabs_img == host)) {
         c.tabs_img.clear();
+        c.xpan_ready = false;
         ++c.img_gen;
         int rc = ensure(c.tabs, total, "tables");
         if (rc) return rc;
@@ -300,6 +320,18 @@ static int upload_tables(Ctx& c, const Plan& plan, cudaStream_t st, TableSet& ts
     ts.t.N = N;
     ts.t.xi = plan.xi;
     ts.Tvals = (const double*)(base + off_T);
+    if (xt) {
+        ts.xvols = (const X64Vol*)(base + off_xvols);
+        ts.xgrps = (const X64Group*)(base + off_xgrps);
+        ts.xcomp = (const uint64_t*)(base + off_xcomp);
+        if (!c.xpan_ready) {
+            int rc = ensure(c.xpan, x64_panel_bytes(N) * (size_t)nv, "convolution panels");
+            if (rc) return rc;
+            launch_panels((const int64_t*)(base + off_xgam), nv, N, (unsigned char*)c.xpan.p, st);
+            RBG_CUDA(cudaGetLastError());
+            c.xpan_ready = true;
+        }
+    }
     return RBG_OK;
 }
 
@@ -362,11 +394,21 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
 {
     TableSet ts;
     int logL = 0;
-    int rc = fp64_conv_log2(o.conv, plan.N, &logL);
+    // Philox normals, no backend asked for: the exact tensor-core convolution and
+    // fixed-point functions wherever the plan's numbers fit their ranges
+    X64Tables xt;
+    const bool fixed = o.conv == RBG_CONV_AUTO && !sobol_vt && x64_prepare(plan, xt);
+    int rc = fixed ? RBG_OK : fp64_conv_log2(o.conv, plan.N, &logL);
     if (rc) return rc;
-    if ((rc = upload_tables(c, plan, st, ts, logL))) return rc;
-    const int no = (int)plan.outs.size(), N = plan.N, ns = mc ? 3 : 2;
+    if ((rc = upload_tables(c, plan, st, ts, logL, fixed ? &xt : nullptr))) return rc;
+    const int no = (int)plan.outs.size(), N = plan.N, ns = mc ? 3 : 2, nv = (int)plan.vols.size();
     const int64_t B = fp64_batch(plan, M, ns);
+    // passes per convolution launch: X within 2 GiB
+    const int vstep = (int)std::max<int64_t>(1, std::min<int64_t>(nv, ((int64_t)1 << 31) / (8 * (int64_t)N * B)));
+    if (fixed) {
+        if ((rc = ensure(c.xdig, x64_digit_bytes(B, N), "normal digits"))) return rc;
+        if ((rc = ensure(c.xbuf, 8 * (size_t)vstep * N * (size_t)B, "Volterra paths"))) return rc;
+    }
     if ((rc = ensure(c.z, sizeof(double) * ns * N * (size_t)B, "normals"))) return rc;
     if ((rc = ensure(c.ivb, sizeof(double) * 2 * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
     if (mc && (rc = ensure(c.ivp, sizeof(double) * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
@@ -374,9 +416,11 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
     const int G = payoff_paths_per_thread(B, device_sms());
     const int64_t max_chunks = (B + 256 * (int64_t)G - 1) / (256 * (int64_t)G);
     if ((rc = ensure(c.part, sizeof(double) * 4 * no * (size_t)max_chunks, "partials"))) return rc;
-    if ((rc = ensure(c.acc, sizeof(double) * 4 * no, "accumulators"))) return rc;
+    // the kernel error word follows the accumulators
+    if ((rc = ensure(c.acc, sizeof(double) * (4 * no + 1), "accumulators"))) return rc;
     if ((rc = ensure(c.res, sizeof(double) * 5 * no, "results"))) return rc;
-    RBG_CUDA(cudaMemsetAsync(c.acc.p, 0, sizeof(double) * 4 * no, st));
+    RBG_CUDA(cudaMemsetAsync(c.acc.p, 0, sizeof(double) * (4 * no + 1), st));
+    unsigned int* err = (unsigned int*)(c.acc.as<double>() + 4 * no);
     for (int64_t m0 = 0; m0 < M; m0 += B) {
         const int64_t b = std::min(B, M - m0);
         {
@@ -384,14 +428,23 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
             if (sobol_vt) {
                 if (launch_sobol_normals(sobol_vt, N, (uint64_t)(o.path_offset + m0 + 1), b, br, c.z.as<double>(), st))
                     return fail(RBG_ERR_UNSUPPORTED, "Brownian bridge shared memory not available for this N");
-            } else {
-                launch_normals(o.seed, o.path_offset + m0, b, N, o.normals == RBG_NORMALS_F32, c.z.as<double>(), st,
-                               ns);
+            } else if (launch_normals_fixed(o.seed, o.path_offset + m0, b, N, o.normals == RBG_NORMALS_F32,
+                                            c.z.as<double>(), fixed ? c.xdig.as<unsigned char>() : nullptr, ns, st)) {
+                return fail(RBG_ERR_CUDA, "normal tables could not be set up");
             }
         }
         {
-            ProfScope ps(kStagePathFp64, st);
-            launch_path_fp64(ts.t, c.z.as<double>(), b, c.ivb.as<double>(), st, ivp);
+            ProfScope ps(kStagePathFp64, st, fixed ? 2 * ((nv + vstep - 1) / vstep) : 1);
+            if (!fixed) launch_path_fp64(ts.t, c.z.as<double>(), b, c.ivb.as<double>(), st, ivp);
+            for (int v0 = 0; fixed && v0 < nv; v0 += vstep) {
+                const int k = std::min(vstep, nv - v0);
+                if (launch_volterra_exact(c.xdig.as<unsigned char>(),
+                                          c.xpan.as<unsigned char>() + (size_t)v0 * x64_panel_bytes(N), ts.xvols + v0, k, N,
+                                          b, c.xbuf.as<uint64_t>(), err, st) ||
+                    launch_variance_fixed(ts.xvols + v0, ts.xgrps, ts.xcomp, c.z.as<double>(), c.xbuf.as<uint64_t>(), k,
+                                          xt.max_groups, ns, N, b, c.ivb.as<double>(), ivp, st))
+                    return fail(RBG_ERR_CUDA, "FP64 path kernels could not be configured");
+            }
         }
         const int nchunks = (int)((b + 256 * (int64_t)G - 1) / (256 * (int64_t)G));
         {
@@ -407,8 +460,12 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
     launch_finalize(c.acc.as<double>(), no, M, ts.t.outs, ts.Tvals, o.compute_iv, c.res.as<double>(), st);
     RBG_CUDA(cudaGetLastError());
     RBG_CUDA(cudaMemcpyAsync(host_res, c.res.p, sizeof(double) * 5 * no, cudaMemcpyDeviceToHost, st));
+    unsigned int word = 0;
+    if (fixed) RBG_CUDA(cudaMemcpyAsync(&word, err, 4, cudaMemcpyDeviceToHost, st));
     RBG_CUDA(cudaStreamSynchronize(st));
-    g_d2h += sizeof(double) * 5 * no;
+    if (word)
+        return fail(RBG_ERR_TIMEOUT, "FP64 convolution: a bounded pipeline wait expired (site " + std::to_string(word) + ")");
+    g_d2h += sizeof(double) * 5 * no + (fixed ? 4 : 0);
     prof_collect();
     return RBG_OK;
 }
@@ -655,7 +712,9 @@ static int price_cv(Ctx& c, const Plan& plan, const rbg_cv_params& p, const rbg_
     if (Zc) {
         RBG_CUDA(cudaMemcpyAsync(c.z.p, Zc, sizeof(double) * 2 * N * Mc, cudaMemcpyHostToDevice, st));
     } else {
-        launch_normals(o.seed, kCvPilotPath0 + o.path_offset, Mc, N, o.normals == RBG_NORMALS_F32, c.z.as<double>(), st);
+        if (launch_normals_fixed(o.seed, kCvPilotPath0 + o.path_offset, Mc, N, o.normals == RBG_NORMALS_F32,
+                                 c.z.as<double>(), nullptr, 2, st))
+            return fail(RBG_ERR_CUDA, "normal tables could not be set up");
     }
     launch_path_fp64(ts.t, c.z.as<double>(), Mc, c.ivb.as<double>(), st);
     launch_cv_pilot(ts.t, c.ivb.as<double>(), Mc, xy, alpha, Q, st);
@@ -668,7 +727,9 @@ static int price_cv(Ctx& c, const Plan& plan, const rbg_cv_params& p, const rbg_
             RBG_CUDA(cudaMemcpyAsync(c.z.p, Z + (size_t)m0 * 2 * N, sizeof(double) * 2 * N * b, cudaMemcpyHostToDevice,
                                      st));
         } else {
-            launch_normals(o.seed, o.path_offset + m0, b, N, o.normals == RBG_NORMALS_F32, c.z.as<double>(), st);
+            if (launch_normals_fixed(o.seed, o.path_offset + m0, b, N, o.normals == RBG_NORMALS_F32, c.z.as<double>(),
+                                     nullptr, 2, st))
+                return fail(RBG_ERR_CUDA, "normal tables could not be set up");
         }
         launch_path_fp64(ts.t, c.z.as<double>(), b, c.ivb.as<double>(), st, nullptr, c.ivp.as<double>());
         const int nchunks = (int)((b + 256 * (int64_t)G - 1) / (256 * (int64_t)G));
@@ -723,7 +784,8 @@ static int price_cv_mixed(Ctx& c, const Plan& plan, const rbg_cv_params& p, cons
     unsigned long long* count = (unsigned long long*)(Q + no);
     double* xy = (double*)(count + no);
     // pilot: one FP64 batch of Mc paths on FP32 normals
-    launch_normals(o.seed, kCvPilotPath0 + o.path_offset, Mc, N, 1, c.z.as<double>(), st);
+    if (launch_normals_fixed(o.seed, kCvPilotPath0 + o.path_offset, Mc, N, 1, c.z.as<double>(), nullptr, 2, st))
+        return fail(RBG_ERR_CUDA, "normal tables could not be set up");
     launch_path_fp64(ts.t, c.z.as<double>(), Mc, c.ivp.as<double>(), st);
     launch_cv_pilot(ts.t, c.ivp.as<double>(), Mc, xy, alpha, Q, st);
     RBG_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned long long) * no, st));
@@ -1053,7 +1115,9 @@ int rbg_generate_normals_streams(uint64_t seed, int64_t path_offset, int64_t M, 
     if ((rc = ensure(c->z, sizeof(double) * ns * N * (size_t)B, "normals"))) return rc;
     for (int64_t m0 = 0; m0 < M; m0 += B) {
         const int64_t b = std::min(B, M - m0);
-        launch_normals(seed, path_offset + m0, b, N, precision == RBG_MIXED, c->z.as<double>(), c->stream, ns);
+        if (launch_normals_fixed(seed, path_offset + m0, b, N, precision == RBG_MIXED, c->z.as<double>(), nullptr, ns,
+                                 c->stream))
+            return fail(RBG_ERR_CUDA, "normal tables could not be set up");
         RBG_CUDA(cudaGetLastError());
         RBG_CUDA(cudaMemcpyAsync(Z + m0 * ns * N, c->z.p, sizeof(double) * ns * N * b, cudaMemcpyDeviceToHost,
                                  c->stream));
@@ -1267,8 +1331,9 @@ int rbg_release(void)
     RBG_CUDA(cudaDeviceSynchronize());
     for (Ctx* c : all) {
         for (DevBuf* b : {&c->z, &c->ivb, &c->ivp, &c->part, &c->acc, &c->tabs, &c->res, &c->pay, &c->mixed_ws,
-                          &c->cv, &c->sobol, &c->sobol32})
+                          &c->cv, &c->sobol, &c->sobol32, &c->xdig, &c->xbuf, &c->xpan})
             b->release();
+        c->xpan_ready = false;
         c->tabs_img.clear();
         c->mixed_img.clear();
         c->sobol_img.clear();

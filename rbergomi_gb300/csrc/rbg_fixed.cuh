@@ -1,0 +1,246 @@
+// rbg_fixed.cuh -- 64-bit fixed-point arithmetic for the FP64 form.
+//
+// GB300 issues an FP64 warp instruction every 64 cycles per SM sub-partition
+// (2 DFMA per clock and SM) and an integer one every cycle, so the FP64 form's
+// elementary functions -- Box-Muller's logarithm, square root and sine /
+// cosine, the variance path's exponential -- are evaluated on 64-bit integers.
+// Each keeps more bits than FP64 evaluation does: a few 2^-58 (absolute for a
+// normal, relative for the exponential) against roundings of 2^-53.
+// Everything here also compiles for the host, where it is tested against
+// quadruple precision.
+#pragma once
+
+#include <cmath>
+#include <cstdint>
+#include <cstring>
+
+#ifdef __CUDACC__
+#define RBG_HD __host__ __device__ __forceinline__
+#else
+#define RBG_HD inline
+#endif
+
+namespace rbg {
+
+RBG_HD uint32_t hi32(uint64_t x) { return (uint32_t)(x >> 32); }
+RBG_HD uint32_t lo32(uint64_t x) { return (uint32_t)x; }
+RBG_HD uint64_t mul32(uint32_t a, uint32_t b) { return (uint64_t)a * b; }
+RBG_HD uint32_t mulhi32(uint32_t a, uint32_t b)
+{
+#ifdef __CUDA_ARCH__
+    return __umulhi(a, b);
+#else
+    return (uint32_t)(((uint64_t)a * b) >> 32);
+#endif
+}
+// High half of a 64 x 64-bit product without the low x low term: three
+// 32 x 32 -> 64 multiplies, 0 to 2 below the exact one.
+RBG_HD uint64_t mulhi64(uint64_t a, uint64_t b)
+{
+    return mul32(hi32(a), hi32(b)) + (mul32(hi32(a), lo32(b)) >> 32) + (mul32(lo32(a), hi32(b)) >> 32);
+}
+RBG_HD int clz64(uint64_t x)
+{
+#ifdef __CUDA_ARCH__
+    return __clzll((long long)x);
+#else
+    return x ? __builtin_clzll(x) : 64;
+#endif
+}
+RBG_HD double bits_double(uint64_t b)
+{
+#ifdef __CUDA_ARCH__
+    return __longlong_as_double((long long)b);
+#else
+    double d;
+    std::memcpy(&d, &b, 8);
+    return d;
+#endif
+}
+RBG_HD uint64_t double_bits(double d)
+{
+#ifdef __CUDA_ARCH__
+    return (uint64_t)__double_as_longlong(d);
+#else
+    uint64_t b;
+    std::memcpy(&b, &d, 8);
+    return b;
+#endif
+}
+
+// ------------------------------------------------------------------ normals
+// Normals in signed fixed point, unit 2^-59 (|z| < 16; Box-Muller on 32-bit
+// uniforms stays below 6.77).
+constexpr int kNormalBits = 59;
+
+// v 2^-59 as a double, rounded to nearest (ties away from zero).
+RBG_HD double fixed_to_double(int64_t v)
+{
+    const uint64_t s = (uint64_t)(v >> 63);
+    const uint64_t a = ((uint64_t)v ^ s) - s;
+    const int n = clz64(a);
+    const uint64_t w = a << (n & 63);
+    // 53 bits of w; their leading one, or the rounding's carry past it, adds to the exponent field
+    const uint64_t m = (w >> 11) + ((w >> 10) & 1u);
+    const uint64_t b = ((uint64_t)(uint32_t)(1023 + 62 - kNormalBits - n) << 52) + m;
+    return bits_double(a ? (b | (s << 63)) : 0ull);
+}
+
+// x in units of 2^-59, exact for 2^-6 <= |x| < 16 and truncated below.
+RBG_HD int64_t double_to_fixed(double x)
+{
+    const uint64_t b = double_bits(x);
+    const int sh = ((int)(b >> 52) & 2047) - (1023 + 52 - kNormalBits);  // <= 11 for |x| < 16
+    const uint64_t m = (b & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
+    const uint64_t a = sh >= 0 ? m << (sh & 63) : (sh > -64 ? m >> (-sh & 63) : 0ull);
+    const uint64_t s = (uint64_t)((int64_t)b >> 63);
+    return (int64_t)((a ^ s) - s);
+}
+
+// Tables of the transform (shared memory on the device).
+//   ln[k], k < 512: centre c = 1 + (k + 1/2) / 512 of m in [1, 2);
+//          x = 2^64 / c, y = ln c in units of 2^-63
+//   trig[k], k < 512: (cos, sin)(pi k / 1024) in units of 2^-63
+//   ln2[n], n <= 33: n ln 2 in units of 2^-58
+struct FixedPair {
+    uint64_t x, y;
+};
+constexpr int kLnTable = 512, kTrigTable = 512, kLn2Table = 34;
+struct NormalTables {
+    FixedPair ln[kLnTable];
+    FixedPair trig[kTrigTable];
+    uint64_t ln2[kLn2Table];
+};
+
+// 1 / sqrt(w 2^-64) from above's reciprocal: an integer y in [2^23, 2^24),
+// y 2^-23 within (1 - 2^-20.4, 1) of it.  w in [2^62, 2^64).
+RBG_HD uint32_t rsqrt_seed(uint64_t w)
+{
+#ifdef __CUDA_ARCH__
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint2float_rz(hi32(w)) * 2.3283064365386963e-10f));
+    return min(__float_as_uint(y) - 0x3f800000u, 0x007fffffu) + 0x00800000u - 4u;
+#else
+    const float y = (float)(1.0 / std::sqrt((double)hi32(w) * 0x1p-32));
+    uint32_t b;
+    std::memcpy(&b, &y, 4);
+    b -= 0x3f800000u;
+    return (b < 0x007fffffu ? b : 0x007fffffu) + 0x00800000u - 4u;
+#endif
+}
+
+// sqrt(w 2^-64) in units of 2^-63 for w in [2^62, 2^64), within a few units.
+// With y just below 1 / sqrt(w): w y^2 = 1 - n, sqrt(w) = w y (1 - n)^(-1/2)
+// = w y (1 + n / 2 + 3 n^2 / 8 + O(2^-62)).
+RBG_HD uint64_t sqrt_fixed(uint64_t w)
+{
+    const uint32_t y = rsqrt_seed(w);
+    const uint64_t n = (1ull << 62) - mulhi64(w, mul32(y, y) << 16);            // n, unit 2^-62, below 2^42
+    const uint64_t wy = (mul32(hi32(w), y) << 8) + (mul32(lo32(w), y) >> 24);  // unit 2^-63
+    const uint32_t n50 = (uint32_t)(n >> 12);                                  // unit 2^-50
+    const uint64_t c = (n >> 1) + ((3ull * mul32(n50, n50)) >> 41);            // unit 2^-62
+    return wy + (mulhi64(c << 21, wy) >> 19);
+}
+
+// Box-Muller of two 32-bit words, u0 = (a + 1/2) 2^-32, u1 = (b + 1/2) 2^-32:
+// sqrt(-2 ln u0) (cos, sin)(2 pi u1) in units of 2^-59.
+RBG_HD void box_muller_fixed(uint32_t a, uint32_t b, const NormalTables& T, int64_t& z0, int64_t& z1)
+{
+    // -2 ln u0 = w 2^-64 2^ex, w in [2^62, 2^64), ex even
+    uint64_t w;
+    int ex;
+    if (a >= 0xFFF00000u) {
+        // 1 - u0 = d 2^-33, d < 2^21: -2 ln u0 = d 2^-32 (1 + x / 2 + x^2 / 3 + x^3 / 4 + x^4 / 5), x = d 2^-33
+        // (relative accuracy to the end of the range)
+        const uint32_t d = 0u - (2u * a + 1u);
+        const uint64_t x = (uint64_t)d << 31;  // unit 2^-64
+        const uint32_t x44 = d << 11;          // unit 2^-44, below 2^32
+        const uint32_t x2 = mulhi32(x44, x44); // unit 2^-56
+        const uint64_t f = (1ull << 63) + (x >> 2) + (mul32(x2, 0x55555555u + (mulhi32(x44, 0x40000000u) >> 12) +
+                                                            (mulhi32(x2, 0x33333333u) >> 24)) >> 25);  // unit 2^-63
+#ifdef __CUDA_ARCH__
+        const int n = __clz((int)d);
+#else
+        const int n = __builtin_clz(d);
+#endif
+        const uint32_t dn = d << n;
+        w = mul32(dn, hi32(f)) + (mul32(dn, lo32(f)) >> 32);  // d f 2^(n - 32): unit of d f is 2^-95
+        ex = 1 - n;                                           // value w 2^(n-dependent): see below
+        // d 2^-32 f = (w 2^(32 - n)) 2^-32 2^-63 = (w 2^-64) 2^(1 - n)
+        if (!(w >> 63)) { w <<= 1; --ex; }
+    } else {
+        // u0 = q 2^-33, q = 2 a + 1 = 2^e m; ln m = ln c + log1p(t), t = (m - c) / c, |t| < 2^-10
+        const uint64_t q = 2ull * a + 1ull;
+        const int s = clz64(q);              // e = 63 - s
+        const uint64_t qn = q << s;          // m, unit 2^-63
+        const FixedPair lc = T.ln[(uint32_t)(qn >> 54) & (kLnTable - 1)];
+        const uint32_t u = (uint32_t)(qn >> 30) & 0xFFFFFFu;  // (m - c) 2^33 + 2^23
+        const int64_t t = (int64_t)((mul32(u, hi32(lc.x)) << 7) + (mul32(u, lo32(lc.x)) >> 25) - (lc.x >> 2));  // unit 2^-72
+        const int32_t th = (int32_t)(t >> 32);                                                    // unit 2^-40
+        const uint64_t t2 = (uint64_t)((int64_t)th * th + (((int64_t)th * (int32_t)(lo32((uint64_t)t) >> 1)) >> 30));  // unit 2^-80
+        const int32_t t3 = (int32_t)(((int64_t)th * (int32_t)hi32(t2)) >> 27);                    // unit 2^-61
+        // 1/3 - t/4 + t^2/5, unit 2^-31
+        const int32_t g = 0x2AAAAAAB - (th >> 11) + (int32_t)(mulhi32(hi32(t2), 0x33333333u) >> 17);
+        // ln m = ln c + t - t^2 / 2 + t^3 g, unit 2^-63
+        const int64_t lm = (int64_t)lc.y + (t >> 9) - (int64_t)(t2 >> 18) + (((int64_t)t3 * g) >> 29);
+        // -ln u0 = (33 - e) ln 2 - ln m: unit 2^-63 for u0 > 1/2, where it is small, else 2^-58
+        const bool top = s == 31;
+        const uint64_t L = top ? 0x58B90BFBE8E7BCD6ull - (uint64_t)lm : T.ln2[s - 30] - (uint64_t)(lm >> 5);
+        const int n = clz64(L);
+        w = L << n;
+        ex = (top ? 2 : 7) - n;  // 2 L 2^-58 = (w 2^-64) 2^(7 - n)
+    }
+    if (ex & 1) { w >>= 1; ++ex; }
+    const uint64_t r = sqrt_fixed(w) << 1;  // sqrt(-2 ln u0) 2^(-ex / 2), unit 2^-64
+
+    // 2 pi u1 = (quadrant) pi / 2 + pi k / 1024 + d, d = p pi 2^-32 with p = 2 (b mod 2^21) + 1
+    const uint32_t p = 2u * (b & 0x1FFFFFu) + 1u;
+    const FixedPair cs = T.trig[(b >> 21) & (kTrigTable - 1)];
+    const uint64_t d = (mul32(p, 0xC90FDAA2u) << 10) + (mul32(p, 0x2168C235u) >> 22);  // unit 2^-72
+    const uint32_t dh = hi32(d);                                                      // unit 2^-40
+    const uint64_t d2 = mul32(dh, dh) + (mul32(dh, lo32(d)) >> 31);                   // unit 2^-80
+    const uint32_t d2h = hi32(d2);                                                    // unit 2^-48
+    // 1 - cos d = d^2 / 2 - d^4 (1/24 - d^2 / 720), unit 2^-81
+    const uint32_t c24 = 0xAAAAAAABu - (mulhi32(d2h, 0x005B05B0u) >> 12);
+    const uint64_t nc = d2 - ((uint64_t)mulhi32(mulhi32(d2h, d2h), c24) << 13);
+    // sin d = d - d^3 (1/6 - d^2 / 120), unit 2^-72
+    const uint32_t c6 = 0xAAAAAAABu - (mulhi32(d2h, 0x02222222u) >> 14);
+    const uint64_t d3 = mul32(dh, d2h);  // unit 2^-88
+    const uint64_t sd = d - ((mul32(hi32(d3), c6) + (mul32(lo32(d3), c6) >> 32)) >> 18);
+    const uint64_t c = cs.x - (mulhi64(cs.x, nc) >> 17) - (mulhi64(cs.y, sd) >> 8);  // unit 2^-63
+    const uint64_t sn = cs.y - (mulhi64(cs.y, nc) >> 17) + (mulhi64(cs.x, sd) >> 8);
+    // quadrant q: (c, s), (-s, c), (-c, -s), (s, -c)
+    const bool odd = (b >> 30) & 1u;
+    const int sh = 4 - ex / 2;  // r 2^(ex / 2) c 2^-63 -> unit 2^-59
+    const uint64_t half = 1ull << (sh - 1);
+    const uint64_t m0 = (mulhi64(r, odd ? sn : c) + half) >> sh;
+    const uint64_t m1 = (mulhi64(r, odd ? c : sn) + half) >> sh;
+    const uint64_t s0 = 0ull - (uint64_t)(((b >> 30) ^ (b >> 31)) & 1u);  // cosine negative in quadrants 1, 2
+    const uint64_t s1 = 0ull - (uint64_t)(b >> 31);                       // sine in 2, 3
+    z0 = (int64_t)((m0 ^ s0) - s0);
+    z1 = (int64_t)((m1 ^ s1) - s1);
+}
+
+// --------------------------------------------------------------- 2^x
+// exp2 table: E[k] = 2^(k / 4096) in units of 2^-63.
+constexpr int kExpTable = 4096;
+
+// 2^(x 2^-ut) for a signed fixed-point x, ut <= 53, as a double: infinity
+// above the range of a double, zero below its normal range.
+RBG_HD double exp2_fixed(int64_t x, int ut, const uint64_t* E)
+{
+    const int64_t e = x >> ut;
+    const uint64_t f = (uint64_t)x << (64 - ut);  // fraction, unit 2^-64
+    const uint64_t T = E[f >> 52];
+    const uint64_t r = f & 0x000FFFFFFFFFFFFFull;  // below 2^-12
+    // 2^r - 1 = c1 r + r^2 (c2 + c3 r + c4 r^2), unit 2^-64
+    const uint32_t rh = (uint32_t)(r >> 20);         // unit 2^-44
+    const uint32_t r2 = mulhi32(rh, rh);             // unit 2^-56
+    const uint32_t c = 0xF5FDEFFDu + ((mulhi32(rh, 0x0E35846Bu) + (mulhi32(r2, 0x0276556Eu) >> 12)) >> 10);  // unit 2^-34
+    const uint64_t p = mulhi64(r, 0xB17217F7D1CF79ACull) + (mul32(r2, c) >> 26);
+    const uint64_t m = T + mulhi64(T, p);            // in [2^63, 2^64)
+    const uint64_t b = ((uint64_t)(e + 1022) << 52) + (m >> 11) + ((m >> 10) & 1u);
+    return bits_double(e > 1023 ? 0x7FF0000000000000ull : (e < -1022 ? 0ull : b));
+}
+
+}  // namespace rbg

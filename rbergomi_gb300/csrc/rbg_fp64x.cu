@@ -1,0 +1,756 @@
+// rbg_fp64x.cu -- the FP64 form on Philox normals: exact convolution on the
+// tensor cores, elementary functions in 64-bit fixed point.
+//
+// GB300's FP64 pipe (2 DFMA per clock and SM) bounds every kernel that does
+// its arithmetic in FP64.  These do it elsewhere, with no less precision:
+//   k_normals_fixed  Philox4x32-10 -> Box-Muller in 64-bit integers
+//                    (rbg_fixed.cuh) -> FP64 normals, quadrature layout, and
+//                    W1 as eight signed 8-bit digits in FP16 for the next
+//   k_volterra_exact X_j = sum_{k<=j} W1_k Gamma'_{j-k}, Gamma' = (a1, Gamma_1,
+//                    ...), as digit products on tcgen05: both operands are
+//                    64-bit fixed-point numbers cut into 8 signed digits, and
+//                    the digit products of weight 2^(-8 d), d = i + j <= 7, are
+//                    summed in one FP32 accumulator each
+//   k_variance_fixed X + a2 W1perp, v = xi 2^t with t and 2^t in 64-bit fixed
+//                    point, FP64 sums of v and sqrt(v) W1 (, Wperp)
+//
+// Exactness of the convolution.  A digit is an integer in [-128, 127], exact in
+// FP16; a product has 14 bits, and an FP32 accumulator holds integers up to
+// 2^24 exactly.  The digits of W1 below the first are uniform over their range
+// and independent between steps (the first is round(8 W1), below 55), so a
+// diagonal of (d + 1) K products has a standard deviation below 74^2 sqrt((d +
+// 1) K): 7.1e5 = 2^19.4 at d = 7 and K = 2048, 24 standard deviations from 2^24
+// (17 at K = 4096).  Left out are the products with d >= 8, below 2^-60 of the
+// operands' product each: the sums are within about 2^-54 of the exact ones,
+// against 2^-45 for an FP64 FFT of 1024 points and 2^-50 for the direct FP64
+// sum of 100 steps.
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <cmath>
+#include <cstring>
+#include <mutex>
+
+#include "rbg_device.cuh"
+#include "rbg_fixed.cuh"
+#include "rbg_fp64x.hpp"
+#include "rbg_tc.cuh"
+
+namespace rbg {
+
+// ------------------------------------------------------------------ tables
+__device__ NormalTables g_normal_tables;
+__device__ uint64_t g_exp_table[kExpTable];
+
+// Fills the device's tables once (extended precision on the host).
+static cudaError_t ensure_fixed_tables()
+{
+    static std::mutex mu;
+    static bool ready[64] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lk(mu);
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    if (ready[dev]) return cudaSuccess;
+    static NormalTables T;
+    static uint64_t E[kExpTable];
+    for (int k = 0; k < kLnTable; ++k) {
+        const long double c = 1.0L + (k + 0.5L) / kLnTable;
+        T.ln[k] = FixedPair{(uint64_t)(std::ldexp(1.0L / c, 64) + 0.5L), (uint64_t)(std::ldexp(std::log(c), 63) + 0.5L)};
+    }
+    const long double pi = 3.14159265358979323846264338327950288L, ln2 = 0.693147180559945309417232121458176568L;
+    for (int k = 0; k < kTrigTable; ++k) {
+        const long double a = pi * k / 1024.0L;
+        T.trig[k] = FixedPair{(uint64_t)(std::ldexp(std::cos(a), 63) + 0.5L),
+                              (uint64_t)(std::ldexp(std::sin(a), 63) + 0.5L)};
+    }
+    for (int n = 0; n < kLn2Table; ++n) T.ln2[n] = (uint64_t)(std::ldexp(ln2 * n, 58) + 0.5L);
+    for (int k = 0; k < kExpTable; ++k) E[k] = (uint64_t)(std::ldexp(std::exp2(k / (long double)kExpTable), 63) + 0.5L);
+    e = cudaMemcpyToSymbol(g_normal_tables, &T, sizeof T);
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_exp_table, E, sizeof E);
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (e == cudaSuccess) ready[dev] = true;
+    return e;
+}
+
+// ----------------------------------------------------------------- normals
+// Digits of W1, [group of 64 paths][16-step chunk][digit][64 paths][16 steps]
+// FP16: one 16 KB block per chunk, the layout the MMA reads (K-major SW32 rows
+// of 32 bytes, row = 64 digit + path, 16-byte halves swapped where row / 4 is
+// odd).
+constexpr int kXPaths = 64, kXSteps = 16, kXDigits = 8;
+constexpr int kXChunkBytes = kXDigits * kXPaths * kXSteps * 2;  // 16 KB
+
+// The signed bytes of four values, digit by digit (most significant first),
+// as FP16: each value plus 0x80 in every byte has digit + 128 as its bytes,
+// and FP16 0x6400 + byte is 1024 + byte.
+__device__ __forceinline__ void store_digits(const int64_t (&v)[4], unsigned char* at)
+{
+    uint32_t w[2][4];  // high, low words
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const uint64_t u = (uint64_t)v[q] + 0x8080808080808080ull;
+        w[0][q] = hi32(u);
+        w[1][q] = lo32(u);
+    }
+    const __half2 off = __halves2half2(__ushort_as_half(0x6480), __ushort_as_half(0x6480));  // 1152
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+#pragma unroll
+        for (int b = 3; b >= 0; b -= 2) {  // bytes b and b - 1 of the word: digits 4 h + 3 - b and the next
+            const uint32_t sel = (uint32_t)(b | ((4 + b) << 4) | ((b - 1) << 8) | ((3 + b) << 12));
+            const uint32_t t01 = __byte_perm(w[h][0], w[h][1], sel), t23 = __byte_perm(w[h][2], w[h][3], sel);
+#pragma unroll
+            for (int z = 0; z < 2; ++z) {
+                const uint32_t s2 = z ? 0x4342u : 0x4140u;
+                uint32_t a = __byte_perm(t01, 0x64646464u, s2), c = __byte_perm(t23, 0x64646464u, s2);
+                const __half2 ha = __hsub2(*reinterpret_cast<__half2*>(&a), off);
+                const __half2 hc = __hsub2(*reinterpret_cast<__half2*>(&c), off);
+                const int digit = 4 * h + 3 - b + z;
+                *(uint2*)(at + digit * (kXPaths * 32)) =
+                    make_uint2(*reinterpret_cast<const uint32_t*>(&ha), *reinterpret_cast<const uint32_t*>(&hc));
+            }
+        }
+    }
+}
+
+// Z[m][s][j], s < NS: W1, W1perp and (plain MC) Wperp on Philox streams 0, 1,
+// 2; dig non-null: also the digits of W1 (zero past N and past B).  A warp
+// takes 8 paths x 16 steps of one stream, four lanes a path and four steps a
+// lane, so a path's 16 doubles and each digit's 8 rows are contiguous.
+// Integer work bounds it: about 220 instructions, 70 of them 32 x 32 -> 64
+// multiplies, for a pair of normals.  2 x 512 steps, 2^17 paths: 1.25 ms,
+// against 5.40 ms for the same draw in FP64 (table-driven logarithm and sine,
+// about 40 FP64 operations a pair).
+constexpr int kNormalThreads = 256;
+template <int F32>
+__global__ void __launch_bounds__(kNormalThreads) k_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int ns,
+                                                                 double* __restrict__ Z,
+                                                                 unsigned char* __restrict__ dig)
+{
+    __shared__ NormalTables T;
+    if (!F32) {
+        const uint64_t* src = reinterpret_cast<const uint64_t*>(&g_normal_tables);
+        uint64_t* dst = reinterpret_cast<uint64_t*>(&T);
+        for (int i = threadIdx.x; i < (int)(sizeof(NormalTables) / 8); i += kNormalThreads) dst[i] = src[i];
+        __syncthreads();
+    }
+    const int lane = threadIdx.x & 31, g = lane & 3, pl = lane >> 2;
+    const int nch = (N + kXSteps - 1) / kXSteps;
+    const int64_t octets = (B + kXPaths - 1) / kXPaths * (kXPaths / 8);
+    const int64_t tasks = octets * ns * nch;
+    const bool vec = (N & 1) == 0;
+    const PhiloxKeys keys = philox_keys(seed);
+    const int64_t warps = (int64_t)gridDim.x * (kNormalThreads / 32);
+    for (int64_t t = blockIdx.x * (int64_t)(kNormalThreads / 32) + (threadIdx.x >> 5); t < tasks; t += warps) {
+        const int c = (int)(t % nch);
+        const int64_t r = t / nch;
+        const int s = (int)(r % ns);
+        const int64_t m = r / ns * 8 + pl;
+        const int j0 = kXSteps * c + 4 * g;
+        const bool valid = m < B;
+        if (!valid && (s != 0 || !dig)) continue;
+        int64_t v[4] = {0, 0, 0, 0};
+        if (valid && j0 < N) {
+            const uint4 x = philox_group(keys, (uint64_t)(path0 + m), (uint32_t)(j0 >> 2), (uint32_t)s);
+            double z[4];
+            if (F32) {
+                float f0, f1, f2, f3;
+                box_muller_f32(x.x, x.y, f0, f1);
+                box_muller_f32(x.z, x.w, f2, f3);
+                z[0] = f0; z[1] = f1; z[2] = f2; z[3] = f3;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) v[q] = double_to_fixed(z[q]);
+            } else {
+                box_muller_fixed(x.x, x.y, T, v[0], v[1]);
+                box_muller_fixed(x.z, x.w, T, v[2], v[3]);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) z[q] = fixed_to_double(v[q]);
+            }
+            double* o = Z + (m * ns + s) * (int64_t)N + j0;
+            if (j0 + 4 <= N) {
+                if (vec) {
+                    *(double2*)o = make_double2(z[0], z[1]);
+                    *(double2*)(o + 2) = make_double2(z[2], z[3]);
+                } else {
+                    o[0] = z[0]; o[1] = z[1]; o[2] = z[2]; o[3] = z[3];
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (j0 + q < N) o[q] = z[q];
+                    else v[q] = 0;
+                }
+            }
+        }
+        if (s == 0 && dig) {
+            const int p = (int)(m & (kXPaths - 1));
+            unsigned char* at = dig + ((m / kXPaths) * nch + c) * kXChunkBytes + p * 32 +
+                                ((((g >> 1) ^ (p >> 2)) & 1) << 4) + ((g & 1) << 3);
+            store_digits(v, at);
+        }
+    }
+}
+
+int launch_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int f32, double* Z, unsigned char* dig, int ns,
+                         cudaStream_t st)
+{
+    if (ensure_fixed_tables() != cudaSuccess) {
+        cudaGetLastError();
+        return -1;
+    }
+    const int64_t octets = (B + kXPaths - 1) / kXPaths * (kXPaths / 8);
+    const int64_t tasks = octets * ns * ((N + kXSteps - 1) / kXSteps);
+    const int64_t need = (tasks + kNormalThreads / 32 - 1) / (kNormalThreads / 32);
+    const int64_t blocks = std::min<int64_t>(need, 8 * (int64_t)device_sms());
+    if (f32) k_normals_fixed<1><<<(unsigned)blocks, kNormalThreads, 0, st>>>(seed, path0, B, N, ns, Z, dig);
+    else k_normals_fixed<0><<<(unsigned)blocks, kNormalThreads, 0, st>>>(seed, path0, B, N, ns, Z, dig);
+    count_launch();
+    return 0;
+}
+
+// ------------------------------------------------------------- convolution
+// D[step][path] per diagonal d: the Toeplitz operand is MMA's A (128 output
+// steps), the W1 digits its B, eight digits x 64 paths = 512 rows of a chunk,
+// so one MMA of N = 256 covers four digit products of one Gamma digit and the
+// accumulators of a block are [d][64 paths] = all 512 TMEM columns.  Gamma
+// digit j multiplies W1 digits 0 .. 7 - j into columns 64 j .. 511.
+//
+// Gamma panels.  Output block b (steps 128 b ..) takes the 16-step chunks of
+// blocks s = 0 .. b; with L = b - s the entries it needs are Gamma'[128 L + i -
+// k], i, k < 128: panel L holds, per digit, rows r < 240 of 16 FP16, P[r][k''] =
+// Gamma'[128 L + r - 112 - k''] (zero for negative indices), and chunk kk of the
+// block reads rows 16 (7 - kk) .. + 127.  60 KB a panel, two in shared memory.
+constexpr int kPanelRows = 240;
+constexpr int kPanelDigit = kPanelRows * 32;           // 7680 B
+constexpr int kPanelBytes = kXDigits * kPanelDigit;    // 61440 B
+constexpr int kXBlock = 128;                           // output steps per block
+constexpr int kXChunks = kXBlock / kXSteps;            // 8 chunks per block of steps
+constexpr int kXStages = 5;
+constexpr int kXEpiWarps = 8;
+constexpr int kXThreads = (kXEpiWarps + 2) * 32;
+constexpr int kXSmem = 2 * kPanelBytes + kXStages * kXChunkBytes + 256 + 1024;
+
+int x64_blocks(int N) { return (N + kXBlock - 1) / kXBlock; }
+size_t x64_panel_bytes(int N) { return (size_t)x64_blocks(N) * kPanelBytes; }
+size_t x64_digit_bytes(int64_t B, int N)
+{
+    return (size_t)((B + kXPaths - 1) / kXPaths) * ((N + kXSteps - 1) / kXSteps) * kXChunkBytes;
+}
+
+// Panels of every pass from its fixed-point Gamma' (unit 2^(e - 62)): one
+// thread per 16-byte half row of one digit.
+__global__ void k_panels(const int64_t* __restrict__ gam, int nv, int N, int nb, unsigned char* __restrict__ panels)
+{
+    const int64_t total = (int64_t)nv * nb * kXDigits * kPanelRows * 2;
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+        const int half = (int)(t & 1);
+        int64_t q = t >> 1;
+        const int r = (int)(q % kPanelRows);
+        q /= kPanelRows;
+        const int digit = (int)(q % kXDigits);
+        q /= kXDigits;
+        const int L = (int)(q % nb), v = (int)(q / nb);
+        uint32_t h[4];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int d = kXBlock * L + r - 112 - (8 * half + i);
+            const uint64_t u = (uint64_t)((d >= 0 && d < N) ? gam[(size_t)v * N + d] : 0) + 0x8080808080808080ull;
+            const int x = (int)((u >> (8 * (7 - digit))) & 255u) - 128;
+            const uint32_t f = __half_as_ushort(__int2half_rn(x));
+            if (i & 1) h[i >> 1] |= f << 16;
+            else h[i >> 1] = f;
+        }
+        unsigned char* at = panels + ((size_t)v * nb + L) * kPanelBytes + digit * kPanelDigit + r * 32 +
+                            ((half ^ (r >> 2)) & 1) * 16;
+        *(uint4*)at = make_uint4(h[0], h[1], h[2], h[3]);
+    }
+}
+
+void launch_panels(const int64_t* gam, int nv, int N, unsigned char* panels, cudaStream_t st)
+{
+    const int nb = x64_blocks(N);
+    const int64_t total = (int64_t)nv * nb * kXDigits * kPanelRows * 2;
+    k_panels<<<(unsigned)std::min<int64_t>((total + 255) / 256, 4096), 256, 0, st>>>(gam, nv, N, nb, panels);
+    count_launch();
+}
+
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+}
+
+// Which of the two panel buffers a panel goes to: the one that holds it, else
+// the one not used last.  The loader and the MMA thread follow the same rule.
+struct PanelSlots {
+    int key0 = -1, key1 = -1, last = 1;
+    __device__ __forceinline__ int use(int key, bool& load)
+    {
+        int b;
+        load = false;
+        if (key == key0) {
+            b = 0;
+        } else if (key == key1) {
+            b = 1;
+        } else {
+            b = 1 - last;
+            load = true;
+            if (b) key1 = key;
+            else key0 = key;
+        }
+        last = b;
+        return b;
+    }
+};
+
+// One (block b, pass v, group of 64 paths) at a time, the longest blocks
+// first.  Warps 0-7 read the accumulators, warp 8 loads, warp 9 issues the
+// MMAs.  WIDE: accumulators may pass 2^22 (N > 1024): converted by F2I, else by
+// adding 1.5 2^23.
+// What bounds it: 2304 columns x 128 steps x 16 per chunk, 1152 MMA cycles,
+// against 16 KB of digits and 7.5 KB of panel from L2; the accumulators fill
+// TMEM, so the next block's MMAs wait for the read-out of this one's.
+// With k_variance_fixed: 512 steps, 2^17 paths, one pass 1.99 ms, against 13.2
+// ms for the FP64 FFT convolution and exponentials; 100 steps, 2^16 paths 0.23
+// ms, against 1.46 ms for the direct FP64 sum.
+template <bool WIDE>
+__global__ void __launch_bounds__(kXThreads, 1) k_volterra_exact(const unsigned char* __restrict__ dig,
+                                                                 const unsigned char* __restrict__ panels,
+                                                                 const X64Vol* __restrict__ vols, int nv, int N,
+                                                                 int64_t B, uint64_t* __restrict__ X,
+                                                                 unsigned int* __restrict__ err)
+{
+    extern __shared__ unsigned char smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw);
+    unsigned char* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
+    unsigned char* stage = base + 2 * kPanelBytes;
+    uint64_t* bars = (uint64_t*)(stage + kXStages * kXChunkBytes);
+    uint64_t* wfull = bars;                 // [kXStages]
+    uint64_t* wempty = bars + kXStages;     // [kXStages]
+    uint64_t* pfull = bars + 2 * kXStages;  // [2]
+    uint64_t* accf = pfull + 2;
+    uint64_t* acce = accf + 1;
+    uint64_t* fin = accf + 2;
+    uint32_t* holder = (uint32_t*)(accf + 3);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nb = (N + kXBlock - 1) / kXBlock, nch = (N + kXSteps - 1) / kXSteps;
+    const int64_t groups = (B + kXPaths - 1) / kXPaths, per = groups * nv, units = per * nb;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kXStages; ++s) {
+            mbar_init(smem_u32(wfull + s), 1);
+            mbar_init(smem_u32(wempty + s), 1);
+        }
+        for (int b = 0; b < 2; ++b) mbar_init(smem_u32(pfull + b), 1);
+        mbar_init(smem_u32(accf), 1);
+        mbar_init(smem_u32(fin), 1);
+        mbar_init(smem_u32(acce), kXEpiWarps);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == kXEpiWarps + 1) {
+        __syncwarp();
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(holder)), "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *holder;
+
+    if (warp == kXEpiWarps) {
+        if (lane == 0) {
+            // ------------------------------------------------------ loader
+            PanelSlots ps;
+            int64_t used[2] = {-1, -1};  // the last chunk (of this thread's count n) that reads each panel buffer
+            int loads[2] = {0, 0};
+            int s = 0;
+            uint32_t ph = 0;
+            int64_t n = 0;
+            bool ok = true;
+            for (int64_t u = blockIdx.x; u < units && ok; u += gridDim.x) {
+                const int b = nb - 1 - (int)(u / per), v = (int)(u % per / groups);
+                const int64_t g = u % groups;
+                const int ke = min(kXChunks * (b + 1), nch);
+                int pb = 0;
+                for (int kc = 0; kc < ke && ok; ++kc, s = (s + 1 == kXStages) ? 0 : s + 1, ph ^= (s == 0)) {
+                    if (kc % kXChunks == 0) {
+                        const int L = b - kc / kXChunks;
+                        bool load;
+                        pb = ps.use(v * nb + L, load);
+                        if (load) {
+                            // every MMA on the buffer's old panel has completed once its last chunk's stage
+                            // is free; chunks before n - kXStages were waited for when their stage was refilled
+                            const int64_t i = used[pb];
+                            if (i >= 0 && i >= n - kXStages &&
+                                !mbar_wait(smem_u32(wempty + (int)(i % kXStages)), (uint32_t)((i / kXStages) & 1), err, 21)) {
+                                ok = false;
+                                break;
+                            }
+                            const uint32_t bar = smem_u32(pfull + pb);
+                            mbar_expect_tx(bar, kPanelBytes);
+                            bulk_g2s(smem_u32(base) + pb * kPanelBytes, panels + ((size_t)v * nb + L) * kPanelBytes,
+                                     kPanelBytes, bar);
+                            ++loads[pb];
+                        }
+                    }
+                    used[pb] = n;
+                    if (!mbar_wait(smem_u32(wempty + s), ph ^ 1u, err, 22)) {
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t bar = smem_u32(wfull + s);
+                    mbar_expect_tx(bar, kXChunkBytes);
+                    bulk_g2s(smem_u32(stage) + s * kXChunkBytes, dig + ((size_t)g * nch + kc) * kXChunkBytes, kXChunkBytes,
+                             bar);
+                    ++n;
+                }
+            }
+            // the copies in flight land before the CTA exits, whatever the error word says
+            for (int64_t i = n > kXStages ? n - kXStages : 0; i < n; ++i)
+                mbar_drain(smem_u32(wfull + (int)(i % kXStages)), (uint32_t)((i / kXStages) & 1));
+            for (int b = 0; b < 2; ++b)
+                if (loads[b]) mbar_drain(smem_u32(pfull + b), (uint32_t)((loads[b] - 1) & 1));
+        }
+    } else if (warp == kXEpiWarps + 1) {
+        if (lane == 0) {
+            // -------------------------------------------------- MMA issuer
+            PanelSlots ps;
+            int loads[2] = {0, 0};
+            int s = 0;
+            uint32_t ph = 0;
+            int64_t done_units = 0;
+            bool ok = true;
+            const uint64_t a_base = sdesc_sw32(smem_u32(base)), b_base = sdesc_sw32(smem_u32(stage));
+            const uint32_t a_lo = (uint32_t)a_base, a_hi = (uint32_t)(a_base >> 32);
+            const uint32_t b_lo = (uint32_t)b_base, b_hi = (uint32_t)(b_base >> 32);
+            for (int64_t u = blockIdx.x; u < units && ok; u += gridDim.x, ++done_units) {
+                const int b = nb - 1 - (int)(u / per), v = (int)(u % per / groups);
+                const int ke = min(kXChunks * (b + 1), nch);
+                if (done_units > 0 && !mbar_wait(smem_u32(acce), (uint32_t)((done_units - 1) & 1), err, 23)) break;
+                int pb = 0;
+                for (int kc = 0; kc < ke; ++kc, s = (s + 1 == kXStages) ? 0 : s + 1, ph ^= (s == 0)) {
+                    if (kc % kXChunks == 0) {
+                        bool load;
+                        pb = ps.use(v * nb + b - kc / kXChunks, load);
+                        if (load) {
+                            if (!mbar_wait(smem_u32(pfull + pb), (uint32_t)(loads[pb] & 1), err, 24)) { ok = false; break; }
+                            ++loads[pb];
+                        }
+                    }
+                    if (!mbar_wait(smem_u32(wfull + s), ph, err, 25)) { ok = false; break; }
+                    tc_fence_after();
+                    // descriptors differ in the start-address field only (address / 16, no carry out of it)
+                    const uint32_t arow = a_lo + (uint32_t)(pb * kPanelBytes + (kXChunks - 1 - kc % kXChunks) * 512) / 16;
+                    const uint32_t brow = b_lo + (uint32_t)(s * kXChunkBytes) / 16;
+#pragma unroll
+                    for (int j = 0; j < kXDigits; ++j) {
+                        const uint64_t da = ((uint64_t)a_hi << 32) | (arow + (uint32_t)(j * kPanelDigit) / 16);
+                        const int n = kXPaths * (kXDigits - j), n1 = n < 256 ? n : 256;
+                        const uint32_t acc = (kc == 0 && j == 0) ? 0u : 1u;
+                        umma_f16(tmem + kXPaths * j, da, ((uint64_t)b_hi << 32) | brow, idesc_f16(n1, 0), acc);
+                        if (n > 256)
+                            umma_f16(tmem + kXPaths * j + 256, da, ((uint64_t)b_hi << 32) | (brow + 256 * 32 / 16),
+                                     idesc_f16(n - 256, 0), acc);
+                    }
+                    umma_commit(smem_u32(wempty + s));
+                }
+                if (ok) umma_commit(smem_u32(accf));
+            }
+            // every issued MMA completes before TMEM is released
+            umma_commit(smem_u32(fin));
+            mbar_wait(smem_u32(fin), 0, err, 26);
+        }
+    } else {
+        // -------------------------------------------------------- read-out
+        const int quad = warp & 3, wg = warp >> 2;
+        const uint32_t tl = tmem + ((uint32_t)(quad * 32) << 16);
+        int64_t n_units = 0;
+        for (int64_t u = blockIdx.x; u < units; u += gridDim.x, ++n_units) {
+            const int b = nb - 1 - (int)(u / per), v = (int)(u % per / groups);
+            const int64_t g = u % groups;
+            const int sh = vols[v].sh;
+            if (!mbar_wait_warp(smem_u32(accf), (uint32_t)(n_units & 1), err, 27)) goto done;
+            tc_fence_after();
+            const int j = kXBlock * b + quad * 32 + lane;
+            uint64_t* Xv = X + (size_t)v * B * N + j;
+#pragma unroll 1
+            for (int q = 0; q < 4; ++q) {
+                const int p0 = wg * 32 + q * 8;
+                uint32_t D[kXDigits][8];
+#pragma unroll
+                for (int d = 0; d < kXDigits; ++d) tmem_ld8(tl + (uint32_t)(kXPaths * d + p0), D[d]);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (q == 3) {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(acce));
+                }
+#pragma unroll
+                for (int p = 0; p < 8; ++p) {
+                    int64_t D8[kXDigits];
+#pragma unroll
+                    for (int d = 0; d < kXDigits; ++d) {
+                        const float f = __uint_as_float(D[d][p]);
+                        D8[d] = WIDE ? __float2int_rn(f) : __float_as_int(f + 12582912.f) - 0x4B400000;
+                    }
+                    // S_hi in units of 2^(e - 33), S_lo of 2^(e - 65); X = S_hi 2^sh + S_lo 2^(sh - 32)
+                    const int64_t hi = (D8[0] << 24) + (D8[1] << 16) + (D8[2] << 8) + D8[3];
+                    const int64_t lo = (D8[4] << 24) + (D8[5] << 16) + (D8[6] << 8) + D8[7];
+                    const uint64_t x = ((uint64_t)hi << sh) + (uint64_t)(lo >> (32 - sh)) + (1ull << 63);
+                    const int64_t m = g * kXPaths + p0 + p;
+                    if (m < B && j < N) Xv[m * N] = x;
+                }
+            }
+        }
+    }
+done:
+    tc_fence_before();
+    __syncthreads();
+    if (warp == kXEpiWarps + 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    }
+}
+
+int launch_volterra_exact(const unsigned char* dig, const unsigned char* panels, const X64Vol* vols, int nv, int N,
+                          int64_t B, uint64_t* X, unsigned int* err, cudaStream_t st)
+{
+    static std::mutex mu;
+    static bool ready[64] = {};
+    {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
+        std::lock_guard<std::mutex> lk(mu);
+        if (!ready[dev]) {
+            if (cudaFuncSetAttribute(k_volterra_exact<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kXSmem) !=
+                    cudaSuccess ||
+                cudaFuncSetAttribute(k_volterra_exact<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kXSmem) !=
+                    cudaSuccess) {
+                cudaGetLastError();
+                return -1;
+            }
+            ready[dev] = true;
+        }
+    }
+    const int64_t units = (B + kXPaths - 1) / kXPaths * nv * x64_blocks(N);
+    const int grid = (int)std::min<int64_t>(units, device_sms());
+    auto* kern = N > 1024 ? k_volterra_exact<true> : k_volterra_exact<false>;
+    kern<<<grid, kXThreads, kXSmem, st>>>(dig, panels, vols, nv, N, B, X, err);
+    count_launch();
+    return 0;
+}
+
+// ----------------------------------------------------------- variance path
+// One warp per path, lanes over steps; GB variance groups of one pass at a
+// time.  sqrt(v_j) = sqrt(xi) 2^t, t = C (X + a2 W1perp)_{j-1} - comp_{j-1} in
+// units of 2^-ut, 2^t by table and polynomial in integers; FP64 only for the
+// two (three) sums, which leaves the FP64 pipe 128 (192) cycles a warp step and
+// the integer pipes about as much.  The lanes' sums of several paths are
+// reduced together through shared memory: one FP64 addition a value and lane
+// instead of five.
+constexpr int kVarThreads = 256, kVarVals = 16;
+constexpr int kVarSmem = kExpTable * 8 + (kVarThreads / 32) * kVarVals * 33 * 8;
+
+template <int NS, int GB>
+__global__ void __launch_bounds__(kVarThreads) k_variance_fixed(const X64Vol* __restrict__ vols,
+                                                               const X64Group* __restrict__ grps,
+                                                               const uint64_t* __restrict__ comp,
+                                                               const double* __restrict__ Z,
+                                                               const uint64_t* __restrict__ X, int nv, int N, int64_t B,
+                                                               double* __restrict__ ivb, double* __restrict__ ivp)
+{
+    constexpr int PB = kVarVals / (GB * NS);  // paths per reduction
+    extern __shared__ uint64_t vsm[];
+    uint64_t* E = vsm;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double* red = reinterpret_cast<double*>(vsm + kExpTable) + (size_t)w * kVarVals * 33;
+    for (int i = threadIdx.x; i < kExpTable; i += kVarThreads) E[i] = g_exp_table[i];
+    __syncthreads();
+    const int64_t runs = (B + PB - 1) / PB, warps = (int64_t)gridDim.x * (kVarThreads / 32);
+    for (int64_t run = blockIdx.x * (int64_t)(kVarThreads / 32) + w; run < runs; run += warps) {
+        for (int v = 0; v < nv; ++v) {
+            const X64Vol vol = vols[v];
+            for (int g0 = vol.vg_begin; g0 < vol.vg_end; g0 += GB) {
+                const int ng = min(GB, vol.vg_end - g0);
+                uint64_t cf[GB];
+                int ut[GB];
+                bool neg[GB];
+#pragma unroll
+                for (int q = 0; q < GB; ++q) {
+                    const X64Group& G = grps[g0 + (q < ng ? q : 0)];
+                    cf[q] = G.cf;
+                    ut[q] = G.ut;
+                    neg[q] = G.neg != 0;
+                }
+#pragma unroll 1
+                for (int pl = 0; pl < PB; ++pl) {
+                    const int64_t m = run * PB + pl;
+                    double acc[GB][NS];
+#pragma unroll
+                    for (int q = 0; q < GB; ++q)
+#pragma unroll
+                        for (int c = 0; c < NS; ++c) acc[q][c] = 0.0;
+                    if (m < B) {
+                        const double* W1 = Z + m * NS * (int64_t)N;
+                        const uint64_t* Xm = X + ((size_t)v * B + m) * N;
+                        for (int j = 1 + lane; j < N; j += 32) {
+                            const double w1 = W1[j];
+                            double wq = 0.0;
+                            if (NS == 3) wq = W1[2 * N + j];
+                            const uint64_t wp = (uint64_t)double_to_fixed(W1[N + j - 1]) ^ (1ull << 63);
+                            const uint64_t x = Xm[j - 1] + mulhi64(wp, vol.a2f) - vol.a2h;
+#pragma unroll
+                            for (int q = 0; q < GB; ++q) {
+                                if (q < ng) {
+                                    const uint64_t t = mulhi64(neg[q] ? 0ull - x : x, cf[q]) -
+                                                       __ldg(comp + (size_t)(g0 + q) * N + j - 1);
+                                    const double su = exp2_fixed((int64_t)t, ut[q], E);
+                                    acc[q][0] = fma(su, su, acc[q][0]);
+                                    acc[q][1] = fma(su, w1, acc[q][1]);
+                                    if (NS == 3) acc[q][2] = fma(su, wq, acc[q][2]);
+                                }
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int q = 0; q < GB; ++q)
+#pragma unroll
+                        for (int c = 0; c < NS; ++c) red[((pl * GB + q) * NS + c) * 33 + lane] = acc[q][c];
+                }
+                __syncwarp();
+                // value lane % 16 over the 16 lanes of half lane / 16, then both halves
+                const int val = lane & 15;
+                double s = 0.0;
+                if (val < PB * GB * NS) {
+                    const double* row = red + val * 33 + (lane >> 4) * 16;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) s += row[i];
+                }
+                s += __shfl_xor_sync(0xffffffffu, s, 16);
+                const int c = val % NS, q = val / NS % GB;
+                const int64_t m = run * PB + val / (NS * GB);
+                if (lane < 16 && val < PB * GB * NS && q < ng && m < B) {
+                    const X64Group& G = grps[g0 + q];
+                    const size_t at = (size_t)(g0 + q) * B + m;
+                    const double* W1 = Z + m * NS * (int64_t)N;
+                    // Ivdt = dt xi (1 + sum), IsvdW = sqrt(dt xi) (W1_0 + sum): v_0 = xi
+                    if (c == 0) ivb[2 * at] = G.dtxi * (1.0 + s);
+                    else if (c == 1) ivb[2 * at + 1] = G.sdtxi * (W1[0] + s);
+                    else ivp[at] = G.sdtxi * (W1[2 * N] + s);
+                }
+                __syncwarp();
+            }
+        }
+    }
+}
+
+int launch_variance_fixed(const X64Vol* vols, const X64Group* grps, const uint64_t* comp, const double* Z,
+                          const uint64_t* X, int nv, int max_groups, int ns, int N, int64_t B, double* ivb, double* ivp,
+                          cudaStream_t st)
+{
+    static std::mutex mu;
+    static bool ready[64] = {};
+    auto* kern = ns == 3 ? (max_groups > 1 ? k_variance_fixed<3, 4> : k_variance_fixed<3, 1>)
+                         : (max_groups > 1 ? k_variance_fixed<2, 4> : k_variance_fixed<2, 1>);
+    {
+        int dev = 0;
+        if (ensure_fixed_tables() != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
+        std::lock_guard<std::mutex> lk(mu);
+        if (!ready[dev]) {
+            for (auto* k : {k_variance_fixed<2, 1>, k_variance_fixed<2, 4>, k_variance_fixed<3, 1>, k_variance_fixed<3, 4>})
+                if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kVarSmem) != cudaSuccess) {
+                    cudaGetLastError();
+                    return -1;
+                }
+            ready[dev] = true;
+        }
+    }
+    const int pb = kVarVals / ((max_groups > 1 ? 4 : 1) * ns);
+    const int64_t runs = (B + pb - 1) / pb;
+    const int64_t blocks = std::min<int64_t>((runs + kVarThreads / 32 - 1) / (kVarThreads / 32), 3 * (int64_t)device_sms());
+    kern<<<(unsigned)blocks, kVarThreads, kVarSmem, st>>>(vols, grps, comp, Z, X, nv, N, B, ivb, ivp);
+    count_launch();
+    return 0;
+}
+
+// -------------------------------------------------------------------- host
+bool x64_prepare(const Plan& plan, X64Tables& out)
+{
+    const int N = plan.N, nv = (int)plan.vols.size(), ng = (int)plan.vgs.size();
+    if (N < 2 || N > kX64MaxN) return false;
+    out.vols.assign(nv, X64Vol{});
+    out.grps.assign(ng, X64Group{});
+    out.gam.assign((size_t)nv * N, 0);
+    out.comp.assign((size_t)ng * N, 0);
+    std::vector<int> ux(nv);
+    const double wmax = 6.9;  // |Box-Muller on 32-bit uniforms| <= sqrt(66 ln 2) = 6.77
+    for (int v = 0; v < nv; ++v) {
+        const VolGroup& V = plan.vols[v];
+        const double* G = plan.gamma.data() + (size_t)v * N;
+        double gmax = std::fabs(V.a1), gsum = std::fabs(V.a1);
+        for (int d = 1; d < N; ++d) {
+            gmax = std::max(gmax, std::fabs(G[d]));
+            gsum += std::fabs(G[d]);
+        }
+        const double bound = wmax * (gsum + std::fabs(V.a2));
+        if (!(gmax > 0.0) || !std::isfinite(bound) || !(V.a2 >= 0.0)) return false;
+        int e = 0, cb = 0;
+        while (std::ldexp(1.0, e) < gmax) ++e;
+        while (std::ldexp(1.0, cb) < bound) ++cb;
+        // X in units of 2^-ux with |X| 2^ux < 2^62; a2 2^(ux - 59) < 1 for its fixed-point factor
+        int u = 62 - cb;
+        while (std::ldexp(V.a2, u - kNormalBits) >= 1.0) --u;
+        const int sh = e - 33 + u;
+        if (sh < 1 || sh > 31) return false;
+        ux[v] = u;
+        out.vols[v].sh = sh;
+        out.vols[v].vg_begin = V.vg_begin;
+        out.vols[v].vg_end = V.vg_end;
+        const uint64_t a2f = (uint64_t)std::ldexp(V.a2, u - kNormalBits + 64);
+        out.vols[v].a2f = a2f;
+        out.vols[v].a2h = (a2f >> 1) - 1;  // the bias's share, and the product's mean truncation
+        // unit 2^(e - 62): |gam| <= 2^62
+        int64_t* q = out.gam.data() + (size_t)v * N;
+        q[0] = (int64_t)std::llrint(std::ldexp(V.a1, 62 - e));
+        for (int d = 1; d < N; ++d) q[d] = (int64_t)std::llrint(std::ldexp(G[d], 62 - e));
+        out.max_groups = std::max(out.max_groups, V.vg_end - V.vg_begin);
+    }
+    const double l2 = 1.4426950408889634074, l2lo = 2.0355273740931033e-17;  // log2 e
+    for (int g = 0; g < ng; ++g) {
+        const VGroup& G = plan.vgs[g];
+        const VolGroup& V = plan.vols[G.vol];
+        const double* c = plan.comp.data() + (size_t)g * N;
+        const double C = 0.5 * G.eta * G.scale * l2, Ca = std::fabs(C);
+        double gsum = std::fabs(V.a1) + std::fabs(V.a2), cmax = 0.0;
+        for (int d = 1; d < N; ++d) gsum += std::fabs(plan.gamma[(size_t)G.vol * N + d]);
+        for (int j = 0; j + 1 < N; ++j) {
+            if (!std::isfinite(c[j])) return false;
+            cmax = std::max(cmax, std::fabs(c[j]));
+        }
+        // t in units of 2^-ut: |t| < 2^(62 - ut), C 2^(ut - ux) < 1 for its factor
+        const double bound = Ca * wmax * gsum + 0.5 * l2 * cmax + 1.0;
+        if (!std::isfinite(bound)) return false;
+        int ut = 53;
+        while (ut > 0 && (std::ldexp(bound, ut) >= std::ldexp(1.0, 62) || std::ldexp(Ca, ut - ux[G.vol]) >= 1.0)) --ut;
+        if (ut < kX64MinUt) return false;
+        X64Group& o = out.grps[g];
+        o.ut = ut;
+        o.neg = C < 0.0;
+        o.cf = (uint64_t)std::ldexp(Ca, ut - ux[G.vol] + 64);
+        o.dtxi = G.dt * G.xi;
+        o.sdtxi = G.sdt * std::sqrt(G.xi);
+        uint64_t* q = out.comp.data() + (size_t)g * N;
+        for (int j = 0; j + 1 < N; ++j) {
+            // comp / 2 log2 e in two parts, so the fixed-point value is rounded once
+            const double hc = 0.5 * c[j], p = hc * l2, lo = std::fma(hc, l2, -p) + hc * l2lo;
+            q[j] = (uint64_t)((int64_t)std::ldexp(p, ut) + (int64_t)std::llrint(std::ldexp(lo, ut))) + (o.cf >> 1) - 1;
+        }
+    }
+    return true;
+}
+
+}  // namespace rbg

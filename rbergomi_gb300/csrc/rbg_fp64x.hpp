@@ -1,0 +1,58 @@
+// rbg_fp64x.hpp -- the FP64 form's fixed-point / tensor-core path pass
+// (rbg_fp64x.cu): its tables and launchers.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdint>
+#include <vector>
+
+#include "rbg_internal.hpp"
+
+namespace rbg {
+
+// Steps the digit convolution takes (its accumulators' exactness, rbg_fp64x.cu).
+constexpr int kX64MaxN = 4096;
+// Fewest fraction bits of the variance exponent: parameters whose worst-case
+// exponent leaves fewer go through the FP64 kernels.
+constexpr int kX64MinUt = 50;
+
+struct X64Vol {
+    int sh;             // X = S_hi 2^sh + S_lo 2^(sh - 32), unit 2^-ux
+    int vg_begin, vg_end, pad;
+    uint64_t a2f, a2h;  // a2 2^(ux - 59 + 64); its half, less the product's mean truncation
+};
+struct X64Group {
+    uint64_t cf;  // |eta scale log2(e) / 2| 2^(ut - ux + 64)
+    int ut, neg;  // fraction bits of the exponent; sign of the factor
+    double dtxi, sdtxi;
+};
+struct X64Tables {
+    std::vector<X64Vol> vols;
+    std::vector<X64Group> grps;
+    std::vector<int64_t> gam;    // [n_vol][N] (a1, Gamma_1, ...), unit 2^(e - 62)
+    std::vector<uint64_t> comp;  // [n_vg][N] compensator in exponent units, plus cf / 2 - 1
+    int max_groups = 0;          // most variance groups of one pass
+};
+// False where the plan's numbers do not fit the fixed-point ranges.
+bool x64_prepare(const Plan& plan, X64Tables& out);
+
+int x64_blocks(int N);
+size_t x64_panel_bytes(int N);  // per Volterra pass
+size_t x64_digit_bytes(int64_t B, int N);
+
+// The launchers return nonzero where the device refuses.
+// Z[m][s][j] as launch_normals; dig non-null: the digits of W1 too.
+int launch_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int f32, double* Z, unsigned char* dig, int ns,
+                         cudaStream_t st);
+void launch_panels(const int64_t* gam, int nv, int N, unsigned char* panels, cudaStream_t st);
+// X[v][m][j] + 2^63
+int launch_volterra_exact(const unsigned char* dig, const unsigned char* panels, const X64Vol* vols, int nv, int N,
+                          int64_t B, uint64_t* X, unsigned int* err, cudaStream_t st);
+// ivb[g][B] (Ivdt, IsvdW); ns = 3: ivp[g][B] IsvdWp too
+int launch_variance_fixed(const X64Vol* vols, const X64Group* grps, const uint64_t* comp, const double* Z,
+                          const uint64_t* X, int nv, int max_groups, int ns, int N, int64_t B, double* ivb, double* ivp,
+                          cudaStream_t st);
+
+}  // namespace rbg

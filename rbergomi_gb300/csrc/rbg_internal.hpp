@@ -106,9 +106,6 @@ int fp64_fft_log2_len(int N);
 // host tables of the FP64 FFT: spec [n_vol][L], tw [L] (complex doubles)
 void fp64_fft_tables(const double* gamma, int n_vol, int N, int logL, double* spec, double* tw);
 
-// ns normal streams per path: 2 (W1, W1perp) for RT, 3 (+ Wperp) for plain MC
-void launch_normals(uint64_t seed, int64_t path0, int64_t B, int N, int f32, double* Z, void* stream, int ns = 2);
-
 // Sobol' quasi-Monte Carlo normals (rbg_qmc.cu).  Direction integers per
 // coordinate: kSobolBits columns; coordinate d of point s is (XOR of
 // V[d][k] over the set bits k of s ^ (s >> 1)) * 2^-62.

@@ -1,0 +1,72 @@
+"""The FP64 form's fixed-point / tensor-core path pass (Philox normals, no
+backend asked for) against the FP64 kernels on the same normals: prices to
+1e-12 relative, the FP64 form's parity bound, at the edges of its tiles (16-step
+chunks, 128-step blocks, 64 paths), over several passes and variance groups,
+and where its ranges end."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+XI, K = 0.235 ** 2, [0.85, 1.0, 1.1]
+
+
+@pytest.fixture(scope="module")
+def R():
+    import rbergomi_gb300 as R
+    return R
+
+
+def close(a, b, tol=1e-12):
+    assert np.all(np.abs(a - b) <= tol * np.abs(b)), np.max(np.abs(a - b) / np.abs(b))
+
+
+@pytest.mark.parametrize("N", [1, 2, 3, 15, 16, 17, 33, 127, 128, 129, 143, 145, 256, 257, 400, 1023, 1025])
+@pytest.mark.parametrize("M", [1, 63, 65, 700])
+def test_against_the_direct_sum(R, N, M):
+    args = (XI, [0.07], [1.9], [-0.9], [1.0] * 3, K, N, M)
+    p, s, _ = R.price_rt(*args, seed=3, path_offset=2 ** 32 - 50)
+    q, t, _ = R.price_rt(*args, seed=3, path_offset=2 ** 32 - 50, conv=R.CONV_DIRECT)
+    close(p, q)
+    if M > 1:
+        close(s, t, 1e-8)
+
+
+@pytest.mark.parametrize("N", [2047, 2049, 4096])
+def test_long_horizons(R, N):
+    args = (XI, [0.1, 0.45], [1.9, 1.0], [-0.9, -0.5], [2.0] * 3, K, N, 300)
+    close(R.price_rt(*args, seed=5)[0], R.price_rt(*args, seed=5, conv=R.CONV_DIRECT)[0])
+
+
+@pytest.mark.parametrize("n_t", [1, 3, 4, 5, 9])  # variance groups per pass: one, short and full batches of four
+@pytest.mark.parametrize("mc", [False, True])
+def test_passes_and_groups(R, n_t, mc):
+    price = R.price_mc if mc else R.price_rt
+    H, eta, rho = [0.05, 0.3, 0.45], [1.5, 2.0, 1.0], [-0.7, -0.3, -0.9]
+    T, Ks = np.repeat(np.linspace(0.1, 2.5, n_t), 2), np.tile([0.9, 1.05], n_t)
+    args = (0.05, H, eta, rho, T, Ks, 150, 333)
+    close(price(*args, seed=8)[0], price(*args, seed=8, conv=R.CONV_DIRECT)[0])
+
+
+@pytest.mark.parametrize("H,eta,T", [(0.01, 3.0, 3.0), (0.5, 0.0, 1.0), (0.9, 0.5, 0.01), (0.3, -1.5, 1.0), (0.2, 40.0, 5.0),
+                                     (0.1, 1e5, 1.0)])
+def test_parameter_corners(R, H, eta, T):
+    # the last ones' exponents do not fit the fixed-point range: the FP64 kernels take them
+    args = (XI, [H], [eta], [-0.5], [T] * 3, K, 200, 500)
+    p, q = R.price_rt(*args, seed=2)[0], R.price_rt(*args, seed=2, conv=R.CONV_DIRECT)[0]
+    assert np.array_equal(np.isnan(p), np.isnan(q))
+    close(p[~np.isnan(q)], q[~np.isnan(q)])
+
+
+@pytest.mark.parametrize("xi", [0.0, -1.0, 1e-300, 1e6])
+def test_forward_variance_corners(R, xi):
+    args = (xi, [0.1], [1.0], [-0.5], [1.0], [1.2], 64, 100)
+    p, q = R.price_rt(*args, seed=2)[0], R.price_rt(*args, seed=2, conv=R.CONV_DIRECT)[0]
+    assert np.array_equal(np.isnan(p), np.isnan(q))
+    ok = ~np.isnan(q)
+    assert np.all(np.abs(p - q)[ok] <= 1e-12 * np.abs(q[ok]) + 1e-300)
+
+
+def test_fp32_normals(R):
+    args = (XI, [0.07], [1.9], [-0.9], [1.0] * 3, K, 130, 500)
+    p = R.price_rt(*args, seed=4, normals=R.NORMALS_F32)[0]
+    close(p, R.price_rt(*args, seed=4, normals=R.NORMALS_F32, conv=R.CONV_DIRECT)[0])
