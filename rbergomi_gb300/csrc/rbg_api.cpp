@@ -449,7 +449,8 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
         const int nchunks = (int)((b + 256 * (int64_t)G - 1) / (256 * (int64_t)G));
         {
             ProfScope ps(kStagePayoff, st);
-            launch_payoff_sums(ts.t, c.ivb.as<double>(), b, b, G, c.part.as<double>(), nchunks, st, ivp);
+            if (launch_payoff_sums(ts.t, c.ivb.as<double>(), b, b, G, c.part.as<double>(), nchunks, st, ivp))
+                return fail(RBG_ERR_CUDA, "FP64 payoff kernel could not be configured");
         }
         {
             ProfScope ps(kStageReduce, st);
@@ -901,7 +902,8 @@ static int payoffs_quadrature(const rbg_params* p, const double* Z, double* payo
             Pd = c->pay.as<double>();
         }
         launch_path_fp64(ts.t, Zd, b, c->ivb.as<double>(), st, ivp);
-        launch_payoff_store(ts.t, c->ivb.as<double>(), b, b, Pd, st, ivp);
+        if (launch_payoff_store(ts.t, c->ivb.as<double>(), b, b, Pd, st, ivp))
+            return fail(RBG_ERR_CUDA, "FP64 payoff kernel could not be configured");
         RBG_CUDA(cudaGetLastError());
         if (!device_ptrs)
             RBG_CUDA(cudaMemcpyAsync(payoff + m0 * no, Pd, sizeof(double) * no * b, cudaMemcpyDeviceToHost, st));

@@ -243,4 +243,148 @@ RBG_HD double exp2_fixed(int64_t x, int ut, const uint64_t* E)
     return bits_double(e > 1023 ? 0x7FF0000000000000ull : (e < -1022 ? 0ull : b));
 }
 
+// 2^x of a double through exp2_fixed, for x < 1022 (infinity from there on):
+// NaN for NaN, zero below the normal range.
+RBG_HD double exp2_double(double x, const uint64_t* E)
+{
+    const uint64_t b = double_bits(x);
+    const uint32_t h = hi32(b) & 0x7FFFFFFFu;
+    if (h >= 0x408FF000u) {  // |x| >= 1022, or NaN
+        if (h > 0x7FF00000u || (h == 0x7FF00000u && lo32(b))) return x;
+        return bits_double((b >> 63) ? 0ull : 0x7FF0000000000000ull);
+    }
+    const int sh = (int)(h >> 20) - (1023 + 52 - 53);  // <= 10
+    const uint64_t m = (b & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
+    const uint64_t a = sh >= 0 ? m << (sh & 63) : (sh > -64 ? m >> (-sh & 63) : 0ull);
+    const uint64_t s = (uint64_t)((int64_t)b >> 63);
+    return exp2_fixed((int64_t)((a ^ s) - s), 53, E);
+}
+
+// ---------------------------------------------------- normal tail, FP64
+// Mills' ratio M(x) = (1 - Phi(x)) / phi(x), x >= 0: polynomials of degree 7
+// about the centres of 64 intervals per octave of y = 1 + x, y < 64: the Taylor
+// series, c_n = (-1)^n / n! times the integral of s^n exp(-x s - s^2 / 2) over s
+// > 0, with its terms 8 and 9 economised (Chebyshev: what is left of them is
+// below 2^-57 of M).
+constexpr int kMillsIntervals = 6 * 64, kMillsCoefs = 8;
+struct MillsTable {
+    double c[kMillsIntervals][kMillsCoefs];
+};
+
+RBG_HD double mills(double x, const MillsTable& T)
+{
+    double y = 1.0 + x;
+    uint32_t h = hi32(double_bits(y));
+    if (h >= 0x404FE000u) {  // y >= 63.75: phi is zero from x = 39 on
+        y = 63.5;
+        h = 0x404FC000u;
+    }
+    const double* c = T.c[(h - 0x3FF00000u) >> 14];
+    const double t = y - bits_double((uint64_t)((h & 0xFFFFC000u) | 0x2000u) << 32);
+    double p = c[7];
+    p = fma(p, t, c[6]);
+    p = fma(p, t, c[5]);
+    p = fma(p, t, c[4]);
+    p = fma(p, t, c[3]);
+    p = fma(p, t, c[2]);
+    p = fma(p, t, c[1]);
+    return fma(p, t, c[0]);
+}
+
+// The integrals I_n(x) of s^n exp(-x s - s^2 / 2): I_{n+1} = n I_{n-1} - x I_n
+// with I_1 = 1 - x I_0.  Forward from erfc for x < 1; above, where that
+// cancels, backward (the I_n are the recurrence's minimal solution) and
+// normalised by I_1 + x I_0 = 1.
+inline void mills_table(MillsTable& T)
+{
+    for (int i = 0; i < kMillsIntervals; ++i) {
+        const uint64_t b = (uint64_t)((0x3FF00000u + ((uint32_t)i << 14)) | 0x2000u) << 32;
+        double yc;
+        std::memcpy(&yc, &b, 8);
+        const long double x = (long double)yc - 1.0L;
+        constexpr int terms = kMillsCoefs + 2;
+        long double I[terms];
+        if (x < 1.0L) {
+            I[0] = std::exp(x * x / 2) * std::erfc(x * 0.707106781186547524400844362104849039L) *
+                   1.25331413731550025120788264240552263L;
+            I[1] = 1.0L - x * I[0];
+            for (int n = 1; n + 1 < terms; ++n) I[n + 1] = n * I[n - 1] - x * I[n];
+        } else {
+            const int top = 30 + (int)(600.0L / (x * x));  // the start value decays as exp(-2 x sqrt(top))
+            long double a = 0.0L, c = 1.0L;  // I_{n+1}, I_n up to a factor
+            for (int n = top; n >= 1; --n) {
+                const long double d = (a + x * c) / n;  // I_{n-1}
+                a = c;
+                c = d;
+                if (n - 1 < terms) I[n - 1] = c;
+                if (c > 1e300L) {  // keep the unnormalised values in range
+                    a *= 1e-300L;
+                    c *= 1e-300L;
+                    for (int k = n - 1; k < terms; ++k) I[k] *= 1e-300L;
+                }
+            }
+            const long double f = 1.0L / (I[1] + x * I[0]);
+            for (int n = 0; n < terms; ++n) I[n] *= f;
+        }
+        // u = t / h on the interval: u^8 = T_8 / 128 + 2 u^6 - 5/4 u^4 + 1/4 u^2 - 1/128,
+        // u^9 = T_9 / 256 + 9/4 u^7 - 27/16 u^5 + 15/32 u^3 - 9/256 u
+        const long double h = std::ldexp(1.0L, i / 64 - 7);
+        long double a[terms], hn = 1.0L, fact = 1.0L;
+        for (int n = 0; n < terms; ++n, hn *= h) {
+            if (n) fact *= -n;
+            a[n] = I[n] / fact * hn;
+        }
+        const long double w8[4] = {-1.0L / 128, 0.25L, -1.25L, 2.0L}, w9[4] = {-9.0L / 256, 15.0L / 32, -27.0L / 16, 2.25L};
+        for (int k = 0; k < 4; ++k) {
+            a[2 * k] += a[8] * w8[k];
+            a[2 * k + 1] += a[9] * w9[k];
+        }
+        hn = 1.0L;
+        for (int n = 0; n < kMillsCoefs; ++n, hn *= h) T.c[i][n] = (double)(a[n] / hn);
+    }
+}
+
+// Every table above, one copy per device.
+struct FixedTables {
+    NormalTables normals;
+    uint64_t exp2[kExpTable];
+    MillsTable mills;
+};
+
+// Their values, in extended precision on the host.
+inline void fill_fixed_tables(FixedTables& F)
+{
+    NormalTables& T = F.normals;
+    for (int k = 0; k < kLnTable; ++k) {
+        const long double c = 1.0L + (k + 0.5L) / kLnTable;
+        T.ln[k] = FixedPair{(uint64_t)(std::ldexp(1.0L / c, 64) + 0.5L), (uint64_t)(std::ldexp(std::log(c), 63) + 0.5L)};
+    }
+    const long double pi = 3.14159265358979323846264338327950288L, ln2 = 0.693147180559945309417232121458176568L;
+    for (int k = 0; k < kTrigTable; ++k) {
+        const long double a = pi * k / (2 * kTrigTable);
+        T.trig[k] = FixedPair{(uint64_t)(std::ldexp(std::cos(a), 63) + 0.5L),
+                              (uint64_t)(std::ldexp(std::sin(a), 63) + 0.5L)};
+    }
+    for (int n = 0; n < kLn2Table; ++n) T.ln2[n] = (uint64_t)(std::ldexp(ln2 * n, 58) + 0.5L);
+    for (int k = 0; k < kExpTable; ++k)
+        F.exp2[k] = (uint64_t)(std::ldexp(std::exp2(k / (long double)kExpTable), 63) + 0.5L);
+    mills_table(F.mills);
+}
+
+// Conditional Black-Scholes call (tau = 1, r = 0) from the parts that do not
+// depend on the strike: S, lnS, vol, rv = 1 / vol.  With S phi(d1) = K phi(d2)
+// and 1 - Phi(x) = phi(x) M(x), the call is
+//   [d1 >= 0] S - [d2 >= 0] K + S phi(d1) (-+ M(|d1|) +- M(|d2|)):
+// one exponential, and tails that keep their relative accuracy.
+RBG_HD double call_mills(double S, double lnS, double vol, double rv, double K, double lnK, const MillsTable& T,
+                         const uint64_t* E)
+{
+    const double d1 = fma(lnS - lnK, rv, 0.5 * vol), d2 = d1 - vol;
+    // S phi(d1) = 2^(log2(e) (lnS - d1^2 / 2) - log2(2 pi) / 2)
+    const double f = exp2_double(fma(fma(-0.5 * d1, d1, lnS), 1.4426950408889634074, -1.3257480647361593990), E);
+    const double m1 = mills(fabs(d1), T), m2 = mills(fabs(d2), T);
+    const double base = (d1 >= 0.0 ? S : 0.0) - (d2 >= 0.0 ? K : 0.0);
+    return fma(f, (d1 >= 0.0 ? -m1 : m1) + (d2 >= 0.0 ? m2 : -m2), base);
+}
+
 }  // namespace rbg

@@ -18,10 +18,14 @@
 // GB300's FP64 pipe (~2 DFMA/clk/SM) bounds every kernel here.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <mutex>
 
 #include "rbg_device.cuh"
+#include "rbg_fixed.cuh"
+#include "rbg_fp64x.hpp"
 #include "rbg_internal.hpp"
 
 namespace rbg {
@@ -363,71 +367,190 @@ void launch_path_fp64(const Fp64Tables& t, const double* Z, int64_t B, double* i
 }
 
 // ------------------------------------------------------------ payoff sums
-constexpr int kOPB = 8;  // outputs per block
+// The conditional Black-Scholes call by Mills' ratio and a fixed-point
+// exponential (rbg_fixed.cuh): about 30 FP64 operations an output and path
+// with the strike-independent parts shared, against about 250 for
+// library log, exp, sqrt and two erfc each time (FP64 pipe: 64 cycles a warp
+// operation).  Blocks keep both tables in shared memory (56 KB) and walk over
+// (chunk, run of 8 outputs) tasks.
+constexpr int kOPB = 8;  // outputs per task
+constexpr int kPayThreads = 256;
 
-// grid (nchunks, ceil(n_out / kOPB)), 256 threads; chunk c covers paths
-// [c G 256, (c+1) G 256) of the batch; part[(c * n_out + i) * 4 + {0,1,2,3}] =
-// (sum, comp, sum2, comp2).
-// MC = 1: plain Monte Carlo payoff from (Ivdt, IsvdW) and ivp = IsvdWp.
+struct OutF64 {
+    double rho, K, lnK;
+    int vg;  // -1 past the last output
+    int ok;  // K in the range of the fast form
+};
 template <int MC>
-__global__ void __launch_bounds__(256) k_payoff_sums(Fp64Tables t, const double2* __restrict__ ivb, int64_t B,
-                                                     int64_t stride, int G, double* __restrict__ part,
-                                                     const double* __restrict__ ivp)
+struct PayoffSmem {
+    uint64_t E[kExpTable];
+    MillsTable T;
+    OutF64 out[kOPB];
+    double red[kPayThreads / 32][2 * kOPB];
+};
+
+template <int MC>
+__device__ __forceinline__ void payoff_tables(PayoffSmem<MC>& sm, const FixedTables* __restrict__ ft)
 {
-    __shared__ double red[8][kOPB][2];
-    const int c = blockIdx.x;
-    const int o0 = blockIdx.y * kOPB;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    double S = 0, CS = 0, S2 = 0, CS2 = 0;  // meaningful in threads q < kOPB
-    OutDev od[kOPB];
-#pragma unroll
-    for (int q = 0; q < kOPB; ++q) {
-        const int i = o0 + q;
-        od[q] = (i < t.n_out) ? t.outs[i] : OutDev{0.0, 1.0, -1, 0};
-    }
-    for (int sub = 0; sub < G; ++sub) {
-        const int64_t m = ((int64_t)c * G + sub) * 256 + threadIdx.x;
-#pragma unroll
-        for (int q = 0; q < kOPB; ++q) {
-            double x = 0.0;
-            if (m < B && od[q].vg >= 0) {
-                const size_t at = (size_t)od[q].vg * stride + m;
-                const double2 iv = ivb[at];
-                x = MC ? mc_payoff(iv.x, iv.y, ivp[at], od[q].rho, od[q].K) : rt_payoff(iv.x, iv.y, od[q].rho, od[q].K);
-            }
-            double x2 = x * x;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                x += __shfl_xor_sync(0xffffffffu, x, o);
-                x2 += __shfl_xor_sync(0xffffffffu, x2, o);
-            }
-            if (lane == 0) { red[w][q][0] = x; red[w][q][1] = x2; }
-        }
-        __syncthreads();
-        if (threadIdx.x < kOPB) {
-            const int q = threadIdx.x;
-            double a = 0, a2 = 0;
-            for (int k = 0; k < 8; ++k) { a += red[k][q][0]; a2 += red[k][q][1]; }
-            neumaier_add(S, CS, a);
-            neumaier_add(S2, CS2, a2);
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x < kOPB && o0 + (int)threadIdx.x < t.n_out) {
-        double* p = part + ((size_t)c * t.n_out + o0 + threadIdx.x) * 4;
-        p[0] = S; p[1] = CS; p[2] = S2; p[3] = CS2;
+    for (int i = threadIdx.x; i < kExpTable; i += kPayThreads) sm.E[i] = ft->exp2[i];
+    if (!MC) {
+        const double* src = ft->mills.c[0];
+        double* dst = reinterpret_cast<double*>(&sm.T);
+        for (int i = threadIdx.x; i < kMillsIntervals * kMillsCoefs; i += kPayThreads) dst[i] = src[i];
     }
 }
 
-void launch_payoff_sums(const Fp64Tables& t, const double* ivb, int64_t B, int64_t stride, int G, double* part,
-                        int nchunks, void* stream, const double* ivp)
+// Outputs o0 .. o0 + 7 of the task, for the whole block.
+template <int MC>
+__device__ __forceinline__ void payoff_outs(PayoffSmem<MC>& sm, const Fp64Tables& t, int o0)
 {
-    dim3 grid(nchunks, (t.n_out + kOPB - 1) / kOPB);
-    if (ivp)
-        k_payoff_sums<1><<<grid, 256, 0, (cudaStream_t)stream>>>(t, (const double2*)ivb, B, stride, G, part, ivp);
-    else
-        k_payoff_sums<0><<<grid, 256, 0, (cudaStream_t)stream>>>(t, (const double2*)ivb, B, stride, G, part, ivp);
+    __syncthreads();  // the previous task's readers (and the tables)
+    if (threadIdx.x < kOPB) {
+        const int i = o0 + (int)threadIdx.x;
+        const OutDev od = (i < t.n_out) ? t.outs[i] : OutDev{0.0, 1.0, -1, 0};
+        const bool ok = od.K > 1e-200 && od.K < 1e200;
+        sm.out[threadIdx.x] = OutF64{od.rho, od.K, ok ? log(od.K) : 0.0, od.vg, ok};
+    }
+    __syncthreads();
+}
+
+// The strike-independent part of a path's conditional call, kept while
+// consecutive outputs share variance group and rho.
+struct RtState {
+    double Iv = 0.0, Is = 0.0, S = 0.0, lnS = 0.0, vol = 0.0, rv = 0.0, rho = 0.0;
+    int vg = -1;
+    bool ok = false;
+};
+
+__device__ __forceinline__ double payoff_rt(RtState& r, const OutF64& o, const double2* __restrict__ ivb, size_t at,
+                                            const PayoffSmem<0>& sm)
+{
+    if (o.vg != r.vg || o.rho != r.rho) {
+        const double2 iv = ivb[at];
+        r.vg = o.vg;
+        r.rho = o.rho;
+        r.Iv = iv.x;
+        r.Is = iv.y;
+        const double v2 = (1.0 - o.rho * o.rho) * iv.x;
+        r.lnS = fma(-0.5 * o.rho * o.rho, iv.x, o.rho * iv.y);
+        r.S = exp2_double(1.4426950408889634074 * r.lnS, sm.E);
+        r.vol = sqrt(v2);
+        r.rv = 1.0 / r.vol;
+        r.ok = v2 > 1e-200 && v2 < 1e200 && r.S > 1e-200 && r.S < 1e200;
+    }
+    // zero or undefined conditional variance, spots and strikes out of range: the plain formula
+    if (!(r.ok && o.ok)) return rt_payoff(r.Iv, r.Is, o.rho, o.K);
+    return call_mills(r.S, r.lnS, r.vol, r.rv, o.K, o.lnK, sm.T, sm.E);
+}
+
+__device__ __forceinline__ double payoff_mc(const OutF64& o, const double2* __restrict__ ivb,
+                                            const double* __restrict__ ivp, size_t at, const PayoffSmem<1>& sm)
+{
+    // mc_payoff's log S, the exponential in fixed point
+    const double2 iv = ivb[at];
+    const double lnS = o.rho * iv.y + sqrt(1.0 - o.rho * o.rho) * ivp[at] - 0.5 * iv.x;
+    const double d = (fabs(lnS) < 700.0 ? exp2_double(1.4426950408889634074 * lnS, sm.E) : exp(lnS)) - o.K;
+    return d > 0.0 ? d : 0.0;
+}
+
+// Warp sums of 16 doubles a lane in the order of the xor tree 16, 8, 4, 2, 1
+// (16 additions a lane instead of 80): value lane >> 1 on every lane.
+__device__ __forceinline__ double warp_sums16_f64(double (&v)[2 * kOPB])
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int n = 8, o = 16; n >= 1; n >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const double send = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+// chunk c covers paths [c G 256, (c+1) G 256) of the batch, G per thread;
+// part[(c * n_out + i) * 4 + {0,1,2,3}] = (sum, comp, sum2, comp2).
+// MC = 1: plain Monte Carlo payoff from (Ivdt, IsvdW) and ivp = IsvdWp.
+template <int MC>
+__global__ void __launch_bounds__(kPayThreads) k_payoff_sums(Fp64Tables t, const double2* __restrict__ ivb, int64_t B,
+                                                     int64_t stride, int G, double* __restrict__ part, int nchunks,
+                                                     const double* __restrict__ ivp, const FixedTables* __restrict__ ft)
+{
+    extern __shared__ uint64_t psm[];
+    PayoffSmem<MC>& sm = *reinterpret_cast<PayoffSmem<MC>*>(psm);
+    payoff_tables<MC>(sm, ft);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t tasks = (int64_t)nchunks * ((t.n_out + kOPB - 1) / kOPB);
+    for (int64_t task = blockIdx.x; task < tasks; task += gridDim.x) {
+        const int c = (int)(task % nchunks), o0 = (int)(task / nchunks) * kOPB;
+        payoff_outs<MC>(sm, t, o0);
+        double s[2 * kOPB];  // sums of x, then of x^2
+#pragma unroll
+        for (int q = 0; q < 2 * kOPB; ++q) s[q] = 0.0;
+        for (int sub = 0; sub < G; ++sub) {
+            const int64_t m = ((int64_t)c * G + sub) * 256 + threadIdx.x;
+            if (m >= B) break;
+            RtState r;
+#pragma unroll
+            for (int q = 0; q < kOPB; ++q) {
+                const OutF64 o = sm.out[q];
+                if (o.vg < 0) continue;
+                const size_t at = (size_t)o.vg * stride + m;
+                double x;
+                if constexpr (MC) x = payoff_mc(o, ivb, ivp, at, sm);
+                else x = payoff_rt(r, o, ivb, at, sm);
+                s[q] += x;
+                s[kOPB + q] = fma(x, x, s[kOPB + q]);
+            }
+        }
+        const double v = warp_sums16_f64(s);
+        if (!(lane & 1)) sm.red[w][lane >> 1] = v;
+        __syncthreads();
+        if (threadIdx.x < 2 * kOPB && o0 + (int)(threadIdx.x & (kOPB - 1)) < t.n_out) {
+            const int q = threadIdx.x & (kOPB - 1), z = threadIdx.x / kOPB;
+            double S = 0, C = 0;
+            for (int k = 0; k < kPayThreads / 32; ++k) neumaier_add(S, C, sm.red[k][threadIdx.x]);
+            double* p = part + ((size_t)c * t.n_out + o0 + q) * 4 + 2 * z;
+            p[0] = S;
+            p[1] = C;
+        }
+    }
+}
+
+// Raises a payoff kernel's shared-memory limit, once per device.
+template <class F>
+static bool payoff_smem_ready(F* kern, size_t bytes, bool (&ready)[64])
+{
+    static std::mutex mu;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    std::lock_guard<std::mutex> lk(mu);
+    if (!ready[dev] && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess)
+        ready[dev] = true;
+    return ready[dev];
+}
+
+int launch_payoff_sums(const Fp64Tables& t, const double* ivb, int64_t B, int64_t stride, int G, double* part,
+                       int nchunks, void* stream, const double* ivp)
+{
+    static bool ready[2][64] = {};
+    const FixedTables* ft = fixed_tables();
+    if (!ft) return -1;
+    const int64_t tasks = (int64_t)nchunks * ((t.n_out + kOPB - 1) / kOPB);
+    const unsigned grid = (unsigned)std::min<int64_t>(tasks, 3 * (int64_t)device_sms());
+    if (ivp) {
+        if (!payoff_smem_ready(k_payoff_sums<1>, sizeof(PayoffSmem<1>), ready[1])) return -1;
+        k_payoff_sums<1><<<grid, kPayThreads, sizeof(PayoffSmem<1>), (cudaStream_t)stream>>>(
+            t, (const double2*)ivb, B, stride, G, part, nchunks, ivp, ft);
+    } else {
+        if (!payoff_smem_ready(k_payoff_sums<0>, sizeof(PayoffSmem<0>), ready[0])) return -1;
+        k_payoff_sums<0><<<grid, kPayThreads, sizeof(PayoffSmem<0>), (cudaStream_t)stream>>>(
+            t, (const double2*)ivb, B, stride, G, part, nchunks, ivp, ft);
+    }
     count_launch();
+    return 0;
 }
 
 // acc[i * 4 + {0..3}] += the batch's chunk sums.  One block per output:
@@ -738,35 +861,54 @@ void launch_implied_vol(int n, const double* price, const double* K, const doubl
 }
 
 // ------------------------------------------------------------ quadrature
+// payoff[m * n_out + i]: tasks of 256 paths x 8 outputs.
 template <int MC>
-__global__ void k_payoff_store(Fp64Tables t, const double2* __restrict__ ivb, int64_t B, int64_t stride,
-                               double* __restrict__ payoff, const double* __restrict__ ivp)
+__global__ void __launch_bounds__(kPayThreads) k_payoff_store(Fp64Tables t, const double2* __restrict__ ivb, int64_t B,
+                               int64_t stride, double* __restrict__ payoff, const double* __restrict__ ivp,
+                               const FixedTables* __restrict__ ft)
 {
-    const int64_t total = B * t.n_out;
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t m = idx / t.n_out;
-        const int i = (int)(idx - m * t.n_out);
-        const OutDev od = t.outs[i];
-        const size_t at = (size_t)od.vg * stride + m;
-        const double2 iv = ivb[at];
-        payoff[idx] = MC ? mc_payoff(iv.x, iv.y, ivp[at], od.rho, od.K) : rt_payoff(iv.x, iv.y, od.rho, od.K);
+    extern __shared__ uint64_t psm[];
+    PayoffSmem<MC>& sm = *reinterpret_cast<PayoffSmem<MC>*>(psm);
+    payoff_tables<MC>(sm, ft);
+    const int64_t tiles = (B + kPayThreads - 1) / kPayThreads, tasks = tiles * ((t.n_out + kOPB - 1) / kOPB);
+    for (int64_t task = blockIdx.x; task < tasks; task += gridDim.x) {
+        const int o0 = (int)(task / tiles) * kOPB;
+        const int64_t m = task % tiles * kPayThreads + threadIdx.x;
+        payoff_outs<MC>(sm, t, o0);
+        if (m >= B) continue;
+        RtState r;
+#pragma unroll
+        for (int q = 0; q < kOPB; ++q) {
+            const OutF64 o = sm.out[q];
+            if (o.vg < 0) continue;
+            const size_t at = (size_t)o.vg * stride + m;
+            double x;
+            if constexpr (MC) x = payoff_mc(o, ivb, ivp, at, sm);
+            else x = payoff_rt(r, o, ivb, at, sm);
+            payoff[m * t.n_out + o0 + q] = x;
+        }
     }
 }
 
-void launch_payoff_store(const Fp64Tables& t, const double* ivb, int64_t B, int64_t stride, double* payoff,
-                         void* stream, const double* ivp)
+int launch_payoff_store(const Fp64Tables& t, const double* ivb, int64_t B, int64_t stride, double* payoff,
+                        void* stream, const double* ivp)
 {
-    const int64_t total = B * t.n_out;
-    int64_t blocks = (total + 255) / 256;
-    if (blocks > (1 << 20)) blocks = 1 << 20;
-    if (ivp)
-        k_payoff_store<1><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(t, (const double2*)ivb, B, stride,
-                                                                             payoff, ivp);
-    else
-        k_payoff_store<0><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(t, (const double2*)ivb, B, stride,
-                                                                             payoff, ivp);
+    static bool ready[2][64] = {};
+    const FixedTables* ft = fixed_tables();
+    if (!ft) return -1;
+    const int64_t tasks = (B + kPayThreads - 1) / kPayThreads * ((t.n_out + kOPB - 1) / kOPB);
+    const unsigned grid = (unsigned)std::min<int64_t>(tasks, 3 * (int64_t)device_sms());
+    if (ivp) {
+        if (!payoff_smem_ready(k_payoff_store<1>, sizeof(PayoffSmem<1>), ready[1])) return -1;
+        k_payoff_store<1><<<grid, kPayThreads, sizeof(PayoffSmem<1>), (cudaStream_t)stream>>>(t, (const double2*)ivb, B,
+                                                                                             stride, payoff, ivp, ft);
+    } else {
+        if (!payoff_smem_ready(k_payoff_store<0>, sizeof(PayoffSmem<0>), ready[0])) return -1;
+        k_payoff_store<0><<<grid, kPayThreads, sizeof(PayoffSmem<0>), (cudaStream_t)stream>>>(t, (const double2*)ivb, B,
+                                                                                             stride, payoff, ivp, ft);
+    }
     count_launch();
+    return 0;
 }
 
 // ------------------------------------------------------- control variate

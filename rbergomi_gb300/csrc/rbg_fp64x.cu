@@ -39,39 +39,32 @@
 namespace rbg {
 
 // ------------------------------------------------------------------ tables
-__device__ NormalTables g_normal_tables;
-__device__ uint64_t g_exp_table[kExpTable];
+__device__ FixedTables g_fixed_tables;
 
-// Fills the device's tables once (extended precision on the host).
-static cudaError_t ensure_fixed_tables()
+// The device's tables, filled on first use; null where that fails.
+const FixedTables* fixed_tables()
 {
     static std::mutex mu;
-    static bool ready[64] = {};
+    static const FixedTables* at[64] = {};
     int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+        cudaGetLastError();
+        return nullptr;
+    }
     std::lock_guard<std::mutex> lk(mu);
-    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    if (ready[dev]) return cudaSuccess;
-    static NormalTables T;
-    static uint64_t E[kExpTable];
-    for (int k = 0; k < kLnTable; ++k) {
-        const long double c = 1.0L + (k + 0.5L) / kLnTable;
-        T.ln[k] = FixedPair{(uint64_t)(std::ldexp(1.0L / c, 64) + 0.5L), (uint64_t)(std::ldexp(std::log(c), 63) + 0.5L)};
+    if (!at[dev]) {
+        static FixedTables T;
+        void* p = nullptr;
+        fill_fixed_tables(T);
+        if (cudaGetSymbolAddress(&p, g_fixed_tables) != cudaSuccess ||
+            cudaMemcpy(p, &T, sizeof T, cudaMemcpyHostToDevice) != cudaSuccess ||
+            cudaDeviceSynchronize() != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        at[dev] = static_cast<const FixedTables*>(p);
     }
-    const long double pi = 3.14159265358979323846264338327950288L, ln2 = 0.693147180559945309417232121458176568L;
-    for (int k = 0; k < kTrigTable; ++k) {
-        const long double a = pi * k / 1024.0L;
-        T.trig[k] = FixedPair{(uint64_t)(std::ldexp(std::cos(a), 63) + 0.5L),
-                              (uint64_t)(std::ldexp(std::sin(a), 63) + 0.5L)};
-    }
-    for (int n = 0; n < kLn2Table; ++n) T.ln2[n] = (uint64_t)(std::ldexp(ln2 * n, 58) + 0.5L);
-    for (int k = 0; k < kExpTable; ++k) E[k] = (uint64_t)(std::ldexp(std::exp2(k / (long double)kExpTable), 63) + 0.5L);
-    e = cudaMemcpyToSymbol(g_normal_tables, &T, sizeof T);
-    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_exp_table, E, sizeof E);
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    if (e == cudaSuccess) ready[dev] = true;
-    return e;
+    return at[dev];
 }
 
 // ----------------------------------------------------------------- normals
@@ -127,11 +120,12 @@ constexpr int kNormalThreads = 256;
 template <int F32>
 __global__ void __launch_bounds__(kNormalThreads) k_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int ns,
                                                                  double* __restrict__ Z,
-                                                                 unsigned char* __restrict__ dig)
+                                                                 unsigned char* __restrict__ dig,
+                                                                 const FixedTables* __restrict__ ft)
 {
     __shared__ NormalTables T;
     if (!F32) {
-        const uint64_t* src = reinterpret_cast<const uint64_t*>(&g_normal_tables);
+        const uint64_t* src = reinterpret_cast<const uint64_t*>(&ft->normals);
         uint64_t* dst = reinterpret_cast<uint64_t*>(&T);
         for (int i = threadIdx.x; i < (int)(sizeof(NormalTables) / 8); i += kNormalThreads) dst[i] = src[i];
         __syncthreads();
@@ -196,16 +190,14 @@ __global__ void __launch_bounds__(kNormalThreads) k_normals_fixed(uint64_t seed,
 int launch_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int f32, double* Z, unsigned char* dig, int ns,
                          cudaStream_t st)
 {
-    if (ensure_fixed_tables() != cudaSuccess) {
-        cudaGetLastError();
-        return -1;
-    }
+    const FixedTables* ft = fixed_tables();
+    if (!ft) return -1;
     const int64_t octets = (B + kXPaths - 1) / kXPaths * (kXPaths / 8);
     const int64_t tasks = octets * ns * ((N + kXSteps - 1) / kXSteps);
     const int64_t need = (tasks + kNormalThreads / 32 - 1) / (kNormalThreads / 32);
     const int64_t blocks = std::min<int64_t>(need, 8 * (int64_t)device_sms());
-    if (f32) k_normals_fixed<1><<<(unsigned)blocks, kNormalThreads, 0, st>>>(seed, path0, B, N, ns, Z, dig);
-    else k_normals_fixed<0><<<(unsigned)blocks, kNormalThreads, 0, st>>>(seed, path0, B, N, ns, Z, dig);
+    if (f32) k_normals_fixed<1><<<(unsigned)blocks, kNormalThreads, 0, st>>>(seed, path0, B, N, ns, Z, dig, ft);
+    else k_normals_fixed<0><<<(unsigned)blocks, kNormalThreads, 0, st>>>(seed, path0, B, N, ns, Z, dig, ft);
     count_launch();
     return 0;
 }
@@ -556,19 +548,20 @@ constexpr int kVarThreads = 256, kVarVals = 16;
 constexpr int kVarSmem = kExpTable * 8 + (kVarThreads / 32) * kVarVals * 33 * 8;
 
 template <int NS, int GB>
-__global__ void __launch_bounds__(kVarThreads) k_variance_fixed(const X64Vol* __restrict__ vols,
+__global__ void __launch_bounds__(kVarThreads, GB > 1 ? 2 : 3) k_variance_fixed(const X64Vol* __restrict__ vols,
                                                                const X64Group* __restrict__ grps,
                                                                const uint64_t* __restrict__ comp,
                                                                const double* __restrict__ Z,
                                                                const uint64_t* __restrict__ X, int nv, int N, int64_t B,
-                                                               double* __restrict__ ivb, double* __restrict__ ivp)
+                                                               double* __restrict__ ivb, double* __restrict__ ivp,
+                                                               const FixedTables* __restrict__ ft)
 {
     constexpr int PB = kVarVals / (GB * NS);  // paths per reduction
     extern __shared__ uint64_t vsm[];
     uint64_t* E = vsm;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     double* red = reinterpret_cast<double*>(vsm + kExpTable) + (size_t)w * kVarVals * 33;
-    for (int i = threadIdx.x; i < kExpTable; i += kVarThreads) E[i] = g_exp_table[i];
+    for (int i = threadIdx.x; i < kExpTable; i += kVarThreads) E[i] = ft->exp2[i];
     __syncthreads();
     const int64_t runs = (B + PB - 1) / PB, warps = (int64_t)gridDim.x * (kVarThreads / 32);
     for (int64_t run = blockIdx.x * (int64_t)(kVarThreads / 32) + w; run < runs; run += warps) {
@@ -654,11 +647,13 @@ int launch_variance_fixed(const X64Vol* vols, const X64Group* grps, const uint64
 {
     static std::mutex mu;
     static bool ready[64] = {};
+    const FixedTables* ft = fixed_tables();
+    if (!ft) return -1;
     auto* kern = ns == 3 ? (max_groups > 1 ? k_variance_fixed<3, 4> : k_variance_fixed<3, 1>)
                          : (max_groups > 1 ? k_variance_fixed<2, 4> : k_variance_fixed<2, 1>);
     {
         int dev = 0;
-        if (ensure_fixed_tables() != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
+        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
         std::lock_guard<std::mutex> lk(mu);
         if (!ready[dev]) {
             for (auto* k : {k_variance_fixed<2, 1>, k_variance_fixed<2, 4>, k_variance_fixed<3, 1>, k_variance_fixed<3, 4>})
@@ -672,7 +667,7 @@ int launch_variance_fixed(const X64Vol* vols, const X64Group* grps, const uint64
     const int pb = kVarVals / ((max_groups > 1 ? 4 : 1) * ns);
     const int64_t runs = (B + pb - 1) / pb;
     const int64_t blocks = std::min<int64_t>((runs + kVarThreads / 32 - 1) / (kVarThreads / 32), 3 * (int64_t)device_sms());
-    kern<<<(unsigned)blocks, kVarThreads, kVarSmem, st>>>(vols, grps, comp, Z, X, nv, N, B, ivb, ivp);
+    kern<<<(unsigned)blocks, kVarThreads, kVarSmem, st>>>(vols, grps, comp, Z, X, nv, N, B, ivb, ivp, ft);
     count_launch();
     return 0;
 }

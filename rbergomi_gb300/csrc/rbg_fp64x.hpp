@@ -42,8 +42,14 @@ int x64_blocks(int N);
 size_t x64_panel_bytes(int N);  // per Volterra pass
 size_t x64_digit_bytes(int64_t B, int N);
 
+// The fixed-point and tail tables of the current device (rbg_fixed.cuh), null
+// where they could not be set up.
+struct FixedTables;
+const FixedTables* fixed_tables();
+
 // The launchers return nonzero where the device refuses.
-// Z[m][s][j] as launch_normals; dig non-null: the digits of W1 too.
+// Philox normals Z[m][s][j] of ns streams per path (W1, W1perp, plain MC: Wperp);
+// f32: the mixed form's FP32 normals, widened; dig non-null: the digits of W1 too.
 int launch_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int f32, double* Z, unsigned char* dig, int ns,
                          cudaStream_t st);
 void launch_panels(const int64_t* gam, int nv, int N, unsigned char* panels, cudaStream_t st);

@@ -139,12 +139,13 @@ void launch_payoff_sums_cv(const Fp64Tables& t, const double* ivb, const double*
 void launch_finalize_cv(const double* acc, int n_out, int64_t M, const OutDev* outs, const double* Tvals,
                         const double* alpha, const double* Q, const unsigned long long* count, double Qmax,
                         int compute_iv, double* res, void* stream);
-void launch_payoff_sums(const Fp64Tables& t, const double* ivb, int64_t B, int64_t ivb_stride, int G,
+// nonzero where the kernel could not be configured
+int launch_payoff_sums(const Fp64Tables& t, const double* ivb, int64_t B, int64_t ivb_stride, int G,
                         double* part, int nchunks, void* stream, const double* ivp = nullptr);
 void launch_accumulate(const double* part, int nchunks, int n_out, double* acc, void* stream);
 void launch_finalize(const double* acc, int n_out, int64_t M, const OutDev* outs, const double* Tvals,
                      int compute_iv, double* res, void* stream);
-void launch_payoff_store(const Fp64Tables& t, const double* ivb, int64_t B, int64_t ivb_stride, double* payoff,
+int launch_payoff_store(const Fp64Tables& t, const double* ivb, int64_t B, int64_t ivb_stride, double* payoff,
                          void* stream, const double* ivp = nullptr);
 void launch_implied_vol(int n, const double* price, const double* K, const double* T, double* iv, void* stream);
 

@@ -10,22 +10,9 @@
 
 using namespace rbg;
 
-static NormalTables T;
-static uint64_t E[kExpTable];
-
-static void tables()
-{
-    const long double pi = 3.14159265358979323846264338327950288L, ln2 = 0.693147180559945309417232121458176568L;
-    for (int k = 0; k < kLnTable; ++k) {
-        const long double c = 1.0L + (k + 0.5L) / kLnTable;
-        T.ln[k] = FixedPair{(uint64_t)(std::ldexp(1.0L / c, 64) + 0.5L), (uint64_t)(std::ldexp(std::log(c), 63) + 0.5L)};
-    }
-    for (int k = 0; k < kTrigTable; ++k)
-        T.trig[k] = FixedPair{(uint64_t)(std::ldexp(std::cos(pi * k / 1024), 63) + 0.5L),
-                              (uint64_t)(std::ldexp(std::sin(pi * k / 1024), 63) + 0.5L)};
-    for (int n = 0; n < kLn2Table; ++n) T.ln2[n] = (uint64_t)(std::ldexp(ln2 * n, 58) + 0.5L);
-    for (int k = 0; k < kExpTable; ++k) E[k] = (uint64_t)(std::ldexp(std::exp2(k / (long double)kExpTable), 63) + 0.5L);
-}
+static FixedTables F;
+static const NormalTables& T = F.normals;
+static const uint64_t* E = F.exp2;
 
 static void check_normal(uint32_t a, uint32_t b)
 {
@@ -61,7 +48,7 @@ static void check_exp2(int64_t x, int ut)
 
 int main()
 {
-    tables();
+    fill_fixed_tables(F);
     const uint32_t ea[] = {0, 1, 2, 0x7FFFFFFFu, 0x80000000u, 0xFFEFFFFFu, 0xFFF00000u, 0xFFFFFFFEu, 0xFFFFFFFFu};
     const uint32_t eb[] = {0, 1, 0x1FFFFFu, 0x200000u, 0x3FFFFFFFu, 0x40000000u, 0x7FFFFFFFu, 0x80000000u, 0xBFFFFFFFu,
                            0xC0000000u, 0xFFFFFFFFu};
