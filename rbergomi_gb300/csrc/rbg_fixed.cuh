@@ -73,17 +73,15 @@ RBG_HD uint64_t double_bits(double d)
 // uniforms stays below 6.77).
 constexpr int kNormalBits = 59;
 
-// v 2^-59 as a double, rounded to nearest (ties away from zero).
+// v 2^-59 as a double, rounded to nearest, in two FP64 additions: the words
+// become the low bits of doubles near 2^25 and 2^-7, whose sum less (2^25 + 2^4
+// + 2^-7) is v 2^-59; only the last addition rounds.  (Where integer
+// instructions are what bounds a kernel, the FP64 pipe is the one to take.)
 RBG_HD double fixed_to_double(int64_t v)
 {
-    const uint64_t s = (uint64_t)(v >> 63);
-    const uint64_t a = ((uint64_t)v ^ s) - s;
-    const int n = clz64(a);
-    const uint64_t w = a << (n & 63);
-    // 53 bits of w; their leading one, or the rounding's carry past it, adds to the exponent field
-    const uint64_t m = (w >> 11) + ((w >> 10) & 1u);
-    const uint64_t b = ((uint64_t)(uint32_t)(1023 + 62 - kNormalBits - n) << 52) + m;
-    return bits_double(a ? (b | (s << 63)) : 0ull);
+    const double a = bits_double(0x4180000000000000ull | (hi32((uint64_t)v) ^ 0x80000000u));
+    const double b = bits_double(0x3F80000000000000ull | lo32((uint64_t)v));
+    return (a - (33554448.0 + 0x1p-7)) + b;
 }
 
 // x in units of 2^-59, exact for 2^-6 <= |x| < 16 and truncated below.
@@ -99,7 +97,8 @@ RBG_HD int64_t double_to_fixed(double x)
 
 // Tables of the transform (shared memory on the device).
 //   ln[k], k < 512: centre c = 1 + (k + 1/2) / 512 of m in [1, 2);
-//          x = 2^64 / c, y = ln c in units of 2^-63
+//          x = the upper and lower 31 bits of 2^62 / c, one in each word, y = ln
+//          c in units of 2^-63
 //   trig[k], k < 512: (cos, sin)(pi k / 1024) in units of 2^-63
 //   ln2[n], n <= 33: n ln 2 in units of 2^-58
 struct FixedPair {
@@ -112,21 +111,47 @@ struct NormalTables {
     uint64_t ln2[kLn2Table];
 };
 
-// 1 / sqrt(w 2^-64) from above's reciprocal: an integer y in [2^23, 2^24),
-// y 2^-23 within (1 - 2^-20.4, 1) of it.  w in [2^62, 2^64).
+RBG_HD int clz32(uint32_t x)
+{
+#ifdef __CUDA_ARCH__
+    return __clz((int)x);
+#else
+    return x ? __builtin_clz(x) : 32;
+#endif
+}
+// 64-bit shifts by 0 .. 31
+RBG_HD uint64_t shl(uint64_t x, int n)
+{
+#ifdef __CUDA_ARCH__
+    return ((uint64_t)__funnelshift_l(lo32(x), hi32(x), n) << 32) | (lo32(x) << n);
+#else
+    return x << n;
+#endif
+}
+RBG_HD uint64_t shr(uint64_t x, int n)
+{
+#ifdef __CUDA_ARCH__
+    return ((uint64_t)(hi32(x) >> n) << 32) | __funnelshift_r(lo32(x), hi32(x), n);
+#else
+    return x >> n;
+#endif
+}
+
+// 1 / sqrt(w 2^-64) from below: y 2^-31 within (1 - 2^-20.4, 1) of it, the low
+// byte of y zero.  w in [2^62, 2^64).
 RBG_HD uint32_t rsqrt_seed(uint64_t w)
 {
 #ifdef __CUDA_ARCH__
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint2float_rz(hi32(w)) * 2.3283064365386963e-10f));
-    return min(__float_as_uint(y) - 0x3f800000u, 0x007fffffu) + 0x00800000u - 4u;
+    float f;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(f) : "f"(__uint2float_rz(hi32(w)) * 2.3283064365386963e-10f));
+    const uint32_t b = __float_as_uint(f) - 0x3f800000u;
 #else
-    const float y = (float)(1.0 / std::sqrt((double)hi32(w) * 0x1p-32));
+    const float f = (float)(1.0 / std::sqrt((double)hi32(w) * 0x1p-32));
     uint32_t b;
-    std::memcpy(&b, &y, 4);
+    std::memcpy(&b, &f, 4);
     b -= 0x3f800000u;
-    return (b < 0x007fffffu ? b : 0x007fffffu) + 0x00800000u - 4u;
 #endif
+    return ((b < 0x007fffffu ? b : 0x007fffffu) << 8) + 0x7ffffc00u;
 }
 
 // sqrt(w 2^-64) in units of 2^-63 for w in [2^62, 2^64), within a few units.
@@ -135,11 +160,11 @@ RBG_HD uint32_t rsqrt_seed(uint64_t w)
 RBG_HD uint64_t sqrt_fixed(uint64_t w)
 {
     const uint32_t y = rsqrt_seed(w);
-    const uint64_t n = (1ull << 62) - mulhi64(w, mul32(y, y) << 16);            // n, unit 2^-62, below 2^42
-    const uint64_t wy = (mul32(hi32(w), y) << 8) + (mul32(lo32(w), y) >> 24);  // unit 2^-63
-    const uint32_t n50 = (uint32_t)(n >> 12);                                  // unit 2^-50
-    const uint64_t c = (n >> 1) + ((3ull * mul32(n50, n50)) >> 41);            // unit 2^-62
-    return wy + (mulhi64(c << 21, wy) >> 19);
+    const uint64_t n = (1ull << 62) - mulhi64(w, mul32(y, y));             // unit 2^-62, below 2^43
+    const uint64_t wy = mul32(hi32(w), y) + (mul32(lo32(w), y) >> 32);    // unit 2^-63
+    const uint32_t n51 = (uint32_t)(n >> 11);                             // unit 2^-51
+    const uint64_t c = (n << 20) + mul32(mulhi32(n51, n51), 3072u);       // n / 2 + 3 n^2 / 8, unit 2^-83
+    return wy + (mulhi64(c, wy) >> 19);
 }
 
 // Box-Muller of two 32-bit words, u0 = (a + 1/2) 2^-32, u1 = (b + 1/2) 2^-32:
@@ -149,49 +174,51 @@ RBG_HD void box_muller_fixed(uint32_t a, uint32_t b, const NormalTables& T, int6
     // -2 ln u0 = w 2^-64 2^ex, w in [2^62, 2^64), ex even
     uint64_t w;
     int ex;
-    if (a >= 0xFFF00000u) {
-        // 1 - u0 = d 2^-33, d < 2^21: -2 ln u0 = d 2^-32 (1 + x / 2 + x^2 / 3 + x^3 / 4 + x^4 / 5), x = d 2^-33
-        // (relative accuracy to the end of the range)
-        const uint32_t d = 0u - (2u * a + 1u);
-        const uint64_t x = (uint64_t)d << 31;  // unit 2^-64
-        const uint32_t x44 = d << 11;          // unit 2^-44, below 2^32
-        const uint32_t x2 = mulhi32(x44, x44); // unit 2^-56
-        const uint64_t f = (1ull << 63) + (x >> 2) + (mul32(x2, 0x55555555u + (mulhi32(x44, 0x40000000u) >> 12) +
-                                                            (mulhi32(x2, 0x33333333u) >> 24)) >> 25);  // unit 2^-63
-#ifdef __CUDA_ARCH__
-        const int n = __clz((int)d);
-#else
-        const int n = __builtin_clz(d);
-#endif
-        const uint32_t dn = d << n;
-        w = mul32(dn, hi32(f)) + (mul32(dn, lo32(f)) >> 32);  // d f 2^(n - 32): unit of d f is 2^-95
-        ex = 1 - n;                                           // value w 2^(n-dependent): see below
-        // d 2^-32 f = (w 2^(32 - n)) 2^-32 2^-63 = (w 2^-64) 2^(1 - n)
-        if (!(w >> 63)) { w <<= 1; --ex; }
+    if (a - 1u >= 0xFFEFFFFFu) {
+        if (a == 0u) {
+            w = 0xB6FDA8B7905DF579ull;  // 66 ln 2 / 64
+            ex = 6;
+        } else {
+            // 1 - u0 = d 2^-33, d < 2^21: -2 ln u0 = d 2^-32 (1 + x / 2 + x^2 / 3 + x^3 / 4 + x^4 / 5), x = d 2^-33
+            // (relative accuracy to the end of the range)
+            const uint32_t d = 0u - (2u * a + 1u);
+            const uint64_t x = (uint64_t)d << 31;   // unit 2^-64
+            const uint32_t x44 = d << 11;           // unit 2^-44, below 2^32
+            const uint32_t x2 = mulhi32(x44, x44);  // unit 2^-56
+            const uint64_t f = (1ull << 63) + (x >> 2) + (mul32(x2, 0x55555555u + (mulhi32(x44, 0x40000000u) >> 12) +
+                                                                (mulhi32(x2, 0x33333333u) >> 24)) >> 25);  // unit 2^-63
+            const int n = clz32(d);
+            const uint32_t dn = d << n;
+            // d 2^-32 f = (w 2^-64) 2^(1 - n)
+            w = mul32(dn, hi32(f)) + (mul32(dn, lo32(f)) >> 32);
+            ex = 1 - n;
+            if (!(w >> 63)) { w <<= 1; --ex; }
+            if (ex & 1) { w >>= 1; ++ex; }
+        }
     } else {
-        // u0 = q 2^-33, q = 2 a + 1 = 2^e m; ln m = ln c + log1p(t), t = (m - c) / c, |t| < 2^-10
-        const uint64_t q = 2ull * a + 1ull;
-        const int s = clz64(q);              // e = 63 - s
-        const uint64_t qn = q << s;          // m, unit 2^-63
-        const FixedPair lc = T.ln[(uint32_t)(qn >> 54) & (kLnTable - 1)];
-        const uint32_t u = (uint32_t)(qn >> 30) & 0xFFFFFFu;  // (m - c) 2^33 + 2^23
-        const int64_t t = (int64_t)((mul32(u, hi32(lc.x)) << 7) + (mul32(u, lo32(lc.x)) >> 25) - (lc.x >> 2));  // unit 2^-72
-        const int32_t th = (int32_t)(t >> 32);                                                    // unit 2^-40
-        const uint64_t t2 = (uint64_t)((int64_t)th * th + (((int64_t)th * (int32_t)(lo32((uint64_t)t) >> 1)) >> 30));  // unit 2^-80
-        const int32_t t3 = (int32_t)(((int64_t)th * (int32_t)hi32(t2)) >> 27);                    // unit 2^-61
+        // u0 = q 2^-33, q = 2 a + 1 = 2^(32 - n) m; ln m = ln c + log1p(t), t = (m - c) / c, |t| < 2^-10
+        const int n = clz32(a);
+        const uint32_t mh = (a << n) | ((1u << n) >> 1);  // m, unit 2^-31 (n = 0: its 2^-32 is added below)
+        const FixedPair lc = T.ln[(mh >> 22) & (kLnTable - 1)];
+        const int32_t u = (int32_t)((mh & 0x3FFFFFu) << 2) + (n ? 0 : 2) - (1 << 23);  // m - c, unit 2^-33
+        const int64_t t = (int64_t)u * (int32_t)hi32(lc.x) + (((int64_t)u * (int32_t)lo32(lc.x)) >> 31);  // unit 2^-64
+        const int32_t th = (int32_t)(t >> 23);                                             // unit 2^-41
+        const int32_t tl = (int32_t)lo32((uint64_t)t) & 0x7FFFFF;
+        const uint64_t t2 = (uint64_t)((int64_t)th * th + (((int64_t)th * tl) >> 22));     // unit 2^-82
+        const int32_t t3 = (int32_t)(((int64_t)th * (int32_t)hi32(t2)) >> 30);             // unit 2^-61
         // 1/3 - t/4 + t^2/5, unit 2^-31
-        const int32_t g = 0x2AAAAAAB - (th >> 11) + (int32_t)(mulhi32(hi32(t2), 0x33333333u) >> 17);
+        const int32_t g = 0x2AAAAAAB - (th >> 12) + (int32_t)(mulhi32(hi32(t2), 0x33333333u) >> 19);
         // ln m = ln c + t - t^2 / 2 + t^3 g, unit 2^-63
-        const int64_t lm = (int64_t)lc.y + (t >> 9) - (int64_t)(t2 >> 18) + (((int64_t)t3 * g) >> 29);
-        // -ln u0 = (33 - e) ln 2 - ln m: unit 2^-63 for u0 > 1/2, where it is small, else 2^-58
-        const bool top = s == 31;
-        const uint64_t L = top ? 0x58B90BFBE8E7BCD6ull - (uint64_t)lm : T.ln2[s - 30] - (uint64_t)(lm >> 5);
-        const int n = clz64(L);
-        w = L << n;
-        ex = (top ? 2 : 7) - n;  // 2 L 2^-58 = (w 2^-64) 2^(7 - n)
+        const int64_t lm = (int64_t)lc.y + (t >> 1) - (int64_t)(t2 >> 20) + (((int64_t)t3 * g) >> 29);
+        // -ln u0 = (n + 1) ln 2 - ln m: unit 2^-63 for u0 > 1/2, where it is small, else 2^-58
+        const uint64_t L = n ? T.ln2[n + 1] - (uint64_t)(lm >> 5) : 0x58B90BFBE8E7BCD6ull - (uint64_t)lm;
+        const int c0 = n ? 7 : 2;  // 2 L = (L << k) 2^-64 2^(c0 - k); the high word is never zero here
+        int k = clz32(hi32(L));
+        k -= (c0 - k) & 1;
+        w = shl(L, k);
+        ex = c0 - k;
     }
-    if (ex & 1) { w >>= 1; ++ex; }
-    const uint64_t r = sqrt_fixed(w) << 1;  // sqrt(-2 ln u0) 2^(-ex / 2), unit 2^-64
+    const uint64_t r = shr(sqrt_fixed(w), 3 - (ex >> 1));  // sqrt(-2 ln u0), unit 2^-60
 
     // 2 pi u1 = (quadrant) pi / 2 + pi k / 1024 + d, d = p pi 2^-32 with p = 2 (b mod 2^21) + 1
     const uint32_t p = 2u * (b & 0x1FFFFFu) + 1u;
@@ -210,13 +237,10 @@ RBG_HD void box_muller_fixed(uint32_t a, uint32_t b, const NormalTables& T, int6
     const uint64_t c = cs.x - (mulhi64(cs.x, nc) >> 17) - (mulhi64(cs.y, sd) >> 8);  // unit 2^-63
     const uint64_t sn = cs.y - (mulhi64(cs.y, nc) >> 17) + (mulhi64(cs.x, sd) >> 8);
     // quadrant q: (c, s), (-s, c), (-c, -s), (s, -c)
-    const bool odd = (b >> 30) & 1u;
-    const int sh = 4 - ex / 2;  // r 2^(ex / 2) c 2^-63 -> unit 2^-59
-    const uint64_t half = 1ull << (sh - 1);
-    const uint64_t m0 = (mulhi64(r, odd ? sn : c) + half) >> sh;
-    const uint64_t m1 = (mulhi64(r, odd ? c : sn) + half) >> sh;
-    const uint64_t s0 = 0ull - (uint64_t)(((b >> 30) ^ (b >> 31)) & 1u);  // cosine negative in quadrants 1, 2
-    const uint64_t s1 = 0ull - (uint64_t)(b >> 31);                       // sine in 2, 3
+    const bool odd = (b & 0x40000000u) != 0u;
+    const uint64_t m0 = mulhi64(r, odd ? sn : c), m1 = mulhi64(r, odd ? c : sn);  // unit 2^-59
+    const uint64_t s0 = (uint64_t)(int64_t)((int32_t)(b ^ (b << 1)) >> 31);  // cosine negative in quadrants 1, 2
+    const uint64_t s1 = (uint64_t)(int64_t)((int32_t)b >> 31);               // sine in 2, 3
     z0 = (int64_t)((m0 ^ s0) - s0);
     z1 = (int64_t)((m1 ^ s1) - s1);
 }
@@ -357,7 +381,8 @@ inline void fill_fixed_tables(FixedTables& F)
     NormalTables& T = F.normals;
     for (int k = 0; k < kLnTable; ++k) {
         const long double c = 1.0L + (k + 0.5L) / kLnTable;
-        T.ln[k] = FixedPair{(uint64_t)(std::ldexp(1.0L / c, 64) + 0.5L), (uint64_t)(std::ldexp(std::log(c), 63) + 0.5L)};
+        const uint64_t x = (uint64_t)(std::ldexp(1.0L / c, 62) + 0.5L);
+        T.ln[k] = FixedPair{((x >> 31) << 32) | (x & 0x7FFFFFFFu), (uint64_t)(std::ldexp(std::log(c), 63) + 0.5L)};
     }
     const long double pi = 3.14159265358979323846264338327950288L, ln2 = 0.693147180559945309417232121458176568L;
     for (int k = 0; k < kTrigTable; ++k) {

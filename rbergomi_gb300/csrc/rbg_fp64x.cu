@@ -108,20 +108,22 @@ __device__ __forceinline__ void store_digits(const int64_t (&v)[4], unsigned cha
     }
 }
 
-// Z[m][s][j], s < NS: W1, W1perp and (plain MC) Wperp on Philox streams 0, 1,
-// 2; dig non-null: also the digits of W1 (zero past N and past B).  A warp
-// takes 8 paths x 16 steps of one stream, four lanes a path and four steps a
-// lane, so a path's 16 doubles and each digit's 8 rows are contiguous.
-// Integer work bounds it: about 220 instructions, 70 of them 32 x 32 -> 64
-// multiplies, for a pair of normals.  2 x 512 steps, 2^17 paths: 1.25 ms,
-// against 5.40 ms for the same draw in FP64 (table-driven logarithm and sine,
-// about 40 FP64 operations a pair).
-constexpr int kNormalThreads = 256;
+// Z[m][s][j], s < ns: W1, W1perp and (plain MC) Wperp on Philox streams 0, 1,
+// 2.  dig non-null (the fixed-point path pass follows): also the digits of W1,
+// zero past N and past B, and W1perp as 64-bit fixed point (unit 2^-59) in
+// place of doubles.
+// A warp takes up to kSeg chunks of 16 steps of 8 paths' stream, four lanes a
+// path and four steps a lane, so a path's 16 values and each digit's 8 rows are
+// contiguous.  Integer instructions bound it: 368 a warp and pair of normals, 64
+// of them 32 x 32 -> 64 multiplies (four cycles each).  2 x 512 steps, 2^17
+// paths: 0.95 ms, against 5.40 ms for the same draw in FP64 (table-driven
+// logarithm and sine, about 40 FP64 operations a pair).
+constexpr int kNormalThreads = 256, kSeg = 8;
 template <int F32>
-__global__ void __launch_bounds__(kNormalThreads) k_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int ns,
-                                                                 double* __restrict__ Z,
-                                                                 unsigned char* __restrict__ dig,
-                                                                 const FixedTables* __restrict__ ft)
+__global__ void __launch_bounds__(kNormalThreads, 4) k_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int ns,
+                                                                    double* __restrict__ Z,
+                                                                    unsigned char* __restrict__ dig,
+                                                                    const FixedTables* __restrict__ ft)
 {
     __shared__ NormalTables T;
     if (!F32) {
@@ -131,58 +133,64 @@ __global__ void __launch_bounds__(kNormalThreads) k_normals_fixed(uint64_t seed,
         __syncthreads();
     }
     const int lane = threadIdx.x & 31, g = lane & 3, pl = lane >> 2;
-    const int nch = (N + kXSteps - 1) / kXSteps;
-    const int64_t octets = (B + kXPaths - 1) / kXPaths * (kXPaths / 8);
-    const int64_t tasks = octets * ns * nch;
+    const int nch = (N + kXSteps - 1) / kXSteps, segs = (nch + kSeg - 1) / kSeg;
+    const int64_t tasks = (B + kXPaths - 1) / kXPaths * (kXPaths / 8) * ns * segs;
     const bool vec = (N & 1) == 0;
     const PhiloxKeys keys = philox_keys(seed);
     const int64_t warps = (int64_t)gridDim.x * (kNormalThreads / 32);
     for (int64_t t = blockIdx.x * (int64_t)(kNormalThreads / 32) + (threadIdx.x >> 5); t < tasks; t += warps) {
-        const int c = (int)(t % nch);
-        const int64_t r = t / nch;
+        const int64_t r = t / segs;
+        const int c0 = (int)(t - r * segs) * kSeg, c1 = min(nch, c0 + kSeg);
         const int s = (int)(r % ns);
         const int64_t m = r / ns * 8 + pl;
-        const int j0 = kXSteps * c + 4 * g;
-        const bool valid = m < B;
-        if (!valid && (s != 0 || !dig)) continue;
-        int64_t v[4] = {0, 0, 0, 0};
-        if (valid && j0 < N) {
-            const uint4 x = philox_group(keys, (uint64_t)(path0 + m), (uint32_t)(j0 >> 2), (uint32_t)s);
-            double z[4];
-            if (F32) {
-                float f0, f1, f2, f3;
-                box_muller_f32(x.x, x.y, f0, f1);
-                box_muller_f32(x.z, x.w, f2, f3);
-                z[0] = f0; z[1] = f1; z[2] = f2; z[3] = f3;
+        const bool valid = m < B, digits = s == 0 && dig != nullptr;
+        if (!valid && !digits) continue;
+        double* zrow = Z + (m * ns + s) * (int64_t)N;
+        const int p = (int)(m & (kXPaths - 1));
+        unsigned char* drow = dig + (m / kXPaths) * nch * kXChunkBytes + p * 32 + ((((g >> 1) ^ (p >> 2)) & 1) << 4) +
+                              ((g & 1) << 3);
+#pragma unroll 1
+        for (int c = c0; c < c1; ++c) {
+            const int j0 = kXSteps * c + 4 * g;
+            int64_t v[4] = {0, 0, 0, 0};
+            if (valid && j0 < N) {
+                const uint4 x = philox_group(keys, (uint64_t)(path0 + m), (uint32_t)(j0 >> 2), (uint32_t)s);
+                double z[4];
+                if (F32) {
+                    float f0, f1, f2, f3;
+                    box_muller_f32(x.x, x.y, f0, f1);
+                    box_muller_f32(x.z, x.w, f2, f3);
+                    z[0] = f0; z[1] = f1; z[2] = f2; z[3] = f3;
 #pragma unroll
-                for (int q = 0; q < 4; ++q) v[q] = double_to_fixed(z[q]);
-            } else {
-                box_muller_fixed(x.x, x.y, T, v[0], v[1]);
-                box_muller_fixed(x.z, x.w, T, v[2], v[3]);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) z[q] = fixed_to_double(v[q]);
-            }
-            double* o = Z + (m * ns + s) * (int64_t)N + j0;
-            if (j0 + 4 <= N) {
-                if (vec) {
-                    *(double2*)o = make_double2(z[0], z[1]);
-                    *(double2*)(o + 2) = make_double2(z[2], z[3]);
+                    for (int q = 0; q < 4; ++q) v[q] = double_to_fixed(z[q]);
                 } else {
-                    o[0] = z[0]; o[1] = z[1]; o[2] = z[2]; o[3] = z[3];
+                    box_muller_fixed(x.x, x.y, T, v[0], v[1]);
+                    box_muller_fixed(x.z, x.w, T, v[2], v[3]);
                 }
-            } else {
+                if (s == 1 && dig) {
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    if (j0 + q < N) o[q] = z[q];
-                    else v[q] = 0;
+                    for (int q = 0; q < 4; ++q) z[q] = __longlong_as_double(v[q]);
+                } else if (!F32) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) z[q] = fixed_to_double(v[q]);
+                }
+                double* o = zrow + j0;
+                if (j0 + 4 <= N) {
+                    if (vec) {
+                        *(double2*)o = make_double2(z[0], z[1]);
+                        *(double2*)(o + 2) = make_double2(z[2], z[3]);
+                    } else {
+                        o[0] = z[0]; o[1] = z[1]; o[2] = z[2]; o[3] = z[3];
+                    }
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        if (j0 + q < N) o[q] = z[q];
+                        else v[q] = 0;
+                    }
                 }
             }
-        }
-        if (s == 0 && dig) {
-            const int p = (int)(m & (kXPaths - 1));
-            unsigned char* at = dig + ((m / kXPaths) * nch + c) * kXChunkBytes + p * 32 +
-                                ((((g >> 1) ^ (p >> 2)) & 1) << 4) + ((g & 1) << 3);
-            store_digits(v, at);
+            if (digits) store_digits(v, drow + (size_t)c * kXChunkBytes);
         }
     }
 }
@@ -192,8 +200,8 @@ int launch_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int f32
 {
     const FixedTables* ft = fixed_tables();
     if (!ft) return -1;
-    const int64_t octets = (B + kXPaths - 1) / kXPaths * (kXPaths / 8);
-    const int64_t tasks = octets * ns * ((N + kXSteps - 1) / kXSteps);
+    const int nch = (N + kXSteps - 1) / kXSteps;
+    const int64_t tasks = (B + kXPaths - 1) / kXPaths * (kXPaths / 8) * ns * ((nch + kSeg - 1) / kSeg);
     const int64_t need = (tasks + kNormalThreads / 32 - 1) / (kNormalThreads / 32);
     const int64_t blocks = std::min<int64_t>(need, 8 * (int64_t)device_sms());
     if (f32) k_normals_fixed<1><<<(unsigned)blocks, kNormalThreads, 0, st>>>(seed, path0, B, N, ns, Z, dig, ft);
@@ -589,13 +597,19 @@ __global__ void __launch_bounds__(kVarThreads, GB > 1 ? 2 : 3) k_variance_fixed(
                         for (int c = 0; c < NS; ++c) acc[q][c] = 0.0;
                     if (m < B) {
                         const double* W1 = Z + m * NS * (int64_t)N;
+                        const uint64_t* Wp = reinterpret_cast<const uint64_t*>(W1 + N);  // fixed point
                         const uint64_t* Xm = X + ((size_t)v * B + m) * N;
-                        for (int j = 1 + lane; j < N; j += 32) {
-                            const double w1 = W1[j];
-                            double wq = 0.0;
-                            if (NS == 3) wq = W1[2 * N + j];
-                            const uint64_t wp = (uint64_t)double_to_fixed(W1[N + j - 1]) ^ (1ull << 63);
-                            const uint64_t x = Xm[j - 1] + mulhi64(wp, vol.a2f) - vol.a2h;
+                        // the next step's operands are loaded while this one's are worked on
+                        int j = 1 + lane;
+                        bool in = j < N;
+                        double w1 = in ? W1[j] : 0.0, wq = (NS == 3 && in) ? W1[2 * N + j] : 0.0;
+                        uint64_t wp = in ? Wp[j - 1] : 0ull, xj = in ? Xm[j - 1] : 0ull;
+                        while (in) {
+                            const int jn = j + 32;
+                            const bool inn = jn < N;
+                            const double w1n = inn ? W1[jn] : 0.0, wqn = (NS == 3 && inn) ? W1[2 * N + jn] : 0.0;
+                            const uint64_t wpn = inn ? Wp[jn - 1] : 0ull, xn = inn ? Xm[jn - 1] : 0ull;
+                            const uint64_t x = xj + mulhi64(wp ^ (1ull << 63), vol.a2f) - vol.a2h;
 #pragma unroll
                             for (int q = 0; q < GB; ++q) {
                                 if (q < ng) {
@@ -607,6 +621,12 @@ __global__ void __launch_bounds__(kVarThreads, GB > 1 ? 2 : 3) k_variance_fixed(
                                     if (NS == 3) acc[q][2] = fma(su, wq, acc[q][2]);
                                 }
                             }
+                            j = jn;
+                            in = inn;
+                            w1 = w1n;
+                            wq = wqn;
+                            wp = wpn;
+                            xj = xn;
                         }
                     }
 #pragma unroll

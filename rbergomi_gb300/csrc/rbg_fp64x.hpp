@@ -49,7 +49,8 @@ const FixedTables* fixed_tables();
 
 // The launchers return nonzero where the device refuses.
 // Philox normals Z[m][s][j] of ns streams per path (W1, W1perp, plain MC: Wperp);
-// f32: the mixed form's FP32 normals, widened; dig non-null: the digits of W1 too.
+// f32: the mixed form's FP32 normals, widened; dig non-null (for the path pass
+// below): the digits of W1 too, and W1perp in 64-bit fixed point.
 int launch_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int f32, double* Z, unsigned char* dig, int ns,
                          cudaStream_t st);
 void launch_panels(const int64_t* gam, int nv, int N, unsigned char* panels, cudaStream_t st);
