@@ -442,7 +442,7 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
                                           c.xpan.as<unsigned char>() + (size_t)v0 * x64_panel_bytes(N), ts.xvols + v0, k, N,
                                           b, c.xbuf.as<uint64_t>(), err, st) ||
                     launch_variance_fixed(ts.xvols + v0, ts.xgrps, ts.xcomp, c.z.as<double>(), c.xbuf.as<uint64_t>(), k,
-                                          xt.max_groups, ns, N, b, c.ivb.as<double>(), ivp, st))
+                                          xt.max_groups, xt.u53, ns, N, b, c.ivb.as<double>(), ivp, st))
                     return fail(RBG_ERR_CUDA, "FP64 path kernels could not be configured");
             }
         }

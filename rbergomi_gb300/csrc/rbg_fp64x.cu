@@ -228,7 +228,7 @@ constexpr int kPanelBytes = kXDigits * kPanelDigit;    // 61440 B
 constexpr int kXBlock = 128;                           // output steps per block
 constexpr int kXChunks = kXBlock / kXSteps;            // 8 chunks per block of steps
 constexpr int kXStages = 5;
-constexpr int kXEpiWarps = 8;
+constexpr int kXEpiWarps = 16;
 constexpr int kXThreads = (kXEpiWarps + 2) * 32;
 constexpr int kXSmem = 2 * kPanelBytes + kXStages * kXChunkBytes + 256 + 1024;
 
@@ -307,7 +307,7 @@ struct PanelSlots {
 };
 
 // One (block b, pass v, group of 64 paths) at a time, the longest blocks
-// first.  Warps 0-7 read the accumulators, warp 8 loads, warp 9 issues the
+// first.  Warps 0-15 read the accumulators, warp 16 loads, warp 17 issues the
 // MMAs.  WIDE: accumulators may pass 2^22 (N > 1024): converted by F2I, else by
 // adding 1.5 2^23.
 // What bounds it: 2304 columns x 128 steps x 16 per chunk, 1152 MMA cycles,
@@ -476,33 +476,44 @@ __global__ void __launch_bounds__(kXThreads, 1) k_volterra_exact(const unsigned 
             if (!mbar_wait_warp(smem_u32(accf), (uint32_t)(n_units & 1), err, 27)) goto done;
             tc_fence_after();
             const int j = kXBlock * b + quad * 32 + lane;
-            uint64_t* Xv = X + (size_t)v * B * N + j;
 #pragma unroll 1
-            for (int q = 0; q < 4; ++q) {
-                const int p0 = wg * 32 + q * 8;
+            for (int q = 0; q < kXPaths / 8 / (kXEpiWarps / 4); ++q) {
+                const int p0 = wg * (kXPaths * 4 / kXEpiWarps) + q * 8;
                 uint32_t D[kXDigits][8];
 #pragma unroll
                 for (int d = 0; d < kXDigits; ++d) tmem_ld8(tl + (uint32_t)(kXPaths * d + p0), D[d]);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (q == 3) {
+                if (q == kXPaths / 8 / (kXEpiWarps / 4) - 1) {
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(acce));
                 }
+                const int64_t m = g * kXPaths + p0;
+                uint64_t* Xm = X + ((size_t)v * B + m) * N + j;
 #pragma unroll
                 for (int p = 0; p < 8; ++p) {
-                    int64_t D8[kXDigits];
-#pragma unroll
-                    for (int d = 0; d < kXDigits; ++d) {
-                        const float f = __uint_as_float(D[d][p]);
-                        D8[d] = WIDE ? __float2int_rn(f) : __float_as_int(f + 12582912.f) - 0x4B400000;
-                    }
                     // S_hi in units of 2^(e - 33), S_lo of 2^(e - 65); X = S_hi 2^sh + S_lo 2^(sh - 32)
-                    const int64_t hi = (D8[0] << 24) + (D8[1] << 16) + (D8[2] << 8) + D8[3];
-                    const int64_t lo = (D8[4] << 24) + (D8[5] << 16) + (D8[6] << 8) + D8[7];
-                    const uint64_t x = ((uint64_t)hi << sh) + (uint64_t)(lo >> (32 - sh)) + (1ull << 63);
-                    const int64_t m = g * kXPaths + p0 + p;
-                    if (m < B && j < N) Xv[m * N] = x;
+                    int64_t hi, lo;
+                    if (WIDE) {
+                        int64_t D8[kXDigits];
+#pragma unroll
+                        for (int d = 0; d < kXDigits; ++d) D8[d] = __float2int_rn(__uint_as_float(D[d][p]));
+                        hi = (D8[0] << 24) + (D8[1] << 16) + (D8[2] << 8) + D8[3];
+                        lo = (D8[4] << 24) + (D8[5] << 16) + (D8[6] << 8) + D8[7];
+                    } else {
+                        // |D| < 2^22: f + 1.5 2^23 has D + 0x4B400000 as its bits, and two neighbours
+                        // make one 32-bit number; the offsets come off modulo 2^32
+                        uint32_t I[kXDigits];
+#pragma unroll
+                        for (int d = 0; d < kXDigits; ++d) I[d] = __float_as_uint(__uint_as_float(D[d][p]) + 12582912.f);
+                        constexpr uint32_t off = 0x4B400000u * 257u;
+                        const int32_t h1 = (int32_t)(I[0] * 256u + I[1] - off), h0 = (int32_t)(I[2] * 256u + I[3] - off);
+                        const int32_t l1 = (int32_t)(I[4] * 256u + I[5] - off), l0 = (int32_t)(I[6] * 256u + I[7] - off);
+                        hi = (int64_t)h1 * 65536 + h0;
+                        lo = (int64_t)l1 * 65536 + l0;
+                    }
+                    const uint64_t x = shl((uint64_t)hi, sh) + (uint64_t)(lo >> (32 - sh)) + (1ull << 63);
+                    if (m + p < B && j < N) Xm[(size_t)p * N] = x;
                 }
             }
         }
@@ -555,7 +566,7 @@ int launch_volterra_exact(const unsigned char* dig, const unsigned char* panels,
 constexpr int kVarThreads = 256, kVarVals = 16;
 constexpr int kVarSmem = kExpTable * 8 + (kVarThreads / 32) * kVarVals * 33 * 8;
 
-template <int NS, int GB>
+template <int NS, int GB, bool U53>
 __global__ void __launch_bounds__(kVarThreads, GB > 1 ? 2 : 3) k_variance_fixed(const X64Vol* __restrict__ vols,
                                                                const X64Group* __restrict__ grps,
                                                                const uint64_t* __restrict__ comp,
@@ -599,34 +610,40 @@ __global__ void __launch_bounds__(kVarThreads, GB > 1 ? 2 : 3) k_variance_fixed(
                         const double* W1 = Z + m * NS * (int64_t)N;
                         const uint64_t* Wp = reinterpret_cast<const uint64_t*>(W1 + N);  // fixed point
                         const uint64_t* Xm = X + ((size_t)v * B + m) * N;
-                        // the next step's operands are loaded while this one's are worked on
-                        int j = 1 + lane;
-                        bool in = j < N;
-                        double w1 = in ? W1[j] : 0.0, wq = (NS == 3 && in) ? W1[2 * N + j] : 0.0;
-                        uint64_t wp = in ? Wp[j - 1] : 0ull, xj = in ? Xm[j - 1] : 0ull;
-                        while (in) {
-                            const int jn = j + 32;
-                            const bool inn = jn < N;
-                            const double w1n = inn ? W1[jn] : 0.0, wqn = (NS == 3 && inn) ? W1[2 * N + jn] : 0.0;
-                            const uint64_t wpn = inn ? Wp[jn - 1] : 0ull, xn = inn ? Xm[jn - 1] : 0ull;
-                            const uint64_t x = xj + mulhi64(wp ^ (1ull << 63), vol.a2f) - vol.a2h;
+                        // operands are loaded two steps ahead: a step's 24 bytes a lane, 24 warps an SM,
+                        // have to cover the latency of device memory
+                        struct Step {
+                            double w1, wq;
+                            uint64_t wp, x;
+                        } s[3];
+                        auto load = [&](int j) {
+                            Step r{0.0, 0.0, 0ull, 0ull};
+                            if (j < N) {
+                                r.w1 = W1[j];
+                                if (NS == 3) r.wq = W1[2 * N + j];
+                                r.wp = Wp[j - 1];
+                                r.x = Xm[j - 1];
+                            }
+                            return r;
+                        };
+                        s[0] = load(1 + lane);
+                        s[1] = load(33 + lane);
+                        for (int j = 1 + lane; j < N; j += 32) {
+                            s[2] = load(j + 64);
+                            const uint64_t x = s[0].x + mulhi64(s[0].wp ^ (1ull << 63), vol.a2f) - vol.a2h;
 #pragma unroll
                             for (int q = 0; q < GB; ++q) {
                                 if (q < ng) {
                                     const uint64_t t = mulhi64(neg[q] ? 0ull - x : x, cf[q]) -
                                                        __ldg(comp + (size_t)(g0 + q) * N + j - 1);
-                                    const double su = exp2_fixed((int64_t)t, ut[q], E);
+                                    const double su = U53 ? exp2_fixed53((int64_t)t, E) : exp2_fixed((int64_t)t, ut[q], E);
                                     acc[q][0] = fma(su, su, acc[q][0]);
-                                    acc[q][1] = fma(su, w1, acc[q][1]);
-                                    if (NS == 3) acc[q][2] = fma(su, wq, acc[q][2]);
+                                    acc[q][1] = fma(su, s[0].w1, acc[q][1]);
+                                    if (NS == 3) acc[q][2] = fma(su, s[0].wq, acc[q][2]);
                                 }
                             }
-                            j = jn;
-                            in = inn;
-                            w1 = w1n;
-                            wq = wqn;
-                            wp = wpn;
-                            xj = xn;
+                            s[0] = s[1];
+                            s[1] = s[2];
                         }
                     }
 #pragma unroll
@@ -662,21 +679,25 @@ __global__ void __launch_bounds__(kVarThreads, GB > 1 ? 2 : 3) k_variance_fixed(
 }
 
 int launch_variance_fixed(const X64Vol* vols, const X64Group* grps, const uint64_t* comp, const double* Z,
-                          const uint64_t* X, int nv, int max_groups, int ns, int N, int64_t B, double* ivb, double* ivp,
-                          cudaStream_t st)
+                          const uint64_t* X, int nv, int max_groups, bool u53, int ns, int N, int64_t B, double* ivb,
+                          double* ivp, cudaStream_t st)
 {
     static std::mutex mu;
     static bool ready[64] = {};
     const FixedTables* ft = fixed_tables();
     if (!ft) return -1;
-    auto* kern = ns == 3 ? (max_groups > 1 ? k_variance_fixed<3, 4> : k_variance_fixed<3, 1>)
-                         : (max_groups > 1 ? k_variance_fixed<2, 4> : k_variance_fixed<2, 1>);
+    auto* kern = ns == 3 ? (max_groups > 1 ? (u53 ? k_variance_fixed<3, 4, true> : k_variance_fixed<3, 4, false>)
+                                           : (u53 ? k_variance_fixed<3, 1, true> : k_variance_fixed<3, 1, false>))
+                         : (max_groups > 1 ? (u53 ? k_variance_fixed<2, 4, true> : k_variance_fixed<2, 4, false>)
+                                           : (u53 ? k_variance_fixed<2, 1, true> : k_variance_fixed<2, 1, false>));
     {
         int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
         std::lock_guard<std::mutex> lk(mu);
         if (!ready[dev]) {
-            for (auto* k : {k_variance_fixed<2, 1>, k_variance_fixed<2, 4>, k_variance_fixed<3, 1>, k_variance_fixed<3, 4>})
+            for (auto* k : {k_variance_fixed<2, 1, true>, k_variance_fixed<2, 4, true>, k_variance_fixed<3, 1, true>,
+                            k_variance_fixed<3, 4, true>, k_variance_fixed<2, 1, false>, k_variance_fixed<2, 4, false>,
+                            k_variance_fixed<3, 1, false>, k_variance_fixed<3, 4, false>})
                 if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kVarSmem) != cudaSuccess) {
                     cudaGetLastError();
                     return -1;
@@ -754,6 +775,7 @@ bool x64_prepare(const Plan& plan, X64Tables& out)
         if (ut < kX64MinUt) return false;
         X64Group& o = out.grps[g];
         o.ut = ut;
+        out.u53 = out.u53 && ut == 53;
         o.neg = C < 0.0;
         o.cf = (uint64_t)std::ldexp(Ca, ut - ux[G.vol] + 64);
         o.dtxi = G.dt * G.xi;

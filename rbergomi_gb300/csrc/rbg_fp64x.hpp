@@ -34,6 +34,7 @@ struct X64Tables {
     std::vector<int64_t> gam;    // [n_vol][N] (a1, Gamma_1, ...), unit 2^(e - 62)
     std::vector<uint64_t> comp;  // [n_vg][N] compensator in exponent units, plus cf / 2 - 1
     int max_groups = 0;          // most variance groups of one pass
+    bool u53 = true;             // every group has 53 fraction bits
 };
 // False where the plan's numbers do not fit the fixed-point ranges.
 bool x64_prepare(const Plan& plan, X64Tables& out);
@@ -59,7 +60,7 @@ int launch_volterra_exact(const unsigned char* dig, const unsigned char* panels,
                           int64_t B, uint64_t* X, unsigned int* err, cudaStream_t st);
 // ivb[g][B] (Ivdt, IsvdW); ns = 3: ivp[g][B] IsvdWp too
 int launch_variance_fixed(const X64Vol* vols, const X64Group* grps, const uint64_t* comp, const double* Z,
-                          const uint64_t* X, int nv, int max_groups, int ns, int N, int64_t B, double* ivb, double* ivp,
-                          cudaStream_t st);
+                          const uint64_t* X, int nv, int max_groups, bool u53, int ns, int N, int64_t B, double* ivb,
+                          double* ivp, cudaStream_t st);
 
 }  // namespace rbg

@@ -44,6 +44,10 @@ static void check_exp2(int64_t x, int ut)
         std::printf("exp2 %lld 2^-%d: %.17g, want %.20Lg\n", (long long)x, ut, d, want);
         std::exit(1);
     }
+    if (ut == 53 && exp2_fixed53(x, E) != d) {
+        std::printf("exp2_fixed53 %lld: %.17g, not %.17g\n", (long long)x, exp2_fixed53(x, E), d);
+        std::exit(1);
+    }
 }
 
 int main()
