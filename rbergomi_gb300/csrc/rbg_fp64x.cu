@@ -563,11 +563,12 @@ int launch_volterra_exact(const unsigned char* dig, const unsigned char* panels,
 // the integer pipes about as much.  The lanes' sums of several paths are
 // reduced together through shared memory: one FP64 addition a value and lane
 // instead of five.
-constexpr int kVarThreads = 256, kVarVals = 16;
-constexpr int kVarSmem = kExpTable * 8 + (kVarThreads / 32) * kVarVals * 33 * 8;
+constexpr int kVarVals = 16, kVarGroups = 4;  // variance groups a batch of a pass with several
+__host__ __device__ constexpr int var_threads(int gb) { return gb > 1 ? 256 : 512; }
+__host__ __device__ constexpr int var_smem(int gb) { return kExpTable * 8 + (var_threads(gb) / 32) * kVarVals * 33 * 8; }
 
 template <int NS, int GB, bool U53>
-__global__ void __launch_bounds__(kVarThreads, GB > 1 ? 2 : 3) k_variance_fixed(const X64Vol* __restrict__ vols,
+__global__ void __launch_bounds__(var_threads(GB), 2) k_variance_fixed(const X64Vol* __restrict__ vols,
                                                                const X64Group* __restrict__ grps,
                                                                const uint64_t* __restrict__ comp,
                                                                const double* __restrict__ Z,
@@ -576,6 +577,7 @@ __global__ void __launch_bounds__(kVarThreads, GB > 1 ? 2 : 3) k_variance_fixed(
                                                                const FixedTables* __restrict__ ft)
 {
     constexpr int PB = kVarVals / (GB * NS);  // paths per reduction
+    constexpr int kVarThreads = var_threads(GB);
     extern __shared__ uint64_t vsm[];
     uint64_t* E = vsm;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -626,16 +628,25 @@ __global__ void __launch_bounds__(kVarThreads, GB > 1 ? 2 : 3) k_variance_fixed(
                             }
                             return r;
                         };
+                        const uint64_t* cg = comp + (size_t)g0 * N - 1;
+                        uint64_t cn[GB];
+#pragma unroll
+                        for (int q = 0; q < GB; ++q) cn[q] = (q < ng && 1 + lane < N) ? __ldg(cg + (size_t)q * N + 1 + lane) : 0ull;
                         s[0] = load(1 + lane);
                         s[1] = load(33 + lane);
                         for (int j = 1 + lane; j < N; j += 32) {
                             s[2] = load(j + 64);
+                            uint64_t cc[GB];
+#pragma unroll
+                            for (int q = 0; q < GB; ++q) {
+                                cc[q] = cn[q];
+                                cn[q] = (q < ng && j + 32 < N) ? __ldg(cg + (size_t)q * N + j + 32) : 0ull;
+                            }
                             const uint64_t x = s[0].x + mulhi64(s[0].wp ^ (1ull << 63), vol.a2f) - vol.a2h;
 #pragma unroll
                             for (int q = 0; q < GB; ++q) {
                                 if (q < ng) {
-                                    const uint64_t t = mulhi64(neg[q] ? 0ull - x : x, cf[q]) -
-                                                       __ldg(comp + (size_t)(g0 + q) * N + j - 1);
+                                    const uint64_t t = mulhi64(neg[q] ? 0ull - x : x, cf[q]) - cc[q];
                                     const double su = U53 ? exp2_fixed53((int64_t)t, E) : exp2_fixed((int64_t)t, ut[q], E);
                                     acc[q][0] = fma(su, su, acc[q][0]);
                                     acc[q][1] = fma(su, s[0].w1, acc[q][1]);
@@ -686,29 +697,35 @@ int launch_variance_fixed(const X64Vol* vols, const X64Group* grps, const uint64
     static bool ready[64] = {};
     const FixedTables* ft = fixed_tables();
     if (!ft) return -1;
-    auto* kern = ns == 3 ? (max_groups > 1 ? (u53 ? k_variance_fixed<3, 4, true> : k_variance_fixed<3, 4, false>)
+    auto* kern = ns == 3 ? (max_groups > 1 ? (u53 ? k_variance_fixed<3, kVarGroups, true> : k_variance_fixed<3, kVarGroups, false>)
                                            : (u53 ? k_variance_fixed<3, 1, true> : k_variance_fixed<3, 1, false>))
-                         : (max_groups > 1 ? (u53 ? k_variance_fixed<2, 4, true> : k_variance_fixed<2, 4, false>)
+                         : (max_groups > 1 ? (u53 ? k_variance_fixed<2, kVarGroups, true> : k_variance_fixed<2, kVarGroups, false>)
                                            : (u53 ? k_variance_fixed<2, 1, true> : k_variance_fixed<2, 1, false>));
     {
         int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
         std::lock_guard<std::mutex> lk(mu);
         if (!ready[dev]) {
-            for (auto* k : {k_variance_fixed<2, 1, true>, k_variance_fixed<2, 4, true>, k_variance_fixed<3, 1, true>,
-                            k_variance_fixed<3, 4, true>, k_variance_fixed<2, 1, false>, k_variance_fixed<2, 4, false>,
-                            k_variance_fixed<3, 1, false>, k_variance_fixed<3, 4, false>})
-                if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kVarSmem) != cudaSuccess) {
-                    cudaGetLastError();
-                    return -1;
-                }
+            const auto allow = [](auto* k, int gb) {
+                return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, var_smem(gb)) == cudaSuccess;
+            };
+            if (!(allow(k_variance_fixed<2, 1, true>, 1) && allow(k_variance_fixed<2, 1, false>, 1) &&
+                  allow(k_variance_fixed<3, 1, true>, 1) && allow(k_variance_fixed<3, 1, false>, 1) &&
+                  allow(k_variance_fixed<2, kVarGroups, true>, kVarGroups) &&
+                  allow(k_variance_fixed<2, kVarGroups, false>, kVarGroups) &&
+                  allow(k_variance_fixed<3, kVarGroups, true>, kVarGroups) &&
+                  allow(k_variance_fixed<3, kVarGroups, false>, kVarGroups))) {
+                cudaGetLastError();
+                return -1;
+            }
             ready[dev] = true;
         }
     }
-    const int pb = kVarVals / ((max_groups > 1 ? 4 : 1) * ns);
+    const int gb = max_groups > 1 ? kVarGroups : 1, pb = kVarVals / (gb * ns), threads = var_threads(gb);
     const int64_t runs = (B + pb - 1) / pb;
-    const int64_t blocks = std::min<int64_t>((runs + kVarThreads / 32 - 1) / (kVarThreads / 32), 3 * (int64_t)device_sms());
-    kern<<<(unsigned)blocks, kVarThreads, kVarSmem, st>>>(vols, grps, comp, Z, X, nv, N, B, ivb, ivp, ft);
+    const int64_t blocks =
+        std::min<int64_t>((runs + threads / 32 - 1) / (threads / 32), 2 * (int64_t)device_sms());
+    kern<<<(unsigned)blocks, threads, var_smem(gb), st>>>(vols, grps, comp, Z, X, nv, N, B, ivb, ivp, ft);
     count_launch();
     return 0;
 }
