@@ -419,8 +419,9 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
     // the kernel error word follows the accumulators
     if ((rc = ensure(c.acc, sizeof(double) * (4 * no + 1), "accumulators"))) return rc;
     if ((rc = ensure(c.res, sizeof(double) * 5 * no, "results"))) return rc;
-    RBG_CUDA(cudaMemsetAsync(c.acc.p, 0, sizeof(double) * (4 * no + 1), st));
     unsigned int* err = (unsigned int*)(c.acc.as<double>() + 4 * no);
+    if (fixed) RBG_CUDA(cudaMemsetAsync(err, 0, sizeof(unsigned int), st));
+    const MergeFinal fin{ts.t.outs, ts.Tvals, c.res.as<double>(), M, o.compute_iv};
     for (int64_t m0 = 0; m0 < M; m0 += B) {
         const int64_t b = std::min(B, M - m0);
         {
@@ -454,12 +455,12 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
         }
         {
             ProfScope ps(kStageReduce, st);
-            launch_accumulate(c.part.as<double>(), nchunks, no, c.acc.as<double>(), st);
+            if (launch_merge(c.part.as<double>(), nchunks, no, c.acc.as<double>(), m0 == 0, st,
+                             m0 + B >= M ? &fin : nullptr))
+                return fail(RBG_ERR_CUDA, "merge tables could not be set up");
         }
         RBG_CUDA(cudaGetLastError());
     }
-    launch_finalize(c.acc.as<double>(), no, M, ts.t.outs, ts.Tvals, o.compute_iv, c.res.as<double>(), st);
-    RBG_CUDA(cudaGetLastError());
     RBG_CUDA(cudaMemcpyAsync(host_res, c.res.p, sizeof(double) * 5 * no, cudaMemcpyDeviceToHost, st));
     unsigned int word = 0;
     if (fixed) RBG_CUDA(cudaMemcpyAsync(&word, err, 4, cudaMemcpyDeviceToHost, st));
@@ -528,7 +529,12 @@ static int mixed_run(Ctx& c, const Plan& plan, const TableSet& ts, const MixedJo
     const double* zext = sz ? c.z.as<double>() : nullptr;
     float* ivq = mc ? c.ivp.as<float>() : nullptr;
     RBG_CUDA(cudaMemsetAsync((unsigned char*)c.mixed_ws.p + job.off_err, 0, 4, st));  // the kernel error word
-    RBG_CUDA(cudaMemsetAsync(c.acc.p, 0, sizeof(double) * 4 * no, st));
+    const MergeFinal fin{ts.t.outs, ts.Tvals, c.res.as<double>(), M, o.compute_iv};
+    auto merge = [&](int rows, int64_t m0) {
+        return launch_merge(c.part.as<double>(), rows, no, c.acc.as<double>(), m0 == 0, st, m0 + B >= M ? &fin : nullptr)
+                   ? fail(RBG_ERR_CUDA, "merge tables could not be set up")
+                   : RBG_OK;
+    };
     for (int64_t m0 = 0; m0 < M; m0 += B) {
         const int64_t b = std::min(B, M - m0);
         if (sz) {
@@ -548,7 +554,7 @@ static int mixed_run(Ctx& c, const Plan& plan, const TableSet& ts, const MixedJo
                     return rc;
             }
             ProfScope ps(kStageReduce, st);
-            launch_accumulate(c.part.as<double>(), rows, no, c.acc.as<double>(), st);
+            if ((rc = merge(rows, m0))) return rc;
         } else {
             {
                 ProfScope ps(kStageMixed, st, (int)job.launches.size());
@@ -563,13 +569,11 @@ static int mixed_run(Ctx& c, const Plan& plan, const TableSet& ts, const MixedJo
             }
             {
                 ProfScope ps(kStageReduce, st);
-                launch_accumulate(c.part.as<double>(), nchunks, no, c.acc.as<double>(), st);
+                if ((rc = merge(nchunks, m0))) return rc;
             }
         }
         RBG_CUDA(cudaGetLastError());
     }
-    launch_finalize(c.acc.as<double>(), no, M, ts.t.outs, ts.Tvals, o.compute_iv, c.res.as<double>(), st);
-    RBG_CUDA(cudaGetLastError());
     // one wait for the whole call: the kernel error word is read after the
     // finalize kernel is queued (finalizing the sums of a launch that gave up
     // is harmless; its results are discarded), so no host round trip sits
@@ -720,7 +724,6 @@ static int price_cv(Ctx& c, const Plan& plan, const rbg_cv_params& p, const rbg_
     launch_path_fp64(ts.t, c.z.as<double>(), Mc, c.ivb.as<double>(), st);
     launch_cv_pilot(ts.t, c.ivb.as<double>(), Mc, xy, alpha, Q, st);
     RBG_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned long long) * no, st));
-    RBG_CUDA(cudaMemsetAsync(c.acc.p, 0, sizeof(double) * 4 * no, st));
     // main paths, antithetic pairs
     for (int64_t m0 = 0; m0 < M; m0 += B) {
         const int64_t b = std::min(B, M - m0);
@@ -736,11 +739,13 @@ static int price_cv(Ctx& c, const Plan& plan, const rbg_cv_params& p, const rbg_
         const int nchunks = (int)((b + 256 * (int64_t)G - 1) / (256 * (int64_t)G));
         launch_payoff_sums_cv(ts.t, c.ivb.as<double>(), c.ivp.as<double>(), b, alpha, Q, p.Q_max, G,
                               c.part.as<double>(), count, nchunks, st);
-        launch_accumulate(c.part.as<double>(), nchunks, no, c.acc.as<double>(), st);
+        if (launch_merge(c.part.as<double>(), nchunks, no, c.acc.as<double>(), m0 == 0, st))
+            return fail(RBG_ERR_CUDA, "merge tables could not be set up");
         RBG_CUDA(cudaGetLastError());
     }
-    launch_finalize_cv(c.acc.as<double>(), no, M, ts.t.outs, ts.Tvals, alpha, Q, count, p.Q_max, o.compute_iv,
-                       c.res.as<double>(), st);
+    if (launch_finalize_cv(c.acc.as<double>(), no, M, ts.t.outs, ts.Tvals, alpha, Q, count, p.Q_max, o.compute_iv,
+                           c.res.as<double>(), st))
+        return fail(RBG_ERR_CUDA, "merge tables could not be set up");
     RBG_CUDA(cudaGetLastError());
     RBG_CUDA(cudaMemcpyAsync(host_res, c.res.p, sizeof(double) * 5 * no, cudaMemcpyDeviceToHost, st));
     RBG_CUDA(cudaStreamSynchronize(st));
@@ -790,7 +795,6 @@ static int price_cv_mixed(Ctx& c, const Plan& plan, const rbg_cv_params& p, cons
     launch_path_fp64(ts.t, c.z.as<double>(), Mc, c.ivp.as<double>(), st);
     launch_cv_pilot(ts.t, c.ivp.as<double>(), Mc, xy, alpha, Q, st);
     RBG_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned long long) * no, st));
-    RBG_CUDA(cudaMemsetAsync(c.acc.p, 0, sizeof(double) * 4 * no, st));
     // main paths: the job as is and its antithetic twin, both with xi = 0 in the final sums
     for (MixedLaunch& L : job.launches) L.args.xi = L.args.sqrt_xi = 0.f;
     MixedJob anti = job;
@@ -821,12 +825,14 @@ static int price_cv_mixed(Ctx& c, const Plan& plan, const rbg_cv_params& p, cons
         }
         {
             ProfScope ps(kStageReduce, st);
-            launch_accumulate(c.part.as<double>(), nchunks, no, c.acc.as<double>(), st);
+            if (launch_merge(c.part.as<double>(), nchunks, no, c.acc.as<double>(), m0 == 0, st))
+                return fail(RBG_ERR_CUDA, "merge tables could not be set up");
         }
         RBG_CUDA(cudaGetLastError());
     }
-    launch_finalize_cv(c.acc.as<double>(), no, M, ts.t.outs, ts.Tvals, alpha, Q, count, p.Q_max, o.compute_iv,
-                       c.res.as<double>(), st);
+    if (launch_finalize_cv(c.acc.as<double>(), no, M, ts.t.outs, ts.Tvals, alpha, Q, count, p.Q_max, o.compute_iv,
+                           c.res.as<double>(), st))
+        return fail(RBG_ERR_CUDA, "merge tables could not be set up");
     RBG_CUDA(cudaGetLastError());
     if ((rc = mixed_check(job, c.mixed_ws.p, st, g_err))) return rc;
     RBG_CUDA(cudaMemcpyAsync(host_res, c.res.p, sizeof(double) * 5 * no, cudaMemcpyDeviceToHost, st));
@@ -1304,7 +1310,8 @@ int rbg_implied_vol(int n, const double* price, const double* K, const double* T
     RBG_CUDA(cudaMemcpyAsync(d, price, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
     RBG_CUDA(cudaMemcpyAsync(d + n, K, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
     RBG_CUDA(cudaMemcpyAsync(d + 2 * n, T, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
-    launch_implied_vol(n, d, d + n, d + 2 * n, d + 3 * n, c->stream);
+    if (launch_implied_vol(n, d, d + n, d + 2 * n, d + 3 * n, c->stream))
+        return fail(RBG_ERR_CUDA, "implied-vol tables could not be set up");
     RBG_CUDA(cudaGetLastError());
     RBG_CUDA(cudaMemcpyAsync(iv, d + 3 * n, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
     RBG_CUDA(cudaStreamSynchronize(c->stream));

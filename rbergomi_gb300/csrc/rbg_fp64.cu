@@ -12,8 +12,8 @@
 //                  sum's N^2 / 2 DFMA per path outgrow it there)
 //   k_payoff_sums  conditional BS per (path, output) and compensated per-chunk
 //                  sums of x and x^2 (rBergomiMT.cpp:598-602, 404-409)
-//   k_accumulate   fixed-order Neumaier merge of chunk sums (deterministic)
-//   k_finalize     price, stat (reference formula), implied vol
+//   k_merge        exact merge of chunk sums (deterministic); after the last
+//                  batch price, stat (reference formula), implied vol
 //   k_payoff_store per-path payoffs for the quadrature entry point
 // GB300's FP64 pipe (~2 DFMA/clk/SM) bounds every kernel here.
 #include <cuda_runtime.h>
@@ -553,98 +553,195 @@ int launch_payoff_sums(const Fp64Tables& t, const double* ivb, int64_t B, int64_
     return 0;
 }
 
-// acc[i * 4 + {0..3}] += the batch's chunk sums.  One block per output:
-// strided Neumaier sums per thread, then a fixed-shape tree, so the result
-// does not depend on scheduling.
-// Output i of a fixed-order merge of chunk sums into acc (fresh: acc holds
-// zeros, read as such -- the job-table launches skip the clearing memset).
-// Shared by the per-request and job-table kernels.
-__device__ __forceinline__ void accumulate_block(const double* __restrict__ part, int nchunks, int n_out,
-                                                 double* __restrict__ acc, int i, bool fresh, double (*sh)[256])
+// ------------------------------------------------------------ chunk merge
+// A call's chunk sums of one output, added exactly: the doubles become 128-bit
+// integers in units of 2^-52 of the largest one's last bit, whose additions
+// cost a few integer instructions and do not depend on their order.  (A
+// compensated FP64 tree of 600 chunks took 14-17 us of serial warp operations
+// on GB300's FP64 pipe.)
+struct Fix128 {
+    uint64_t lo;
+    int64_t hi;
+};
+
+__device__ __forceinline__ void fix_add(Fix128& a, uint64_t lo, int64_t hi)
 {
-    double S = 0, C = 0, S2 = 0, C2 = 0;
-    for (int c = threadIdx.x; c < nchunks; c += blockDim.x) {
-        const double* p = part + ((size_t)c * n_out + i) * 4;
-        neumaier_add(S, C, p[0]);
-        neumaier_add(S, C, p[1]);
-        neumaier_add(S2, C2, p[2]);
-        neumaier_add(S2, C2, p[3]);
+    const uint64_t s = a.lo + lo;
+    a.hi += hi + (s < lo ? 1 : 0);
+    a.lo = s;
+}
+
+__device__ __forceinline__ int double_exp(double x) { return (int)((double_bits(x) >> 52) & 2047u); }
+
+// a += x, x's exponent field at most emax (< 2047); bits more than 52 places
+// below emax's last one are dropped.
+__device__ __forceinline__ void fix_add_double(Fix128& a, double x, int emax)
+{
+    const uint64_t b = double_bits(x);
+    const int e = (int)(b >> 52) & 2047;
+    uint64_t m = b & 0x000FFFFFFFFFFFFFull;
+    if (e) m |= 0x0010000000000000ull;
+    const int sh = 52 - (emax - (e ? e : 1));  // left shift of the significand in the 128-bit frame
+    uint64_t lo = 0, hi = 0;
+    if (sh > 0) {
+        lo = m << sh;
+        hi = m >> (64 - sh);
+    } else if (sh > -64) {
+        lo = m >> -sh;
     }
-    sh[0][threadIdx.x] = S; sh[1][threadIdx.x] = C; sh[2][threadIdx.x] = S2; sh[3][threadIdx.x] = C2;
-    __syncthreads();
-    for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-        if ((int)threadIdx.x < h) {
-            const int j = threadIdx.x + h;
-            double a = sh[0][threadIdx.x], ac = sh[1][threadIdx.x];
-            neumaier_add(a, ac, sh[0][j]);
-            neumaier_add(a, ac, sh[1][j]);
-            double b = sh[2][threadIdx.x], bc = sh[3][threadIdx.x];
-            neumaier_add(b, bc, sh[2][j]);
-            neumaier_add(b, bc, sh[3][j]);
-            sh[0][threadIdx.x] = a; sh[1][threadIdx.x] = ac; sh[2][threadIdx.x] = b; sh[3][threadIdx.x] = bc;
+    if (b >> 63) {  // two's complement
+        lo = ~lo + 1;
+        hi = ~hi + (lo == 0 ? 1 : 0);
+    }
+    fix_add(a, lo, (int64_t)hi);
+}
+
+// a in the frame of emax as S + C, S its leading 53 bits.
+__device__ void fix_split(const Fix128& a, int emax, double& S, double& C)
+{
+    uint64_t lo = a.lo, hi = (uint64_t)a.hi;
+    const bool neg = a.hi < 0;
+    if (neg) {
+        lo = ~lo + 1;
+        hi = ~hi + (lo == 0 ? 1 : 0);
+    }
+    S = C = 0.0;
+    const int unit = emax - 1075 - 52;  // the frame's last bit is 2^unit
+    double part[2] = {0.0, 0.0};
+    for (int k = 0; k < 2 && (hi | lo); ++k) {
+        const int top = hi ? 127 - __clzll((long long)hi) : 63 - __clzll((long long)lo);
+        const int cut = top > 52 ? top - 52 : 0;  // the 53 bits from `top` down
+        uint64_t m;
+        if (cut >= 64) {
+            m = hi >> (cut - 64);
+            hi &= (1ull << (cut - 64)) - 1;
+        } else {
+            m = cut ? ((lo >> cut) | (hi << (64 - cut))) : lo;
+            hi = 0;
+            lo &= cut ? ((1ull << cut) - 1) : 0ull;
         }
-        __syncthreads();
+        part[k] = ldexp((double)(long long)m, unit + cut);
     }
-    if (threadIdx.x == 0) {
-        double a = 0, ac = 0, b = 0, bc = 0;
-        if (!fresh) { a = acc[i * 4 + 0]; ac = acc[i * 4 + 1]; b = acc[i * 4 + 2]; bc = acc[i * 4 + 3]; }
-        neumaier_add(a, ac, sh[0][0]);
-        neumaier_add(a, ac, sh[1][0]);
-        neumaier_add(b, bc, sh[2][0]);
-        neumaier_add(b, bc, sh[3][0]);
-        acc[i * 4 + 0] = a; acc[i * 4 + 1] = ac; acc[i * 4 + 2] = b; acc[i * 4 + 3] = bc;
+    S = neg ? -part[0] : part[0];
+    C = neg ? -part[1] : part[1];
+}
+
+constexpr int kMergeThreads = 128;
+struct MergeSmem {
+    Fix128 s[kMergeThreads / 32][2];
+    int emax[kMergeThreads / 32][2];
+    double out[4];
+};
+
+// Output i: acc (S, C, S2, C2) plus every chunk's, or just these where `fresh`;
+// stored to acc and, on every thread, in v.  A sum with a NaN or infinity in
+// it is added up in FP64 by one thread.
+__device__ void merge_block(const double* __restrict__ part, int nchunks, int n_out, double* __restrict__ acc, int i,
+                            bool fresh, MergeSmem& sm, double (&v)[4])
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    // the largest exponent of either sum
+    int em[2] = {0, 0};
+    for (int c = threadIdx.x; c < nchunks; c += kMergeThreads) {
+        const double2* p = reinterpret_cast<const double2*>(part + ((size_t)c * n_out + i) * 4);
+        const double2 x = p[0], y = p[1];
+        em[0] = max(em[0], max(double_exp(x.x), double_exp(x.y)));
+        em[1] = max(em[1], max(double_exp(y.x), double_exp(y.y)));
     }
-}
-
-__global__ void __launch_bounds__(256) k_accumulate(const double* __restrict__ part, int nchunks, int n_out,
-                                                    double* __restrict__ acc)
-{
-    __shared__ double sh[4][256];
-    accumulate_block(part, nchunks, n_out, acc, blockIdx.x, false, sh);
-}
-
-// Job-table form: block b merges output b - jobs[k].block0 of job k.
-__global__ void __launch_bounds__(256) k_accumulate_jobs(const AccJob* __restrict__ jobs, int n_jobs)
-{
-    __shared__ double sh[4][256];
-    int lo = 0, hi = n_jobs - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (jobs[mid].block0 <= (int64_t)blockIdx.x) lo = mid; else hi = mid - 1;
+    if (!fresh)
+        for (int z = 0; z < 2; ++z) em[z] = max(em[z], max(double_exp(acc[i * 4 + 2 * z]), double_exp(acc[i * 4 + 2 * z + 1])));
+#pragma unroll
+    for (int z = 0; z < 2; ++z) {
+        em[z] = __reduce_max_sync(0xffffffffu, em[z]);
+        if (lane == 0) sm.emax[w][z] = em[z];
     }
-    const AccJob& J = jobs[lo];
-    accumulate_block(J.part, J.nchunks, J.n_out, J.acc, (int)((int64_t)blockIdx.x - J.block0), true, sh);
-}
-
-void launch_accumulate_jobs(const AccJob* jobs, int n_jobs, int64_t blocks, void* stream)
-{
-    k_accumulate_jobs<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(jobs, n_jobs);
-    count_launch();
-}
-
-void launch_accumulate(const double* part, int nchunks, int n_out, double* acc, void* stream)
-{
-    k_accumulate<<<n_out, 256, 0, (cudaStream_t)stream>>>(part, nchunks, n_out, acc);
-    count_launch();
+    __syncthreads();
+#pragma unroll
+    for (int z = 0; z < 2; ++z)
+#pragma unroll
+        for (int k = 0; k < kMergeThreads / 32; ++k) em[z] = max(em[z], sm.emax[k][z]);
+    Fix128 s[2] = {{0, 0}, {0, 0}};
+    for (int c = threadIdx.x; c < nchunks; c += kMergeThreads) {
+        const double2* p = reinterpret_cast<const double2*>(part + ((size_t)c * n_out + i) * 4);
+        const double2 x = p[0], y = p[1];
+        fix_add_double(s[0], x.x, em[0]);
+        fix_add_double(s[0], x.y, em[0]);
+        fix_add_double(s[1], y.x, em[1]);
+        fix_add_double(s[1], y.y, em[1]);
+    }
+    if (!fresh && threadIdx.x == 0) {
+        for (int z = 0; z < 2; ++z) {
+            fix_add_double(s[z], acc[i * 4 + 2 * z], em[z]);
+            fix_add_double(s[z], acc[i * 4 + 2 * z + 1], em[z]);
+        }
+    }
+#pragma unroll
+    for (int z = 0; z < 2; ++z) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            fix_add(s[z], __shfl_xor_sync(0xffffffffu, s[z].lo, o), __shfl_xor_sync(0xffffffffu, s[z].hi, o));
+        if (lane == 0) sm.s[w][z] = s[z];
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        const int z = threadIdx.x;
+        double S, C;
+        if (em[z] < 2047) {
+            Fix128 t = sm.s[0][z];
+            for (int k = 1; k < kMergeThreads / 32; ++k) fix_add(t, sm.s[k][z].lo, sm.s[k][z].hi);
+            fix_split(t, em[z], S, C);
+        } else {
+            S = fresh ? 0.0 : acc[i * 4 + 2 * z] + acc[i * 4 + 2 * z + 1];
+            C = 0.0;
+            for (int c = 0; c < nchunks; ++c) S += part[((size_t)c * n_out + i) * 4 + 2 * z];
+        }
+        acc[i * 4 + 2 * z] = sm.out[2 * z] = S;
+        acc[i * 4 + 2 * z + 1] = sm.out[2 * z + 1] = C;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = sm.out[k];
 }
 
 // ------------------------------------------------------------- IV (FP64)
-__device__ double bs_gen(double K, double T, double s, int put)
+// The out-of-the-money Black-Scholes price (S0 = 1, r = 0; put for K < 1) and
+// what its derivatives need: f = phi(d1), vega = f sqrt(T).  lnK = ln K.
+struct OtmPrice {
+    double p, f, d1, d2;
+};
+
+__device__ __forceinline__ OtmPrice otm_price(double K, double lnK, double v, bool put, const FixedTables* __restrict__ ft)
 {
-    const double sq = sqrt(T);
-    const double d1 = (log(1.0 / K) + 0.5 * s * s * T) / (s * sq);
-    const double d2 = d1 - s * sq;
-    return put ? (-phi_cdf(-d1) + phi_cdf(-d2) * K) : (phi_cdf(d1) - phi_cdf(d2) * K);
+    OtmPrice r;
+    r.d1 = fma(-lnK, 1.0 / v, 0.5 * v);
+    r.d2 = r.d1 - v;
+    r.f = exp2_double(fma(-0.5 * r.d1 * r.d1, 1.4426950408889634074, -1.3257480647361593990), ft->exp2);
+    const double m1 = mills(fabs(r.d1), ft->mills), m2 = mills(fabs(r.d2), ft->mills);
+    // call: [d1 >= 0] - K [d2 >= 0] + f (-+ M1 +- M2); put: less 1 - K, which only leaves K [d2 < 0]
+    const double base = put ? (r.d2 < 0.0 ? K : 0.0) : (r.d1 >= 0.0 ? 1.0 : 0.0);
+    r.p = fma(r.f, (r.d1 >= 0.0 ? -m1 : m1) + (r.d2 >= 0.0 ? m2 : -m2), base);
+    return r;
 }
 
-// The out-of-the-money Black-Scholes price in FP32 (S0 = 1, r = 0): the
-// bracketing rounds of implied_vol_warp.  lnK1 = ln(1 / K), sqT = sqrt(T).
+// The same price in FP32: the bracketing rounds of implied_vol_warp.  lnK1 =
+// ln(1 / K), sqT = sqrt(T).
 __device__ __forceinline__ float bs_gen_f32(float lnK1, float sqT, float K, float s, int put)
 {
     const float ssq = s * sqT;
     const float d1 = fmaf(0.5f, ssq, lnK1 * rcp_approx(ssq));
     const float d2 = d1 - ssq;
     return put ? fmaf(K, phi_f32(-d2), -phi_f32(-d1)) : fmaf(-K, phi_f32(d2), phi_f32(d1));
+}
+
+// log(p / target) for e = p / target - 1
+__device__ __forceinline__ double log_ratio(double e)
+{
+    if (fabs(e) > 1e-3) return log1p(e);
+    double s = fma(e, -1.0 / 6, 1.0 / 5);
+    s = fma(e, s, -1.0 / 4);
+    s = fma(e, s, 1.0 / 3);
+    s = fma(e, s, -1.0 / 2);
+    return fma(e * e, s, e);
 }
 
 // Implied vol by a warp: inverts on the out-of-the-money side (put-call
@@ -655,18 +752,20 @@ __device__ __forceinline__ float bs_gen_f32(float lnK1, float sqT, float K, floa
 //      FP64 decides (no bracket there: no volatility fits, NaN);
 //   2. three 33-section rounds in FP32 narrow the bracket ~36,000-fold (FP32
 //      resolves it no further);
-//   3. one FP64 step checks the narrowed bracket (lanes 0 and 1 price its
-//      ends, widened by 1e-6) while lane 2 prices its middle; if the check
-//      fails -- FP32 cannot resolve the price, e.g. far in a wing -- the FP64
-//      grid and FP64 33-section rounds (to 1e-6) take over;
+//   3. one FP64 step checks the narrowed bracket, widened by 1e-4 (near the
+//      money FP32 prices cancel to a few 1e-6: a margin of 1e-6 sent those
+//      outputs to step 4's search, 60 us longer): lanes 0 and 1 price its
+//      ends, the others its middle; if the check fails -- FP32 cannot resolve
+//      the price, e.g. far in a wing -- the FP64 grid and FP64 33-section
+//      rounds (to 1e-6) take over;
 //   4. from the checked bracket's middle one Halley step on the log price
-//      (cubic: from a 1e-5 bracket the error left is 1e-15 near the money,
-//      below ~1e-12 in the wings), then safeguarded Newton on the
-//      log price where a step is still larger than that.
-// The search is a chain of serial FP64 evaluations on GB300's slow FP64 pipe,
-// so fewer of them is what makes it fast: two on the common path.  All lanes
+//      (cubic: from 1e-5 the error left is 1e-15 near the money, below ~1e-12
+//      in the wings), then safeguarded Newton on the log price where a step is
+//      still larger than that.
+// Prices are Mills' ratios (otm_price): the density they contain is the vega,
+// so an FP64 step is one chain of about 30 dependent operations.  All lanes
 // return the same value; NaN when no volatility fits.
-__device__ double implied_vol_warp(double price, double K, double T)
+__device__ double implied_vol_warp(double price, double K, double T, const FixedTables* __restrict__ ft)
 {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -675,17 +774,17 @@ __device__ double implied_vol_warp(double price, double K, double T)
     const double upper = put ? K : 1.0;
     const double nan = __longlong_as_double(0x7ff8000000000000ll);
     if (!(target > 0.0) || !(target < upper) || !(T > 0.0)) return nan;
-    const float lnK1 = (float)log(1.0 / K), sqT32 = (float)sqrt(T), K32 = (float)K, t32 = (float)target;
-    double lo = 0.0, hi = 0.0;
+    const double lnK = log(K), sqT = sqrt(T);
+    const float lnK1 = -log1pf((float)(K - 1.0)), sqT32 = sqrtf((float)T), K32 = (float)K, t32 = (float)target;
+    double lo = 0.0, hi = 0.0, s = 0.0;
     bool narrowed = false;
-    double s = 0.0, p0 = 0.0;
+    OtmPrice q{};
     {
         // FP32 grid and rounds, then the FP64 check
         const unsigned b32 = __ballot_sync(FULL, bs_gen_f32(lnK1, sqT32, K32, 1e-3f * exp2f(0.5f * lane), put) >= t32);
         if (b32 != 0u) {
             const int f = __ffs(b32) - 1;
-            const double glo = (f > 0) ? 1e-3 * exp2(0.5 * (f - 1)) : 0.0, ghi = 1e-3 * exp2(0.5 * f);
-            float lo32 = (float)glo, hi32 = (float)ghi;
+            float lo32 = (f > 0) ? 1e-3f * exp2f(0.5f * (f - 1)) : 0.f, hi32 = 1e-3f * exp2f(0.5f * f);
 #pragma unroll 1
             for (int it = 0; it < 3; ++it) {
                 const float sl = fmaf(hi32 - lo32, (float)(lane + 1) * (1.0f / 33.0f), lo32);
@@ -696,17 +795,16 @@ __device__ double implied_vol_warp(double price, double K, double T)
                 if (ff > 0) lo32 = nlo;
                 if (ff < 32) hi32 = nhi;
             }
-            const double lo2 = fmax(glo, (double)lo32 * (1.0 - 1e-6)), hi2 = fmin(ghi, (double)hi32 * (1.0 + 1e-6));
-            const double sv = lane == 0 ? lo2 : (lane == 1 ? hi2 : 0.5 * (lo2 + hi2));
-            const double pv = (sv > 0.0) ? bs_gen(K, T, sv, put) : 0.0;  // zero volatility: the OTM price is 0
-            const double plo = __shfl_sync(FULL, pv, 0), phi_ = __shfl_sync(FULL, pv, 1);
-            const double pmid = __shfl_sync(FULL, pv, 2);
-            if (lo2 < hi2 && plo < target && phi_ >= target) {
+            const double mid = 0.5 * ((double)lo32 + (double)hi32);
+            const double lo2 = fmax((double)lo32 - 1e-4 * mid, 1e-12), hi2 = (double)hi32 + 1e-4 * mid;
+            const double sv = lane == 0 ? lo2 : (lane == 1 ? hi2 : mid);
+            q = otm_price(K, lnK, sv * sqT, put, ft);
+            const double plo = __shfl_sync(FULL, q.p, 0), phi_ = __shfl_sync(FULL, q.p, 1);
+            if (plo < target && phi_ >= target) {
                 narrowed = true;
                 lo = lo2;
                 hi = hi2;
-                s = 0.5 * (lo2 + hi2);
-                p0 = pmid;
+                s = mid;
             }
         }
     }
@@ -714,14 +812,14 @@ __device__ double implied_vol_warp(double price, double K, double T)
         // FP64 grid, then FP64 33-section rounds (one evaluation per lane)
         // until the bracket is within 1e-6 relative
         const double sig = 1e-3 * exp2(0.5 * lane);
-        unsigned b = __ballot_sync(FULL, bs_gen(K, T, sig, put) >= target);
+        unsigned b = __ballot_sync(FULL, otm_price(K, lnK, sig * sqT, put, ft).p >= target);
         if (b == 0u) return nan;
         int f = __ffs(b) - 1;
         lo = (f > 0) ? 1e-3 * exp2(0.5 * (f - 1)) : 0.0;
         hi = 1e-3 * exp2(0.5 * f);
         for (int it = 0; it < 14 && hi - lo > 1e-6 * hi; ++it) {
             const double sl = lo + (hi - lo) * (double)(lane + 1) / 33.0;
-            b = __ballot_sync(FULL, bs_gen(K, T, sl, put) >= target);
+            b = __ballot_sync(FULL, otm_price(K, lnK, sl * sqT, put, ft).p >= target);
             f = b ? __ffs(b) - 1 : 32;
             const double nlo = __shfl_sync(FULL, sl, f > 0 ? f - 1 : 0);
             const double nhi = __shfl_sync(FULL, sl, f < 32 ? f : 31);
@@ -730,22 +828,27 @@ __device__ double implied_vol_warp(double price, double K, double T)
         }
         s = 0.5 * (lo + hi);
     }
-    const double lt = log(target), sqT = sqrt(T);
-    if (narrowed && p0 > 0.0) {
-        // Halley on g(s) = log p(s) - log target: g' = vega / p and
-        // g'' = (vomma p - vega^2) / p^2 with vomma = vega d1 d2 / s
-        const double d1 = (log(1.0 / K) + 0.5 * s * s * T) / (s * sqT);
-        const double d2 = d1 - s * sqT;
-        const double vega = exp(-0.5 * d1 * d1) * 0.39894228040143267794 * sqT;
-        const double g = log(p0) - lt, g1 = vega / p0, g2 = (vega * d1 * d2 / s) / p0 - g1 * g1;
-        const double nt = s - 2.0 * g * g1 / (2.0 * g1 * g1 - g * g2);
+    if (narrowed) {
+        // Halley on g(s) = log p(s) - log target: with r = g / g', g'' / g' = d1 d2 / s - vega / p,
+        // the step is r / (1 - r g'' / (2 g')); the bracket's ends move to the middle's side.
+        // (Lanes 0 and 1 hold the ends' prices: lane 2's values decide.)
+        const double vega = q.f * sqT;
+        const double r = log_ratio((q.p - target) / target) * (q.p / vega);
+        const float h = 0.5f * (float)r * ((float)(q.d1 * q.d2) / (float)s - (float)vega / (float)q.p);
+        const double step = r + r * (double)(h / (1.0f - h));
+        double nt = __shfl_sync(FULL, s - step, 2);
+        const bool above = __shfl_sync(FULL, q.p > target ? 1 : 0, 2) != 0;
         if (nt > lo && nt < hi) {
             if (fabs(nt - s) <= 1e-5 * s) return nt;  // cubic: the error left is below ~1e-12 relative
+            if (above) hi = s;
+            else lo = s;
+            if (!(nt > lo && nt < hi)) nt = 0.5 * (lo + hi);
             s = nt;
+        } else {
+            if (above) hi = s;
+            else lo = s;
+            s = 0.5 * (lo + hi);
         }
-        if (p0 > target) hi = 0.5 * (lo + hi);
-        else lo = 0.5 * (lo + hi);
-        if (!(s > lo && s < hi)) s = 0.5 * (lo + hi);
     }
     // safeguarded Newton on the log price (every lane computes the same
     // iterate).  A Newton step below 1e-14 relative ends the search: the
@@ -753,15 +856,13 @@ __device__ double implied_vol_warp(double price, double K, double T)
     // step that leaves the bracket, or a vanishing price, falls back to
     // bisection; 40 halvings take a 1e-6 bracket below 1e-15 on their own.
     for (int it = 0; it < 40; ++it) {
-        const double p = bs_gen(K, T, s, put);
-        if (p == target) break;
-        if (p > target) hi = s;
+        q = otm_price(K, lnK, s * sqT, put, ft);
+        if (q.p == target) break;
+        if (q.p > target) hi = s;
         else lo = s;
         double sn = 0.5 * (lo + hi);
-        if (p > 0.0) {
-            const double d1 = (log(1.0 / K) + 0.5 * s * s * T) / (s * sqT);
-            const double vega = exp(-0.5 * d1 * d1) * 0.39894228040143267794 * sqT;
-            const double nt = s - (log(p) - lt) * p / vega;
+        if (q.p > 0.0) {
+            const double nt = s - log_ratio((q.p - target) / target) * q.p / (q.f * sqT);
             if (fabs(nt - s) <= 1e-14 * s) {
                 s = nt;
                 break;
@@ -774,21 +875,20 @@ __device__ double implied_vol_warp(double price, double K, double T)
     return s;
 }
 
+// Output i's price, stat and implied vol from its sums v (one warp).
 // res: [0,n) price, [n,2n) stat, [2n,3n) iv, [3n,4n) sum, [4n,5n) sum2.
-// One warp per output.
-// Output i (one warp) of the price / stat / implied vol; shared by the
-// per-request and job-table kernels.
-__device__ __forceinline__ void finalize_warp(const double* __restrict__ acc, int n_out, int64_t M,
+__device__ __forceinline__ void finalize_warp(const double (&v)[4], int n_out, double invM, double isqM,
                                               const OutDev* __restrict__ outs, const double* __restrict__ Tv,
-                                              int compute_iv, double* __restrict__ res, int i)
+                                              int compute_iv, double* __restrict__ res, int i,
+                                              const FixedTables* __restrict__ ft)
 {
-    const double S = acc[i * 4 + 0] + acc[i * 4 + 1];
-    const double S2 = acc[i * 4 + 2] + acc[i * 4 + 3];
+    const double S = v[0] + v[1];
+    const double S2 = v[2] + v[3];
     // rBergLib/rBergomiMT.cpp:404-409
-    const double price = S * (1.0 / (double)M);
-    const double var = 1.0 * (S2 * (1.0 / (double)M)) + -1.0 * (price * price);
-    const double stat = sqrt(var) * (1.0 / sqrt((double)M));
-    const double iv = compute_iv ? implied_vol_warp(price, outs[i].K, Tv[i]) : 0.0;
+    const double price = S * invM;
+    const double var = 1.0 * (S2 * invM) + -1.0 * (price * price);
+    const double stat = sqrt(var) * isqM;
+    const double iv = compute_iv ? implied_vol_warp(price, outs[i].K, Tv[i], ft) : 0.0;
     if ((threadIdx.x & 31) == 0) {
         res[i] = price;
         res[n_out + i] = stat;
@@ -798,66 +898,87 @@ __device__ __forceinline__ void finalize_warp(const double* __restrict__ acc, in
     }
 }
 
-__global__ void k_finalize(const double* __restrict__ acc, int n_out, int64_t M, const OutDev* __restrict__ outs,
-                           const double* __restrict__ Tv, int compute_iv, double* __restrict__ res)
+// One block per output: its chunk sums into acc and, after the call's last
+// batch (res non-null), the price, stat and implied vol by the first warp.
+__global__ void __launch_bounds__(kMergeThreads) k_merge(const double* __restrict__ part, int nchunks, int n_out,
+                                                        double* __restrict__ acc, int fresh, double invM, double isqM,
+                                                        const OutDev* __restrict__ outs, const double* __restrict__ Tv,
+                                                        int compute_iv, double* __restrict__ res,
+                                                        const FixedTables* __restrict__ ft)
 {
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (i >= n_out) return;  // whole warps leave together
-    finalize_warp(acc, n_out, M, outs, Tv, compute_iv, res, i);
+    __shared__ MergeSmem sm;
+    double v[4];
+    merge_block(part, nchunks, n_out, acc, blockIdx.x, fresh != 0, sm, v);
+    if (res && threadIdx.x < 32) finalize_warp(v, n_out, invM, isqM, outs, Tv, compute_iv, res, blockIdx.x, ft);
 }
 
-// Job-table form: one warp (block) per output, block b finalizes output
-// b - jobs[k].block0 of job k.
-__global__ void k_finalize_jobs(const FinJob* __restrict__ jobs, int n_jobs)
+// Job-table form: block b is output b - jobs[k].block0 of job k (both tables).
+__global__ void __launch_bounds__(kMergeThreads) k_merge_jobs(const AccJob* __restrict__ jobs,
+                                                             const FinJob* __restrict__ fins, int n_jobs,
+                                                             const FixedTables* __restrict__ ft)
 {
+    __shared__ MergeSmem sm;
     int lo = 0, hi = n_jobs - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if (jobs[mid].block0 <= (int64_t)blockIdx.x) lo = mid; else hi = mid - 1;
     }
-    const FinJob& J = jobs[lo];
-    finalize_warp(J.acc, J.n_out, J.M, J.outs, J.Tv, J.compute_iv, J.res, (int)((int64_t)blockIdx.x - J.block0));
+    const AccJob& J = jobs[lo];
+    const FinJob& F = fins[lo];
+    const int i = (int)((int64_t)blockIdx.x - J.block0);
+    double v[4];
+    merge_block(J.part, J.nchunks, J.n_out, J.acc, i, true, sm, v);
+    if (threadIdx.x < 32) finalize_warp(v, J.n_out, F.invM, F.isqM, F.outs, F.Tv, F.compute_iv, F.res, i, ft);
 }
 
-void launch_finalize_jobs(const FinJob* jobs, int n_jobs, int64_t blocks, void* stream)
+int launch_merge_jobs(const AccJob* jobs, const FinJob* fins, int n_jobs, int64_t blocks, void* stream)
 {
-    k_finalize_jobs<<<(unsigned)blocks, 32, 0, (cudaStream_t)stream>>>(jobs, n_jobs);
+    const FixedTables* ft = fixed_tables();
+    if (!ft) return -1;
+    k_merge_jobs<<<(unsigned)blocks, kMergeThreads, 0, (cudaStream_t)stream>>>(jobs, fins, n_jobs, ft);
     count_launch();
+    return 0;
 }
 
+// Loads the merge kernels and their tables (a serving loop's first request
+// must not meet either).
 void reduce_preload()
 {
     cudaFuncAttributes fa;
-    cudaFuncGetAttributes(&fa, k_accumulate);
-    cudaFuncGetAttributes(&fa, k_accumulate_jobs);
-    cudaFuncGetAttributes(&fa, k_finalize);
-    cudaFuncGetAttributes(&fa, k_finalize_jobs);
+    cudaFuncGetAttributes(&fa, k_merge);
+    cudaFuncGetAttributes(&fa, k_merge_jobs);
+    fixed_tables();
     cudaGetLastError();
 }
 
-void launch_finalize(const double* acc, int n_out, int64_t M, const OutDev* outs, const double* Tvals,
-                     int compute_iv, double* res, void* stream)
+int launch_merge(const double* part, int nchunks, int n_out, double* acc, bool fresh, void* stream, const MergeFinal* fin)
 {
-    // one output (one warp) per block: the implied-vol search is FP64-bound,
-    // and GB300's FP64 pipe is per SM, so the outputs spread over the SMs
-    const int threads = 32;
-    const int blocks = (int)(((int64_t)n_out * 32 + threads - 1) / threads);
-    k_finalize<<<blocks, threads, 0, (cudaStream_t)stream>>>(acc, n_out, M, outs, Tvals, compute_iv, res);
+    const FixedTables* ft = fixed_tables();
+    if (!ft) return -1;
+    const MergeFinal f = fin ? *fin : MergeFinal{};
+    k_merge<<<n_out, kMergeThreads, 0, (cudaStream_t)stream>>>(
+        part, nchunks, n_out, acc, fresh ? 1 : 0, fin ? 1.0 / (double)f.M : 0.0, fin ? 1.0 / std::sqrt((double)f.M) : 0.0,
+        f.outs, f.Tv, f.compute_iv, f.res, ft);
     count_launch();
+    return 0;
 }
 
-__global__ void k_implied_vol(int n, const double* price, const double* K, const double* T, double* iv)
+__global__ void k_implied_vol(int n, const double* price, const double* K, const double* T, double* iv,
+                              const FixedTables* __restrict__ ft)
 {
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (i >= n) return;
-    const double v = implied_vol_warp(price[i], K[i], T[i]);
+    const double v = implied_vol_warp(price[i], K[i], T[i], ft);
     if ((threadIdx.x & 31) == 0) iv[i] = v;
 }
 
-void launch_implied_vol(int n, const double* price, const double* K, const double* T, double* iv, void* stream)
+int launch_implied_vol(int n, const double* price, const double* K, const double* T, double* iv, void* stream)
 {
-    k_implied_vol<<<n, 32, 0, (cudaStream_t)stream>>>(n, price, K, T, iv);  // one warp (output) per block
+    const FixedTables* ft = fixed_tables();
+    if (!ft) return -1;
+    k_implied_vol<<<n, 32, 0, (cudaStream_t)stream>>>(n, price, K, T, iv, ft);  // one warp (output) per block
     count_launch();
+    return 0;
 }
 
 // ------------------------------------------------------------ quadrature
@@ -1078,7 +1199,8 @@ void launch_payoff_sums_cv(const Fp64Tables& t, const double* ivb, const double*
 __global__ void k_finalize_cv(const double* __restrict__ acc, int n_out, int64_t M, const OutDev* __restrict__ outs,
                               const double* __restrict__ Tv, const double* __restrict__ alpha,
                               const double* __restrict__ Q, const unsigned long long* __restrict__ count,
-                              double Qmax, int compute_iv, double* __restrict__ res)
+                              double Qmax, int compute_iv, double* __restrict__ res,
+                              const FixedTables* __restrict__ ft)
 {
     const int i = blockIdx.x;
     if (i >= n_out) return;
@@ -1090,7 +1212,7 @@ __global__ void k_finalize_cv(const double* __restrict__ acc, int n_out, int64_t
     const double p = (double)count[i] / (double)M, r = outs[i].rho, K = outs[i].K;
     const double adj = (1.0 - p) * bs_call_tau1(1.0, K, sqrt(r * r * Q[i])) + p * bs_call_tau1(1.0, K, sqrt(r * r * Qmax));
     const double price = mean - alpha[i] * adj;
-    const double iv = compute_iv ? implied_vol_warp(price, K, Tv[i]) : 0.0;
+    const double iv = compute_iv ? implied_vol_warp(price, K, Tv[i], ft) : 0.0;
     if ((threadIdx.x & 31) == 0) {
         res[i] = price;
         res[n_out + i] = stat;
@@ -1100,13 +1222,16 @@ __global__ void k_finalize_cv(const double* __restrict__ acc, int n_out, int64_t
     }
 }
 
-void launch_finalize_cv(const double* acc, int n_out, int64_t M, const OutDev* outs, const double* Tvals,
+int launch_finalize_cv(const double* acc, int n_out, int64_t M, const OutDev* outs, const double* Tvals,
                         const double* alpha, const double* Q, const unsigned long long* count, double Qmax,
                         int compute_iv, double* res, void* stream)
 {
+    const FixedTables* ft = fixed_tables();
+    if (!ft) return -1;
     k_finalize_cv<<<n_out, 32, 0, (cudaStream_t)stream>>>(acc, n_out, M, outs, Tvals, alpha, Q, count, Qmax,
-                                                          compute_iv, res);
+                                                          compute_iv, res, ft);
     count_launch();
+    return 0;
 }
 
 }  // namespace rbg

@@ -136,18 +136,27 @@ void launch_cv_pilot(const Fp64Tables& t, const double* ivb, int64_t Mc, double*
 void launch_payoff_sums_cv(const Fp64Tables& t, const double* ivb, const double* ivn, int64_t B, const double* alpha,
                            const double* Q, double Qmax, int G, double* part, unsigned long long* count, int nchunks,
                            void* stream);
-void launch_finalize_cv(const double* acc, int n_out, int64_t M, const OutDev* outs, const double* Tvals,
+int launch_finalize_cv(const double* acc, int n_out, int64_t M, const OutDev* outs, const double* Tvals,
                         const double* alpha, const double* Q, const unsigned long long* count, double Qmax,
                         int compute_iv, double* res, void* stream);
 // nonzero where the kernel could not be configured
 int launch_payoff_sums(const Fp64Tables& t, const double* ivb, int64_t B, int64_t ivb_stride, int G,
                         double* part, int nchunks, void* stream, const double* ivp = nullptr);
-void launch_accumulate(const double* part, int nchunks, int n_out, double* acc, void* stream);
-void launch_finalize(const double* acc, int n_out, int64_t M, const OutDev* outs, const double* Tvals,
-                     int compute_iv, double* res, void* stream);
+// Merges a batch's chunk sums into acc[n_out][4] (fresh: the first batch, acc
+// need not be cleared); fin (the last batch): price, stat, implied vol, sum and
+// sum2 of every output into res[5 n_out].
+struct MergeFinal {
+    const OutDev* outs = nullptr;
+    const double* Tv = nullptr;
+    double* res = nullptr;
+    int64_t M = 1;
+    int compute_iv = 0;
+};
+int launch_merge(const double* part, int nchunks, int n_out, double* acc, bool fresh, void* stream,
+                 const MergeFinal* fin = nullptr);
 int launch_payoff_store(const Fp64Tables& t, const double* ivb, int64_t B, int64_t ivb_stride, double* payoff,
                          void* stream, const double* ivp = nullptr);
-void launch_implied_vol(int n, const double* price, const double* K, const double* T, double* iv, void* stream);
+int launch_implied_vol(int n, const double* price, const double* K, const double* T, double* iv, void* stream);
 
 // ---- job-table forms of the payoff, merge and finalize kernels ----------
 // (the serving loop's shared launches: one launch serves many requests; each
@@ -160,23 +169,21 @@ struct PayoffJob {      // FP32 RT payoff sums, nchunks x ceil(n_out / 8) blocks
     int64_t B, block0;
     int n_out, G, nchunks, pad;
 };
-struct AccJob {  // fixed-order merge of the chunk sums into acc (written, not added to), n_out blocks
+struct AccJob {  // merge of the chunk sums into acc (written, not added to), n_out blocks
     const double* part;
     double* acc;
     int64_t block0;
     int nchunks, n_out;
 };
-struct FinJob {  // price, stat, implied vol, n_out blocks of one warp
-    const double* acc;
+struct FinJob {  // then its price, stat, implied vol; invM = 1 / M, isqM = 1 / sqrt(M)
     const OutDev* outs;
     const double* Tv;
     double* res;
-    int64_t M, block0;
-    int n_out, compute_iv;
+    double invM, isqM;
+    int compute_iv, pad;
 };
-void launch_accumulate_jobs(const AccJob* jobs, int n_jobs, int64_t blocks, void* stream);
-void launch_finalize_jobs(const FinJob* jobs, int n_jobs, int64_t blocks, void* stream);
-// Loads the merge and finalize kernels (modules load lazily, on first use).
+int launch_merge_jobs(const AccJob* jobs, const FinJob* fins, int n_jobs, int64_t blocks, void* stream);
+// Loads the merge kernels and their tables (modules load lazily, on first use).
 void reduce_preload();
 
 // Kernel-launch counter shared by all launchers.

@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <atomic>
 #include <chrono>
 #include <condition_variable>
@@ -326,26 +327,30 @@ int Server::launch(Slot& s, Req& r, std::string& err)
     }
     std::string kerr;
     rc = RBG_OK;
-    cudaMemsetAsync(s.acc.p, 0, sizeof(double) * 4 * no, st);
+    const MergeFinal fin{d_outs, d_T, (double*)s.res.p, r.M, r.opt.compute_iv};
     for (int64_t m0 = 0; m0 < r.M && rc == RBG_OK; m0 += B) {
         const int64_t b = std::min(B, r.M - m0);
+        const MergeFinal* last = m0 + B >= r.M ? &fin : nullptr;
         if (job.fused) {
             const int nr = mixed_part_rows(job, b);
             cudaMemsetAsync(s.part.p, 0, sizeof(double) * 4 * no * (size_t)nr, st);
             rc = mixed_launch(job, s.ws.p, r.opt.seed, r.opt.path_offset + m0, b, nullptr, st, kerr, nullptr,
                               nullptr, (double*)s.part.p);
-            if (rc == RBG_OK) launch_accumulate((const double*)s.part.p, nr, no, (double*)s.acc.p, st);
+            if (rc == RBG_OK && launch_merge((const double*)s.part.p, nr, no, (double*)s.acc.p, m0 == 0, st, last))
+                rc = RBG_ERR_CUDA;
         } else {
             rc = mixed_launch(job, s.ws.p, r.opt.seed, r.opt.path_offset + m0, b, s.ivb.p, st, kerr);
             const int nchunks = (int)((b + 256 * (int64_t)G - 1) / (256 * (int64_t)G));
             if (rc == RBG_OK) {
                 launch_payoff_sums_f32(d_outs, no, s.ivb.p, b, G, (double*)s.part.p, nchunks, st);
-                launch_accumulate((const double*)s.part.p, nchunks, no, (double*)s.acc.p, st);
+                if (launch_merge((const double*)s.part.p, nchunks, no, (double*)s.acc.p, m0 == 0, st, last)) {
+                    kerr = "merge tables could not be set up";
+                    rc = RBG_ERR_CUDA;
+                }
             }
         }
     }
     if (rc == RBG_OK) {
-        launch_finalize((const double*)s.acc.p, no, r.M, d_outs, d_T, r.opt.compute_iv, (double*)s.res.p, st);
         cudaMemcpyAsync(s.pin, (unsigned char*)s.ws.p + job.off_err, 4, cudaMemcpyDeviceToHost, st);
         cudaMemcpyAsync(s.pin + 1, s.res.p, sizeof(double) * 5 * no, cudaMemcpyDeviceToHost, st);
     }
@@ -553,7 +558,8 @@ int Server::launch_batch(BatchSlot& b, std::vector<Req*>& rs, std::string& err)
                           nch[k], 0};
         pblocks += (int64_t)nch[k] * ((no + 7) / 8);
         aj[k] = AccJob{(const double*)(dpart + o_part[k]), acc, ablocks, nch[k], no};
-        fj[k] = FinJob{acc, outs, (const double*)(din + o_T[k]), dres + o_res[k], r.M, ablocks, no, r.opt.compute_iv};
+        fj[k] = FinJob{outs, (const double*)(din + o_T[k]), dres + o_res[k], 1.0 / (double)r.M,
+                       1.0 / std::sqrt((double)r.M), r.opt.compute_iv, 0};
         ablocks += no;
     }
     MixedArgs LA;
@@ -577,8 +583,10 @@ int Server::launch_batch(BatchSlot& b, std::vector<Req*>& rs, std::string& err)
     int rc = mixed_launch_jobs(LA, rs[0]->job.split, grid, st, err);
     if (rc == RBG_OK) {
         launch_payoff_sums_f32_jobs((const PayoffJob*)(din + off_pj), n, pblocks, st);
-        launch_accumulate_jobs((const AccJob*)(din + off_aj), n, ablocks, st);
-        launch_finalize_jobs((const FinJob*)(din + off_fj), n, ablocks, st);
+        if (launch_merge_jobs((const AccJob*)(din + off_aj), (const FinJob*)(din + off_fj), n, ablocks, st)) {
+            err = "merge tables could not be set up";
+            rc = RBG_ERR_CUDA;
+        }
         cudaMemcpyAsync(b.pin, din, 4, cudaMemcpyDeviceToHost, st);
         cudaMemcpyAsync(b.pin + 1, dres, sizeof(double) * 5 * kBatchOutputs, cudaMemcpyDeviceToHost, st);
     }

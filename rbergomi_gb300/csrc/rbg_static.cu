@@ -159,8 +159,13 @@ int rbg_price_rt_static(const rbg_params* p, const rbg_options* o, double* price
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(s + off_outs, outs.data(), sizeof(OutDev) * n_out, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(s + off_T, Tv.data(), sizeof(double) * n_out, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(s + off_acc, 0, sizeof(double) * 4 * n_out, st);
     if (e != cudaSuccess) return fail_queued(RBG_ERR_CUDA, std::string("static scratch upload: ") + cudaGetErrorString(e));
+    const MergeFinal fin{(const OutDev*)(s + off_outs), (const double*)(s + off_T), (double*)(s + off_res), p->M,
+                         o->compute_iv};
+    auto merge = [&](int rows, int64_t m0) {
+        return launch_merge((const double*)(s + off_part), rows, n_out, (double*)(s + off_acc), m0 == 0, st,
+                            m0 + B >= p->M ? &fin : nullptr);
+    };
     for (int64_t m0 = 0; m0 < p->M; m0 += B) {
         const int64_t b = std::min(B, p->M - m0);
         if (job.fused) {
@@ -171,7 +176,7 @@ int rbg_price_rt_static(const rbg_params* p, const rbg_options* o, double* price
             rc = mixed_launch(job, s + off_ws, o->seed, o->path_offset + m0, b, nullptr, st, err, nullptr, nullptr,
                               (double*)(s + off_part));
             if (rc) return fail_queued(rc, err);
-            launch_accumulate((const double*)(s + off_part), rows, n_out, (double*)(s + off_acc), st);
+            if (merge(rows, m0)) return fail_queued(RBG_ERR_CUDA, "merge tables could not be set up");
             continue;
         }
         rc = mixed_launch(job, s + off_ws, o->seed, o->path_offset + m0, b, s + off_ivb, st, err);
@@ -179,10 +184,8 @@ int rbg_price_rt_static(const rbg_params* p, const rbg_options* o, double* price
         const int nchunks = (int)((b + chunk - 1) / chunk);
         launch_payoff_sums_f32((const OutDev*)(s + off_outs), n_out, s + off_ivb, b, G, (double*)(s + off_part),
                                nchunks, st);
-        launch_accumulate((const double*)(s + off_part), nchunks, n_out, (double*)(s + off_acc), st);
+        if (merge(nchunks, m0)) return fail_queued(RBG_ERR_CUDA, "merge tables could not be set up");
     }
-    launch_finalize((const double*)(s + off_acc), n_out, p->M, (const OutDev*)(s + off_outs),
-                    (const double*)(s + off_T), o->compute_iv, (double*)(s + off_res), st);
     // the error word after the finalize is queued: one wait for the whole call
     if ((rc = mixed_check(job, s + off_ws, st, err))) return fail_queued(rc, err);
     std::vector<double> res(5 * (size_t)n_out);

@@ -70,3 +70,20 @@ def test_fp32_normals(R):
     args = (XI, [0.07], [1.9], [-0.9], [1.0] * 3, K, 130, 500)
     p = R.price_rt(*args, seed=4, normals=R.NORMALS_F32)[0]
     close(p, R.price_rt(*args, seed=4, normals=R.NORMALS_F32, conv=R.CONV_DIRECT)[0])
+
+
+@pytest.mark.parametrize("M", [1, 255, 257, 5000])
+def test_sums_are_the_payoffs_sums(R, M):
+    """The exact merge of the chunk sums against fsum over the per-path payoffs
+    of the same normals (another path pass: 1e-12), and shards against the whole
+    (the same payoffs in other chunks: additions of up to 256 values, 1e-13)."""
+    import math
+    args = (XI, [0.07], [1.9], [-0.9], [1.0] * 3, [0.5, 1.0, 2.5], 60)
+    s1, s2 = R.price_rt_sums(*args, M, seed=6)
+    pay = R.payoffs_rt(*args[:6], R.generate_normals(6, M, 60))
+    close(s1, np.array([math.fsum(pay[:, i]) for i in range(3)]))
+    close(s2, np.array([math.fsum(pay[:, i] ** 2) for i in range(3)]))
+    if M > 1:
+        a, b = R.price_rt_sums(*args, M // 2, seed=6), R.price_rt_sums(*args, M - M // 2, seed=6, path_offset=M // 2)
+        close(a[0] + b[0], s1, 1e-13)
+        close(a[1] + b[1], s2, 1e-13)
