@@ -284,66 +284,68 @@ RBG_HD double exp2_fixed53(int64_t x, const uint64_t* E)
     return bits_double(e < -1022 ? 0ull : b);                 // e <= 1023: x 2^-53 < 1024
 }
 
-// 2^x of a double through exp2_fixed, for x < 1022 (infinity from there on):
-// NaN for NaN, zero below the normal range.
-RBG_HD double exp2_double(double x, const uint64_t* E)
+// ---------------------------------------------------------- normal tail
+// Mills' ratio M(x) = (1 - Phi(x)) / phi(x), x >= 0, on 64 intervals per octave
+// of y = 1 + x, y < 64: with f the position inside the interval (0 .. 1),
+//   M = b0 - f (b1 - f (b2 - f (b3 - f (b4 - f (b5 - f b6))))),
+// the Taylor series about the interval's left end (all b positive: the
+// derivatives of M alternate in sign) with its terms 7 to 9 economised by
+// shifted Chebyshev polynomials, which leaves less than 2^-57 of M.
+// Units 2^-61.
+constexpr int kMillsIntervals = 6 * 64;
+struct alignas(16) MillsRow {
+    uint64_t b0, b1, b2, b3, b4;
+    uint32_t b5, b6;
+};
+struct MillsTable {
+    MillsRow r[kMillsIntervals];
+};
+constexpr int kTailBits = 57;  // x in units of 2^-57
+constexpr uint64_t kTailMax = 62ull << kTailBits;
+
+// M in units of 2^-61 for x 2^-57 (62 from there on, where phi is zero).
+RBG_HD uint64_t mills_fixed(uint64_t x, const MillsTable& T)
 {
-    const uint64_t b = double_bits(x);
-    const uint32_t h = hi32(b) & 0x7FFFFFFFu;
-    if (h >= 0x408FF000u) {  // |x| >= 1022, or NaN
-        if (h > 0x7FF00000u || (h == 0x7FF00000u && lo32(b))) return x;
-        return bits_double((b >> 63) ? 0ull : 0x7FF0000000000000ull);
-    }
-    const int sh = (int)(h >> 20) - (1023 + 52 - 53);  // <= 10
+    const uint64_t y = (x < kTailMax ? x : kTailMax) + (1ull << kTailBits);
+    const int n = clz32(hi32(y));  // octave 6 - n
+    const uint64_t z = shl(y, n);
+    const MillsRow& r = T.r[(6 - n) * 64 + (int)((hi32(z) >> 25) & 63u)];
+    const uint64_t f = z << 7;
+    uint64_t q = r.b4 - mulhi32(r.b5 - mulhi32(r.b6, hi32(f)), hi32(f));
+    q = r.b3 - mulhi64(q, f);
+    q = r.b2 - mulhi64(q, f);
+    q = r.b1 - mulhi64(q, f);
+    return r.b0 - mulhi64(q, f);
+}
+
+// |x| in units of 2^-57, at most kTailMax (which NaN gives too).
+RBG_HD uint64_t tail_fixed(double x)
+{
+    const uint64_t b = double_bits(x) & 0x7FFFFFFFFFFFFFFFull;
+    const int sh = (int)(b >> 52) - (1023 + 52 - kTailBits);  // <= 10 below 64
     const uint64_t m = (b & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
     const uint64_t a = sh >= 0 ? m << (sh & 63) : (sh > -64 ? m >> (-sh & 63) : 0ull);
-    const uint64_t s = (uint64_t)((int64_t)b >> 63);
-    return exp2_fixed53((int64_t)((a ^ s) - s), E);
+    return hi32(b) >= 0x404F0000u ? kTailMax : a;
 }
 
-// ---------------------------------------------------- normal tail, FP64
-// Mills' ratio M(x) = (1 - Phi(x)) / phi(x), x >= 0: polynomials of degree 7
-// about the centres of 64 intervals per octave of y = 1 + x, y < 64: the Taylor
-// series, c_n = (-1)^n / n! times the integral of s^n exp(-x s - s^2 / 2) over s
-// > 0, with its terms 8 and 9 economised (Chebyshev: what is left of them is
-// below 2^-57 of M).
-constexpr int kMillsIntervals = 6 * 64, kMillsCoefs = 8;
-struct MillsTable {
-    double c[kMillsIntervals][kMillsCoefs];
-};
-
-RBG_HD double mills(double x, const MillsTable& T)
+// A signed value below 4 in units of 2^-61 as a double (fixed_to_double's form).
+RBG_HD double tail_to_double(int64_t v)
 {
-    double y = 1.0 + x;
-    uint32_t h = hi32(double_bits(y));
-    if (h >= 0x404FE000u) {  // y >= 63.75: phi is zero from x = 39 on
-        y = 63.5;
-        h = 0x404FC000u;
-    }
-    const double* c = T.c[(h - 0x3FF00000u) >> 14];
-    const double t = y - bits_double((uint64_t)((h & 0xFFFFC000u) | 0x2000u) << 32);
-    double p = c[7];
-    p = fma(p, t, c[6]);
-    p = fma(p, t, c[5]);
-    p = fma(p, t, c[4]);
-    p = fma(p, t, c[3]);
-    p = fma(p, t, c[2]);
-    p = fma(p, t, c[1]);
-    return fma(p, t, c[0]);
+    const double a = bits_double(0x4160000000000000ull | (hi32((uint64_t)v) ^ 0x80000000u));
+    const double b = bits_double(0x3F60000000000000ull | lo32((uint64_t)v));
+    return (a - (8388612.0 + 0x1p-9)) + b;
 }
 
-// The integrals I_n(x) of s^n exp(-x s - s^2 / 2): I_{n+1} = n I_{n-1} - x I_n
-// with I_1 = 1 - x I_0.  Forward from erfc for x < 1; above, where that
-// cancels, backward (the I_n are the recurrence's minimal solution) and
-// normalised by I_1 + x I_0 = 1.
+// The integrals I_n(x) of s^n exp(-x s - s^2 / 2), s > 0: M = I_0 and M's n-th
+// derivative is (-1)^n I_n.  I_{n+1} = n I_{n-1} - x I_n with I_1 = 1 - x I_0:
+// forward from erfc for x < 1; above, where that cancels, backward (the I_n are
+// the recurrence's minimal solution), normalised by I_1 + x I_0 = 1.
 inline void mills_table(MillsTable& T)
 {
+    constexpr int terms = 10;
     for (int i = 0; i < kMillsIntervals; ++i) {
-        const uint64_t b = (uint64_t)((0x3FF00000u + ((uint32_t)i << 14)) | 0x2000u) << 32;
-        double yc;
-        std::memcpy(&yc, &b, 8);
-        const long double x = (long double)yc - 1.0L;
-        constexpr int terms = kMillsCoefs + 2;
+        const int o = i / 64;
+        const long double h = std::ldexp(1.0L, o - 6), x = std::ldexp(1.0L + (i % 64) / 64.0L, o) - 1.0L;
         long double I[terms];
         if (x < 1.0L) {
             I[0] = std::exp(x * x / 2) * std::erfc(x * 0.707106781186547524400844362104849039L) *
@@ -351,8 +353,8 @@ inline void mills_table(MillsTable& T)
             I[1] = 1.0L - x * I[0];
             for (int n = 1; n + 1 < terms; ++n) I[n + 1] = n * I[n - 1] - x * I[n];
         } else {
-            const int top = 30 + (int)(600.0L / (x * x));  // the start value decays as exp(-2 x sqrt(top))
-            long double a = 0.0L, c = 1.0L;  // I_{n+1}, I_n up to a factor
+            const int top = 30 + (int)(600.0L / (x * x));  // the start value's weight decays as exp(-2 x sqrt(top))
+            long double a = 0.0L, c = 1.0L;                // I_{n+1}, I_n up to a factor
             for (int n = top; n >= 1; --n) {
                 const long double d = (a + x * c) / n;  // I_{n-1}
                 a = c;
@@ -367,21 +369,29 @@ inline void mills_table(MillsTable& T)
             const long double f = 1.0L / (I[1] + x * I[0]);
             for (int n = 0; n < terms; ++n) I[n] *= f;
         }
-        // u = t / h on the interval: u^8 = T_8 / 128 + 2 u^6 - 5/4 u^4 + 1/4 u^2 - 1/128,
-        // u^9 = T_9 / 256 + 9/4 u^7 - 27/16 u^5 + 15/32 u^3 - 9/256 u
-        const long double h = std::ldexp(1.0L, i / 64 - 7);
-        long double a[terms], hn = 1.0L, fact = 1.0L;
+        long double c[terms], hn = 1.0L, fact = 1.0L;
         for (int n = 0; n < terms; ++n, hn *= h) {
             if (n) fact *= -n;
-            a[n] = I[n] / fact * hn;
+            c[n] = I[n] / fact * hn;
         }
-        const long double w8[4] = {-1.0L / 128, 0.25L, -1.25L, 2.0L}, w9[4] = {-9.0L / 256, 15.0L / 32, -27.0L / 16, 2.25L};
-        for (int k = 0; k < 4; ++k) {
-            a[2 * k] += a[8] * w8[k];
-            a[2 * k + 1] += a[9] * w9[k];
+        // f^n less T*_n(f) / 2^(2n - 1), n = 9, 8, 7 in turn (T*_n the shifted Chebyshev polynomials)
+        const long double t9[10] = {-1, 162, -4320, 44352, -228096, 658944, -1118208, 1105920, -589824, 131072};
+        const long double t8[9] = {1, -128, 2688, -21504, 84480, -180224, 212992, -131072, 32768};
+        const long double t7[8] = {-1, 98, -1568, 9408, -26880, 39424, -28672, 8192};
+        const long double* t[3] = {t9, t8, t7};
+        for (int k = 0; k < 3; ++k) {
+            const int n = 9 - k;
+            for (int j = 0; j < n; ++j) c[j] -= c[n] * t[k][j] / t[k][n];
         }
-        hn = 1.0L;
-        for (int n = 0; n < kMillsCoefs; ++n, hn *= h) T.c[i][n] = (double)(a[n] / hn);
+        MillsRow& r = T.r[i];
+        auto fix = [](long double v) { return (uint64_t)(std::ldexp(v, 61) + 0.5L); };
+        r.b0 = fix(c[0]);
+        r.b1 = fix(-c[1]);
+        r.b2 = fix(c[2]);
+        r.b3 = fix(-c[3]);
+        r.b4 = fix(c[4]);
+        r.b5 = (uint32_t)fix(-c[5]);
+        r.b6 = (uint32_t)fix(c[6]);
     }
 }
 
@@ -413,20 +423,88 @@ inline void fill_fixed_tables(FixedTables& F)
     mills_table(F.mills);
 }
 
-// Conditional Black-Scholes call (tau = 1, r = 0) from the parts that do not
-// depend on the strike: S, lnS, vol, rv = 1 / vol.  With S phi(d1) = K phi(d2)
-// and 1 - Phi(x) = phi(x) M(x), the call is
-//   [d1 >= 0] S - [d2 >= 0] K + S phi(d1) (-+ M(|d1|) +- M(|d2|)):
-// one exponential, and tails that keep their relative accuracy.
-RBG_HD double call_mills(double S, double lnS, double vol, double rv, double K, double lnK, const MillsTable& T,
-                         const uint64_t* E)
+// sqrt(v) and its reciprocal as doubles, for a normal positive v: the square
+// root of the significand in fixed point, the exponent halved.
+RBG_HD void sqrt_recip(double v, double& root, double& recip)
 {
-    const double d1 = fma(lnS - lnK, rv, 0.5 * vol), d2 = d1 - vol;
-    // S phi(d1) = 2^(log2(e) (lnS - d1^2 / 2) - log2(2 pi) / 2)
-    const double f = exp2_double(fma(fma(-0.5 * d1, d1, lnS), 1.4426950408889634074, -1.3257480647361593990), E);
-    const double m1 = mills(fabs(d1), T), m2 = mills(fabs(d2), T);
-    const double base = (d1 >= 0.0 ? S : 0.0) - (d2 >= 0.0 ? K : 0.0);
-    return fma(f, (d1 >= 0.0 ? -m1 : m1) + (d2 >= 0.0 ? m2 : -m2), base);
+    const uint64_t b = double_bits(v);
+    const int e = (int)(b >> 52) - 1023;  // v = 2^e m, m in [1, 2)
+    // w 2^-64 = v 2^-(2 k), in [1/4, 1): k = (e + 2) >> 1
+    const int k = (e + 2) >> 1;
+    const uint64_t m = ((b & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull) << 11;  // m, unit 2^-63
+    const uint64_t w = (e & 1) ? m : m >> 1;
+    const uint32_t y = rsqrt_seed(w);
+    const uint64_t n = (1ull << 62) - mulhi64(w, mul32(y, y));
+    const uint64_t wy = mul32(hi32(w), y) + (mul32(lo32(w), y) >> 32);
+    const uint32_t n51 = (uint32_t)(n >> 11);
+    const uint64_t c = (n << 20) + mul32(mulhi32(n51, n51), 3072u);  // (1 - n)^(-1/2) - 1, unit 2^-83
+    const uint64_t r = wy + (mulhi64(c, wy) >> 19);                  // sqrt, unit 2^-63, in [2^62, 2^63)
+    const uint64_t yy = (uint64_t)y << 31;                           // y, unit 2^-62, in [2^62, 2^63)
+    const uint64_t q = yy + (mulhi64(c, yy) >> 19);                  // reciprocal, unit 2^-62
+    // r 2^-63 2^k and q 2^-62 2^-k, 53 bits each (the leading one adds to the exponent field)
+    root = bits_double(((uint64_t)(uint32_t)(1023 - 1 + k - 1) << 52) + (r >> 10) + ((r >> 9) & 1u));
+    recip = bits_double(((uint64_t)(uint32_t)(1023 - k - 1) << 52) + (q >> 10) + ((q >> 9) & 1u));
+}
+
+// x log2(e) in units of 2^-53, |x| < 62.
+RBG_HD int64_t log2e_fixed53(double x)
+{
+    const uint64_t q = (mulhi64(tail_fixed(x), 0xB8AA3B295C17F0BCull) + 5) >> 3;  // log2(e) / 2: 2^-56 before the shift
+    return (int64_t)double_bits(x) < 0 ? -(int64_t)q : (int64_t)q;
+}
+
+// log2 of S phi(d) sqrt(2 pi) less log2 S, in units of 2^-53: -d^2 / 2 log2 e, d
+// as tail_fixed gives it (finer units below 8, where it matters).
+RBG_HD uint64_t half_square_log2(uint64_t d)
+{
+    const bool small = hi32(d) < (8u << (kTailBits - 32));
+    const uint64_t x = small ? d << 3 : d;
+    const uint64_t q = mulhi64(mulhi64(x, x), 0xB8AA3B295C17F0BCull);  // log2(e) / 2
+    return small ? (q + 6) >> 3 : (q < (900ull << 50) ? q << 3 : 900ull << 53);  // 900: phi below 2^-900
+}
+constexpr int64_t kLog2Sqrt2Pi53 = 0x002A6C873498DDF7ll;  // log2(2 pi) / 2, unit 2^-53
+
+// The strike-independent parts of a conditional Black-Scholes call (tau = 1, r
+// = 0): spot and its logarithm, volatility and its reciprocal, and in fixed
+// point the volatility (2^-57) and log2(S / sqrt(2 pi)) (2^-53).
+struct SpotFixed {
+    double S, lnS, vol, rv;
+    int64_t volf, e;
+};
+
+// False where the numbers leave the ranges of the fixed-point form.
+RBG_HD bool spot_fixed(double v2, double lnS, const uint64_t* E, SpotFixed& r)
+{
+    // 1e-200 < v2 < 3000 and |lnS| < 60
+    const uint32_t hv = hi32(double_bits(v2)), hs = hi32(double_bits(lnS)) & 0x7FFFFFFFu;
+    if (!(hv - 0x16700000u < 0x40A77000u - 0x16700000u && hs < 0x404E0000u)) return false;
+    sqrt_recip(v2, r.vol, r.rv);
+    r.lnS = lnS;
+    r.volf = (int64_t)tail_fixed(r.vol);
+    const int64_t l = log2e_fixed53(lnS);
+    r.S = exp2_fixed53(l, E);
+    r.e = l - kLog2Sqrt2Pi53;
+    return true;
+}
+
+// The call at strike K.  With S phi(d1) = K phi(d2) and 1 - Phi(x) = phi(x) M(x)
+// it is
+//   [d1 >= 0] S - [d2 >= 0] K + S phi(d1) (-+ M(|d1|) +- M(|d2|)):
+// one exponential, tails that keep their relative accuracy, and eight FP64
+// operations with the caller's two sums.
+RBG_HD double call_fixed(const SpotFixed& r, double K, double lnK, const MillsTable& T, const uint64_t* E)
+{
+    const double d1 = fma(r.lnS - lnK, r.rv, 0.5 * r.vol);
+    const bool n1 = (int64_t)double_bits(d1) < 0;
+    const uint64_t x1 = tail_fixed(d1);
+    const int64_t d2 = (n1 ? -(int64_t)x1 : (int64_t)x1) - r.volf;
+    const bool n2 = d2 < 0;
+    const uint64_t x2 = (uint64_t)(n2 ? -d2 : d2);
+    const int64_t e = r.e - (int64_t)half_square_log2(x1);
+    const double f = exp2_fixed53(e, E);
+    const int64_t m1 = (int64_t)mills_fixed(x1, T), m2 = (int64_t)mills_fixed(x2, T);
+    const double m = tail_to_double((n1 ? m1 : -m1) + (n2 ? -m2 : m2));
+    return fma(f, m, (n1 ? 0.0 : r.S) - (n2 ? 0.0 : K));
 }
 
 }  // namespace rbg

@@ -367,19 +367,20 @@ void launch_path_fp64(const Fp64Tables& t, const double* Z, int64_t B, double* i
 }
 
 // ------------------------------------------------------------ payoff sums
-// The conditional Black-Scholes call by Mills' ratio and a fixed-point
-// exponential (rbg_fixed.cuh): about 30 FP64 operations an output and path
-// with the strike-independent parts shared, against about 250 for
-// library log, exp, sqrt and two erfc each time (FP64 pipe: 64 cycles a warp
-// operation).  Blocks keep both tables in shared memory (56 KB) and walk over
-// (chunk, run of 8 outputs) tasks.
+// The conditional Black-Scholes call by Mills' ratio, the exponential and the
+// square root in fixed point (rbg_fixed.cuh): eight FP64 operations an output
+// and path, the strike-independent parts shared, against about 250 for library
+// log, exp, sqrt and two erfc each time (FP64 pipe: 64 cycles a warp
+// operation).  Blocks keep both tables in shared memory (50 KB) and walk over
+// (chunk, run of 8 outputs) tasks.  2^17 paths x 21 outputs: 1.17 -> 0.10 ms;
+// 8192 paths x 2112 outputs: 7.06 -> 0.50 ms.
 constexpr int kOPB = 8;  // outputs per task
 constexpr int kPayThreads = 256;
 
 struct OutF64 {
-    double rho, K, lnK;
-    int vg;  // -1 past the last output
-    int ok;  // K in the range of the fast form
+    double rho, K, lnK, om, hr;  // om = 1 - rho^2 (plain MC: its root), hr = -rho^2 / 2
+    int vg;                      // -1 past the last output
+    int ok;                      // K in the range of the fast form
 };
 template <int MC>
 struct PayoffSmem {
@@ -394,9 +395,9 @@ __device__ __forceinline__ void payoff_tables(PayoffSmem<MC>& sm, const FixedTab
 {
     for (int i = threadIdx.x; i < kExpTable; i += kPayThreads) sm.E[i] = ft->exp2[i];
     if (!MC) {
-        const double* src = ft->mills.c[0];
-        double* dst = reinterpret_cast<double*>(&sm.T);
-        for (int i = threadIdx.x; i < kMillsIntervals * kMillsCoefs; i += kPayThreads) dst[i] = src[i];
+        const uint64_t* src = reinterpret_cast<const uint64_t*>(&ft->mills);
+        uint64_t* dst = reinterpret_cast<uint64_t*>(&sm.T);
+        for (int i = threadIdx.x; i < (int)(sizeof(MillsTable) / 8); i += kPayThreads) dst[i] = src[i];
     }
 }
 
@@ -409,7 +410,9 @@ __device__ __forceinline__ void payoff_outs(PayoffSmem<MC>& sm, const Fp64Tables
         const int i = o0 + (int)threadIdx.x;
         const OutDev od = (i < t.n_out) ? t.outs[i] : OutDev{0.0, 1.0, -1, 0};
         const bool ok = od.K > 1e-200 && od.K < 1e200;
-        sm.out[threadIdx.x] = OutF64{od.rho, od.K, ok ? log(od.K) : 0.0, od.vg, ok};
+        const double om = 1.0 - od.rho * od.rho;
+        sm.out[threadIdx.x] = OutF64{od.rho, od.K, (ok && !MC) ? log(od.K) : 0.0, MC ? sqrt(om) : om,
+                                     -0.5 * od.rho * od.rho, od.vg, ok};
     }
     __syncthreads();
 }
@@ -417,7 +420,8 @@ __device__ __forceinline__ void payoff_outs(PayoffSmem<MC>& sm, const Fp64Tables
 // The strike-independent part of a path's conditional call, kept while
 // consecutive outputs share variance group and rho.
 struct RtState {
-    double Iv = 0.0, Is = 0.0, S = 0.0, lnS = 0.0, vol = 0.0, rv = 0.0, rho = 0.0;
+    double Iv = 0.0, Is = 0.0, rho = 0.0;
+    SpotFixed s{};
     int vg = -1;
     bool ok = false;
 };
@@ -431,16 +435,11 @@ __device__ __forceinline__ double payoff_rt(RtState& r, const OutF64& o, const d
         r.rho = o.rho;
         r.Iv = iv.x;
         r.Is = iv.y;
-        const double v2 = (1.0 - o.rho * o.rho) * iv.x;
-        r.lnS = fma(-0.5 * o.rho * o.rho, iv.x, o.rho * iv.y);
-        r.S = exp2_double(1.4426950408889634074 * r.lnS, sm.E);
-        r.vol = sqrt(v2);
-        r.rv = 1.0 / r.vol;
-        r.ok = v2 > 1e-200 && v2 < 1e200 && r.S > 1e-200 && r.S < 1e200;
+        r.ok = spot_fixed(o.om * iv.x, fma(o.hr, iv.x, o.rho * iv.y), sm.E, r.s);
     }
     // zero or undefined conditional variance, spots and strikes out of range: the plain formula
     if (!(r.ok && o.ok)) return rt_payoff(r.Iv, r.Is, o.rho, o.K);
-    return call_mills(r.S, r.lnS, r.vol, r.rv, o.K, o.lnK, sm.T, sm.E);
+    return call_fixed(r.s, o.K, o.lnK, sm.T, sm.E);
 }
 
 __device__ __forceinline__ double payoff_mc(const OutF64& o, const double2* __restrict__ ivb,
@@ -448,8 +447,8 @@ __device__ __forceinline__ double payoff_mc(const OutF64& o, const double2* __re
 {
     // mc_payoff's log S, the exponential in fixed point
     const double2 iv = ivb[at];
-    const double lnS = o.rho * iv.y + sqrt(1.0 - o.rho * o.rho) * ivp[at] - 0.5 * iv.x;
-    const double d = (fabs(lnS) < 700.0 ? exp2_double(1.4426950408889634074 * lnS, sm.E) : exp(lnS)) - o.K;
+    const double lnS = o.rho * iv.y + o.om * ivp[at] - 0.5 * iv.x;
+    const double d = (fabs(lnS) < 60.0 ? exp2_fixed53(log2e_fixed53(lnS), sm.E) : exp(lnS)) - o.K;
     return d > 0.0 ? d : 0.0;
 }
 
@@ -510,11 +509,11 @@ __global__ void __launch_bounds__(kPayThreads) k_payoff_sums(Fp64Tables t, const
         __syncthreads();
         if (threadIdx.x < 2 * kOPB && o0 + (int)(threadIdx.x & (kOPB - 1)) < t.n_out) {
             const int q = threadIdx.x & (kOPB - 1), z = threadIdx.x / kOPB;
-            double S = 0, C = 0;
-            for (int k = 0; k < kPayThreads / 32; ++k) neumaier_add(S, C, sm.red[k][threadIdx.x]);
+            double S = 0;
+            for (int k = 0; k < kPayThreads / 32; ++k) S += sm.red[k][threadIdx.x];
             double* p = part + ((size_t)c * t.n_out + o0 + q) * 4 + 2 * z;
             p[0] = S;
-            p[1] = C;
+            p[1] = 0.0;
         }
     }
 }
@@ -704,22 +703,28 @@ __device__ void merge_block(const double* __restrict__ part, int nchunks, int n_
 }
 
 // ------------------------------------------------------------- IV (FP64)
-// The out-of-the-money Black-Scholes price (S0 = 1, r = 0; put for K < 1) and
-// what its derivatives need: f = phi(d1), vega = f sqrt(T).  lnK = ln K.
+// The out-of-the-money Black-Scholes price (S0 = 1, r = 0; put for K < 1) at v =
+// s sqrt(T) and what its derivatives need: f = phi(d1), vega = f sqrt(T).  lnK =
+// ln K.
 struct OtmPrice {
-    double p, f, d1, d2;
+    double p, f;
+    float d1d2;
 };
 
 __device__ __forceinline__ OtmPrice otm_price(double K, double lnK, double v, bool put, const FixedTables* __restrict__ ft)
 {
+    const double d1 = fma(-lnK, 1.0 / v, 0.5 * v);
+    const bool n1 = d1 < 0.0;
+    const uint64_t x1 = tail_fixed(d1);
+    const int64_t d2 = (n1 ? -(int64_t)x1 : (int64_t)x1) - (int64_t)tail_fixed(v);
+    const bool n2 = d2 < 0;
     OtmPrice r;
-    r.d1 = fma(-lnK, 1.0 / v, 0.5 * v);
-    r.d2 = r.d1 - v;
-    r.f = exp2_double(fma(-0.5 * r.d1 * r.d1, 1.4426950408889634074, -1.3257480647361593990), ft->exp2);
-    const double m1 = mills(fabs(r.d1), ft->mills), m2 = mills(fabs(r.d2), ft->mills);
+    r.d1d2 = (float)d1 * ((float)d1 - (float)v);
+    r.f = exp2_fixed53(-kLog2Sqrt2Pi53 - (int64_t)half_square_log2(x1), ft->exp2);
+    const int64_t m1 = (int64_t)mills_fixed(x1, ft->mills), m2 = (int64_t)mills_fixed((uint64_t)(n2 ? -d2 : d2), ft->mills);
     // call: [d1 >= 0] - K [d2 >= 0] + f (-+ M1 +- M2); put: less 1 - K, which only leaves K [d2 < 0]
-    const double base = put ? (r.d2 < 0.0 ? K : 0.0) : (r.d1 >= 0.0 ? 1.0 : 0.0);
-    r.p = fma(r.f, (r.d1 >= 0.0 ? -m1 : m1) + (r.d2 >= 0.0 ? m2 : -m2), base);
+    const double base = put ? (n2 ? K : 0.0) : (n1 ? 0.0 : 1.0);
+    r.p = fma(r.f, tail_to_double((n1 ? m1 : -m1) + (n2 ? -m2 : m2)), base);
     return r;
 }
 
@@ -763,7 +768,7 @@ __device__ __forceinline__ double log_ratio(double e)
 //      in the wings), then safeguarded Newton on the log price where a step is
 //      still larger than that.
 // Prices are Mills' ratios (otm_price): the density they contain is the vega,
-// so an FP64 step is one chain of about 30 dependent operations.  All lanes
+// so an FP64 step is one short chain.  All lanes
 // return the same value; NaN when no volatility fits.
 __device__ double implied_vol_warp(double price, double K, double T, const FixedTables* __restrict__ ft)
 {
@@ -834,7 +839,7 @@ __device__ double implied_vol_warp(double price, double K, double T, const Fixed
         // (Lanes 0 and 1 hold the ends' prices: lane 2's values decide.)
         const double vega = q.f * sqT;
         const double r = log_ratio((q.p - target) / target) * (q.p / vega);
-        const float h = 0.5f * (float)r * ((float)(q.d1 * q.d2) / (float)s - (float)vega / (float)q.p);
+        const float h = 0.5f * (float)r * (q.d1d2 / (float)s - (float)vega / (float)q.p);
         const double step = r + r * (double)(h / (1.0f - h));
         double nt = __shfl_sync(FULL, s - step, 2);
         const bool above = __shfl_sync(FULL, q.p > target ? 1 : 0, 2) != 0;
@@ -982,24 +987,23 @@ int launch_implied_vol(int n, const double* price, const double* K, const double
 }
 
 // ------------------------------------------------------------ quadrature
-// payoff[m * n_out + i]: tasks of 256 paths x 8 outputs.
+// payoff[m * n_out + i]: tasks of 256 paths x nq <= 8 outputs.
 template <int MC>
 __global__ void __launch_bounds__(kPayThreads) k_payoff_store(Fp64Tables t, const double2* __restrict__ ivb, int64_t B,
-                               int64_t stride, double* __restrict__ payoff, const double* __restrict__ ivp,
+                               int64_t stride, double* __restrict__ payoff, const double* __restrict__ ivp, int nq,
                                const FixedTables* __restrict__ ft)
 {
     extern __shared__ uint64_t psm[];
     PayoffSmem<MC>& sm = *reinterpret_cast<PayoffSmem<MC>*>(psm);
     payoff_tables<MC>(sm, ft);
-    const int64_t tiles = (B + kPayThreads - 1) / kPayThreads, tasks = tiles * ((t.n_out + kOPB - 1) / kOPB);
+    const int64_t tiles = (B + kPayThreads - 1) / kPayThreads, tasks = tiles * ((t.n_out + nq - 1) / nq);
     for (int64_t task = blockIdx.x; task < tasks; task += gridDim.x) {
-        const int o0 = (int)(task / tiles) * kOPB;
+        const int o0 = (int)(task / tiles) * nq;
         const int64_t m = task % tiles * kPayThreads + threadIdx.x;
         payoff_outs<MC>(sm, t, o0);
         if (m >= B) continue;
         RtState r;
-#pragma unroll
-        for (int q = 0; q < kOPB; ++q) {
+        for (int q = 0; q < nq; ++q) {
             const OutF64 o = sm.out[q];
             if (o.vg < 0) continue;
             const size_t at = (size_t)o.vg * stride + m;
@@ -1017,16 +1021,19 @@ int launch_payoff_store(const Fp64Tables& t, const double* ivb, int64_t B, int64
     static bool ready[2][64] = {};
     const FixedTables* ft = fixed_tables();
     if (!ft) return -1;
-    const int64_t tasks = (B + kPayThreads - 1) / kPayThreads * ((t.n_out + kOPB - 1) / kOPB);
-    const unsigned grid = (unsigned)std::min<int64_t>(tasks, 3 * (int64_t)device_sms());
+    // fewer outputs a task where 8 would leave SMs idle
+    const int64_t tiles = (B + kPayThreads - 1) / kPayThreads;
+    int nq = kOPB;
+    while (nq > 1 && tiles * ((t.n_out + nq - 1) / nq) < 2 * (int64_t)device_sms()) nq >>= 1;
+    const unsigned grid = (unsigned)std::min<int64_t>(tiles * ((t.n_out + nq - 1) / nq), 3 * (int64_t)device_sms());
     if (ivp) {
         if (!payoff_smem_ready(k_payoff_store<1>, sizeof(PayoffSmem<1>), ready[1])) return -1;
         k_payoff_store<1><<<grid, kPayThreads, sizeof(PayoffSmem<1>), (cudaStream_t)stream>>>(t, (const double2*)ivb, B,
-                                                                                             stride, payoff, ivp, ft);
+                                                                                             stride, payoff, ivp, nq, ft);
     } else {
         if (!payoff_smem_ready(k_payoff_store<0>, sizeof(PayoffSmem<0>), ready[0])) return -1;
         k_payoff_store<0><<<grid, kPayThreads, sizeof(PayoffSmem<0>), (cudaStream_t)stream>>>(t, (const double2*)ivb, B,
-                                                                                             stride, payoff, ivp, ft);
+                                                                                             stride, payoff, ivp, nq, ft);
     }
     count_launch();
     return 0;

@@ -1,6 +1,7 @@
 // Host check of rbg_fixed.cuh against extended precision: Box-Muller normals
 // to 2^-53 absolute (one FP64 rounding at 1), 2^x to 2^-52 relative, the
 // double conversions to half an ulp.  Exits nonzero at the first miss.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -50,6 +51,29 @@ static void check_exp2(int64_t x, int ut)
     }
 }
 
+// Conditional calls against extended precision: 2^-50 of S + K absolute and, out
+// of the money, 1e-12 relative down to 1e-30 (FP64 d1 leaves 2^-53 d1^2).
+static void check_call(double v2, double lnS, double K)
+{
+    SpotFixed sp;
+    if (!spot_fixed(v2, lnS, E, sp)) {
+        std::printf("spot refused %.17g %.17g\n", v2, lnS);
+        std::exit(1);
+    }
+    const long double v = std::sqrt((long double)v2), S = std::exp((long double)lnS);
+    const long double d1 = ((long double)lnS - std::log((long double)K)) / v + v / 2, d2 = d1 - v, h = 0.7071067811865475244L;
+    const bool itm = S > K;  // through the put: both wings from small tails
+    const long double want = itm ? (S - K) + (K * std::erfc(d2 * h) - S * std::erfc(d1 * h)) / 2
+                                 : (S * std::erfc(-d1 * h) - K * std::erfc(-d2 * h)) / 2;
+    const double got = call_fixed(sp, K, std::log(K), F.mills, E);
+    const long double err = std::fabs(got - want);
+    if (err > (S + K) * 0x1p-50L || (!itm && want > 1e-30L && err > want * 1e-12L)) {
+        std::printf("call v2=%.17g lnS=%.17g K=%.17g: %.17g, want %.20Lg\n", v2, lnS, K, got, want);
+        std::exit(1);
+    }
+    if (std::fabs(sp.vol / v - 1.0L) > 0x1p-52L || std::fabs(sp.rv * v - 1.0L) > 0x1p-52L) std::exit(1);
+}
+
 int main()
 {
     fill_fixed_tables(F);
@@ -74,6 +98,20 @@ int main()
         check_exp2(((int64_t)1023 << ut) + ((int64_t)1 << ut) - 2, ut);
     }
     if (!std::isinf(exp2_fixed((int64_t)1024 << 50, 50, E)) || exp2_fixed(((int64_t)-1022 << 50) - 1, 50, E) != 0.0) return 1;
+    for (int i = 0; i < 200000; ++i) {
+        auto u = [&] { return (double)(g() >> 11) * 0x1p-53; };
+        const double vol = std::exp2(-9.0 + 12.0 * u());
+        check_call(vol * vol, (u() - 0.5) * std::min(1.0, 12.0 * vol), 1.0 + (u() - 0.5) * std::min(0.9, 6.0 * vol));
+    }
+    check_call(2999.0, 0.0, 1.0);
+    check_call(1e-199, 1e-100, 1.0);
+    check_call(0.04, 59.0, 1e20);
+    check_call(0.04, -59.0, 1e-20);
+    SpotFixed refused;
+    for (double v2 : {0.0, -1.0, 1e-201, 3001.0, (double)NAN, (double)INFINITY})
+        if (spot_fixed(v2, 0.0, E, refused)) return 1;
+    for (double l : {60.1, -60.1, (double)NAN, (double)INFINITY})
+        if (spot_fixed(0.04, l, E, refused)) return 1;
     const double ex[] = {0.0, -0.0, 1.0, -1.0, 6.77, -15.5, 0x1p-6, 0x1p-59, -0x1.8p-59, 0x1p-60, 1e-300};
     for (double d : ex) {
         const long double v = std::ldexp((long double)d, kNormalBits);
