@@ -141,6 +141,31 @@ struct DevBuf {
     T* as() const { return (T*)p; }
 };
 
+// Grow-only pinned host buffer (results read back after a call's one wait).
+struct PinBuf {
+    void* p = nullptr;
+    size_t n = 0;
+    int ensure(size_t bytes)
+    {
+        if (bytes <= n) return 0;
+        release();
+        const size_t want = std::max(bytes, (size_t)4096);
+        if (cudaMallocHost(&p, want) != cudaSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+            return -1;
+        }
+        n = want;
+        return 0;
+    }
+    void release()
+    {
+        if (p) cudaFreeHost(p);
+        p = nullptr;
+        n = 0;
+    }
+};
+
 // Device views of the FP64 tables of one call (pointers into Ctx::tabs).
 struct TableSet {
     Fp64Tables t{};
@@ -157,6 +182,7 @@ struct Ctx {
     DevBuf z, ivb, ivp, part, acc, tabs, res, pay, mixed_ws, cv, sobol, sobol32;
     // fixed-point FP64 path pass: digits of W1, X, and the Toeplitz panels of the tables in `tabs`
     DevBuf xdig, xbuf, xpan;
+    PinBuf pin;
     bool xpan_ready = false;
     // host images of what `tabs`, `mixed_ws` and `sobol` hold, so that a call
     // with the same tables (a calibration loop, a benchmark) uploads nothing
@@ -247,8 +273,10 @@ static int fp64_conv_log2(int conv, int N, int* logL)
 // logL > 0: also the FP64 FFT convolution's spectra (one per distinct H) and
 // twiddles; xt: also the fixed-point path pass's tables, and its Toeplitz
 // panels (built on the device, kept with the tables)
+// fp64: the FP64 path kernels' Gamma and compensators too (the other path
+// passes bring their own).
 static int upload_tables(Ctx& c, const Plan& plan, cudaStream_t st, TableSet& ts, int logL = 0,
-                         const X64Tables* xt = nullptr)
+                         const X64Tables* xt = nullptr, bool fp64 = true)
 {
     const int nv = (int)plan.vols.size(), ng = (int)plan.vgs.size(), no = (int)plan.outs.size(), N = plan.N;
     std::vector<VolDev> vols(nv);
@@ -269,9 +297,9 @@ static int upload_tables(Ctx& c, const Plan& plan, cudaStream_t st, TableSet& ts
     size_t off_outs = align_up(off_vgs + sizeof(VGDev) * ng, 256);
     size_t off_T = align_up(off_outs + sizeof(OutDev) * no, 256);
     size_t off_gamma = align_up(off_T + sizeof(double) * no, 256);
-    size_t off_comp = align_up(off_gamma + sizeof(double) * plan.gamma.size(), 256);
+    size_t off_comp = align_up(off_gamma + (fp64 ? sizeof(double) * plan.gamma.size() : 0), 256);
     const size_t L = logL > 0 ? (size_t)1 << logL : 0;
-    size_t off_spec = align_up(off_comp + sizeof(double) * plan.comp.size(), 256);
+    size_t off_spec = align_up(off_comp + (fp64 ? sizeof(double) * plan.comp.size() : 0), 256);
     size_t off_tw = align_up(off_spec + 2 * sizeof(double) * L * nv, 256);
     size_t off_xvols = align_up(off_tw + 2 * sizeof(double) * L, 256);
     size_t off_xgrps = align_up(off_xvols + (xt ? sizeof(X64Vol) * nv : 0), 256);
@@ -292,8 +320,10 @@ static int upload_tables(Ctx& c, const Plan& plan, cudaStream_t st, TableSet& ts
     std::memcpy(host.data() + off_vgs, vgs.data(), sizeof(VGDev) * ng);
     std::memcpy(host.data() + off_outs, outs.data(), sizeof(OutDev) * no);
     std::memcpy(host.data() + off_T, Tv.data(), sizeof(double) * no);
-    std::memcpy(host.data() + off_gamma, plan.gamma.data(), sizeof(double) * plan.gamma.size());
-    std::memcpy(host.data() + off_comp, plan.comp.data(), sizeof(double) * plan.comp.size());
+    if (fp64) {
+        std::memcpy(host.data() + off_gamma, plan.gamma.data(), sizeof(double) * plan.gamma.size());
+        std::memcpy(host.data() + off_comp, plan.comp.data(), sizeof(double) * plan.comp.size());
+    }
     if (!(c.tabs.p && c.tabs_img == host)) {
         c.tabs_img.clear();
         c.xpan_ready = false;
@@ -309,8 +339,8 @@ static int upload_tables(Ctx& c, const Plan& plan, cudaStream_t st, TableSet& ts
     ts.t.vols = (const VolDev*)(base + off_vols);
     ts.t.vgs = (const VGDev*)(base + off_vgs);
     ts.t.outs = (const OutDev*)(base + off_outs);
-    ts.t.gamma = (const double*)(base + off_gamma);
-    ts.t.comp = (const double*)(base + off_comp);
+    ts.t.gamma = fp64 ? (const double*)(base + off_gamma) : nullptr;
+    ts.t.comp = fp64 ? (const double*)(base + off_comp) : nullptr;
     ts.t.spec = logL > 0 ? (const double2*)(base + off_spec) : nullptr;
     ts.t.tw = logL > 0 ? (const double2*)(base + off_tw) : nullptr;
     ts.t.logL = logL;
@@ -383,6 +413,28 @@ static int64_t fp64_batch(const Plan& plan, int64_t M, int ns = 2)
     return std::min(B, M);
 }
 
+// The call's results (5 n_out doubles at c.res) and its kernel error word (err,
+// or null) through pinned memory, with one wait; `what` names the kernels whose
+// bounded waits the word reports.
+static int read_back(Ctx& c, int no, const unsigned int* err, const char* what, cudaStream_t st, double* host_res)
+{
+    const size_t bytes = sizeof(double) * 5 * (size_t)no;
+    if (c.pin.ensure(bytes + sizeof(double))) return fail(RBG_ERR_NOMEM, "pinned result buffer");
+    unsigned int* word = (unsigned int*)c.pin.p;
+    double* res = (double*)c.pin.p + 1;
+    *word = 0;
+    if (err) RBG_CUDA(cudaMemcpyAsync(word, err, sizeof *word, cudaMemcpyDeviceToHost, st));
+    RBG_CUDA(cudaMemcpyAsync(res, c.res.p, bytes, cudaMemcpyDeviceToHost, st));
+    RBG_CUDA(cudaStreamSynchronize(st));
+    if (*word)
+        return fail(RBG_ERR_TIMEOUT,
+                    std::string(what) + ": a bounded pipeline wait expired (site " + std::to_string(*word) + ")");
+    std::memcpy(host_res, res, bytes);
+    g_d2h += bytes + (err ? sizeof *word : 0);
+    prof_collect();
+    return RBG_OK;
+}
+
 // mc: the plain Monte Carlo estimator (third normal stream Wperp, payoff
 // max(S_T - K, 0)) instead of the Romano-Touzi conditional price.
 // sobol_vt: Sobol' quasi-Monte Carlo normals (device direction table
@@ -400,7 +452,7 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
     const bool fixed = o.conv == RBG_CONV_AUTO && !sobol_vt && x64_prepare(plan, xt);
     int rc = fixed ? RBG_OK : fp64_conv_log2(o.conv, plan.N, &logL);
     if (rc) return rc;
-    if ((rc = upload_tables(c, plan, st, ts, logL, fixed ? &xt : nullptr))) return rc;
+    if ((rc = upload_tables(c, plan, st, ts, logL, fixed ? &xt : nullptr, !fixed))) return rc;
     const int no = (int)plan.outs.size(), N = plan.N, ns = mc ? 3 : 2, nv = (int)plan.vols.size();
     const int64_t B = fp64_batch(plan, M, ns);
     // passes per convolution launch: X within 2 GiB
@@ -461,15 +513,7 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
         }
         RBG_CUDA(cudaGetLastError());
     }
-    RBG_CUDA(cudaMemcpyAsync(host_res, c.res.p, sizeof(double) * 5 * no, cudaMemcpyDeviceToHost, st));
-    unsigned int word = 0;
-    if (fixed) RBG_CUDA(cudaMemcpyAsync(&word, err, 4, cudaMemcpyDeviceToHost, st));
-    RBG_CUDA(cudaStreamSynchronize(st));
-    if (word)
-        return fail(RBG_ERR_TIMEOUT, "FP64 convolution: a bounded pipeline wait expired (site " + std::to_string(word) + ")");
-    g_d2h += sizeof(double) * 5 * no + (fixed ? 4 : 0);
-    prof_collect();
-    return RBG_OK;
+    return read_back(c, no, fixed ? err : nullptr, "FP64 convolution", st, host_res);
 }
 
 // Sobol' normals materialized per batch on the device and read by the mixed
@@ -488,7 +532,7 @@ struct SobolZ {
 static int mixed_setup(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M, cudaStream_t st, bool mc,
                        const unsigned int* sob, const SobolZ* sz, TableSet& ts, MixedJob& job)
 {
-    int rc = upload_tables(c, plan, st, ts);
+    int rc = upload_tables(c, plan, st, ts, 0, nullptr, false);
     if (rc) return rc;
     const int no = (int)plan.outs.size();
     // materialized normals: 2 N doubles per path, at most 2 GiB per batch
@@ -574,17 +618,10 @@ static int mixed_run(Ctx& c, const Plan& plan, const TableSet& ts, const MixedJo
         }
         RBG_CUDA(cudaGetLastError());
     }
-    // one wait for the whole call: the kernel error word is read after the
-    // finalize kernel is queued (finalizing the sums of a launch that gave up
-    // is harmless; its results are discarded), so no host round trip sits
-    // between the path kernels and the finalize
-    if ((rc = mixed_check(job, c.mixed_ws.p, st, g_err))) return rc;
-    g_d2h += 4;
-    RBG_CUDA(cudaMemcpyAsync(host_res, c.res.p, sizeof(double) * 5 * no, cudaMemcpyDeviceToHost, st));
-    RBG_CUDA(cudaStreamSynchronize(st));
-    g_d2h += sizeof(double) * 5 * no;
-    prof_collect();
-    return RBG_OK;
+    // one wait for the whole call: the kernel error word is read with the results
+    // (finalizing the sums of a launch that gave up is harmless; its results are
+    // discarded)
+    return read_back(c, no, (const unsigned int*)((unsigned char*)c.mixed_ws.p + job.off_err), "mixed kernel", st, host_res);
 }
 
 // Mixed form: tcgen05 fused path kernel writes FP32 (Ivdt, IsvdW) per
@@ -934,7 +971,7 @@ static int payoffs_quadrature_mixed(const rbg_params* p, const rbg_options& o, c
     std::lock_guard<std::mutex> lk(c->mu);
     cudaStream_t st = o.stream ? (cudaStream_t)o.stream : c->stream;
     TableSet ts;
-    if ((rc = upload_tables(*c, plan, st, ts))) return rc;
+    if ((rc = upload_tables(*c, plan, st, ts, 0, nullptr, false))) return rc;
     const int no = (int)plan.outs.size(), N = plan.N, ns = mc ? 3 : 2;
     const int64_t M = p->M;
     MixedJob job;
@@ -1342,6 +1379,7 @@ int rbg_release(void)
         for (DevBuf* b : {&c->z, &c->ivb, &c->ivp, &c->part, &c->acc, &c->tabs, &c->res, &c->pay, &c->mixed_ws,
                           &c->cv, &c->sobol, &c->sobol32, &c->xdig, &c->xbuf, &c->xpan})
             b->release();
+        c->pin.release();
         c->xpan_ready = false;
         c->tabs_img.clear();
         c->mixed_img.clear();

@@ -740,6 +740,7 @@ bool x64_prepare(const Plan& plan, X64Tables& out)
     out.gam.assign((size_t)nv * N, 0);
     out.comp.assign((size_t)ng * N, 0);
     std::vector<int> ux(nv);
+    std::vector<double> xbound(nv);  // |X + a2 W1perp| at most
     const double wmax = 6.9;  // |Box-Muller on 32-bit uniforms| <= sqrt(66 ln 2) = 6.77
     for (int v = 0; v < nv; ++v) {
         const VolGroup& V = plan.vols[v];
@@ -751,6 +752,7 @@ bool x64_prepare(const Plan& plan, X64Tables& out)
         }
         const double bound = wmax * (gsum + std::fabs(V.a2));
         if (!(gmax > 0.0) || !std::isfinite(bound) || !(V.a2 >= 0.0)) return false;
+        xbound[v] = bound;
         int e = 0, cb = 0;
         while (std::ldexp(1.0, e) < gmax) ++e;
         while (std::ldexp(1.0, cb) < bound) ++cb;
@@ -768,25 +770,25 @@ bool x64_prepare(const Plan& plan, X64Tables& out)
         out.vols[v].a2h = (a2f >> 1) - 1;  // the bias's share, and the product's mean truncation
         // unit 2^(e - 62): |gam| <= 2^62
         int64_t* q = out.gam.data() + (size_t)v * N;
-        q[0] = (int64_t)std::llrint(std::ldexp(V.a1, 62 - e));
-        for (int d = 1; d < N; ++d) q[d] = (int64_t)std::llrint(std::ldexp(G[d], 62 - e));
+        const double unit = std::ldexp(1.0, 62 - e);
+        q[0] = (int64_t)(V.a1 * unit);  // whole units from 2^(e - 10) up, truncated below
+        for (int d = 1; d < N; ++d) q[d] = (int64_t)(G[d] * unit);
         out.max_groups = std::max(out.max_groups, V.vg_end - V.vg_begin);
     }
     const double l2 = 1.4426950408889634074, l2lo = 2.0355273740931033e-17;  // log2 e
     for (int g = 0; g < ng; ++g) {
         const VGroup& G = plan.vgs[g];
-        const VolGroup& V = plan.vols[G.vol];
         const double* c = plan.comp.data() + (size_t)g * N;
         const double C = 0.5 * G.eta * G.scale * l2, Ca = std::fabs(C);
-        double gsum = std::fabs(V.a1) + std::fabs(V.a2), cmax = 0.0;
-        for (int d = 1; d < N; ++d) gsum += std::fabs(plan.gamma[(size_t)G.vol * N + d]);
+        double cmax = 0.0;
+        bool finite = true;
         for (int j = 0; j + 1 < N; ++j) {
-            if (!std::isfinite(c[j])) return false;
+            finite = finite && std::fabs(c[j]) <= 1e300;
             cmax = std::max(cmax, std::fabs(c[j]));
         }
         // t in units of 2^-ut: |t| < 2^(62 - ut), C 2^(ut - ux) < 1 for its factor
-        const double bound = Ca * wmax * gsum + 0.5 * l2 * cmax + 1.0;
-        if (!std::isfinite(bound)) return false;
+        const double bound = Ca * xbound[G.vol] + 0.5 * l2 * cmax + 1.0;
+        if (!finite || !std::isfinite(bound)) return false;
         int ut = 53;
         while (ut > 0 && (std::ldexp(bound, ut) >= std::ldexp(1.0, 62) || std::ldexp(Ca, ut - ux[G.vol]) >= 1.0)) --ut;
         if (ut < kX64MinUt) return false;
@@ -798,10 +800,12 @@ bool x64_prepare(const Plan& plan, X64Tables& out)
         o.dtxi = G.dt * G.xi;
         o.sdtxi = G.sdt * std::sqrt(G.xi);
         uint64_t* q = out.comp.data() + (size_t)g * N;
+        const double unit = std::ldexp(1.0, ut);
+        const uint64_t bias = (o.cf >> 1) - 1;
         for (int j = 0; j + 1 < N; ++j) {
             // comp / 2 log2 e in two parts, so the fixed-point value is rounded once
-            const double hc = 0.5 * c[j], p = hc * l2, lo = std::fma(hc, l2, -p) + hc * l2lo;
-            q[j] = (uint64_t)((int64_t)std::ldexp(p, ut) + (int64_t)std::llrint(std::ldexp(lo, ut))) + (o.cf >> 1) - 1;
+            const double hc = 0.5 * c[j], p = hc * l2, lo = (std::fma(hc, l2, -p) + hc * l2lo) * unit;
+            q[j] = (uint64_t)((int64_t)(p * unit) + (int64_t)(lo + (lo < 0.0 ? -0.5 : 0.5))) + bias;
         }
     }
     return true;

@@ -38,7 +38,12 @@ void gamma_table(double H, int N, double* G)
 {
     double alpha = H - 0.5;
     G[0] = 0.0;
-    for (int i = 1; i < N; ++i) G[i] = (std::pow(i + 1.0, alpha + 1.0) - std::pow(i, alpha + 1.0)) / (alpha + 1.0);
+    double below = 1.0;  // i^(alpha + 1)
+    for (int i = 1; i < N; ++i) {
+        const double above = std::pow(i + 1.0, alpha + 1.0);
+        G[i] = (above - below) / (alpha + 1.0);
+        below = above;
+    }
 }
 // One Volterra pass for H (rBergLib/rBergomiMT.cpp:83-109).
 VolGroup make_vol(double H, int N)
@@ -95,13 +100,21 @@ void fill_tables(Plan& plan)
     plan.gamma.assign((size_t)plan.vols.size() * N, 0.0);
     for (size_t v = 0; v < plan.vols.size(); ++v) gamma_table(plan.vols[v].H, N, plan.gamma.data() + v * N);
     plan.comp.assign((size_t)plan.vgs.size() * N, 0.0);
+    // updateV's compensator, evaluated as the reference writes it:
+    // 0.5 * eta * eta * pow((i - 1 + comp_shift) * dt, 2 * H) with j = i - 1.  Groups
+    // that differ in eta alone share the powers (of 16 groups a pass on a grid of
+    // four maturities and four etas, four take them).
+    std::map<std::pair<double, double>, std::vector<double>> powers;
     for (size_t g = 0; g < plan.vgs.size(); ++g) {
         const VGroup& G = plan.vgs[g];
         double* c = plan.comp.data() + g * N;
-        // updateV's compensator, evaluated as the reference writes it:
-        // 0.5 * eta * eta * pow((i - 1 + comp_shift) * dt, 2 * H) with j = i - 1
-        for (int j = 0; j + 1 < N; ++j)
-            c[j] = 0.5 * G.eta * G.eta * std::pow((j + plan.comp_shift) * G.dt, 2 * G.Hv);
+        std::vector<double>& w = powers[{G.dt, G.Hv}];
+        if (w.empty() && N > 1) {
+            w.resize(N - 1);
+            for (int j = 0; j + 1 < N; ++j) w[j] = std::pow((j + plan.comp_shift) * G.dt, 2 * G.Hv);
+        }
+        const double k = 0.5 * G.eta * G.eta;
+        for (int j = 0; j + 1 < N; ++j) c[j] = k * w[j];
     }
 }
 }  // namespace
