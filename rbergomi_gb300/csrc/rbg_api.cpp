@@ -493,9 +493,9 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
                 const int k = std::min(vstep, nv - v0);
                 if (launch_volterra_exact(c.xdig.as<unsigned char>(),
                                           c.xpan.as<unsigned char>() + (size_t)v0 * x64_panel_bytes(N), ts.xvols + v0, k, N,
-                                          b, c.xbuf.as<uint64_t>(), err, st) ||
+                                          b, false, c.xbuf.as<uint64_t>(), err, st) ||
                     launch_variance_fixed(ts.xvols + v0, ts.xgrps, ts.xcomp, c.z.as<double>(), c.xbuf.as<uint64_t>(), k,
-                                          xt.max_groups, xt.u53, ns, N, b, c.ivb.as<double>(), ivp, st))
+                                          xt.max_groups, xt.u53, false, ns, N, b, c.ivb.as<double>(), ivp, st))
                     return fail(RBG_ERR_CUDA, "FP64 path kernels could not be configured");
             }
         }
@@ -917,20 +917,33 @@ static int payoffs_quadrature(const rbg_params* p, const double* Z, double* payo
     cudaStream_t st = user_stream ? user_stream : c->stream;
     TableSet ts;
     int logL = 0;
-    if ((rc = fp64_conv_log2(conv, plan.N, &logL))) return rc;
-    if ((rc = upload_tables(*c, plan, st, ts, logL))) return rc;
-    const int no = (int)plan.outs.size(), N = plan.N, ns = mc ? 3 : 2;
+    // no backend asked for: the exact tensor-core convolution and fixed-point
+    // functions; a batch with normals outside their range takes the direct FP64 sum
+    X64Tables xt;
+    const bool fixed = conv == RBG_CONV_AUTO && x64_prepare(plan, xt, true);
+    if (!fixed && (rc = fp64_conv_log2(conv, plan.N, &logL))) return rc;
+    if ((rc = upload_tables(*c, plan, st, ts, logL, fixed ? &xt : nullptr))) return rc;
+    const int no = (int)plan.outs.size(), N = plan.N, ns = mc ? 3 : 2, nv = (int)plan.vols.size();
     const int64_t M = p->M;
     int64_t B = fp64_batch(plan, M, ns);
     // payoffs of a batch within 1 GiB too
     B = std::min<int64_t>(B, std::max<int64_t>(256, ((int64_t)1 << 30) / (8 * (int64_t)no)));
+    const int vstep = (int)std::max<int64_t>(1, std::min<int64_t>(nv, ((int64_t)1 << 31) / (8 * (int64_t)N * B)));
     if ((rc = ensure(c->ivb, sizeof(double) * 2 * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
     if (mc && (rc = ensure(c->ivp, sizeof(double) * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
     double* ivp = mc ? c->ivp.as<double>() : nullptr;
+    if (fixed) {
+        if ((rc = ensure(c->xdig, x64_digit_bytes(B, N), "normal digits"))) return rc;
+        if ((rc = ensure(c->xbuf, 8 * (size_t)vstep * N * (size_t)B, "Volterra paths"))) return rc;
+    }
     if (!device_ptrs) {
         if ((rc = ensure(c->z, sizeof(double) * ns * N * (size_t)B, "normals"))) return rc;
         if ((rc = ensure(c->pay, sizeof(double) * no * (size_t)B, "payoffs"))) return rc;
     }
+    // device words: kernel error, normals out of range
+    if ((rc = ensure(c->acc, 2 * sizeof(unsigned int), "accumulators"))) return rc;
+    unsigned int* words = c->acc.as<unsigned int>();
+    if (fixed) RBG_CUDA(cudaMemsetAsync(words, 0, 2 * sizeof(unsigned int), st));
     for (int64_t m0 = 0; m0 < M; m0 += B) {
         const int64_t b = std::min(B, M - m0);
         const double* Zd;
@@ -944,14 +957,34 @@ static int payoffs_quadrature(const rbg_params* p, const double* Z, double* payo
             Zd = c->z.as<double>();
             Pd = c->pay.as<double>();
         }
-        launch_path_fp64(ts.t, Zd, b, c->ivb.as<double>(), st, ivp);
+        if (fixed) {
+            if (m0) RBG_CUDA(cudaMemsetAsync(words + 1, 0, sizeof(unsigned int), st));
+            launch_digits(Zd, b, N, ns, c->xdig.as<unsigned char>(), words + 1, st);
+            for (int v0 = 0; v0 < nv; v0 += vstep) {
+                const int k = std::min(vstep, nv - v0);
+                if (launch_volterra_exact(c->xdig.as<unsigned char>(),
+                                          c->xpan.as<unsigned char>() + (size_t)v0 * x64_panel_bytes(N), ts.xvols + v0, k, N,
+                                          b, true, c->xbuf.as<uint64_t>(), words, st) ||
+                    launch_variance_fixed(ts.xvols + v0, ts.xgrps, ts.xcomp, Zd, c->xbuf.as<uint64_t>(), k, xt.max_groups,
+                                          xt.u53, true, ns, N, b, c->ivb.as<double>(), ivp, st))
+                    return fail(RBG_ERR_CUDA, "FP64 path kernels could not be configured");
+            }
+        }
+        launch_path_fp64(ts.t, Zd, b, c->ivb.as<double>(), st, ivp, nullptr, fixed ? words + 1 : nullptr);
         if (launch_payoff_store(ts.t, c->ivb.as<double>(), b, b, Pd, st, ivp))
             return fail(RBG_ERR_CUDA, "FP64 payoff kernel could not be configured");
         RBG_CUDA(cudaGetLastError());
         if (!device_ptrs)
             RBG_CUDA(cudaMemcpyAsync(payoff + m0 * no, Pd, sizeof(double) * no * b, cudaMemcpyDeviceToHost, st));
     }
+    if (fixed) {
+        if (c->pin.ensure(sizeof(unsigned int))) return fail(RBG_ERR_NOMEM, "pinned result buffer");
+        RBG_CUDA(cudaMemcpyAsync(c->pin.p, words, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
+    }
     RBG_CUDA(cudaStreamSynchronize(st));
+    if (fixed && *(unsigned int*)c->pin.p)
+        return fail(RBG_ERR_TIMEOUT, "FP64 convolution: a bounded pipeline wait expired (site " +
+                                         std::to_string(*(unsigned int*)c->pin.p) + ")");
     return RBG_OK;
 }
 

@@ -30,6 +30,7 @@
 #include <cmath>
 #include <cstring>
 #include <mutex>
+#include <set>
 
 #include "rbg_device.cuh"
 #include "rbg_fixed.cuh"
@@ -210,6 +211,58 @@ int launch_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int f32
     return 0;
 }
 
+// Digits of the caller's W1 (Z[m][s][j] as k_normals_fixed's), zero past N and
+// past B.  W1 and W1perp below kExtMax in size, which finite normals are, fit the
+// fixed-point ranges; *flag is set where one is not (or is NaN), and the FP64
+// path kernels take the batch.
+__global__ void __launch_bounds__(kNormalThreads) k_digits(const double* __restrict__ Z, int64_t B, int N, int ns,
+                                                          unsigned char* __restrict__ dig, unsigned int* __restrict__ flag)
+{
+    const int lane = threadIdx.x & 31, g = lane & 3, pl = lane >> 2;
+    const int nch = (N + kXSteps - 1) / kXSteps, segs = (nch + kSeg - 1) / kSeg;
+    const int64_t tasks = (B + kXPaths - 1) / kXPaths * (kXPaths / 8) * segs;
+    const int64_t warps = (int64_t)gridDim.x * (kNormalThreads / 32);
+    bool bad = false;
+    for (int64_t t = blockIdx.x * (int64_t)(kNormalThreads / 32) + (threadIdx.x >> 5); t < tasks; t += warps) {
+        const int64_t r = t / segs, m = r * 8 + pl;
+        const int c0 = (int)(t - r * segs) * kSeg, c1 = min(nch, c0 + kSeg);
+        const double* z0 = Z + m * ns * (int64_t)N;
+        const int p = (int)(m & (kXPaths - 1));
+        unsigned char* drow = dig + (m / kXPaths) * nch * kXChunkBytes + p * 32 + ((((g >> 1) ^ (p >> 2)) & 1) << 4) +
+                              ((g & 1) << 3);
+        for (int c = c0; c < c1; ++c) {
+            const int j0 = kXSteps * c + 4 * g;
+            double z[4] = {0.0, 0.0, 0.0, 0.0}, w[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (m < B && j0 + q < N) {
+                    z[q] = z0[j0 + q];
+                    w[q] = z0[N + j0 + q];
+                }
+            }
+            int64_t v[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                // a double's size as the integer of its bits; NaN compares above every number
+                constexpr uint64_t lim = 0x402F000000000000ull;  // kExtMax
+                bad |= (double_bits(z[q]) & ~(1ull << 63)) >= lim || (double_bits(w[q]) & ~(1ull << 63)) >= lim;
+                v[q] = double_to_fixed(z[q]);
+            }
+            store_digits(v, drow + (size_t)c * kXChunkBytes);
+        }
+    }
+    if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(flag, 1u);
+}
+
+void launch_digits(const double* Z, int64_t B, int N, int ns, unsigned char* dig, unsigned int* flag, cudaStream_t st)
+{
+    const int nch = (N + kXSteps - 1) / kXSteps;
+    const int64_t tasks = (B + kXPaths - 1) / kXPaths * (kXPaths / 8) * ((nch + kSeg - 1) / kSeg);
+    const int64_t need = (tasks + kNormalThreads / 32 - 1) / (kNormalThreads / 32);
+    k_digits<<<(unsigned)std::min<int64_t>(need, 8 * (int64_t)device_sms()), kNormalThreads, 0, st>>>(Z, B, N, ns, dig, flag);
+    count_launch();
+}
+
 // ------------------------------------------------------------- convolution
 // D[step][path] per diagonal d: the Toeplitz operand is MMA's A (128 output
 // steps), the W1 digits its B, eight digits x 64 paths = 512 rows of a chunk,
@@ -230,6 +283,8 @@ constexpr int kXChunks = kXBlock / kXSteps;            // 8 chunks per block of 
 constexpr int kXStages = 5;
 constexpr int kXEpiWarps = 16;
 constexpr int kXThreads = (kXEpiWarps + 2) * 32;
+// SEG: steps a sum takes where the digits may be anything: 8 digit pairs x 128 x 2^14 = 2^24
+constexpr int kAnyChunks = 128 / kXSteps;
 constexpr int kXSmem = 2 * kPanelBytes + kXStages * kXChunkBytes + 256 + 1024;
 
 int x64_blocks(int N) { return (N + kXBlock - 1) / kXBlock; }
@@ -309,14 +364,16 @@ struct PanelSlots {
 // One (block b, pass v, group of 64 paths) at a time, the longest blocks
 // first.  Warps 0-15 read the accumulators, warp 16 loads, warp 17 issues the
 // MMAs.  WIDE: accumulators may pass 2^22 (N > 1024): converted by F2I, else by
-// adding 1.5 2^23.
+// adding 1.5 2^23.  SEG: the caller's normals, whose digits may add up: the
+// accumulators are read out every 128 steps and X summed in integers, which is
+// exact for any digits.
 // What bounds it: 2304 columns x 128 steps x 16 per chunk, 1152 MMA cycles,
 // against 16 KB of digits and 7.5 KB of panel from L2; the accumulators fill
 // TMEM, so the next block's MMAs wait for the read-out of this one's.
 // With k_variance_fixed: 512 steps, 2^17 paths, one pass 1.99 ms, against 13.2
 // ms for the FP64 FFT convolution and exponentials; 100 steps, 2^16 paths 0.23
 // ms, against 1.46 ms for the direct FP64 sum.
-template <bool WIDE>
+template <bool WIDE, bool SEG>
 __global__ void __launch_bounds__(kXThreads, 1) k_volterra_exact(const unsigned char* __restrict__ dig,
                                                                  const unsigned char* __restrict__ panels,
                                                                  const X64Vol* __restrict__ vols, int nv, int N,
@@ -422,17 +479,22 @@ __global__ void __launch_bounds__(kXThreads, 1) k_volterra_exact(const unsigned 
             int loads[2] = {0, 0};
             int s = 0;
             uint32_t ph = 0;
-            int64_t done_units = 0;
+            int64_t drains = 0;  // accumulator read-outs asked for
             bool ok = true;
             const uint64_t a_base = sdesc_sw32(smem_u32(base)), b_base = sdesc_sw32(smem_u32(stage));
             const uint32_t a_lo = (uint32_t)a_base, a_hi = (uint32_t)(a_base >> 32);
             const uint32_t b_lo = (uint32_t)b_base, b_hi = (uint32_t)(b_base >> 32);
-            for (int64_t u = blockIdx.x; u < units && ok; u += gridDim.x, ++done_units) {
+            for (int64_t u = blockIdx.x; u < units && ok; u += gridDim.x) {
                 const int b = nb - 1 - (int)(u / per), v = (int)(u % per / groups);
                 const int ke = min(kXChunks * (b + 1), nch);
-                if (done_units > 0 && !mbar_wait(smem_u32(acce), (uint32_t)((done_units - 1) & 1), err, 23)) break;
-                int pb = 0;
+                int pb = 0, sc = 0;  // SEG: chunks of the current sum so far
+                // (kept out of the chunk loop where a unit is one sum: inside it they cost the convolution 10 %)
+                if (!SEG && drains > 0 && !mbar_wait(smem_u32(acce), (uint32_t)((drains - 1) & 1), err, 23)) break;
                 for (int kc = 0; kc < ke; ++kc, s = (s + 1 == kXStages) ? 0 : s + 1, ph ^= (s == 0)) {
+                    if (SEG && sc == 0 && drains > 0 && !mbar_wait(smem_u32(acce), (uint32_t)((drains - 1) & 1), err, 23)) {
+                        ok = false;
+                        break;
+                    }
                     if (kc % kXChunks == 0) {
                         bool load;
                         pb = ps.use(v * nb + b - kc / kXChunks, load);
@@ -450,15 +512,23 @@ __global__ void __launch_bounds__(kXThreads, 1) k_volterra_exact(const unsigned 
                     for (int j = 0; j < kXDigits; ++j) {
                         const uint64_t da = ((uint64_t)a_hi << 32) | (arow + (uint32_t)(j * kPanelDigit) / 16);
                         const int n = kXPaths * (kXDigits - j), n1 = n < 256 ? n : 256;
-                        const uint32_t acc = (kc == 0 && j == 0) ? 0u : 1u;
+                        const uint32_t acc = ((SEG ? sc : kc) == 0 && j == 0) ? 0u : 1u;
                         umma_f16(tmem + kXPaths * j, da, ((uint64_t)b_hi << 32) | brow, idesc_f16(n1, 0), acc);
                         if (n > 256)
                             umma_f16(tmem + kXPaths * j + 256, da, ((uint64_t)b_hi << 32) | (brow + 256 * 32 / 16),
                                      idesc_f16(n - 256, 0), acc);
                     }
                     umma_commit(smem_u32(wempty + s));
+                    if (SEG && (++sc == kAnyChunks || kc == ke - 1)) {
+                        umma_commit(smem_u32(accf));
+                        ++drains;
+                        sc = 0;
+                    }
                 }
-                if (ok) umma_commit(smem_u32(accf));
+                if (!SEG) {
+                    if (ok) umma_commit(smem_u32(accf));
+                    ++drains;
+                }
             }
             // every issued MMA completes before TMEM is released
             umma_commit(smem_u32(fin));
@@ -468,14 +538,16 @@ __global__ void __launch_bounds__(kXThreads, 1) k_volterra_exact(const unsigned 
         // -------------------------------------------------------- read-out
         const int quad = warp & 3, wg = warp >> 2;
         const uint32_t tl = tmem + ((uint32_t)(quad * 32) << 16);
-        int64_t n_units = 0;
-        for (int64_t u = blockIdx.x; u < units; u += gridDim.x, ++n_units) {
+        int64_t drains = 0;
+        for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {
             const int b = nb - 1 - (int)(u / per), v = (int)(u % per / groups);
             const int64_t g = u % groups;
-            const int sh = vols[v].sh;
-            if (!mbar_wait_warp(smem_u32(accf), (uint32_t)(n_units & 1), err, 27)) goto done;
-            tc_fence_after();
+            const int sh = vols[v].sh, ke = min(kXChunks * (b + 1), nch);
             const int j = kXBlock * b + quad * 32 + lane;
+          for (int k0 = 0; k0 < (SEG ? ke : 1); k0 += kAnyChunks, ++drains) {
+            if (!mbar_wait_warp(smem_u32(accf), (uint32_t)(drains & 1), err, 27)) goto done;
+            tc_fence_after();
+            const bool add = SEG && k0 > 0;  // a further segment of the same sums
 #pragma unroll 1
             for (int q = 0; q < kXPaths / 8 / (kXEpiWarps / 4); ++q) {
                 const int p0 = wg * (kXPaths * 4 / kXEpiWarps) + q * 8;
@@ -512,10 +584,14 @@ __global__ void __launch_bounds__(kXThreads, 1) k_volterra_exact(const unsigned 
                         hi = (int64_t)h1 * 65536 + h0;
                         lo = (int64_t)l1 * 65536 + l0;
                     }
-                    const uint64_t x = shl((uint64_t)hi, sh) + (uint64_t)(lo >> (32 - sh)) + (1ull << 63);
-                    if (m + p < B && j < N) Xm[(size_t)p * N] = x;
+                    const uint64_t x = shl((uint64_t)hi, sh) + (uint64_t)(lo >> (32 - sh));
+                    if (m + p < B && j < N) {
+                        uint64_t* at = Xm + (size_t)p * N;
+                        *at = x + (add ? *at : 1ull << 63);
+                    }
                 }
             }
+          }
         }
     }
 done:
@@ -528,7 +604,7 @@ done:
 }
 
 int launch_volterra_exact(const unsigned char* dig, const unsigned char* panels, const X64Vol* vols, int nv, int N,
-                          int64_t B, uint64_t* X, unsigned int* err, cudaStream_t st)
+                          int64_t B, bool any, uint64_t* X, unsigned int* err, cudaStream_t st)
 {
     static std::mutex mu;
     static bool ready[64] = {};
@@ -537,19 +613,18 @@ int launch_volterra_exact(const unsigned char* dig, const unsigned char* panels,
         if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
         std::lock_guard<std::mutex> lk(mu);
         if (!ready[dev]) {
-            if (cudaFuncSetAttribute(k_volterra_exact<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kXSmem) !=
-                    cudaSuccess ||
-                cudaFuncSetAttribute(k_volterra_exact<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kXSmem) !=
-                    cudaSuccess) {
-                cudaGetLastError();
-                return -1;
-            }
+            for (auto* k : {k_volterra_exact<false, false>, k_volterra_exact<true, false>, k_volterra_exact<true, true>})
+                if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kXSmem) != cudaSuccess) {
+                    cudaGetLastError();
+                    return -1;
+                }
             ready[dev] = true;
         }
     }
     const int64_t units = (B + kXPaths - 1) / kXPaths * nv * x64_blocks(N);
     const int grid = (int)std::min<int64_t>(units, device_sms());
-    auto* kern = N > 1024 ? k_volterra_exact<true> : k_volterra_exact<false>;
+    // any digits: sums of at most 128 steps, whose diagonals stay within 2^24 whatever the digits are
+    auto* kern = any ? k_volterra_exact<true, true> : (N > 1024 ? k_volterra_exact<true, false> : k_volterra_exact<false, false>);
     kern<<<grid, kXThreads, kXSmem, st>>>(dig, panels, vols, nv, N, B, X, err);
     count_launch();
     return 0;
@@ -567,7 +642,7 @@ constexpr int kVarVals = 16, kVarGroups = 4;  // variance groups a batch of a pa
 __host__ __device__ constexpr int var_threads(int gb) { return gb > 1 ? 256 : 512; }
 __host__ __device__ constexpr int var_smem(int gb) { return kExpTable * 8 + (var_threads(gb) / 32) * kVarVals * 33 * 8; }
 
-template <int NS, int GB, bool U53>
+template <int NS, int GB, bool U53, bool EXT>
 __global__ void __launch_bounds__(var_threads(GB), 2) k_variance_fixed(const X64Vol* __restrict__ vols,
                                                                const X64Group* __restrict__ grps,
                                                                const uint64_t* __restrict__ comp,
@@ -610,7 +685,7 @@ __global__ void __launch_bounds__(var_threads(GB), 2) k_variance_fixed(const X64
                         for (int c = 0; c < NS; ++c) acc[q][c] = 0.0;
                     if (m < B) {
                         const double* W1 = Z + m * NS * (int64_t)N;
-                        const uint64_t* Wp = reinterpret_cast<const uint64_t*>(W1 + N);  // fixed point
+                        const uint64_t* Wp = reinterpret_cast<const uint64_t*>(W1 + N);  // fixed point, EXT: doubles
                         const uint64_t* Xm = X + ((size_t)v * B + m) * N;
                         // operands are loaded two steps ahead: a step's 24 bytes a lane, 24 warps an SM,
                         // have to cover the latency of device memory
@@ -642,7 +717,8 @@ __global__ void __launch_bounds__(var_threads(GB), 2) k_variance_fixed(const X64
                                 cc[q] = cn[q];
                                 cn[q] = (q < ng && j + 32 < N) ? __ldg(cg + (size_t)q * N + j + 32) : 0ull;
                             }
-                            const uint64_t x = s[0].x + mulhi64(s[0].wp ^ (1ull << 63), vol.a2f) - vol.a2h;
+                            const uint64_t wp = EXT ? (uint64_t)double_to_fixed(bits_double(s[0].wp)) : s[0].wp;
+                            const uint64_t x = s[0].x + mulhi64(wp ^ (1ull << 63), vol.a2f) - vol.a2h;
 #pragma unroll
                             for (int q = 0; q < GB; ++q) {
                                 if (q < ng) {
@@ -689,36 +765,38 @@ __global__ void __launch_bounds__(var_threads(GB), 2) k_variance_fixed(const X64
     }
 }
 
-int launch_variance_fixed(const X64Vol* vols, const X64Group* grps, const uint64_t* comp, const double* Z,
-                          const uint64_t* X, int nv, int max_groups, bool u53, int ns, int N, int64_t B, double* ivb,
-                          double* ivp, cudaStream_t st)
+template <bool EXT>
+static auto* variance_kernel(int ns, bool many, bool u53)
 {
-    static std::mutex mu;
-    static bool ready[64] = {};
+    if (ns == 3)
+        return many ? (u53 ? k_variance_fixed<3, kVarGroups, true, EXT> : k_variance_fixed<3, kVarGroups, false, EXT>)
+                    : (u53 ? k_variance_fixed<3, 1, true, EXT> : k_variance_fixed<3, 1, false, EXT>);
+    return many ? (u53 ? k_variance_fixed<2, kVarGroups, true, EXT> : k_variance_fixed<2, kVarGroups, false, EXT>)
+                : (u53 ? k_variance_fixed<2, 1, true, EXT> : k_variance_fixed<2, 1, false, EXT>);
+}
+
+int launch_variance_fixed(const X64Vol* vols, const X64Group* grps, const uint64_t* comp, const double* Z,
+                          const uint64_t* X, int nv, int max_groups, bool u53, bool ext, int ns, int N, int64_t B,
+                          double* ivb, double* ivp, cudaStream_t st)
+{
     const FixedTables* ft = fixed_tables();
     if (!ft) return -1;
-    auto* kern = ns == 3 ? (max_groups > 1 ? (u53 ? k_variance_fixed<3, kVarGroups, true> : k_variance_fixed<3, kVarGroups, false>)
-                                           : (u53 ? k_variance_fixed<3, 1, true> : k_variance_fixed<3, 1, false>))
-                         : (max_groups > 1 ? (u53 ? k_variance_fixed<2, kVarGroups, true> : k_variance_fixed<2, kVarGroups, false>)
-                                           : (u53 ? k_variance_fixed<2, 1, true> : k_variance_fixed<2, 1, false>));
+    auto* kern = ext ? variance_kernel<true>(ns, max_groups > 1, u53) : variance_kernel<false>(ns, max_groups > 1, u53);
     {
+        // each kernel's shared-memory limit, once per device
+        static std::mutex mu;
+        static std::set<std::pair<int, uintptr_t>> done;
         int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
+        if (cudaGetDevice(&dev) != cudaSuccess) return -1;
         std::lock_guard<std::mutex> lk(mu);
-        if (!ready[dev]) {
-            const auto allow = [](auto* k, int gb) {
-                return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, var_smem(gb)) == cudaSuccess;
-            };
-            if (!(allow(k_variance_fixed<2, 1, true>, 1) && allow(k_variance_fixed<2, 1, false>, 1) &&
-                  allow(k_variance_fixed<3, 1, true>, 1) && allow(k_variance_fixed<3, 1, false>, 1) &&
-                  allow(k_variance_fixed<2, kVarGroups, true>, kVarGroups) &&
-                  allow(k_variance_fixed<2, kVarGroups, false>, kVarGroups) &&
-                  allow(k_variance_fixed<3, kVarGroups, true>, kVarGroups) &&
-                  allow(k_variance_fixed<3, kVarGroups, false>, kVarGroups))) {
+        const std::pair<int, uintptr_t> key{dev, reinterpret_cast<uintptr_t>(kern)};
+        if (!done.count(key)) {
+            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     var_smem(max_groups > 1 ? kVarGroups : 1)) != cudaSuccess) {
                 cudaGetLastError();
                 return -1;
             }
-            ready[dev] = true;
+            done.insert(key);
         }
     }
     const int gb = max_groups > 1 ? kVarGroups : 1, pb = kVarVals / (gb * ns), threads = var_threads(gb);
@@ -731,7 +809,7 @@ int launch_variance_fixed(const X64Vol* vols, const X64Group* grps, const uint64
 }
 
 // -------------------------------------------------------------------- host
-bool x64_prepare(const Plan& plan, X64Tables& out)
+bool x64_prepare(const Plan& plan, X64Tables& out, bool ext)
 {
     const int N = plan.N, nv = (int)plan.vols.size(), ng = (int)plan.vgs.size();
     if (N < 2 || N > kX64MaxN) return false;
@@ -741,7 +819,8 @@ bool x64_prepare(const Plan& plan, X64Tables& out)
     out.comp.assign((size_t)ng * N, 0);
     std::vector<int> ux(nv);
     std::vector<double> xbound(nv);  // |X + a2 W1perp| at most
-    const double wmax = 6.9;  // |Box-Muller on 32-bit uniforms| <= sqrt(66 ln 2) = 6.77
+    // |Box-Muller on 32-bit uniforms| <= sqrt(66 ln 2) = 6.77; the caller's normals below kExtMax
+    const double wmax = ext ? kExtMax : 6.9;
     for (int v = 0; v < nv; ++v) {
         const VolGroup& V = plan.vols[v];
         const double* G = plan.gamma.data() + (size_t)v * N;

@@ -36,8 +36,11 @@ struct X64Tables {
     int max_groups = 0;          // most variance groups of one pass
     bool u53 = true;             // every group has 53 fraction bits
 };
-// False where the plan's numbers do not fit the fixed-point ranges.
-bool x64_prepare(const Plan& plan, X64Tables& out);
+// Size that the caller's normals (ext) stay below: 15.5.
+constexpr double kExtMax = 15.5;
+// False where the plan's numbers do not fit the fixed-point ranges; ext: for the
+// caller's normals.
+bool x64_prepare(const Plan& plan, X64Tables& out, bool ext = false);
 
 int x64_blocks(int N);
 size_t x64_panel_bytes(int N);  // per Volterra pass
@@ -55,12 +58,17 @@ const FixedTables* fixed_tables();
 int launch_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int f32, double* Z, unsigned char* dig, int ns,
                          cudaStream_t st);
 void launch_panels(const int64_t* gam, int nv, int N, unsigned char* panels, cudaStream_t st);
-// X[v][m][j] + 2^63
+// Digits of the caller's W1; *flag |= 1 where W1 or W1perp is kExtMax or more in
+// size, or NaN.
+void launch_digits(const double* Z, int64_t B, int N, int ns, unsigned char* dig, unsigned int* flag, cudaStream_t st);
+// X[v][m][j] + 2^63; any: exact for any digits, not only for those of independent
+// normals
 int launch_volterra_exact(const unsigned char* dig, const unsigned char* panels, const X64Vol* vols, int nv, int N,
-                          int64_t B, uint64_t* X, unsigned int* err, cudaStream_t st);
-// ivb[g][B] (Ivdt, IsvdW); ns = 3: ivp[g][B] IsvdWp too
+                          int64_t B, bool any, uint64_t* X, unsigned int* err, cudaStream_t st);
+// ivb[g][B] (Ivdt, IsvdW); ns = 3: ivp[g][B] IsvdWp too; ext: Z holds doubles
+// throughout
 int launch_variance_fixed(const X64Vol* vols, const X64Group* grps, const uint64_t* comp, const double* Z,
-                          const uint64_t* X, int nv, int max_groups, bool u53, int ns, int N, int64_t B, double* ivb,
-                          double* ivp, cudaStream_t st);
+                          const uint64_t* X, int nv, int max_groups, bool u53, bool ext, int ns, int N, int64_t B,
+                          double* ivb, double* ivp, cudaStream_t st);
 
 }  // namespace rbg

@@ -87,3 +87,42 @@ def test_sums_are_the_payoffs_sums(R, M):
         a, b = R.price_rt_sums(*args, M // 2, seed=6), R.price_rt_sums(*args, M - M // 2, seed=6, path_offset=M // 2)
         close(a[0] + b[0], s1, 1e-13)
         close(a[1] + b[1], s2, 1e-13)
+
+
+@pytest.mark.parametrize("kind", ["normal", "constant", "extreme digits", "zero"])
+@pytest.mark.parametrize("N,M", [(1, 5), (2, 64), (17, 65), (128, 63), (129, 70), (300, 130), (1030, 20)])
+def test_caller_normals(R, N, M, kind):
+    """Per-path payoffs of the caller's normals against the FP64 direct sum's:
+    2e-13 of the larger of the payoff and 1 (FP64 roundoff of the exponent over
+    N steps), for inputs whose digits add up as well as for normals."""
+    g = np.random.default_rng(N + M)
+    Z = {"normal": lambda: g.standard_normal((M, 2, N)), "zero": lambda: np.zeros((M, 2, N)),
+         "constant": lambda: np.broadcast_to(g.uniform(-1, 1, (M, 2, 1)), (M, 2, N)).copy(),
+         # every lower digit of W1 at an end of its range
+         "extreme digits": lambda: np.where(g.random((M, 2, 1)) < 0.5, -1, 1) * np.full((M, 2, N), 0x7f7f7f7f7f7f7 / 2.0 ** 51)
+         }[kind]()
+    eta = 1.9 if kind in ("normal", "zero") else 1.9 / np.sqrt(N)
+    args = (XI, [0.07, 0.4], [eta, eta], [-0.9, 0.3], [1.0, 0.5], [0.9, 1.1], Z)
+    p, q = R.payoffs_rt(*args), R.payoffs_rt(*args, conv=R.CONV_DIRECT)
+    assert np.all(np.abs(p - q) <= 2e-13 * np.maximum(np.abs(q), 1.0)), np.max(np.abs(p - q))
+
+
+@pytest.mark.parametrize("bad", [15.5, -16.0, 1e3, np.inf, np.nan])
+@pytest.mark.parametrize("stream", [0, 1])
+def test_caller_normals_out_of_range_take_the_fp64_kernels(R, bad, stream):
+    Z = np.random.default_rng(1).standard_normal((70, 2, 40))
+    Z[66, stream, 21] = bad
+    args = (XI, [0.1], [0.5], [-0.7], [1.0], [1.0], Z)
+    p, q = R.payoffs_rt(*args), R.payoffs_rt(*args, conv=R.CONV_DIRECT)
+    assert np.array_equal(p, q, equal_nan=True)  # the whole batch is the direct sum's
+    Zm = np.concatenate([Z, np.random.default_rng(2).standard_normal((70, 1, 40))], 1)
+    p, q = R.payoffs_mc(*args[:6], Zm), R.payoffs_mc(*args[:6], Zm, conv=R.CONV_DIRECT)
+    assert np.array_equal(p, q, equal_nan=True)
+
+
+def test_caller_normals_plain_mc(R):
+    Z = np.random.default_rng(3).standard_normal((130, 3, 150))
+    Z[5, 2, 7] = 1e3  # Wperp only meets FP64 sums: no range
+    args = (XI, [0.1, 0.3], [1.5, 1.0], [-0.7, 0.2], [1.0, 0.5, 2.0], [1.0, 0.9, 1.1], Z)
+    p, q = R.payoffs_mc(*args), R.payoffs_mc(*args, conv=R.CONV_DIRECT)
+    assert np.all(np.abs(p - q) <= 2e-13 * np.maximum(np.abs(q), 1.0))
