@@ -282,7 +282,7 @@ constexpr int kXBlock = 128;                           // output steps per block
 constexpr int kXChunks = kXBlock / kXSteps;            // 8 chunks per block of steps
 constexpr int kXStages = 5;
 constexpr int kXEpiWarps = 16;
-constexpr int kXThreads = (kXEpiWarps + 2) * 32;
+constexpr int kXThreads = (kXEpiWarps + 3) * 32;
 // SEG: steps a sum takes where the digits may be anything: 8 digit pairs x 128 x 2^14 = 2^24
 constexpr int kAnyChunks = 128 / kXSteps;
 constexpr int kXSmem = 2 * kPanelBytes + kXStages * kXChunkBytes + 256 + 1024;
@@ -362,8 +362,8 @@ struct PanelSlots {
 };
 
 // One (block b, pass v, group of 64 paths) at a time, the longest blocks
-// first.  Warps 0-15 read the accumulators, warp 16 loads, warp 17 issues the
-// MMAs.  WIDE: accumulators may pass 2^22 (N > 1024): converted by F2I, else by
+// first.  Warps 0-15 read the accumulators, warp 16 loads, warps 17 and 18 issue
+// the MMAs.  WIDE: accumulators may pass 2^22 (N > 1024): converted by F2I, else by
 // adding 1.5 2^23.  SEG: the caller's normals, whose digits may add up: the
 // accumulators are read out every 128 steps and X summed in integers, which is
 // exact for any digits.
@@ -399,11 +399,11 @@ __global__ void __launch_bounds__(kXThreads, 1) k_volterra_exact(const unsigned 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kXStages; ++s) {
             mbar_init(smem_u32(wfull + s), 1);
-            mbar_init(smem_u32(wempty + s), 1);
+            mbar_init(smem_u32(wempty + s), 2);
         }
         for (int b = 0; b < 2; ++b) mbar_init(smem_u32(pfull + b), 1);
-        mbar_init(smem_u32(accf), 1);
-        mbar_init(smem_u32(fin), 1);
+        mbar_init(smem_u32(accf), 2);
+        mbar_init(smem_u32(fin), 2);
         mbar_init(smem_u32(acce), kXEpiWarps);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -472,9 +472,12 @@ __global__ void __launch_bounds__(kXThreads, 1) k_volterra_exact(const unsigned 
             for (int b = 0; b < 2; ++b)
                 if (loads[b]) mbar_drain(smem_u32(pfull + b), (uint32_t)((loads[b] - 1) & 1));
         }
-    } else if (warp == kXEpiWarps + 1) {
+    } else if (warp > kXEpiWarps) {
         if (lane == 0) {
-            // -------------------------------------------------- MMA issuer
+            // ------------------------------------------------- MMA issuers
+            // Thread 0 accumulates the diagonals 0 .. 3 (four MMAs a chunk), thread 1 the
+            // diagonals 4 .. 7 (eight): one thread issuing all twelve held the tensor pipe.
+            const int me = warp - kXEpiWarps - 1;
             PanelSlots ps;
             int loads[2] = {0, 0};
             int s = 0;
@@ -508,15 +511,21 @@ __global__ void __launch_bounds__(kXThreads, 1) k_volterra_exact(const unsigned 
                     // descriptors differ in the start-address field only (address / 16, no carry out of it)
                     const uint32_t arow = a_lo + (uint32_t)(pb * kPanelBytes + (kXChunks - 1 - kc % kXChunks) * 512) / 16;
                     const uint32_t brow = b_lo + (uint32_t)(s * kXChunkBytes) / 16;
+                    const uint32_t first = (SEG ? sc : kc) == 0 ? 0u : 1u;
+                    if (me == 0) {
 #pragma unroll
-                    for (int j = 0; j < kXDigits; ++j) {
-                        const uint64_t da = ((uint64_t)a_hi << 32) | (arow + (uint32_t)(j * kPanelDigit) / 16);
-                        const int n = kXPaths * (kXDigits - j), n1 = n < 256 ? n : 256;
-                        const uint32_t acc = ((SEG ? sc : kc) == 0 && j == 0) ? 0u : 1u;
-                        umma_f16(tmem + kXPaths * j, da, ((uint64_t)b_hi << 32) | brow, idesc_f16(n1, 0), acc);
-                        if (n > 256)
-                            umma_f16(tmem + kXPaths * j + 256, da, ((uint64_t)b_hi << 32) | (brow + 256 * 32 / 16),
-                                     idesc_f16(n - 256, 0), acc);
+                        for (int j = 0; j < 4; ++j)  // W1 digits 0 .. 3 - j into diagonals j .. 3
+                            umma_f16(tmem + kXPaths * j, ((uint64_t)a_hi << 32) | (arow + (uint32_t)(j * kPanelDigit) / 16),
+                                     ((uint64_t)b_hi << 32) | brow, idesc_f16(kXPaths * (4 - j), 0), j ? 1u : first);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < kXDigits; ++j) {  // W1 digits max(0, 4 - j) .. 7 - j into diagonals max(4, j) .. 7
+                            const int i0 = j < 4 ? 4 - j : 0, n = j < 4 ? 4 : kXDigits - j;
+                            umma_f16(tmem + kXPaths * (i0 + j),
+                                     ((uint64_t)a_hi << 32) | (arow + (uint32_t)(j * kPanelDigit) / 16),
+                                     ((uint64_t)b_hi << 32) | (brow + (uint32_t)(i0 * kXPaths * 32) / 16),
+                                     idesc_f16(kXPaths * n, 0), j ? 1u : first);
+                        }
                     }
                     umma_commit(smem_u32(wempty + s));
                     if (SEG && (++sc == kAnyChunks || kc == ke - 1)) {
