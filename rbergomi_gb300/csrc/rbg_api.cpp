@@ -455,11 +455,17 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
     if ((rc = upload_tables(c, plan, st, ts, logL, fixed ? &xt : nullptr, !fixed))) return rc;
     const int no = (int)plan.outs.size(), N = plan.N, ns = mc ? 3 : 2, nv = (int)plan.vols.size();
     const int64_t B = fp64_batch(plan, M, ns);
-    // passes per convolution launch: X within 2 GiB
-    const int vstep = (int)std::max<int64_t>(1, std::min<int64_t>(nv, ((int64_t)1 << 31) / (8 * (int64_t)N * B)));
+    // The variance pass inside the convolution's read-out for up to x64_fuse_groups
+    // variance groups a pass, where its sums (one value per group, path and 32 steps)
+    // stay within X's limit of 2 GiB for one pass.
+    const size_t sums = (size_t)std::max(xt.max_groups, 1) * x64_slot_bytes(B, N, ns);
+    const bool fused = fixed && xt.u53 && xt.max_groups <= x64_fuse_groups(ns) && sums <= ((size_t)1 << 31);
+    const size_t per = fused ? sums : 8 * (size_t)N * (size_t)B;
+    // passes per convolution launch: X or the sums within 2 GiB
+    const int vstep = (int)std::max<int64_t>(1, std::min<int64_t>(nv, ((int64_t)1 << 31) / (int64_t)per));
     if (fixed) {
         if ((rc = ensure(c.xdig, x64_digit_bytes(B, N), "normal digits"))) return rc;
-        if ((rc = ensure(c.xbuf, 8 * (size_t)vstep * N * (size_t)B, "Volterra paths"))) return rc;
+        if ((rc = ensure(c.xbuf, (size_t)vstep * per, "Volterra paths"))) return rc;
     }
     if ((rc = ensure(c.z, sizeof(double) * ns * N * (size_t)B, "normals"))) return rc;
     if ((rc = ensure(c.ivb, sizeof(double) * 2 * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
@@ -482,7 +488,8 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
                 if (launch_sobol_normals(sobol_vt, N, (uint64_t)(o.path_offset + m0 + 1), b, br, c.z.as<double>(), st))
                     return fail(RBG_ERR_UNSUPPORTED, "Brownian bridge shared memory not available for this N");
             } else if (launch_normals_fixed(o.seed, o.path_offset + m0, b, N, o.normals == RBG_NORMALS_F32,
-                                            c.z.as<double>(), fixed ? c.xdig.as<unsigned char>() : nullptr, ns, st)) {
+                                            c.z.as<double>(), fixed ? c.xdig.as<unsigned char>() : nullptr,
+                                            fused ? kFixAll : (fixed ? kFixW1perp : 0), ns, st)) {
                 return fail(RBG_ERR_CUDA, "normal tables could not be set up");
             }
         }
@@ -491,12 +498,20 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
             if (!fixed) launch_path_fp64(ts.t, c.z.as<double>(), b, c.ivb.as<double>(), st, ivp);
             for (int v0 = 0; fixed && v0 < nv; v0 += vstep) {
                 const int k = std::min(vstep, nv - v0);
-                if (launch_volterra_exact(c.xdig.as<unsigned char>(),
-                                          c.xpan.as<unsigned char>() + (size_t)v0 * x64_panel_bytes(N), ts.xvols + v0, k, N,
-                                          b, false, c.xbuf.as<uint64_t>(), err, st) ||
-                    launch_variance_fixed(ts.xvols + v0, ts.xgrps, ts.xcomp, c.z.as<double>(), c.xbuf.as<uint64_t>(), k,
-                                          xt.max_groups, xt.u53, false, ns, N, b, c.ivb.as<double>(), ivp, st))
+                const unsigned char* pan = c.xpan.as<unsigned char>() + (size_t)v0 * x64_panel_bytes(N);
+                if (fused) {
+                    const int g0 = plan.vols[v0].vg_begin, ng = plan.vols[v0 + k - 1].vg_end - g0;
+                    if (launch_volterra_variance(c.xdig.as<unsigned char>(), pan, ts.xvols + v0, ts.xgrps, ts.xcomp,
+                                                 c.z.as<double>(), k, g0, ng, ns, N, b, c.xbuf.as<double>(),
+                                                 c.ivb.as<double>(), ivp, err, st))
+                        return fail(RBG_ERR_CUDA, "FP64 path kernels could not be configured");
+                } else if (launch_volterra_exact(c.xdig.as<unsigned char>(), pan, ts.xvols + v0, k, N, b, false,
+                                                 c.xbuf.as<uint64_t>(), err, st) ||
+                           launch_variance_fixed(ts.xvols + v0, ts.xgrps, ts.xcomp, c.z.as<double>(),
+                                                 c.xbuf.as<uint64_t>(), k, xt.max_groups, xt.u53, false, ns, N, b,
+                                                 c.ivb.as<double>(), ivp, st)) {
                     return fail(RBG_ERR_CUDA, "FP64 path kernels could not be configured");
+                }
             }
         }
         const int nchunks = (int)((b + 256 * (int64_t)G - 1) / (256 * (int64_t)G));
@@ -755,7 +770,7 @@ static int price_cv(Ctx& c, const Plan& plan, const rbg_cv_params& p, const rbg_
         RBG_CUDA(cudaMemcpyAsync(c.z.p, Zc, sizeof(double) * 2 * N * Mc, cudaMemcpyHostToDevice, st));
     } else {
         if (launch_normals_fixed(o.seed, kCvPilotPath0 + o.path_offset, Mc, N, o.normals == RBG_NORMALS_F32,
-                                 c.z.as<double>(), nullptr, 2, st))
+                                 c.z.as<double>(), nullptr, 0, 2, st))
             return fail(RBG_ERR_CUDA, "normal tables could not be set up");
     }
     launch_path_fp64(ts.t, c.z.as<double>(), Mc, c.ivb.as<double>(), st);
@@ -769,7 +784,7 @@ static int price_cv(Ctx& c, const Plan& plan, const rbg_cv_params& p, const rbg_
                                      st));
         } else {
             if (launch_normals_fixed(o.seed, o.path_offset + m0, b, N, o.normals == RBG_NORMALS_F32, c.z.as<double>(),
-                                     nullptr, 2, st))
+                                     nullptr, 0, 2, st))
                 return fail(RBG_ERR_CUDA, "normal tables could not be set up");
         }
         launch_path_fp64(ts.t, c.z.as<double>(), b, c.ivb.as<double>(), st, nullptr, c.ivp.as<double>());
@@ -827,7 +842,7 @@ static int price_cv_mixed(Ctx& c, const Plan& plan, const rbg_cv_params& p, cons
     unsigned long long* count = (unsigned long long*)(Q + no);
     double* xy = (double*)(count + no);
     // pilot: one FP64 batch of Mc paths on FP32 normals
-    if (launch_normals_fixed(o.seed, kCvPilotPath0 + o.path_offset, Mc, N, 1, c.z.as<double>(), nullptr, 2, st))
+    if (launch_normals_fixed(o.seed, kCvPilotPath0 + o.path_offset, Mc, N, 1, c.z.as<double>(), nullptr, 0, 2, st))
         return fail(RBG_ERR_CUDA, "normal tables could not be set up");
     launch_path_fp64(ts.t, c.z.as<double>(), Mc, c.ivp.as<double>(), st);
     launch_cv_pilot(ts.t, c.ivp.as<double>(), Mc, xy, alpha, Q, st);
@@ -1193,7 +1208,7 @@ int rbg_generate_normals_streams(uint64_t seed, int64_t path_offset, int64_t M, 
     if ((rc = ensure(c->z, sizeof(double) * ns * N * (size_t)B, "normals"))) return rc;
     for (int64_t m0 = 0; m0 < M; m0 += B) {
         const int64_t b = std::min(B, M - m0);
-        if (launch_normals_fixed(seed, path_offset + m0, b, N, precision == RBG_MIXED, c->z.as<double>(), nullptr, ns,
+        if (launch_normals_fixed(seed, path_offset + m0, b, N, precision == RBG_MIXED, c->z.as<double>(), nullptr, 0, ns,
                                  c->stream))
             return fail(RBG_ERR_CUDA, "normal tables could not be set up");
         RBG_CUDA(cudaGetLastError());

@@ -267,11 +267,11 @@ RBG_HD double exp2_fixed(int64_t x, int ut, const uint64_t* E)
     return bits_double(e > 1023 ? 0x7FF0000000000000ull : (e < -1022 ? 0ull : b));
 }
 
-// exp2_fixed(x, 53, E), its shifts constants.
-RBG_HD double exp2_fixed53(int64_t x, const uint64_t* E)
+// 2^(x 2^-53) = m 2^(e - 63), m in [2^63, 2^64).
+RBG_HD uint64_t exp2_mantissa53(int64_t x, const uint64_t* E, int32_t& e)
 {
     const uint32_t h = hi32((uint64_t)x), l = lo32((uint64_t)x);
-    const int32_t e = (int32_t)h >> 21;
+    e = (int32_t)h >> 21;
     const uint64_t T = E[(h >> 9) & (kExpTable - 1)];
     const uint32_t rt = h & 511u;                             // remainder below 2^-12: 9 + 32 bits, unit 2^-53
     const uint32_t rh = (rt << 23) | (l >> 9);                // unit 2^-44
@@ -279,7 +279,14 @@ RBG_HD double exp2_fixed53(int64_t x, const uint64_t* E)
     const uint32_t r2 = mulhi32(rh, rh);                      // unit 2^-56
     const uint32_t c = 0xF5FDEFFDu + ((mulhi32(rh, 0x0E35846Bu) + (mulhi32(r2, 0x0276556Eu) >> 12)) >> 10);  // unit 2^-34
     const uint64_t p = mulhi64(r, 0xB17217F7D1CF79ACull) + (mul32(r2, c) >> 26);
-    const uint64_t m = T + mulhi64(T, p);
+    return T + mulhi64(T, p);
+}
+
+// exp2_fixed(x, 53, E), its shifts constants.
+RBG_HD double exp2_fixed53(int64_t x, const uint64_t* E)
+{
+    int32_t e;
+    const uint64_t m = exp2_mantissa53(x, E, e);
     const uint64_t b = ((uint64_t)((uint32_t)(e + 1022) << 20) << 32) + (m >> 11) + ((m >> 10) & 1u);
     return bits_double(e < -1022 ? 0ull : b);                 // e <= 1023: x 2^-53 < 1024
 }

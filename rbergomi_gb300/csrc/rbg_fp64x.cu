@@ -111,8 +111,8 @@ __device__ __forceinline__ void store_digits(const int64_t (&v)[4], unsigned cha
 
 // Z[m][s][j], s < ns: W1, W1perp and (plain MC) Wperp on Philox streams 0, 1,
 // 2.  dig non-null (the fixed-point path pass follows): also the digits of W1,
-// zero past N and past B, and W1perp as 64-bit fixed point (unit 2^-59) in
-// place of doubles.
+// zero past N and past B.  Streams s with bit s of fix set are stored as 64-bit
+// fixed point (unit 2^-59) in place of doubles.
 // A warp takes up to kSeg chunks of 16 steps of 8 paths' stream, four lanes a
 // path and four steps a lane, so a path's 16 values and each digit's 8 rows are
 // contiguous.  Integer instructions bound it: 368 a warp and pair of normals, 64
@@ -123,7 +123,7 @@ constexpr int kNormalThreads = 256, kSeg = 8;
 template <int F32>
 __global__ void __launch_bounds__(kNormalThreads, 4) k_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int ns,
                                                                     double* __restrict__ Z,
-                                                                    unsigned char* __restrict__ dig,
+                                                                    unsigned char* __restrict__ dig, int fix,
                                                                     const FixedTables* __restrict__ ft)
 {
     __shared__ NormalTables T;
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kNormalThreads, 4) k_normals_fixed(uint64_t se
                     box_muller_fixed(x.x, x.y, T, v[0], v[1]);
                     box_muller_fixed(x.z, x.w, T, v[2], v[3]);
                 }
-                if (s == 1 && dig) {
+                if ((fix >> s) & 1) {
 #pragma unroll
                     for (int q = 0; q < 4; ++q) z[q] = __longlong_as_double(v[q]);
                 } else if (!F32) {
@@ -196,8 +196,8 @@ __global__ void __launch_bounds__(kNormalThreads, 4) k_normals_fixed(uint64_t se
     }
 }
 
-int launch_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int f32, double* Z, unsigned char* dig, int ns,
-                         cudaStream_t st)
+int launch_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int f32, double* Z, unsigned char* dig, int fix,
+                         int ns, cudaStream_t st)
 {
     const FixedTables* ft = fixed_tables();
     if (!ft) return -1;
@@ -205,8 +205,8 @@ int launch_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int f32
     const int64_t tasks = (B + kXPaths - 1) / kXPaths * (kXPaths / 8) * ns * ((nch + kSeg - 1) / kSeg);
     const int64_t need = (tasks + kNormalThreads / 32 - 1) / (kNormalThreads / 32);
     const int64_t blocks = std::min<int64_t>(need, 8 * (int64_t)device_sms());
-    if (f32) k_normals_fixed<1><<<(unsigned)blocks, kNormalThreads, 0, st>>>(seed, path0, B, N, ns, Z, dig, ft);
-    else k_normals_fixed<0><<<(unsigned)blocks, kNormalThreads, 0, st>>>(seed, path0, B, N, ns, Z, dig, ft);
+    if (f32) k_normals_fixed<1><<<(unsigned)blocks, kNormalThreads, 0, st>>>(seed, path0, B, N, ns, Z, dig, fix, ft);
+    else k_normals_fixed<0><<<(unsigned)blocks, kNormalThreads, 0, st>>>(seed, path0, B, N, ns, Z, dig, fix, ft);
     count_launch();
     return 0;
 }
@@ -280,12 +280,13 @@ constexpr int kPanelDigit = kPanelRows * 32;           // 7680 B
 constexpr int kPanelBytes = kXDigits * kPanelDigit;    // 61440 B
 constexpr int kXBlock = 128;                           // output steps per block
 constexpr int kXChunks = kXBlock / kXSteps;            // 8 chunks per block of steps
-constexpr int kXStages = 5;
+constexpr int kXStagesPlain = 5, kXStagesFused = 4;
 constexpr int kXEpiWarps = 16;
 constexpr int kXThreads = (kXEpiWarps + 3) * 32;
 // SEG: steps a sum takes where the digits may be anything: 8 digit pairs x 128 x 2^14 = 2^24
 constexpr int kAnyChunks = 128 / kXSteps;
-constexpr int kXSmem = 2 * kPanelBytes + kXStages * kXChunkBytes + 256 + 1024;
+constexpr int kXSmemPlain = 2 * kPanelBytes + kXStagesPlain * kXChunkBytes + 256 + 1024;
+constexpr int kXSmemFused = 2 * kPanelBytes + kXStagesFused * kXChunkBytes + 256 + kExpTable * 8 + 1024;
 
 int x64_blocks(int N) { return (N + kXBlock - 1) / kXBlock; }
 size_t x64_panel_bytes(int N) { return (size_t)x64_blocks(N) * kPanelBytes; }
@@ -338,6 +339,109 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8])
                  : "r"(taddr));
 }
 
+// Warp sums of NV integers a lane (a power of two up to 32): each halving step
+// hands half of the values to the partner lane.  Value lane / (32 / NV) of every
+// lane's sum on return.
+template <int NV>
+__device__ __forceinline__ int64_t warp_sums_i64(int64_t (&v)[NV])
+{
+    const int lane = threadIdx.x & 31;
+    int o = 16;
+#pragma unroll
+    for (int n = NV / 2; n >= 1; n >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const int64_t send = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+#pragma unroll
+    for (; o >= 1; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return v[0];
+}
+
+// What a fused variance pass needs beside the convolution's arguments; its sums
+// go to part[group of the launch][4 block + warp quadrant][path][NS].
+struct FuseArgs {
+    const X64Group* grps;
+    const uint64_t* comp;
+    const uint64_t* Z;
+    double* part;
+    const FixedTables* ft;
+    int slots;
+};
+
+// The variance pass of a read-out warp on X of its 16 paths (x, without the
+// offset of 2^63), step j of the unit in lane order: per group and path the
+// warp's sums of 2^(2 t) and 2^t W over its 32 steps, v = xi 2^(2 t) (k_variance_fixed).
+// The sums are taken in integers: with 2^t = m 2^(e - 63) and E the largest e of
+// the 32 steps, m^2 is shifted right by 2 (E - e) + 5 and m W by E - e + 4, so 32
+// terms fit 64 bits, with a half unit back for the truncation (16 units of 32
+// terms).  The square's unit is 2^-57 of the largest term or less, the product's
+// 2^-54 2^E; an FP64 sum rounds every product to 2^-53 of itself and every partial
+// sum likewise.  The same in FP64 (two products, the lanes' additions) holds the
+// FP64 pipe: 2^16 paths of 250 steps, three sums, 313 us for the path pass against
+// 261.  132 warp instructions a path and group; four warps a scheduler do not hide
+// their latencies (0.55 a cycle).
+template <int NS>
+__device__ __forceinline__ void fused_variance(uint64_t (&x)[2][8], const X64Vol& vol, int grp0, const FuseArgs& fa,
+                                               const uint64_t* E, int N, int64_t B, int64_t m0, int j, int slot)
+{
+    const int lane = threadIdx.x & 31;
+    const bool in = j + 1 < N;
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        const int64_t m = m0 + 4 * h;
+        uint64_t xs[4], w1[4], wq[NS == 3 ? 4 : 1];
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            const bool ok = in && m + p < B;
+            const uint64_t* W1 = fa.Z + (m + p) * NS * (int64_t)N + j;
+            const uint64_t wp = ok ? W1[N] : 0ull;
+            w1[p] = ok ? W1[1] ^ (1ull << 63) : 0ull;
+            if (NS == 3) wq[p] = ok ? W1[2 * N + 1] ^ (1ull << 63) : 0ull;
+            xs[p] = x[h >> 1][(4 * h + p) & 7] + (1ull << 63) + mulhi64(wp ^ (1ull << 63), vol.a2f) - vol.a2h;
+        }
+#pragma unroll 1
+        for (int g = vol.vg_begin; g < vol.vg_end; ++g) {
+            const uint64_t cf = fa.grps[g].cf;
+            const bool neg = fa.grps[g].neg != 0;
+            const uint64_t cj = in ? __ldg(fa.comp + (size_t)g * N + j) : 0ull;
+            int64_t s[8], sq[4];
+            int top[4];
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                const bool ok = in && m + p < B;
+                int32_t e;
+                uint64_t mt = exp2_mantissa53((int64_t)(mulhi64(neg ? 0ull - xs[p] : xs[p], cf) - cj), E, e);
+                if (!ok) {
+                    mt = 0ull;
+                    e = -1000;
+                }
+                top[p] = __reduce_max_sync(0xffffffffu, e);
+                const int d = top[p] - e;
+                const uint64_t hh = mul32(hi32(mt), lo32(mt)) >> 31;
+                const uint64_t sqr = mul32(hi32(mt), hi32(mt)) + hh;  // m^2 2^-64
+                s[2 * p] = (int64_t)(sqr >> min(5 + 2 * d, 63));
+                s[2 * p + 1] = (int64_t)(mulhi64(mt, w1[p]) - (mt >> 1)) >> min(4 + d, 63);
+                if (NS == 3) sq[p] = (int64_t)(mulhi64(mt, wq[p]) - (mt >> 1)) >> min(4 + d, 63);
+            }
+            const int64_t i0 = warp_sums_i64<8>(s) + 16;  // value lane / 4 = 2 path + sum
+            const int pa = lane >> 3, c = (lane >> 2) & 1;
+            const int tp = pa & 2 ? (pa & 1 ? top[3] : top[2]) : (pa & 1 ? top[1] : top[0]);
+            const double sc = bits_double((uint64_t)(uint32_t)(tp + 1023) << 52);
+            double* out = fa.part + (((size_t)(g - grp0) * fa.slots + slot) * B + m + pa) * NS;
+            const double r = (c ? (double)i0 * 0x1p-54 : (double)(uint64_t)i0 * 0x1p-57 * sc) * sc;
+            if (!(lane & 3) && m + pa < B) out[c] = r;
+            if constexpr (NS == 3) {
+                const int64_t i2 = warp_sums_i64<4>(sq) + 16;
+                if (!(lane & 7) && m + pa < B) out[2] = (double)i2 * 0x1p-54 * sc;
+            }
+        }
+    }
+}
+
 // Which of the two panel buffers a panel goes to: the one that holds it, else
 // the one not used last.  The loader and the MMA thread follow the same rule.
 struct PanelSlots {
@@ -370,21 +474,26 @@ struct PanelSlots {
 // What bounds it: 2304 columns x 128 steps x 16 per chunk, 1152 MMA cycles,
 // against 16 KB of digits and 7.5 KB of panel from L2; the accumulators fill
 // TMEM, so the next block's MMAs wait for the read-out of this one's.
-// With k_variance_fixed: 512 steps, 2^17 paths, one pass 1.99 ms, against 13.2
-// ms for the FP64 FFT convolution and exponentials; 100 steps, 2^16 paths 0.23
-// ms, against 1.46 ms for the direct FP64 sum.
-template <bool WIDE, bool SEG>
+// FUSE = NS > 0: the read-out warps also do the variance pass on their X, in
+// registers, while the next unit's MMAs run, and write the sums of their 32
+// steps per path and group instead of X: 512 steps, 2^17 paths, one group 1.06 ms
+// with k_slot_sums, against 0.88 + 0.38 ms with X through memory and
+// k_variance_fixed, and 13.2 ms for the FP64 FFT convolution and exponentials; 100
+// steps, 2^16 paths 0.122 ms, against 0.133 and, for the direct FP64 sum, 1.46 ms.
+template <bool WIDE, bool SEG, int FUSE>
 __global__ void __launch_bounds__(kXThreads, 1) k_volterra_exact(const unsigned char* __restrict__ dig,
                                                                  const unsigned char* __restrict__ panels,
                                                                  const X64Vol* __restrict__ vols, int nv, int N,
                                                                  int64_t B, uint64_t* __restrict__ X,
-                                                                 unsigned int* __restrict__ err)
+                                                                 unsigned int* __restrict__ err, const FuseArgs fa)
 {
+    constexpr int kXStages = FUSE ? kXStagesFused : kXStagesPlain;
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     unsigned char* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
     unsigned char* stage = base + 2 * kPanelBytes;
     uint64_t* bars = (uint64_t*)(stage + kXStages * kXChunkBytes);
+    uint64_t* E = bars + 32;  // FUSE: the exponential's table
     uint64_t* wfull = bars;                 // [kXStages]
     uint64_t* wempty = bars + kXStages;     // [kXStages]
     uint64_t* pfull = bars + 2 * kXStages;  // [2]
@@ -407,6 +516,8 @@ __global__ void __launch_bounds__(kXThreads, 1) k_volterra_exact(const unsigned 
         mbar_init(smem_u32(acce), kXEpiWarps);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (FUSE)
+        for (int i = threadIdx.x; i < kExpTable; i += kXThreads) E[i] = fa.ft->exp2[i];
     if (warp == kXEpiWarps + 1) {
         __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(holder)), "r"(512)
@@ -557,20 +668,17 @@ __global__ void __launch_bounds__(kXThreads, 1) k_volterra_exact(const unsigned 
             if (!mbar_wait_warp(smem_u32(accf), (uint32_t)(drains & 1), err, 27)) goto done;
             tc_fence_after();
             const bool add = SEG && k0 > 0;  // a further segment of the same sums
-#pragma unroll 1
-            for (int q = 0; q < kXPaths / 8 / (kXEpiWarps / 4); ++q) {
-                const int p0 = wg * (kXPaths * 4 / kXEpiWarps) + q * 8;
+            // X of 8 paths (from column p0), the unit's step j
+            auto read8 = [&](int p0, uint64_t (&xv)[8], bool last) {
                 uint32_t D[kXDigits][8];
 #pragma unroll
                 for (int d = 0; d < kXDigits; ++d) tmem_ld8(tl + (uint32_t)(kXPaths * d + p0), D[d]);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (q == kXPaths / 8 / (kXEpiWarps / 4) - 1) {
+                if (last) {
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(acce));
                 }
-                const int64_t m = g * kXPaths + p0;
-                uint64_t* Xm = X + ((size_t)v * B + m) * N + j;
 #pragma unroll
                 for (int p = 0; p < 8; ++p) {
                     // S_hi in units of 2^(e - 33), S_lo of 2^(e - 65); X = S_hi 2^sh + S_lo 2^(sh - 32)
@@ -593,12 +701,32 @@ __global__ void __launch_bounds__(kXThreads, 1) k_volterra_exact(const unsigned 
                         hi = (int64_t)h1 * 65536 + h0;
                         lo = (int64_t)l1 * 65536 + l0;
                     }
-                    const uint64_t x = shl((uint64_t)hi, sh) + (uint64_t)(lo >> (32 - sh));
-                    if (m + p < B && j < N) {
-                        uint64_t* at = Xm + (size_t)p * N;
-                        *at = x + (add ? *at : 1ull << 63);
+                    xv[p] = shl((uint64_t)hi, sh) + (uint64_t)(lo >> (32 - sh));
+                }
+            };
+            if constexpr (FUSE == 0) {
+#pragma unroll 1
+                for (int q = 0; q < kXPaths / 8 / (kXEpiWarps / 4); ++q) {
+                    const int p0 = wg * (kXPaths * 4 / kXEpiWarps) + q * 8;
+                    uint64_t xv[8];
+                    read8(p0, xv, q == kXPaths / 8 / (kXEpiWarps / 4) - 1);
+                    const int64_t m = g * kXPaths + p0;
+                    uint64_t* Xm = X + ((size_t)v * B + m) * N + j;
+#pragma unroll
+                    for (int p = 0; p < 8; ++p) {
+                        if (m + p < B && j < N) {
+                            uint64_t* at = Xm + (size_t)p * N;
+                            *at = xv[p] + (add ? *at : 1ull << 63);
+                        }
                     }
                 }
+            } else {
+                static_assert(kXPaths * 4 / kXEpiWarps == 16, "two read-outs of 8 paths a warp");
+                const int p0 = wg * 16;
+                uint64_t xs[2][8];
+                read8(p0, xs[0], false);
+                read8(p0 + 8, xs[1], true);
+                fused_variance<FUSE>(xs, vols[v], vols[0].vg_begin, fa, E, N, B, g * kXPaths + p0, j, 4 * b + quad);
             }
           }
         }
@@ -612,29 +740,87 @@ done:
     }
 }
 
+// (Ivdt, IsvdW (, IsvdWp)) per path and group from the fused pass's sums over
+// its slots of 32 steps; groups grp0 .. grp0 + ng - 1.
+template <int NS>
+__global__ void __launch_bounds__(256) k_slot_sums(const X64Group* __restrict__ grps, const double* __restrict__ part,
+                                                  const int64_t* __restrict__ Z, int grp0, int ng, int slots, int N,
+                                                  int64_t B, double* __restrict__ ivb, double* __restrict__ ivp)
+{
+    for (int64_t t = blockIdx.x * (int64_t)256 + threadIdx.x; t < B * ng; t += (int64_t)gridDim.x * 256) {
+        const int g = (int)(t / B);
+        const int64_t m = t - (int64_t)g * B;
+        const double* p = part + ((size_t)g * slots * B + m) * NS;
+        double s[NS];
+#pragma unroll
+        for (int c = 0; c < NS; ++c) s[c] = 0.0;
+        for (int k = 0; k < slots; ++k, p += (size_t)B * NS) {
+#pragma unroll
+            for (int c = 0; c < NS; ++c) s[c] += p[c];
+        }
+        const X64Group& G = grps[grp0 + g];
+        const size_t at = (size_t)(grp0 + g) * B + m;
+        const int64_t* W1 = Z + m * NS * (int64_t)N;
+        // Ivdt = dt xi (1 + sum), IsvdW = sqrt(dt xi) (W1_0 + sum): v_0 = xi
+        ivb[2 * at] = G.dtxi * (1.0 + s[0]);
+        ivb[2 * at + 1] = G.sdtxi * (fixed_to_double(W1[0]) + s[1]);
+        if (NS == 3) ivp[at] = G.sdtxi * (fixed_to_double(W1[2 * N]) + s[NS - 1]);
+    }
+}
+
+size_t x64_slot_bytes(int64_t B, int N, int ns) { return (size_t)4 * x64_blocks(N) * (size_t)B * ns * sizeof(double); }
+
+// Raises a kernel's shared-memory limit, once per (device, kernel).
+static bool allow_smem(const void* kern, int bytes)
+{
+    static std::mutex mu;
+    static std::set<std::pair<int, const void*>> done;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    std::lock_guard<std::mutex> lk(mu);
+    if (done.count({dev, kern})) return true;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    done.insert({dev, kern});
+    return true;
+}
+
+static int volterra_grid(int64_t B, int N, int nv)
+{
+    const int64_t units = (B + kXPaths - 1) / kXPaths * nv * x64_blocks(N);
+    return (int)std::min<int64_t>(units, device_sms());
+}
+
+int launch_volterra_variance(const unsigned char* dig, const unsigned char* panels, const X64Vol* vols,
+                             const X64Group* grps, const uint64_t* comp, const double* Z, int nv, int grp0, int ng, int ns,
+                             int N, int64_t B, double* part, double* ivb, double* ivp, unsigned int* err, cudaStream_t st)
+{
+    const FixedTables* ft = fixed_tables();
+    if (!ft) return -1;
+    const bool wide = N > 1024;
+    auto* kern = ns == 3 ? (wide ? k_volterra_exact<true, false, 3> : k_volterra_exact<false, false, 3>)
+                         : (wide ? k_volterra_exact<true, false, 2> : k_volterra_exact<false, false, 2>);
+    if (!allow_smem((const void*)kern, kXSmemFused)) return -1;
+    const int slots = 4 * x64_blocks(N);
+    kern<<<volterra_grid(B, N, nv), kXThreads, kXSmemFused, st>>>(
+        dig, panels, vols, nv, N, B, nullptr, err, FuseArgs{grps, comp, (const uint64_t*)Z, part, ft, slots});
+    const unsigned blocks = (unsigned)std::min<int64_t>((B * ng + 255) / 256, 8 * (int64_t)device_sms());
+    auto* sums = ns == 3 ? k_slot_sums<3> : k_slot_sums<2>;
+    sums<<<blocks, 256, 0, st>>>(grps, part, (const int64_t*)Z, grp0, ng, slots, N, B, ivb, ivp);
+    count_launch(2);
+    return 0;
+}
+
 int launch_volterra_exact(const unsigned char* dig, const unsigned char* panels, const X64Vol* vols, int nv, int N,
                           int64_t B, bool any, uint64_t* X, unsigned int* err, cudaStream_t st)
 {
-    static std::mutex mu;
-    static bool ready[64] = {};
-    {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
-        std::lock_guard<std::mutex> lk(mu);
-        if (!ready[dev]) {
-            for (auto* k : {k_volterra_exact<false, false>, k_volterra_exact<true, false>, k_volterra_exact<true, true>})
-                if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kXSmem) != cudaSuccess) {
-                    cudaGetLastError();
-                    return -1;
-                }
-            ready[dev] = true;
-        }
-    }
-    const int64_t units = (B + kXPaths - 1) / kXPaths * nv * x64_blocks(N);
-    const int grid = (int)std::min<int64_t>(units, device_sms());
     // any digits: sums of at most 128 steps, whose diagonals stay within 2^24 whatever the digits are
-    auto* kern = any ? k_volterra_exact<true, true> : (N > 1024 ? k_volterra_exact<true, false> : k_volterra_exact<false, false>);
-    kern<<<grid, kXThreads, kXSmem, st>>>(dig, panels, vols, nv, N, B, X, err);
+    auto* kern = any ? k_volterra_exact<true, true, 0>
+                     : (N > 1024 ? k_volterra_exact<true, false, 0> : k_volterra_exact<false, false, 0>);
+    if (!allow_smem((const void*)kern, kXSmemPlain)) return -1;
+    kern<<<volterra_grid(B, N, nv), kXThreads, kXSmemPlain, st>>>(dig, panels, vols, nv, N, B, X, err, FuseArgs{});
     count_launch();
     return 0;
 }
@@ -791,23 +977,7 @@ int launch_variance_fixed(const X64Vol* vols, const X64Group* grps, const uint64
     const FixedTables* ft = fixed_tables();
     if (!ft) return -1;
     auto* kern = ext ? variance_kernel<true>(ns, max_groups > 1, u53) : variance_kernel<false>(ns, max_groups > 1, u53);
-    {
-        // each kernel's shared-memory limit, once per device
-        static std::mutex mu;
-        static std::set<std::pair<int, uintptr_t>> done;
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess) return -1;
-        std::lock_guard<std::mutex> lk(mu);
-        const std::pair<int, uintptr_t> key{dev, reinterpret_cast<uintptr_t>(kern)};
-        if (!done.count(key)) {
-            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     var_smem(max_groups > 1 ? kVarGroups : 1)) != cudaSuccess) {
-                cudaGetLastError();
-                return -1;
-            }
-            done.insert(key);
-        }
-    }
+    if (!allow_smem((const void*)kern, var_smem(max_groups > 1 ? kVarGroups : 1))) return -1;
     const int gb = max_groups > 1 ? kVarGroups : 1, pb = kVarVals / (gb * ns), threads = var_threads(gb);
     const int64_t runs = (B + pb - 1) / pb;
     const int64_t blocks =

@@ -53,10 +53,13 @@ const FixedTables* fixed_tables();
 
 // The launchers return nonzero where the device refuses.
 // Philox normals Z[m][s][j] of ns streams per path (W1, W1perp, plain MC: Wperp);
-// f32: the mixed form's FP32 normals, widened; dig non-null (for the path pass
-// below): the digits of W1 too, and W1perp in 64-bit fixed point.
-int launch_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int f32, double* Z, unsigned char* dig, int ns,
-                         cudaStream_t st);
+// f32: the mixed form's FP32 normals, widened; dig non-null (for the path passes
+// below): the digits of W1 too; fix: streams (bit s: stream s) stored in 64-bit
+// fixed point, unit 2^-59, in place of doubles: kFixAll for the fused pass, kFixW1perp
+// for the separate one, whose FP64 sums take the doubles.
+constexpr int kFixAll = 7, kFixW1perp = 2;
+int launch_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int f32, double* Z, unsigned char* dig, int fix,
+                         int ns, cudaStream_t st);
 void launch_panels(const int64_t* gam, int nv, int N, unsigned char* panels, cudaStream_t st);
 // Digits of the caller's W1; *flag |= 1 where W1 or W1perp is kExtMax or more in
 // size, or NaN.
@@ -65,6 +68,17 @@ void launch_digits(const double* Z, int64_t B, int N, int ns, unsigned char* dig
 // normals
 int launch_volterra_exact(const unsigned char* dig, const unsigned char* panels, const X64Vol* vols, int nv, int N,
                           int64_t B, bool any, uint64_t* X, unsigned int* err, cudaStream_t st);
+// Both passes in one kernel, for groups with 53 fraction bits; the passes'
+// groups are grp0 .. grp0 + ng - 1, part holds x64_slot_bytes per group.
+// Worth it up to x64_fuse_groups groups a pass (path pass in microseconds, fused
+// against separate; 512 steps, 2^16 paths): two sums 1 group 550 / 775, 3 groups 912 /
+// 1001, 4 groups 1146 / 1117, 8 groups 1908 / 1773; three sums 1 group 606 / 967, 4
+// groups 1496 / 1506, 6 groups 2052 / 2215, 8 groups 2582 / 2549.
+constexpr int x64_fuse_groups(int ns) { return ns == 3 ? 6 : 3; }
+size_t x64_slot_bytes(int64_t B, int N, int ns);
+int launch_volterra_variance(const unsigned char* dig, const unsigned char* panels, const X64Vol* vols,
+                             const X64Group* grps, const uint64_t* comp, const double* Z, int nv, int grp0, int ng, int ns,
+                             int N, int64_t B, double* part, double* ivb, double* ivp, unsigned int* err, cudaStream_t st);
 // ivb[g][B] (Ivdt, IsvdW); ns = 3: ivp[g][B] IsvdWp too; ext: Z holds doubles
 // throughout
 int launch_variance_fixed(const X64Vol* vols, const X64Group* grps, const uint64_t* comp, const double* Z,

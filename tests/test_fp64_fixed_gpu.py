@@ -126,3 +126,15 @@ def test_caller_normals_plain_mc(R):
     args = (XI, [0.1, 0.3], [1.5, 1.0], [-0.7, 0.2], [1.0, 0.5, 2.0], [1.0, 0.9, 1.1], Z)
     p, q = R.payoffs_mc(*args), R.payoffs_mc(*args, conv=R.CONV_DIRECT)
     assert np.all(np.abs(p - q) <= 2e-13 * np.maximum(np.abs(q), 1.0))
+
+
+@pytest.mark.parametrize("mc,n_t", [(False, 2), (False, 3), (True, 6), (True, 7)])  # around the last fused group count
+@pytest.mark.parametrize("N,M", [(2, 65), (31, 129), (33, 64), (161, 700), (1100, 130)])
+def test_variance_in_the_read_out(R, mc, n_t, N, M):
+    """Variance groups up to and past the count the convolution's read-out takes,
+    at the edges of its 32-step sums, 128-step blocks and 16-path shares: the FP64
+    form's parity bound against the direct sum."""
+    price = R.price_mc if mc else R.price_rt
+    T = np.linspace(0.1, 3.0, n_t)
+    args = (XI, [0.08, 0.35], [2.2, -1.0], [-0.8, 0.4], T, [1.0] * n_t, N, M)
+    close(price(*args, seed=9)[0], price(*args, seed=9, conv=R.CONV_DIRECT)[0])
