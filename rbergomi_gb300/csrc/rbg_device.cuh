@@ -48,6 +48,42 @@ __device__ __forceinline__ uint4 philox_group(const PhiloxKeys& k, uint64_t p, u
     return philox4x32_10(make_uint4(g, (uint32_t)p, (uint32_t)(p >> 32), s), k);
 }
 
+// philox_group in parts.  Rounds 0 to 2 multiply either the path's word alone
+// (once a path) or the group's and stream's (the same for every path of one
+// upper counter word): philox_entry holds the latter's share, three of the 20
+// multiplications and what is XORed to them, philox_path the former's, and
+// philox_from_entry does the rest.
+struct PhiloxPath {
+    uint32_t hi, lo;
+};
+__device__ __forceinline__ uint4 philox_entry(uint64_t seed, uint32_t path_hi, uint32_t g, uint32_t s)
+{
+    const PhiloxKeys k = philox_keys(seed);
+    const uint64_t g0 = (uint64_t)0xD2511F53u * g;
+    const uint64_t g1 = (uint64_t)0xCD9E8D57u * ((uint32_t)(g0 >> 32) ^ s ^ k.b[0]);
+    const uint64_t g2 = (uint64_t)0xD2511F53u * ((uint32_t)(g1 >> 32) ^ (0xCD9E8D57u * path_hi) ^ k.a[1]);
+    return make_uint4((uint32_t)g0 ^ k.b[1], (uint32_t)g1 ^ k.a[2], (uint32_t)(g2 >> 32) ^ k.b[2], (uint32_t)g2);
+}
+__device__ __forceinline__ PhiloxPath philox_path(const PhiloxKeys& k, uint64_t p)
+{
+    const uint32_t h = (uint32_t)(((uint64_t)0xCD9E8D57u * (uint32_t)(p >> 32)) >> 32);
+    const uint64_t m = (uint64_t)0xD2511F53u * (h ^ (uint32_t)p ^ k.a[0]);
+    return PhiloxPath{(uint32_t)(m >> 32), (uint32_t)m};
+}
+__device__ __forceinline__ uint4 philox_from_entry(const PhiloxKeys& k, const PhiloxPath& p, const uint4& e)
+{
+    const uint64_t m = (uint64_t)0xCD9E8D57u * (p.hi ^ e.x);
+    uint4 c = make_uint4((uint32_t)(m >> 32) ^ e.y, (uint32_t)m, e.z ^ p.lo, e.w);
+#pragma unroll
+    for (int r = 3; r < 10; ++r) {
+        const uint64_t p0 = (uint64_t)0xD2511F53u * c.x;
+        const uint64_t p1 = (uint64_t)0xCD9E8D57u * c.z;
+        c = make_uint4((uint32_t)(p1 >> 32) ^ c.y ^ k.a[r], (uint32_t)p1, (uint32_t)(p0 >> 32) ^ c.w ^ k.b[r],
+                       (uint32_t)p0);
+    }
+    return c;
+}
+
 __device__ __forceinline__ uint4 philox_group(uint64_t seed, uint64_t p, uint32_t g, uint32_t s)
 {
     return philox_group(philox_keys(seed), p, g, s);
@@ -138,6 +174,28 @@ __device__ __forceinline__ void box_muller_f32(uint32_t a, uint32_t b, float& z0
     z0 = nr * c;
     z1 = nr * s;
 }
+
+// Two FP32 values in a register pair: one instruction for both, each rounded
+// as the scalar operation's.
+__device__ __forceinline__ uint64_t f2_pack(float x, float y)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 f2_unpack(uint64_t v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t f2_dup(float x) { return f2_pack(x, x); }
 
 // Normal CDF and BS call, rBergLib/BlackScholes.cpp:11-21 with tau = 1, r = 0
 // (the RT payoff always calls BS_call_price(spot, K, 1.0, vol)).

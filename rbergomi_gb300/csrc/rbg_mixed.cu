@@ -397,6 +397,32 @@ __device__ __forceinline__ float rt_payoff_f32(float Ivdt, float IsvdW, float rh
     return r.spot * phi_f32(d1) - K * phi_f32(d2);
 }
 
+// The launch's Philox entries, [upper word of the path: the first path's, the
+// next][stream][4-step group], filled by every CTA that reads them (all write
+// the same values; its threads read after a barrier of their own).  A producer
+// reads one broadcast 16 bytes, in L1, in place of three multiplications and four
+// XORs a draw: 1001 -> 963 million warp instructions at 512 steps, 2^20 paths.
+// With the role and the producer's share known as warp-uniform and the paired
+// FP32 operations of X, 2^22 paths of 512 steps take 5.33 ms against 5.52 (1024
+// steps 4.90 / 5.11, 2000 steps 2.81 / 2.93, sixteen variance groups 1.91 / 2.05).
+// Pairing the FP32 operations of Box-Muller, of the split or of the exponent too
+// was slower (5.70 ms at 512 steps), as were sixteen producer warps (5.59 ms).
+__device__ __forceinline__ void fill_entries(const MixedArgs& a, int ns, int t, int threads)
+{
+    const int ng = a.Np / 4;
+    const uint32_t hi = (uint32_t)((uint64_t)a.path0 >> 32);
+    const int n = (hi == (uint32_t)((uint64_t)(a.path0 + a.B - 1) >> 32) ? 1 : 2) * ns * ng;
+    for (int i = t; i < n; i += threads) {
+        const int g = i % ng, s = i / ng % ns;
+        a.ent[i] = philox_entry(a.seed, hi + i / (ng * ns), (uint32_t)g, (uint32_t)s);
+    }
+}
+// Those of a path.
+__device__ __forceinline__ const uint4* path_entries(const MixedArgs& a, int ns, uint64_t gpath)
+{
+    return a.ent + ((uint32_t)(gpath >> 32) == (uint32_t)((uint64_t)a.path0 >> 32) ? 0 : ns * (a.Np / 4));
+}
+
 // One producer thread's share of a chunk: Philox -> FP32 normals for steps
 // [32 c + SPT h, + SPT) of path p, its hi/lo row of the A tile and, unless
 // REDRAW (a first-pass chunk drawn again for the second pass), the FP32 W1 /
@@ -405,7 +431,8 @@ __device__ __forceinline__ float rt_payoff_f32(float Ivdt, float IsvdW, float rh
 // FW1 = false (pass mode 3): no FP32 W1 tile, W1perp at the start of the
 // stage's FP32 region (the epilogue reads W1 back from the A tile).
 template <int SK, bool REDRAW, bool MC, bool FW1 = true>
-__device__ __forceinline__ void produce_chunk(const MixedArgs& a, const PhiloxKeys& keys, uint64_t gpath, bool valid,
+__device__ __forceinline__ void produce_chunk(const MixedArgs& a, const PhiloxKeys& keys, const PhiloxPath& pp,
+                                              const uint4* ent, bool valid,
                                               int64_t m, int p, int h, int c, bool bnd, unsigned char* st,
                                               float* w1s)
 {
@@ -418,16 +445,16 @@ __device__ __forceinline__ void produce_chunk(const MixedArgs& a, const PhiloxKe
 #pragma unroll
     for (int q = 0; q < SPT / 4; ++q) {
         const uint32_t g = (uint32_t)((step0 >> 2) + q);
-        const uint4 x0 = philox_group(keys, gpath, g, 0);
+        const uint4 x0 = philox_from_entry(keys, pp, ent[g]);
         box_muller_f32(x0.x, x0.y, w[4 * q], w[4 * q + 1]);
         box_muller_f32(x0.z, x0.w, w[4 * q + 2], w[4 * q + 3]);
         if (!REDRAW) {
-            const uint4 x1 = philox_group(keys, gpath, g, 1);
+            const uint4 x1 = philox_from_entry(keys, pp, ent[Np / 4 + g]);
             box_muller_f32(x1.x, x1.y, wp[4 * q], wp[4 * q + 1]);
             box_muller_f32(x1.z, x1.w, wp[4 * q + 2], wp[4 * q + 3]);
         }
         if (MC && !REDRAW) {  // plain Monte Carlo: Wperp on stream 2
-            const uint4 x2 = philox_group(keys, gpath, g, 2);
+            const uint4 x2 = philox_from_entry(keys, pp, ent[2 * (Np / 4) + g]);
             box_muller_f32(x2.x, x2.y, wq[4 * q], wq[4 * q + 1]);
             box_muller_f32(x2.z, x2.w, wq[4 * q + 2], wq[4 * q + 3]);
         }
@@ -479,12 +506,12 @@ __device__ __forceinline__ void produce_chunk(const MixedArgs& a, const PhiloxKe
         // c + 1) follows the next pass's redrawn chunks, so W1 at step 32 (c + 1)
         // for the last column's sqrt(v) dW goes into this stage's boundary row
         if (bnd && h == kHPerPath - 1) {
-            const uint4 xb = philox_group(keys, gpath, (uint32_t)(8 * (c + 1)), 0);
+            const uint4 xb = philox_from_entry(keys, pp, ent[8 * (c + 1)]);
             float b0, b1;
             box_muller_f32(xb.x, xb.y, b0, b1);
             w1s[kFBnd + p] = valid ? b0 : 0.f;
             if (MC) {
-                const uint4 xq = philox_group(keys, gpath, (uint32_t)(8 * (c + 1)), 2);
+                const uint4 xq = philox_from_entry(keys, pp, ent[2 * (Np / 4) + 8 * (c + 1)]);
                 box_muller_f32(xq.x, xq.y, b0, b1);
                 w1s[kFWqBnd + p] = valid ? b0 : 0.f;
             }
@@ -743,7 +770,9 @@ __global__ void __launch_bounds__(PM > 0 ? kThreads + 32 : kThreads, 1) k_mixed_
     uint64_t* cempty = bars + 17;  // [kCSlots]
     uint64_t* ydone = bars + 20;   // thread 1's far-field of a pass complete
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // (read from lane 0: the compiler then knows it is the same for the warp, and keeps what
+    // follows from it in uniform registers)
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int Np = a.Np, nc = a.nc;
     const PassPlan<PM> pp(a);
     const int FB = (PM == 2 || PM == 3) ? L.fstride : kStageFB;  // bytes per stage of the FP32-tile region
@@ -789,6 +818,7 @@ __global__ void __launch_bounds__(PM > 0 ? kThreads + 32 : kThreads, 1) k_mixed_
     }
     for (int i = threadIdx.x; i < a.n_g * a.Np; i += blockDim.x) beta_s[i] = a.beta[i];
     for (int i = threadIdx.x; i < a.n_o; i += blockDim.x) otab[i] = a.otab[i];
+    if (SRC == 0) fill_entries(a, NS, threadIdx.x, blockDim.x);
     for (int i = threadIdx.x; i < kEpiWarps * a.n_o * 4; i += blockDim.x) osum[i] = 0.f;
     tc_fence_before();
     __syncthreads();
@@ -799,7 +829,7 @@ __global__ void __launch_bounds__(PM > 0 ? kThreads + 32 : kThreads, 1) k_mixed_
     if (warp < kProdWarps) {
         // ------------------------------------------------------- producers
         const int p = threadIdx.x & (kTileM - 1);
-        const int h = threadIdx.x >> 7;  // which kStepsPerThread steps of the chunk
+        const int h = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 7), 0);  // which kStepsPerThread steps of the chunk
         const PhiloxKeys keys = philox_keys(a.seed);
         // stage s and its phase parity ph run over the chunks of all tiles
         int s = 0;
@@ -807,7 +837,10 @@ __global__ void __launch_bounds__(PM > 0 ? kThreads + 32 : kThreads, 1) k_mixed_
         for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
             const int64_t m = tile * kTileM + p;
             const bool valid = m < a.B;
-            const uint64_t gpath = (uint64_t)(a.path0 + m);
+            // (paths past the last one share its entries)
+            const uint64_t gpath = (uint64_t)(a.path0 + (valid ? m : a.B - 1));
+            const PhiloxPath path = philox_path(keys, gpath);
+            const uint4* ent = SRC == 0 ? path_entries(a, NS, gpath) : nullptr;
             for (int q = 0; q < pp.np; ++q) {
                 const int cb = pp.begin(q), ce = pp.end(q);
                 // pass mode 3 draws each chunk once: no redrawn chunks, no boundary rows
@@ -842,11 +875,11 @@ __global__ void __launch_bounds__(PM > 0 ? kThreads + 32 : kThreads, 1) k_mixed_
                         else
                             produce_chunk_ext<SK, false, MC>(a, tile, c, bnd, st, w1s);
                     } else if (PM == 3) {
-                        produce_chunk<SK, false, MC, false>(a, keys, gpath, valid, m, p, h, c, bnd, st, w1s);
+                        produce_chunk<SK, false, MC, false>(a, keys, path, ent, valid, m, p, h, c, bnd, st, w1s);
                     } else if (PM > 0 && redraw) {
-                        produce_chunk<SK, true, MC>(a, keys, gpath, valid, m, p, h, c, bnd, st, w1s);
+                        produce_chunk<SK, true, MC>(a, keys, path, ent, valid, m, p, h, c, bnd, st, w1s);
                     } else {
-                        produce_chunk<SK, false, MC>(a, keys, gpath, valid, m, p, h, c, bnd, st, w1s);
+                        produce_chunk<SK, false, MC>(a, keys, path, ent, valid, m, p, h, c, bnd, st, w1s);
                     }
                     fence_proxy_async();
                     __syncwarp();
@@ -960,10 +993,17 @@ __global__ void __launch_bounds__(PM > 0 ? kThreads + 32 : kThreads, 1) k_mixed_
                         if (lane == 0) mbar_arrive(smem_u32((PM == 3 && (gpass & 1)) ? tmem_empty1 : tmem_empty));
                     }
                     float wn[16];
+                    // X = x + a1 W1 + a2 W1perp, two columns an instruction
+#pragma unroll
+                    for (int jj = 0; jj < 16; jj += 2) {
+                        const uint64_t y = f2_fma(f2_dup(a.a1), f2_pack(w1v[jj], w1v[jj + 1]), f2_pack(x[jj], x[jj + 1]));
+                        const float2 xx = f2_unpack(f2_fma(f2_dup(a.a2), f2_pack(w1pv[jj], w1pv[jj + 1]), y));
+                        x[jj] = xx.x;
+                        x[jj + 1] = xx.y;
+                    }
 #pragma unroll
                     for (int jj = 0; jj < 16; ++jj) {
                         const float w1 = w1v[jj];
-                        x[jj] = x[jj] + a.a1 * w1 + a.a2 * w1pv[jj];
                         if (jj > 0) wn[jj - 1] = w1;
                         if (jj == 0 && j0 == 0 && c == 0) {
                             w10_s[p] = w1;
@@ -1415,7 +1455,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_mixed_gemm_jobs(const __grid_co
     uint64_t* final_bar = bars + 11;
     uint32_t* tmem_holder = (uint32_t*)(bars + 12);
     uint64_t* strip_free = bars + 13;  // every MMA issued on the old strip has completed
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // (read from lane 0: the compiler then knows it is the same for the warp, and keeps what
+    // follows from it in uniform registers)
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
 
     // this CTA's tiles [t_first, t_last), starting in job jb
     const int64_t T = a.job_tile0[a.n_jobs];
@@ -1448,6 +1490,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_mixed_gemm_jobs(const __grid_co
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     for (int i = threadIdx.x; i < J0.n_g * J0.Np; i += blockDim.x) beta_s[i] = J0.beta[i];
+    fill_entries(J0, 2, threadIdx.x, blockDim.x);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -1456,23 +1499,29 @@ __global__ void __launch_bounds__(kThreads, 1) k_mixed_gemm_jobs(const __grid_co
     if (warp < kProdWarps) {
         // ------------------------------------------------------- producers
         const int p = threadIdx.x & (kTileM - 1);
-        const int h = threadIdx.x >> 7;
+        const int h = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 7), 0);
         PhiloxKeys keys = philox_keys(J0.seed);
         int s = 0, j = jb;
         uint32_t ph = 0;
         for (int64_t it = t_first; it < t_last; ++it) {
             const int jp = j;
             while (it >= a.job_tile0[j + 1]) ++j;
-            if (j != jp) keys = philox_keys(a.jobs[j].seed);
             const MixedArgs& J = a.jobs[j];
+            if (j != jp) {
+                keys = philox_keys(J.seed);
+                fill_entries(J, 2, lane, 32);  // each warp all of them: no barrier among the producers
+                __syncwarp();
+            }
             const int64_t m = (it - a.job_tile0[j]) * kTileM + p;
             const bool valid = m < J.B;
-            const uint64_t gpath = (uint64_t)(J.path0 + m);
+            const uint64_t gpath = (uint64_t)(J.path0 + (valid ? m : J.B - 1));
+            const PhiloxPath path = philox_path(keys, gpath);
+            const uint4* ent = path_entries(J, 2, gpath);
             for (int c = 0; c < J.nc; ++c, s = (s + 1 == S) ? 0 : s + 1, ph ^= (s == 0)) {
                 if (!mbar_wait_warp(smem_u32(empty + s), ph ^ 1u, a.err, 1)) goto done;
                 unsigned char* st = base + L.a0 + s * kStageA;
                 float* w1s = (float*)(base + L.f0 + s * kStageFB);
-                produce_chunk<SK, false, false>(J, keys, gpath, valid, m, p, h, c, false, st, w1s);
+                produce_chunk<SK, false, false>(J, keys, path, ent, valid, m, p, h, c, false, st, w1s);
                 fence_proxy_async();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(full + s));
@@ -1538,9 +1587,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_mixed_gemm_jobs(const __grid_co
                     }
                     float wn[16];
 #pragma unroll
+                    for (int jj = 0; jj < 16; jj += 2) {
+                        const uint64_t y = f2_fma(f2_dup(J.a1), f2_pack(w1v[jj], w1v[jj + 1]), f2_pack(x[jj], x[jj + 1]));
+                        const float2 xx = f2_unpack(f2_fma(f2_dup(J.a2), f2_pack(w1pv[jj], w1pv[jj + 1]), y));
+                        x[jj] = xx.x;
+                        x[jj + 1] = xx.y;
+                    }
+#pragma unroll
                     for (int jj = 0; jj < 16; ++jj) {
                         const float w1 = w1v[jj];
-                        x[jj] = x[jj] + J.a1 * w1 + J.a2 * w1pv[jj];
                         if (jj > 0) wn[jj - 1] = w1;
                         if (jj == 0 && j0 == 0 && c == 0) w10_s[p] = w1;
                     }
@@ -2262,6 +2317,11 @@ int mixed_prepare(const Plan& plan, const rbg_options& o, int64_t M, MixedJob& j
 
     size_t off = 256;  // the error word lives at offset 0
     job.off_err = 0;
+    if (backend == RBG_CONV_GEMM) {
+        job.off_ent = off;
+        off += (size_t)2 * ns * (Np / 4) * sizeof(uint4);
+        off = (off + 255) / 256 * 256;
+    }
     const double log2e = 1.4426950408889634;
     for (int v = 0; v < job.n_vol; ++v) {
         const VolGroup& vol = plan.vols[v];
@@ -2491,6 +2551,7 @@ int mixed_launch(const MixedJob& job, void* ws, uint64_t seed, int64_t path0, in
         A.sob = job.sob;
         A.ext = ext;
         mixed_set_seed(A, seed);
+        A.ent = (uint4*)(base + job.off_ent);
         A.path0 = path0;
         A.B = B;
         int pm = job.backend == RBG_CONV_GEMM ? pass_mode(A.Np) : 0;
@@ -2586,6 +2647,7 @@ int mixed_jobs_prepare(const std::vector<MixedJobRef>& jobs, void* table, unsign
         A.dbg_x = nullptr;
         A.n_o = 0;
         mixed_set_seed(A, r.seed);
+        A.ent = (uint4*)((unsigned char*)r.ws + r.job->off_ent);
         A.path0 = r.path0;
         A.B = r.B;
         A.jobs = nullptr;

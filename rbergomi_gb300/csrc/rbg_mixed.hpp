@@ -65,6 +65,7 @@ struct MixedArgs {
     // chunks of 16 KB per CTA (CTA b's at acache + b * ncache * 16 KB).
     unsigned char* acache;
     int ncache;
+    uint4* ent;  // GEMM backend, Philox: the launch's entries (philox_entry), [2][streams][Np / 4], written by the kernel
 };
 
 // Sets a.seed and its Philox round keys a.pk.
@@ -101,6 +102,7 @@ struct MixedJob {
     // past the uploaded image)
     int pmode = 0;
     size_t off_acache = 0;
+    size_t off_ent = 0;  // Philox entries, written by the kernel (inside the uploaded image, GEMM backend)
     std::vector<MixedLaunch> launches;   // one per (Volterra pass, <= 16 groups)
     std::vector<const void*> table_dev;  // optional device copies of each launch's strip / spectrum
     std::vector<unsigned char> host_ws;  // image uploaded by mixed_upload
@@ -156,7 +158,7 @@ bool mixed_job_batchable(const MixedJob& job);
 // device, its paths and its (Ivdt, IsvdW) buffer.
 struct MixedJobRef {
     const MixedJob* job;
-    const void* ws;
+    void* ws;
     uint64_t seed;
     int64_t path0, B;
     void* ivb;
