@@ -68,6 +68,17 @@ RBG_HD uint64_t double_bits(double d)
 #endif
 }
 
+RBG_HD float bits_float(uint32_t b)
+{
+#ifdef __CUDA_ARCH__
+    return __uint_as_float(b);
+#else
+    float d;
+    std::memcpy(&d, &b, 4);
+    return d;
+#endif
+}
+
 // ------------------------------------------------------------------ normals
 // Normals in signed fixed point, unit 2^-59 (|z| < 16; Box-Muller on 32-bit
 // uniforms stays below 6.77).
@@ -93,6 +104,18 @@ RBG_HD int64_t double_to_fixed(double x)
     const uint64_t a = sh >= 0 ? m << (sh & 63) : (sh > -64 ? m >> (-sh & 63) : 0ull);
     const uint64_t s = (uint64_t)((int64_t)b >> 63);
     return (int64_t)((a ^ s) - s);
+}
+
+// x as a float, rounded to nearest even: integers in place of the conversion,
+// which holds the FP64 pipe 64 cycles a warp, wherever the result is a normal float.
+RBG_HD float double_to_float(double x)
+{
+    const uint64_t b = double_bits(x);
+    const uint32_t h = hi32(b), l = lo32(b), a = h & 0x7FFFFFFFu;
+    if (a - 0x38100000u >= 0x47EFFFFFu - 0x38100000u) return (float)x;  // zero, below 2^-126, near 2^128 and above, NaN
+    uint32_t f = ((a - 0x38000000u) << 3) | (l >> 29);
+    f += ((l << 3) | (f & 1u)) > 0x80000000u ? 1u : 0u;
+    return bits_float(f | (h & 0x80000000u));
 }
 
 // Tables of the transform (shared memory on the device).

@@ -69,6 +69,7 @@
 #include <mutex>
 
 #include "rbg_device.cuh"
+#include "rbg_fixed.cuh"
 #include "rbg_mixed.hpp"
 #include "rbg_tc.cuh"
 
@@ -644,60 +645,96 @@ __device__ __forceinline__ void produce_chunk_sobol(const MixedArgs& a, int64_t 
 // Caller-normals producer (the mixed quadrature entry points): the caller's
 // FP64 normals in the quadrature layout, path m's stream s at a.ext +
 // (m NS + s) N.  Warp w of the producers takes paths 16 w .. 16 w + 15 of the
-// tile and lane l step j = 32 c + l, so each load instruction reads 32
-// consecutive doubles of one row (256 B, coalesced; no alignment beyond the
-// doubles' own).  Writes the FP32 W1 / W1perp (/ Wperp) tiles and the 16-bit
-// hi/lo A tile (REDRAW: W1 and the A tile only).
+// tile, four at a time, eight lanes a path and four steps a lane: a row's 32
+// steps are 256 contiguous bytes, a lane's share two 16-byte loads where every
+// row starts on a 16-byte boundary (N even, a.ext aligned) and four of 8 bytes
+// otherwise.  Writes the FP32 W1 / W1perp (/ Wperp) tiles and the hi/lo A tile
+// (REDRAW: W1 and the A tile only).
+// What bounds it: loads in flight (two batches of four paths ahead, and the
+// second next chunk's rows asked into L2), then instructions: with one step a lane,
+// 2-byte stores and conversions on the FP64 pipe it took 100 of them a path-step. A
+// call with 2^16 paths of 512 steps on the device, 21 strikes: 328 -> 251 us (270 with one
+// batch ahead), 81 of them the floor of reading the normals.
 template <int SK, bool REDRAW, bool MC>
 __device__ __forceinline__ void produce_chunk_ext(const MixedArgs& a, int64_t tile, int c, bool bnd, unsigned char* st,
                                                   float* w1s)
 {
     constexpr int NS = MC ? 3 : 2;
+    constexpr int RD = REDRAW ? 1 : NS;       // streams read
+    constexpr int LA = RD == 3 ? 1 : 2;       // batches loaded ahead
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int N = a.N, Np = a.Np;
-    const int j = kChunk * c + lane;
-    const bool jin = j < N;
-    const int64_t m0 = tile * kTileM + 16 * w;
+    const int k0 = 4 * (lane & 7), j0 = kChunk * c + k0;
+    const int64_t m0 = tile * kTileM + 16 * w + (lane >> 3);
+    const bool whole = j0 + 4 <= N, vec = whole && (((uintptr_t)a.ext | (uintptr_t)(8 * N)) & 15) == 0;
     float* w1ps = w1s + kFW1p;
-#pragma unroll 4
-    for (int i = 0; i < 16; ++i) {
-        const int p = 16 * w + i;
-        const int64_t m = m0 + i;
-        const bool ok = jin && m < a.B;
-        const double* z = a.ext + (size_t)m * NS * N + j;
-        const float z0 = ok ? (float)__ldg(z) : 0.f;
-        if (!REDRAW) {
-            w1s[ftile_at(p, lane)] = z0;
-            w1ps[ftile_at(p, lane)] = ok ? (float)__ldg(z + N) : 0.f;
-            if (MC) w1s[kFWq + ftile_at(p, lane)] = ok ? (float)__ldg(z + 2 * N) : 0.f;
-            if (a.dbg_w && m < a.B) {
-                a.dbg_w[(m * 2 + 0) * Np + j] = z0;
-                a.dbg_w[(m * 2 + 1) * Np + j] = w1ps[ftile_at(p, lane)];
+    double z[4][RD][4];
+    auto load = [&](int k) {
+        const int64_t m = m0 + 4 * k;
+        const double* row = a.ext + (size_t)m * NS * N + j0;
+#pragma unroll
+        for (int s = 0; s < RD; ++s) {
+            if (m < a.B && vec) {
+                const double2 u = __ldg((const double2*)(row + (size_t)s * N)), v = __ldg((const double2*)(row + (size_t)s * N) + 1);
+                z[k][s][0] = u.x; z[k][s][1] = u.y; z[k][s][2] = v.x; z[k][s][3] = v.y;
+            } else {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) z[k][s][q] = (m < a.B && j0 + q < N) ? __ldg(row + (size_t)s * N + q) : 0.0;
             }
         }
-        a_tile_store1<SK>(st, p, lane, z0);
-    }
-    // the next chunk's rows into L2 while this one is consumed: the loads above
-    // keep too few bytes in flight to cover HBM latency on their own.  One
-    // 128-byte line per 16 lanes; every address stays inside its row.
-    if ((lane & 15) == 0 && j + kChunk < N) {
-#pragma unroll 4
-        for (int i = 0; i < 16; ++i) {
-            if (m0 + i >= a.B) break;
-            const double* z = a.ext + (size_t)(m0 + i) * NS * N + j + kChunk;
+    };
 #pragma unroll
-            for (int s = 0; s < (REDRAW ? 1 : NS); ++s)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(z + (size_t)s * N));
+    for (int k = 0; k < LA; ++k) load(k);
+    // the rows of the chunk after the next into L2: one 128-byte line per 16 steps; every
+    // address stays inside its row
+    const int jp = kChunk * (c + 2) + 16 * (lane & 1), mp = 16 * w + (lane >> 1);
+    if (jp < N && tile * kTileM + mp < a.B) {
+        const double* row = a.ext + (size_t)(tile * kTileM + mp) * NS * N + jp;
+#pragma unroll
+        for (int s = 0; s < RD; ++s) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + (size_t)s * N));
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (k + LA < 4) load(k + LA);
+        const int p = 16 * w + 4 * k + (lane >> 3);
+        float f[RD][4];
+#pragma unroll
+        for (int s = 0; s < RD; ++s)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) f[s][q] = double_to_float(z[k][s][q]);
+        if (!REDRAW) {
+            const int at = ftile_at(p, k0);
+            *(float4*)(w1s + at) = make_float4(f[0][0], f[0][1], f[0][2], f[0][3]);
+            *(float4*)(w1ps + at) = make_float4(f[1][0], f[1][1], f[1][2], f[1][3]);
+            if (MC) *(float4*)(w1s + kFWq + at) = make_float4(f[RD - 1][0], f[RD - 1][1], f[RD - 1][2], f[RD - 1][3]);
+            if (a.dbg_w && m0 + 4 * k < a.B) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    a.dbg_w[((m0 + 4 * k) * 2 + 0) * Np + j0 + q] = f[0][q];
+                    a.dbg_w[((m0 + 4 * k) * 2 + 1) * Np + j0 + q] = f[1][q];
+                }
+            }
+        }
+        if constexpr (SK == 2) {
+            *(uint4*)(st + p * 128 + (((lane & 7) ^ (p & 7)) << 4)) =
+                make_uint4(tf32_rn(f[0][0]), tf32_rn(f[0][1]), tf32_rn(f[0][2]), tf32_rn(f[0][3]));
+        } else {
+            uint32_t h0, h1, l0, l1;
+            split2<SK>(f[0][0], f[0][1], h0, l0);
+            split2<SK>(f[0][2], f[0][3], h1, l1);
+            const int off = p * 64 + ((((lane & 7) >> 1) ^ ((p >> 1) & 3)) << 4) + ((lane & 1) << 3);
+            *(uint2*)(st + off) = make_uint2(h0, h1);
+            *(uint2*)(st + kTileBytes + off) = make_uint2(l0, l1);
         }
     }
     // last real chunk of a pass before the last: W1 (and Wperp) at step 32 (c + 1)
     // for the boundary rows
     if (!REDRAW && bnd && lane < 16) {
         const int p = 16 * w + lane;
-        const int64_t m = m0 + lane;
-        const double* z = a.ext + (size_t)m * NS * N + kChunk * (c + 1);
-        w1s[kFBnd + p] = m < a.B ? (float)__ldg(z) : 0.f;
-        if (MC) w1s[kFWqBnd + p] = m < a.B ? (float)__ldg(z + 2 * N) : 0.f;
+        const int64_t m = tile * kTileM + p;
+        const double* row = a.ext + (size_t)m * NS * N + kChunk * (c + 1);
+        w1s[kFBnd + p] = m < a.B ? (float)__ldg(row) : 0.f;
+        if (MC) w1s[kFWqBnd + p] = m < a.B ? (float)__ldg(row + 2 * N) : 0.f;
     }
 }
 
