@@ -375,68 +375,66 @@ struct FuseArgs {
 // The variance pass of a read-out warp on X of its 16 paths (x, without the
 // offset of 2^63), step j of the unit in lane order: per group and path the
 // warp's sums of 2^(2 t) and 2^t W over its 32 steps, v = xi 2^(2 t) (k_variance_fixed).
-// The sums are taken in integers: with 2^t = m 2^(e - 63) and E the largest e of
-// the 32 steps, m^2 is shifted right by 2 (E - e) + 5 and m W by E - e + 4, so 32
-// terms fit 64 bits, with a half unit back for the truncation (16 units of 32
-// terms).  The square's unit is 2^-57 of the largest term or less, the product's
-// 2^-54 2^E; an FP64 sum rounds every product to 2^-53 of itself and every partial
-// sum likewise.  The same in FP64 (two products, the lanes' additions) holds the
-// FP64 pipe: 2^16 paths of 250 steps, three sums, 313 us for the path pass against
-// 261.  132 warp instructions a path and group; four warps a scheduler do not hide
-// their latencies (0.55 a cycle).
+// The sums are taken in integers: with 2^t = m 2^(e - 63), E the largest e of the
+// 32 steps and m' = m >> (E - e + 3), 32 terms m'^2 and m' W / 2 fit 64 bits, and
+// half a unit a term goes back for the truncation.  The square's unit is 2^-54 of
+// the largest term or less, the product's 2^-54 2^E; an FP64 sum rounds every product
+// to 2^-53 of itself and every partial sum likewise.  The same in FP64 (two
+// products, the lanes' additions) holds the FP64 pipe: 2^16 paths of 250 steps, three
+// sums, 313 us for the path pass against 254.  Instructions and their latencies
+// bound it: four warps a scheduler issue one every second cycle.
+// Loads past the last step or path are clamped to it, and m is zero there.
 template <int NS>
 __device__ __forceinline__ void fused_variance(uint64_t (&x)[2][8], const X64Vol& vol, int grp0, const FuseArgs& fa,
                                                const uint64_t* E, int N, int64_t B, int64_t m0, int j, int slot)
 {
     const int lane = threadIdx.x & 31;
     const bool in = j + 1 < N;
+    const int jc = min(j, N - 2), left = (int)min(B - m0, (int64_t)16);  // paths of the warp's 16
+    const bool whole = left == 16 && __all_sync(0xffffffffu, in);
+    if (left <= 0) return;
+    const uint64_t* z0 = fa.Z + m0 * NS * (int64_t)N + jc;
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
-        const int64_t m = m0 + 4 * h;
         uint64_t xs[4], w1[4], wq[NS == 3 ? 4 : 1];
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
-            const bool ok = in && m + p < B;
-            const uint64_t* W1 = fa.Z + (m + p) * NS * (int64_t)N + j;
-            const uint64_t wp = ok ? W1[N] : 0ull;
-            w1[p] = ok ? W1[1] ^ (1ull << 63) : 0ull;
-            if (NS == 3) wq[p] = ok ? W1[2 * N + 1] ^ (1ull << 63) : 0ull;
-            xs[p] = x[h >> 1][(4 * h + p) & 7] + (1ull << 63) + mulhi64(wp ^ (1ull << 63), vol.a2f) - vol.a2h;
+            const uint64_t* W1 = z0 + (size_t)(min(4 * h + p, left - 1) * NS) * N;
+            // a signed w as 2^63 + w, and half of it
+            w1[p] = (W1[1] ^ (1ull << 63)) >> 1;
+            if (NS == 3) wq[p] = (W1[2 * N + 1] ^ (1ull << 63)) >> 1;
+            xs[p] = x[h >> 1][(4 * h + p) & 7] + (1ull << 63) + mulhi64(W1[N] ^ (1ull << 63), vol.a2f) - vol.a2h;
         }
 #pragma unroll 1
         for (int g = vol.vg_begin; g < vol.vg_end; ++g) {
-            const uint64_t cf = fa.grps[g].cf;
-            const bool neg = fa.grps[g].neg != 0;
-            const uint64_t cj = in ? __ldg(fa.comp + (size_t)g * N + j) : 0ull;
+            const uint64_t cf = fa.grps[g].cf, flip = fa.grps[g].neg ? ~0ull : 0ull;  // -x less one unit
+            const uint64_t cj = __ldg(fa.comp + (size_t)g * N + jc);
             int64_t s[8], sq[4];
             int top[4];
 #pragma unroll
             for (int p = 0; p < 4; ++p) {
-                const bool ok = in && m + p < B;
                 int32_t e;
-                uint64_t mt = exp2_mantissa53((int64_t)(mulhi64(neg ? 0ull - xs[p] : xs[p], cf) - cj), E, e);
-                if (!ok) {
+                uint64_t mt = exp2_mantissa53((int64_t)(mulhi64(xs[p] ^ flip, cf) - cj), E, e);
+                if (!whole && !(in && 4 * h + p < left)) {
                     mt = 0ull;
                     e = -1000;
                 }
                 top[p] = __reduce_max_sync(0xffffffffu, e);
-                const int d = top[p] - e;
-                const uint64_t hh = mul32(hi32(mt), lo32(mt)) >> 31;
-                const uint64_t sqr = mul32(hi32(mt), hi32(mt)) + hh;  // m^2 2^-64
-                s[2 * p] = (int64_t)(sqr >> min(5 + 2 * d, 63));
-                s[2 * p + 1] = (int64_t)(mulhi64(mt, w1[p]) - (mt >> 1)) >> min(4 + d, 63);
-                if (NS == 3) sq[p] = (int64_t)(mulhi64(mt, wq[p]) - (mt >> 1)) >> min(4 + d, 63);
+                mt >>= min(top[p] - e + 3, 63);
+                s[2 * p] = (int64_t)(mul32(hi32(mt), hi32(mt)) + (mul32(hi32(mt), lo32(mt)) >> 31));  // m'^2 2^-64
+                s[2 * p + 1] = (int64_t)(mulhi64(mt, w1[p]) - (mt >> 2));
+                if (NS == 3) sq[p] = (int64_t)(mulhi64(mt, wq[p]) - (mt >> 2));
             }
             const int64_t i0 = warp_sums_i64<8>(s) + 16;  // value lane / 4 = 2 path + sum
             const int pa = lane >> 3, c = (lane >> 2) & 1;
             const int tp = pa & 2 ? (pa & 1 ? top[3] : top[2]) : (pa & 1 ? top[1] : top[0]);
             const double sc = bits_double((uint64_t)(uint32_t)(tp + 1023) << 52);
-            double* out = fa.part + (((size_t)(g - grp0) * fa.slots + slot) * B + m + pa) * NS;
-            const double r = (c ? (double)i0 * 0x1p-54 : (double)(uint64_t)i0 * 0x1p-57 * sc) * sc;
-            if (!(lane & 3) && m + pa < B) out[c] = r;
+            double* out = fa.part + (((size_t)(g - grp0) * fa.slots + slot) * B + m0 + 4 * h + pa) * NS;
+            const double r = (c ? (double)i0 * 0x1p-54 : (double)i0 * 0x1p-56 * sc) * sc;
+            if (!(lane & 3) && 4 * h + pa < left) out[c] = r;
             if constexpr (NS == 3) {
                 const int64_t i2 = warp_sums_i64<4>(sq) + 16;
-                if (!(lane & 7) && m + pa < B) out[2] = (double)i2 * 0x1p-54 * sc;
+                if (!(lane & 7) && 4 * h + pa < left) out[2] = (double)i2 * 0x1p-54 * sc;
             }
         }
     }
@@ -476,10 +474,10 @@ struct PanelSlots {
 // TMEM, so the next block's MMAs wait for the read-out of this one's.
 // FUSE = NS > 0: the read-out warps also do the variance pass on their X, in
 // registers, while the next unit's MMAs run, and write the sums of their 32
-// steps per path and group instead of X: 512 steps, 2^17 paths, one group 1.06 ms
+// steps per path and group instead of X: 512 steps, 2^17 paths, one group 1.04 ms
 // with k_slot_sums, against 0.88 + 0.38 ms with X through memory and
 // k_variance_fixed, and 13.2 ms for the FP64 FFT convolution and exponentials; 100
-// steps, 2^16 paths 0.122 ms, against 0.133 and, for the direct FP64 sum, 1.46 ms.
+// steps, 2^17 paths 0.119 ms, against 0.133 and, for the direct FP64 sum, 1.46 ms.
 template <bool WIDE, bool SEG, int FUSE>
 __global__ void __launch_bounds__(kXThreads, 1) k_volterra_exact(const unsigned char* __restrict__ dig,
                                                                  const unsigned char* __restrict__ panels,
