@@ -89,6 +89,31 @@ __device__ __forceinline__ uint4 philox_group(uint64_t seed, uint64_t p, uint32_
     return philox_group(philox_keys(seed), p, g, s);
 }
 
+// A table of BYTES from global to shared memory by THREADS threads, 16 bytes a
+// load, every load in flight at once: store() after what else there is to do.
+template <int THREADS, int BYTES>
+struct TableCopy {
+    static_assert(BYTES % 16 == 0, "whole 16-byte words");
+    static constexpr int kPer = (BYTES / 16 + THREADS - 1) / THREADS;
+    uint4 r[kPer];
+    __device__ __forceinline__ explicit TableCopy(const void* src)
+    {
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const int i = threadIdx.x + k * THREADS;
+            if (i < BYTES / 16) r[k] = __ldg(static_cast<const uint4*>(src) + i);
+        }
+    }
+    __device__ __forceinline__ void store(void* dst) const
+    {
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const int i = threadIdx.x + k * THREADS;
+            if (i < BYTES / 16) static_cast<uint4*>(dst)[i] = r[k];
+        }
+    }
+};
+
 // Hardware approximations (PTX .approx instructions on the MUFU pipe).
 __device__ __forceinline__ float ex2_approx(float x)
 {

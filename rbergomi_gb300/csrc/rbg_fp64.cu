@@ -373,8 +373,8 @@ void launch_path_fp64(const Fp64Tables& t, const double* Z, int64_t B, double* i
 // and path, the strike-independent parts shared, against about 250 for library
 // log, exp, sqrt and two erfc each time (FP64 pipe: 64 cycles a warp
 // operation).  Blocks keep both tables in shared memory (50 KB) and walk over
-// (chunk, run of 8 outputs) tasks.  2^17 paths x 21 outputs: 1.17 -> 0.10 ms;
-// 8192 paths x 2112 outputs: 7.06 -> 0.50 ms.
+// (chunk, run of 8 outputs) tasks.  2^17 paths x 21 outputs: 1.17 -> 0.095
+// ms; 8192 paths x 2112 outputs: 7.06 -> 0.49 ms.
 constexpr int kOPB = 8;  // outputs per task
 constexpr int kPayThreads = 256;
 
@@ -391,22 +391,10 @@ struct PayoffSmem {
     double red[kPayThreads / 32][2 * kOPB];
 };
 
-template <int MC>
-__device__ __forceinline__ void payoff_tables(PayoffSmem<MC>& sm, const FixedTables* __restrict__ ft)
-{
-    for (int i = threadIdx.x; i < kExpTable; i += kPayThreads) sm.E[i] = ft->exp2[i];
-    if (!MC) {
-        const uint64_t* src = reinterpret_cast<const uint64_t*>(&ft->mills);
-        uint64_t* dst = reinterpret_cast<uint64_t*>(&sm.T);
-        for (int i = threadIdx.x; i < (int)(sizeof(MillsTable) / 8); i += kPayThreads) dst[i] = src[i];
-    }
-}
-
-// Outputs o0 .. o0 + 7 of the task, for the whole block.
+// Outputs o0 .. o0 + 7 of the task, by the first threads of the block.
 template <int MC>
 __device__ __forceinline__ void payoff_outs(PayoffSmem<MC>& sm, const Fp64Tables& t, int o0)
 {
-    __syncthreads();  // the previous task's readers (and the tables)
     if (threadIdx.x < kOPB) {
         const int i = o0 + (int)threadIdx.x;
         const OutDev od = (i < t.n_out) ? t.outs[i] : OutDev{0.0, 1.0, -1, 0};
@@ -415,6 +403,20 @@ __device__ __forceinline__ void payoff_outs(PayoffSmem<MC>& sm, const Fp64Tables
         sm.out[threadIdx.x] = OutF64{od.rho, od.K, (ok && !MC) ? log(od.K) : 0.0, MC ? sqrt(om) : om,
                                      -0.5 * od.rho * od.rho, od.vg, ok};
     }
+}
+
+// The tables, and the first task's outputs while they are on their way.  With 8-byte
+// loads a few at a time a block's first task waited 10 us longer: 2^16 paths x 5
+// outputs 32.8 -> 22.5 us.
+template <int MC>
+__device__ __forceinline__ void payoff_start(PayoffSmem<MC>& sm, const Fp64Tables& t, int o0,
+                                             const FixedTables* __restrict__ ft)
+{
+    const TableCopy<kPayThreads, kExpTable * 8> e(ft->exp2);
+    const TableCopy<kPayThreads, MC ? 16 : (int)sizeof(MillsTable)> m(&ft->mills);
+    payoff_outs<MC>(sm, t, o0);
+    e.store(sm.E);
+    if (!MC) m.store(&sm.T);
     __syncthreads();
 }
 
@@ -480,12 +482,16 @@ __global__ void __launch_bounds__(kPayThreads) k_payoff_sums(Fp64Tables t, const
 {
     extern __shared__ uint64_t psm[];
     PayoffSmem<MC>& sm = *reinterpret_cast<PayoffSmem<MC>*>(psm);
-    payoff_tables<MC>(sm, ft);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t tasks = (int64_t)nchunks * ((t.n_out + kOPB - 1) / kOPB);
+    payoff_start<MC>(sm, t, (int)(blockIdx.x / nchunks) * kOPB, ft);
     for (int64_t task = blockIdx.x; task < tasks; task += gridDim.x) {
         const int c = (int)(task % nchunks), o0 = (int)(task / nchunks) * kOPB;
-        payoff_outs<MC>(sm, t, o0);
+        if (task != blockIdx.x) {
+            __syncthreads();  // the previous task's readers
+            payoff_outs<MC>(sm, t, o0);
+            __syncthreads();
+        }
         double s[2 * kOPB];  // sums of x, then of x^2
 #pragma unroll
         for (int q = 0; q < 2 * kOPB; ++q) s[q] = 0.0;
@@ -996,12 +1002,16 @@ __global__ void __launch_bounds__(kPayThreads) k_payoff_store(Fp64Tables t, cons
 {
     extern __shared__ uint64_t psm[];
     PayoffSmem<MC>& sm = *reinterpret_cast<PayoffSmem<MC>*>(psm);
-    payoff_tables<MC>(sm, ft);
     const int64_t tiles = (B + kPayThreads - 1) / kPayThreads, tasks = tiles * ((t.n_out + nq - 1) / nq);
+    payoff_start<MC>(sm, t, (int)(blockIdx.x / tiles) * nq, ft);
     for (int64_t task = blockIdx.x; task < tasks; task += gridDim.x) {
         const int o0 = (int)(task / tiles) * nq;
         const int64_t m = task % tiles * kPayThreads + threadIdx.x;
-        payoff_outs<MC>(sm, t, o0);
+        if (task != blockIdx.x) {
+            __syncthreads();  // the previous task's readers
+            payoff_outs<MC>(sm, t, o0);
+            __syncthreads();
+        }
         if (m >= B) continue;
         RtState r;
         for (int q = 0; q < nq; ++q) {

@@ -128,9 +128,7 @@ __global__ void __launch_bounds__(kNormalThreads, 4) k_normals_fixed(uint64_t se
 {
     __shared__ NormalTables T;
     if (!F32) {
-        const uint64_t* src = reinterpret_cast<const uint64_t*>(&ft->normals);
-        uint64_t* dst = reinterpret_cast<uint64_t*>(&T);
-        for (int i = threadIdx.x; i < (int)(sizeof(NormalTables) / 8); i += kNormalThreads) dst[i] = src[i];
+        TableCopy<kNormalThreads, (int)sizeof(NormalTables)>(&ft->normals).store(&T);
         __syncthreads();
     }
     const int lane = threadIdx.x & 31, g = lane & 3, pl = lane >> 2;
@@ -380,8 +378,8 @@ struct FuseArgs {
 // half a unit a term goes back for the truncation.  The square's unit is 2^-54 of
 // the largest term or less, the product's 2^-54 2^E; an FP64 sum rounds every product
 // to 2^-53 of itself and every partial sum likewise.  The same in FP64 (two
-// products, the lanes' additions) holds the FP64 pipe: 2^16 paths of 250 steps, three
-// sums, 313 us for the path pass against 254.  Instructions and their latencies
+// products, the lanes' additions) holds the FP64 pipe: 30011 paths of 250 steps, two
+// passes, three sums, 313 us for the path pass against 254.  Instructions and their latencies
 // bound it: four warps a scheduler issue one every second cycle.
 // Loads past the last step or path are clamped to it, and m is zero there.
 template <int NS>
@@ -477,7 +475,7 @@ struct PanelSlots {
 // steps per path and group instead of X: 512 steps, 2^17 paths, one group 1.04 ms
 // with k_slot_sums, against 0.88 + 0.38 ms with X through memory and
 // k_variance_fixed, and 13.2 ms for the FP64 FFT convolution and exponentials; 100
-// steps, 2^17 paths 0.119 ms, against 0.133 and, for the direct FP64 sum, 1.46 ms.
+// steps, 2^16 paths 0.119 ms, against 0.133 and, for the direct FP64 sum, 1.46 ms.
 template <bool WIDE, bool SEG, int FUSE>
 __global__ void __launch_bounds__(kXThreads, 1) k_volterra_exact(const unsigned char* __restrict__ dig,
                                                                  const unsigned char* __restrict__ panels,
@@ -515,7 +513,7 @@ __global__ void __launch_bounds__(kXThreads, 1) k_volterra_exact(const unsigned 
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (FUSE)
-        for (int i = threadIdx.x; i < kExpTable; i += kXThreads) E[i] = fa.ft->exp2[i];
+        TableCopy<kXThreads, kExpTable * 8>(fa.ft->exp2).store(E);
     if (warp == kXEpiWarps + 1) {
         __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(holder)), "r"(512)
