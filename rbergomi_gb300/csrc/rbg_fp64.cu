@@ -632,7 +632,8 @@ __device__ void fix_split(const Fix128& a, int emax, double& S, double& C)
     C = neg ? -part[1] : part[1];
 }
 
-constexpr int kMergeThreads = 128;
+constexpr int kMergeThreads = 128;                  // that add up the chunks
+constexpr int kMergeBlock = kMergeThreads + 32;     // and the warp of the implied volatility
 struct MergeSmem {
     Fix128 s[kMergeThreads / 32][2];
     int emax[kMergeThreads / 32][2];
@@ -646,6 +647,13 @@ __device__ void merge_block(const double* __restrict__ part, int nchunks, int n_
                             bool fresh, MergeSmem& sm, double (&v)[4])
 {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (w >= kMergeThreads / 32) {  // waits for the sums with the others
+#pragma unroll
+        for (int k = 0; k < 3; ++k) __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = sm.out[k];
+        return;
+    }
     // the largest exponent of either sum
     int em[2] = {0, 0};
     for (int c = threadIdx.x; c < nchunks; c += kMergeThreads) {
@@ -756,6 +764,23 @@ __device__ __forceinline__ double log_ratio(double e)
     return fma(e * e, s, e);
 }
 
+// What implied_vol_warp needs of strike and maturity alone; p0: the lane's price
+// on the geometric grid.
+struct IvStart {
+    double lnK, sqT;
+    float lnK1, sqT32, p0;
+};
+__device__ __forceinline__ IvStart iv_start(double K, double T)
+{
+    IvStart r;
+    r.lnK = log(K);
+    r.sqT = sqrt(T);
+    r.lnK1 = -log1pf((float)(K - 1.0));
+    r.sqT32 = sqrtf((float)T);
+    r.p0 = bs_gen_f32(r.lnK1, r.sqT32, (float)K, 1e-3f * exp2f(0.5f * (threadIdx.x & 31)), 1.0 > K);
+    return r;
+}
+
 // Implied vol by a warp: inverts on the out-of-the-money side (put-call
 // parity for K < 1, as rBergLib/BlackScholes.cpp:38-41 does).  The 32 lanes
 // price 32 volatilities at once:
@@ -777,7 +802,8 @@ __device__ __forceinline__ double log_ratio(double e)
 // Prices are Mills' ratios (otm_price): the density they contain is the vega,
 // so an FP64 step is one short chain.  All lanes
 // return the same value; NaN when no volatility fits.
-__device__ double implied_vol_warp(double price, double K, double T, const FixedTables* __restrict__ ft)
+__device__ double implied_vol_warp(double price, double K, double T, const IvStart& st,
+                                   const FixedTables* __restrict__ ft)
 {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -786,14 +812,14 @@ __device__ double implied_vol_warp(double price, double K, double T, const Fixed
     const double upper = put ? K : 1.0;
     const double nan = __longlong_as_double(0x7ff8000000000000ll);
     if (!(target > 0.0) || !(target < upper) || !(T > 0.0)) return nan;
-    const double lnK = log(K), sqT = sqrt(T);
-    const float lnK1 = -log1pf((float)(K - 1.0)), sqT32 = sqrtf((float)T), K32 = (float)K, t32 = (float)target;
+    const double lnK = st.lnK, sqT = st.sqT;
+    const float lnK1 = st.lnK1, sqT32 = st.sqT32, K32 = (float)K, t32 = (float)target;
     double lo = 0.0, hi = 0.0, s = 0.0;
     bool narrowed = false;
     OtmPrice q{};
     {
         // FP32 grid and rounds, then the FP64 check
-        const unsigned b32 = __ballot_sync(FULL, bs_gen_f32(lnK1, sqT32, K32, 1e-3f * exp2f(0.5f * lane), put) >= t32);
+        const unsigned b32 = __ballot_sync(FULL, st.p0 >= t32);
         if (b32 != 0u) {
             const int f = __ffs(b32) - 1;
             float lo32 = (f > 0) ? 1e-3f * exp2f(0.5f * (f - 1)) : 0.f, hi32 = 1e-3f * exp2f(0.5f * f);
@@ -887,47 +913,59 @@ __device__ double implied_vol_warp(double price, double K, double T, const Fixed
     return s;
 }
 
-// Output i's price, stat and implied vol from its sums v (one warp).
+// Output i of a merge: its sums, price and stat by the first thread, its implied
+// volatility by the last warp, which takes what depends on strike and maturity
+// alone (logarithm, root, the FP32 grid) while the others add up the chunks.
 // res: [0,n) price, [n,2n) stat, [2n,3n) iv, [3n,4n) sum, [4n,5n) sum2.
-__device__ __forceinline__ void finalize_warp(const double (&v)[4], int n_out, double invM, double isqM,
-                                              const OutDev* __restrict__ outs, const double* __restrict__ Tv,
-                                              int compute_iv, double* __restrict__ res, int i,
-                                              const FixedTables* __restrict__ ft)
+__device__ __forceinline__ void merge_finish(const double* __restrict__ part, int nchunks, int n_out,
+                                             double* __restrict__ acc, int i, bool fresh, double invM, double isqM,
+                                             const OutDev* __restrict__ outs, const double* __restrict__ Tv,
+                                             int compute_iv, double* __restrict__ res,
+                                             const FixedTables* __restrict__ ft, MergeSmem& sm)
 {
+    double v[4];
+    const bool solve = threadIdx.x >= kMergeThreads && res;
+    double K = 1.0, T = 1.0;
+    IvStart start{};
+    if (solve && compute_iv) {
+        K = outs[i].K;
+        T = Tv[i];
+        start = iv_start(K, T);
+    }
+    merge_block(part, nchunks, n_out, acc, i, fresh, sm, v);
+    if (!res) return;
     const double S = v[0] + v[1];
-    const double S2 = v[2] + v[3];
-    // rBergLib/rBergomiMT.cpp:404-409
     const double price = S * invM;
-    const double var = 1.0 * (S2 * invM) + -1.0 * (price * price);
-    const double stat = sqrt(var) * isqM;
-    const double iv = compute_iv ? implied_vol_warp(price, outs[i].K, Tv[i], ft) : 0.0;
-    if ((threadIdx.x & 31) == 0) {
+    if (solve) {
+        const double iv = compute_iv ? implied_vol_warp(price, K, T, start, ft) : 0.0;
+        if (threadIdx.x == kMergeThreads) res[2 * n_out + i] = iv;
+    } else if (threadIdx.x == 0) {
+        // rBergLib/rBergomiMT.cpp:404-409
+        const double S2 = v[2] + v[3];
+        const double var = 1.0 * (S2 * invM) + -1.0 * (price * price);
         res[i] = price;
-        res[n_out + i] = stat;
-        res[2 * n_out + i] = iv;
+        res[n_out + i] = sqrt(var) * isqM;
         res[3 * n_out + i] = S;
         res[4 * n_out + i] = S2;
     }
 }
 
 // One block per output: its chunk sums into acc and, after the call's last
-// batch (res non-null), the price, stat and implied vol by the first warp.
-__global__ void __launch_bounds__(kMergeThreads) k_merge(const double* __restrict__ part, int nchunks, int n_out,
-                                                        double* __restrict__ acc, int fresh, double invM, double isqM,
-                                                        const OutDev* __restrict__ outs, const double* __restrict__ Tv,
-                                                        int compute_iv, double* __restrict__ res,
-                                                        const FixedTables* __restrict__ ft)
+// batch (res non-null), the price, stat and implied vol.
+__global__ void __launch_bounds__(kMergeBlock) k_merge(const double* __restrict__ part, int nchunks, int n_out,
+                                                      double* __restrict__ acc, int fresh, double invM, double isqM,
+                                                      const OutDev* __restrict__ outs, const double* __restrict__ Tv,
+                                                      int compute_iv, double* __restrict__ res,
+                                                      const FixedTables* __restrict__ ft)
 {
     __shared__ MergeSmem sm;
-    double v[4];
-    merge_block(part, nchunks, n_out, acc, blockIdx.x, fresh != 0, sm, v);
-    if (res && threadIdx.x < 32) finalize_warp(v, n_out, invM, isqM, outs, Tv, compute_iv, res, blockIdx.x, ft);
+    merge_finish(part, nchunks, n_out, acc, blockIdx.x, fresh != 0, invM, isqM, outs, Tv, compute_iv, res, ft, sm);
 }
 
 // Job-table form: block b is output b - jobs[k].block0 of job k (both tables).
-__global__ void __launch_bounds__(kMergeThreads) k_merge_jobs(const AccJob* __restrict__ jobs,
-                                                             const FinJob* __restrict__ fins, int n_jobs,
-                                                             const FixedTables* __restrict__ ft)
+__global__ void __launch_bounds__(kMergeBlock) k_merge_jobs(const AccJob* __restrict__ jobs,
+                                                           const FinJob* __restrict__ fins, int n_jobs,
+                                                           const FixedTables* __restrict__ ft)
 {
     __shared__ MergeSmem sm;
     int lo = 0, hi = n_jobs - 1;
@@ -938,16 +976,14 @@ __global__ void __launch_bounds__(kMergeThreads) k_merge_jobs(const AccJob* __re
     const AccJob& J = jobs[lo];
     const FinJob& F = fins[lo];
     const int i = (int)((int64_t)blockIdx.x - J.block0);
-    double v[4];
-    merge_block(J.part, J.nchunks, J.n_out, J.acc, i, true, sm, v);
-    if (threadIdx.x < 32) finalize_warp(v, J.n_out, F.invM, F.isqM, F.outs, F.Tv, F.compute_iv, F.res, i, ft);
+    merge_finish(J.part, J.nchunks, J.n_out, J.acc, i, true, F.invM, F.isqM, F.outs, F.Tv, F.compute_iv, F.res, ft, sm);
 }
 
 int launch_merge_jobs(const AccJob* jobs, const FinJob* fins, int n_jobs, int64_t blocks, void* stream)
 {
     const FixedTables* ft = fixed_tables();
     if (!ft) return -1;
-    k_merge_jobs<<<(unsigned)blocks, kMergeThreads, 0, (cudaStream_t)stream>>>(jobs, fins, n_jobs, ft);
+    k_merge_jobs<<<(unsigned)blocks, kMergeBlock, 0, (cudaStream_t)stream>>>(jobs, fins, n_jobs, ft);
     count_launch();
     return 0;
 }
@@ -968,7 +1004,7 @@ int launch_merge(const double* part, int nchunks, int n_out, double* acc, bool f
     const FixedTables* ft = fixed_tables();
     if (!ft) return -1;
     const MergeFinal f = fin ? *fin : MergeFinal{};
-    k_merge<<<n_out, kMergeThreads, 0, (cudaStream_t)stream>>>(
+    k_merge<<<n_out, kMergeBlock, 0, (cudaStream_t)stream>>>(
         part, nchunks, n_out, acc, fresh ? 1 : 0, fin ? 1.0 / (double)f.M : 0.0, fin ? 1.0 / std::sqrt((double)f.M) : 0.0,
         f.outs, f.Tv, f.compute_iv, f.res, ft);
     count_launch();
@@ -980,7 +1016,7 @@ __global__ void k_implied_vol(int n, const double* price, const double* K, const
 {
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (i >= n) return;
-    const double v = implied_vol_warp(price[i], K[i], T[i], ft);
+    const double v = implied_vol_warp(price[i], K[i], T[i], iv_start(K[i], T[i]), ft);
     if ((threadIdx.x & 31) == 0) iv[i] = v;
 }
 
@@ -1230,7 +1266,7 @@ __global__ void k_finalize_cv(const double* __restrict__ acc, int n_out, int64_t
     const double p = (double)count[i] / (double)M, r = outs[i].rho, K = outs[i].K;
     const double adj = (1.0 - p) * bs_call_tau1(1.0, K, sqrt(r * r * Q[i])) + p * bs_call_tau1(1.0, K, sqrt(r * r * Qmax));
     const double price = mean - alpha[i] * adj;
-    const double iv = compute_iv ? implied_vol_warp(price, K, Tv[i], ft) : 0.0;
+    const double iv = compute_iv ? implied_vol_warp(price, K, Tv[i], iv_start(K, Tv[i]), ft) : 0.0;
     if ((threadIdx.x & 31) == 0) {
         res[i] = price;
         res[n_out + i] = stat;
