@@ -39,14 +39,6 @@ RBG_HD uint64_t mulhi64(uint64_t a, uint64_t b)
 {
     return mul32(hi32(a), hi32(b)) + (mul32(hi32(a), lo32(b)) >> 32) + (mul32(lo32(a), hi32(b)) >> 32);
 }
-RBG_HD int clz64(uint64_t x)
-{
-#ifdef __CUDA_ARCH__
-    return __clzll((long long)x);
-#else
-    return x ? __builtin_clzll(x) : 64;
-#endif
-}
 RBG_HD double bits_double(uint64_t b)
 {
 #ifdef __CUDA_ARCH__

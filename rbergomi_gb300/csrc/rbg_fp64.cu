@@ -10,12 +10,13 @@
 //   k_path_fp64_fft  the same pass with Y2 as an FP64 FFT convolution, two
 //                  paths per complex transform (from 200 steps; the direct
 //                  sum's N^2 / 2 DFMA per path outgrow it there)
-//   k_payoff_sums  conditional BS per (path, output) and compensated per-chunk
-//                  sums of x and x^2 (rBergomiMT.cpp:598-602, 404-409)
+//   k_payoff_sums  conditional BS per (path, output) and per-chunk sums of x and
+//                  x^2 (rBergomiMT.cpp:598-602, 404-409)
 //   k_merge        exact merge of chunk sums (deterministic); after the last
 //                  batch price, stat (reference formula), implied vol
 //   k_payoff_store per-path payoffs for the quadrature entry point
-// GB300's FP64 pipe (~2 DFMA/clk/SM) bounds every kernel here.
+// GB300's FP64 pipe (~2 DFMA/clk/SM) bounds the path kernels here, and the payoffs
+// although their elementary functions are in fixed point (rbg_fixed.cuh).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -445,10 +446,13 @@ __device__ __forceinline__ double payoff_rt(RtState& r, const OutF64& o, const d
     return call_fixed(r.s, o.K, o.lnK, sm.T, sm.E);
 }
 
+// Plain Monte Carlo payoff (rBergLib/rBergomiMT.cpp:134-136 updateZ, :129-132
+// scaleZ, :111-116 updateS, aux.h:31-34 posPart): with Z = rho W1 + sqrt(1 - rho^2) Wperp,
+// log S = sum sqrt(v) sdt Z - dt/2 sum v = rho IsvdW + sqrt(1 - rho^2) IsvdWp
+// - Ivdt / 2, the same sum regrouped by normal stream; the exponential in fixed point.
 __device__ __forceinline__ double payoff_mc(const OutF64& o, const double2* __restrict__ ivb,
                                             const double* __restrict__ ivp, size_t at, const PayoffSmem<1>& sm)
 {
-    // mc_payoff's log S, the exponential in fixed point
     const double2 iv = ivb[at];
     const double lnS = o.rho * iv.y + o.om * ivp[at] - 0.5 * iv.x;
     const double d = (fabs(lnS) < 60.0 ? exp2_fixed53(log2e_fixed53(lnS), sm.E) : exp(lnS)) - o.K;

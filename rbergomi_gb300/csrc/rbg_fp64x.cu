@@ -1,18 +1,22 @@
-// rbg_fp64x.cu -- the FP64 form on Philox normals: exact convolution on the
-// tensor cores, elementary functions in 64-bit fixed point.
+// rbg_fp64x.cu -- the FP64 form on Philox normals and on the caller's: exact
+// convolution on the tensor cores, elementary functions in 64-bit fixed point.
 //
 // GB300's FP64 pipe (2 DFMA per clock and SM) bounds every kernel that does
 // its arithmetic in FP64.  These do it elsewhere, with no less precision:
 //   k_normals_fixed  Philox4x32-10 -> Box-Muller in 64-bit integers
-//                    (rbg_fixed.cuh) -> FP64 normals, quadrature layout, and
-//                    W1 as eight signed 8-bit digits in FP16 for the next
+//                    (rbg_fixed.cuh) -> normals, quadrature layout, FP64 or
+//                    fixed point, and W1 as eight signed 8-bit digits in FP16
+//                    for the next
+//   k_digits         the digits of the caller's W1
 //   k_volterra_exact X_j = sum_{k<=j} W1_k Gamma'_{j-k}, Gamma' = (a1, Gamma_1,
 //                    ...), as digit products on tcgen05: both operands are
 //                    64-bit fixed-point numbers cut into 8 signed digits, and
 //                    the digit products of weight 2^(-8 d), d = i + j <= 7, are
 //                    summed in one FP32 accumulator each
 //   k_variance_fixed X + a2 W1perp, v = xi 2^t with t and 2^t in 64-bit fixed
-//                    point, FP64 sums of v and sqrt(v) W1 (, Wperp)
+//                    point, FP64 sums of v and sqrt(v) W1 (, Wperp); with few
+//                    variance groups inside k_volterra_exact instead, k_slot_sums
+//                    adding up its parts
 //
 // Exactness of the convolution.  A digit is an integer in [-128, 127], exact in
 // FP16; a product has 14 bits, and an FP32 accumulator holds integers up to
@@ -117,7 +121,7 @@ __device__ __forceinline__ void store_digits(const int64_t (&v)[4], unsigned cha
 // path and four steps a lane, so a path's 16 values and each digit's 8 rows are
 // contiguous.  Integer instructions bound it: 368 a warp and pair of normals, 64
 // of them 32 x 32 -> 64 multiplies (four cycles each).  2 x 512 steps, 2^17
-// paths: 0.95 ms, against 5.40 ms for the same draw in FP64 (table-driven
+// paths: 0.95 ms (0.91 left in fixed point), against 5.40 ms for the same draw in FP64 (table-driven
 // logarithm and sine, about 40 FP64 operations a pair).
 constexpr int kNormalThreads = 256, kSeg = 8;
 template <int F32>

@@ -1776,7 +1776,7 @@ done:
 constexpr int kOPB32 = 8;
 
 // Plain Monte Carlo payoff in FP32: S_T = exp(rho IsvdW + sqrt(1 - rho^2) IsvdWp
-// - Ivdt / 2) (the FP64 form's mc_payoff), payoff max(S_T - K, 0).
+// - Ivdt / 2) (the FP64 form's payoff_mc), payoff max(S_T - K, 0).
 __device__ __forceinline__ float mc_payoff_f32(float Ivdt, float IsvdW, float IsvdWp, float rho, float K)
 {
     const float lnS = fmaf(rho, IsvdW, fmaf(sqrtf(fmaxf(1.0f - rho * rho, 0.0f)), IsvdWp, -0.5f * Ivdt));
