@@ -343,6 +343,10 @@ def run_gpu(args, w):
         return
     stage = R.STAGE_MIXED if prec == R.MIXED else R.STAGE_PATH_FP64
     kms, kn = R.profile_read(stage)
+    # the FP64 form's own path pass is two kernels a batch (convolution with the variance pass, its sums)
+    fp64_exact = prec != R.MIXED and args.conv == "auto" and 2 <= w["N"] <= 4096
+    if fp64_exact:
+        kn //= 2
     avg_kernel_ms = kms / max(kn, 1)
     bf16_peak, hbm_peak, peak_src = peaks()
     algo_flops = w["M"] * w["N"] * (w["N"] - 1) * len(set(w["H"])) / max(1, kn // args.steps)
@@ -353,7 +357,8 @@ def run_gpu(args, w):
     exec_flops = (4.0 if args.split == 2 else 6.0) * 32 * 32 * nc * (nc + 1) / 2 * w["M"] / max(1, kn // args.steps)
     fp64_fft = args.conv == "fft" or (args.conv == "auto" and 200 <= w["N"] <= 2048)
     kname = ("k_mixed_fft" if (args.conv == "fft" or (args.conv == "auto" and w["N"] > 1024))
-             else "k_mixed_gemm") if prec == R.MIXED else ("k_path_fp64_fft" if fp64_fft else "k_path_fp64")
+             else "k_mixed_gemm") if prec == R.MIXED else ("k_volterra_exact + k_slot_sums" if fp64_exact else
+                                                "k_path_fp64_fft" if fp64_fft else "k_path_fp64")
     roof = {"bound": "tensor", "achieved": achieved_tf, "peak": bf16_peak, "unit": "TFLOP/s",
             "frac": achieved_tf / bf16_peak, "traffic": traffic_per_launch(kname, w),
             "kernel": kname,
