@@ -119,10 +119,11 @@ __device__ __forceinline__ void store_digits(const int64_t (&v)[4], unsigned cha
 // fixed point (unit 2^-59) in place of doubles.
 // A warp takes up to kSeg chunks of 16 steps of 8 paths' stream, four lanes a
 // path and four steps a lane, so a path's 16 values and each digit's 8 rows are
-// contiguous.  Integer instructions bound it: 368 a warp and pair of normals, 64
-// of them 32 x 32 -> 64 multiplies (four cycles each).  2 x 512 steps, 2^17
-// paths: 0.95 ms (0.91 left in fixed point), against 5.40 ms for the same draw in FP64 (table-driven
-// logarithm and sine, about 40 FP64 operations a pair).
+// contiguous.  Integer instructions bound it: 330 a warp and pair of normals, 57
+// of them 32 x 32 -> 64 multiplies (four cycles each): the FMA-heavy pipe is 78 %
+// busy.  2 x 512 steps, 2^17 paths, left in fixed point: 0.84 ms, against 5.40 ms
+// for the same draw in FP64 (table-driven logarithm and sine, about 40 FP64
+// operations a pair).
 constexpr int kNormalThreads = 256, kSeg = 8;
 template <int F32>
 __global__ void __launch_bounds__(kNormalThreads, 4) k_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int ns,
