@@ -387,7 +387,10 @@ struct FuseArgs {
 // passes, three sums, 313 us for the path pass against 254.  Instructions and their latencies
 // bound it: four warps a scheduler issue one every second cycle.
 // Loads past the last step or path are clamped to it, and m is zero there.
-template <int NS>
+// ONE: the pass has one group; without the loop over groups the four quarters
+// of the paths overlap (two sums, 100 steps, 2^16 paths 117 -> 111 us; 512 steps, 2^17
+// 1.045 -> 1.03 ms; with three sums it is slower, 254 -> 266 us for the case above).
+template <int NS, bool ONE>
 __device__ __forceinline__ void fused_variance(uint64_t (&x)[2][8], const X64Vol& vol, int grp0, const FuseArgs& fa,
                                                const uint64_t* E, int N, int64_t B, int64_t m0, int j, int slot)
 {
@@ -409,7 +412,7 @@ __device__ __forceinline__ void fused_variance(uint64_t (&x)[2][8], const X64Vol
             xs[p] = x[h >> 1][(4 * h + p) & 7] + (1ull << 63) + mulhi64(W1[N] ^ (1ull << 63), vol.a2f) - vol.a2h;
         }
 #pragma unroll 1
-        for (int g = vol.vg_begin; g < vol.vg_end; ++g) {
+        for (int g = vol.vg_begin; g < (ONE ? vol.vg_begin + 1 : vol.vg_end); ++g) {
             const uint64_t cf = fa.grps[g].cf, flip = fa.grps[g].neg ? ~0ull : 0ull;  // -x less one unit
             const uint64_t cj = __ldg(fa.comp + (size_t)g * N + jc);
             int64_t s[8], sq[4];
@@ -475,12 +478,12 @@ struct PanelSlots {
 // What bounds it: 2304 columns x 128 steps x 16 per chunk, 1152 MMA cycles,
 // against 16 KB of digits and 7.5 KB of panel from L2; the accumulators fill
 // TMEM, so the next block's MMAs wait for the read-out of this one's.
-// FUSE = NS > 0: the read-out warps also do the variance pass on their X, in
+// FUSE > 0 (sums per path: 2 or 3; 1: two, one group a pass): the read-out warps also do the variance pass on their X, in
 // registers, while the next unit's MMAs run, and write the sums of their 32
-// steps per path and group instead of X: 512 steps, 2^17 paths, one group 1.04 ms
+// steps per path and group instead of X: 512 steps, 2^17 paths, one group 1.03 ms
 // with k_slot_sums, against 0.88 + 0.38 ms with X through memory and
 // k_variance_fixed, and 13.2 ms for the FP64 FFT convolution and exponentials; 100
-// steps, 2^16 paths 0.119 ms, against 0.133 and, for the direct FP64 sum, 1.46 ms.
+// steps, 2^16 paths 0.111 ms, against 0.133 and, for the direct FP64 sum, 1.46 ms.
 template <bool WIDE, bool SEG, int FUSE>
 __global__ void __launch_bounds__(kXThreads, 1) k_volterra_exact(const unsigned char* __restrict__ dig,
                                                                  const unsigned char* __restrict__ panels,
@@ -727,7 +730,7 @@ __global__ void __launch_bounds__(kXThreads, 1) k_volterra_exact(const unsigned 
                 uint64_t xs[2][8];
                 read8(p0, xs[0], false);
                 read8(p0 + 8, xs[1], true);
-                fused_variance<FUSE>(xs, vols[v], vols[0].vg_begin, fa, E, N, B, g * kXPaths + p0, j, 4 * b + quad);
+                fused_variance<FUSE == 1 ? 2 : FUSE, FUSE == 1>(xs, vols[v], vols[0].vg_begin, fa, E, N, B, g * kXPaths + p0, j, 4 * b + quad);
             }
           }
         }
@@ -801,7 +804,9 @@ int launch_volterra_variance(const unsigned char* dig, const unsigned char* pane
     const FixedTables* ft = fixed_tables();
     if (!ft) return -1;
     const bool wide = N > 1024;
+    const bool one = ng == nv;  // every pass has at least one group
     auto* kern = ns == 3 ? (wide ? k_volterra_exact<true, false, 3> : k_volterra_exact<false, false, 3>)
+                 : one   ? (wide ? k_volterra_exact<true, false, 1> : k_volterra_exact<false, false, 1>)
                          : (wide ? k_volterra_exact<true, false, 2> : k_volterra_exact<false, false, 2>);
     if (!allow_smem((const void*)kern, kXSmemFused)) return -1;
     const int slots = 4 * x64_blocks(N);
