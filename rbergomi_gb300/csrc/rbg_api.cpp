@@ -250,6 +250,16 @@ static int ensure(DevBuf& b, size_t bytes, const char* what)
     return RBG_OK;
 }
 
+// The FP64 form's digit and X (or sum) buffers.  Without room for them the call
+// goes on with the FP64 kernels, which need neither.
+static bool ensure_fixed(Ctx& c, size_t digits, size_t paths)
+{
+    if (!c.xdig.ensure(digits) && !c.xbuf.ensure(paths)) return true;
+    c.xdig.release();
+    c.xbuf.release();
+    return false;
+}
+
 // ---------------------------------------------------------------- tables
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
@@ -449,28 +459,28 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
     // Philox normals, no backend asked for: the exact tensor-core convolution and
     // fixed-point functions wherever the plan's numbers fit their ranges
     X64Tables xt;
-    const bool fixed = o.conv == RBG_CONV_AUTO && !sobol_vt && x64_prepare(plan, xt);
+    bool fixed = o.conv == RBG_CONV_AUTO && !sobol_vt && x64_prepare(plan, xt);
     int rc = fixed ? RBG_OK : fp64_conv_log2(o.conv, plan.N, &logL);
     if (rc) return rc;
-    if ((rc = upload_tables(c, plan, st, ts, logL, fixed ? &xt : nullptr, !fixed))) return rc;
     const int no = (int)plan.outs.size(), N = plan.N, ns = mc ? 3 : 2, nv = (int)plan.vols.size();
     const int64_t B = fp64_batch(plan, M, ns);
-    // The variance pass inside the convolution's read-out for up to x64_fuse_groups
-    // variance groups a pass, where its sums (one value per group, path and 32 steps)
-    // stay within X's limit of 2 GiB for one pass.
-    const size_t sums = (size_t)std::max(xt.max_groups, 1) * x64_slot_bytes(B, N, ns);
-    const bool fused = fixed && xt.u53 && xt.max_groups <= x64_fuse_groups(ns) && sums <= ((size_t)1 << 31);
-    const size_t per = fused ? sums : 8 * (size_t)N * (size_t)B;
-    // passes per convolution launch: X or the sums within 2 GiB
-    const int vstep = (int)std::max<int64_t>(1, std::min<int64_t>(nv, ((int64_t)1 << 31) / (int64_t)per));
-    if (fixed) {
-        if ((rc = ensure(c.xdig, x64_digit_bytes(B, N), "normal digits"))) return rc;
-        if ((rc = ensure(c.xbuf, (size_t)vstep * per, "Volterra paths"))) return rc;
-    }
     if ((rc = ensure(c.z, sizeof(double) * ns * N * (size_t)B, "normals"))) return rc;
     if ((rc = ensure(c.ivb, sizeof(double) * 2 * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
     if (mc && (rc = ensure(c.ivp, sizeof(double) * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
     double* ivp = mc ? c.ivp.as<double>() : nullptr;
+    // The variance pass inside the convolution's read-out for up to x64_fuse_groups
+    // variance groups a pass, where its sums (one value per group, path and 32 steps)
+    // stay within X's limit of 2 GiB for one pass.
+    const size_t sums = (size_t)std::max(xt.max_groups, 1) * x64_slot_bytes(B, N, ns);
+    const bool fused = xt.u53 && xt.max_groups <= x64_fuse_groups(ns) && sums <= ((size_t)1 << 31);
+    const size_t per = fused ? sums : 8 * (size_t)N * (size_t)B;
+    // passes per convolution launch: X or the sums within 2 GiB
+    const int vstep = (int)std::max<int64_t>(1, std::min<int64_t>(nv, ((int64_t)1 << 31) / (int64_t)per));
+    if (fixed && !ensure_fixed(c, x64_digit_bytes(B, N), (size_t)vstep * per)) {
+        fixed = false;
+        if ((rc = fp64_conv_log2(o.conv, N, &logL))) return rc;
+    }
+    if ((rc = upload_tables(c, plan, st, ts, logL, fixed ? &xt : nullptr, !fixed))) return rc;
     const int G = payoff_paths_per_thread(B, device_sms());
     const int64_t max_chunks = (B + 256 * (int64_t)G - 1) / (256 * (int64_t)G);
     if ((rc = ensure(c.part, sizeof(double) * 4 * no * (size_t)max_chunks, "partials"))) return rc;
@@ -489,7 +499,7 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
                     return fail(RBG_ERR_UNSUPPORTED, "Brownian bridge shared memory not available for this N");
             } else if (launch_normals_fixed(o.seed, o.path_offset + m0, b, N, o.normals == RBG_NORMALS_F32,
                                             c.z.as<double>(), fixed ? c.xdig.as<unsigned char>() : nullptr,
-                                            fused ? kFixAll : (fixed ? kFixW1perp : 0), ns, st)) {
+                                            !fixed ? 0 : (fused ? kFixAll : kFixW1perp), ns, st)) {
                 return fail(RBG_ERR_CUDA, "normal tables could not be set up");
             }
         }
@@ -935,9 +945,8 @@ static int payoffs_quadrature(const rbg_params* p, const double* Z, double* payo
     // no backend asked for: the exact tensor-core convolution and fixed-point
     // functions; a batch with normals outside their range takes the direct FP64 sum
     X64Tables xt;
-    const bool fixed = conv == RBG_CONV_AUTO && x64_prepare(plan, xt, true);
+    bool fixed = conv == RBG_CONV_AUTO && x64_prepare(plan, xt, true);
     if (!fixed && (rc = fp64_conv_log2(conv, plan.N, &logL))) return rc;
-    if ((rc = upload_tables(*c, plan, st, ts, logL, fixed ? &xt : nullptr))) return rc;
     const int no = (int)plan.outs.size(), N = plan.N, ns = mc ? 3 : 2, nv = (int)plan.vols.size();
     const int64_t M = p->M;
     int64_t B = fp64_batch(plan, M, ns);
@@ -947,14 +956,15 @@ static int payoffs_quadrature(const rbg_params* p, const double* Z, double* payo
     if ((rc = ensure(c->ivb, sizeof(double) * 2 * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
     if (mc && (rc = ensure(c->ivp, sizeof(double) * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
     double* ivp = mc ? c->ivp.as<double>() : nullptr;
-    if (fixed) {
-        if ((rc = ensure(c->xdig, x64_digit_bytes(B, N), "normal digits"))) return rc;
-        if ((rc = ensure(c->xbuf, 8 * (size_t)vstep * N * (size_t)B, "Volterra paths"))) return rc;
-    }
     if (!device_ptrs) {
         if ((rc = ensure(c->z, sizeof(double) * ns * N * (size_t)B, "normals"))) return rc;
         if ((rc = ensure(c->pay, sizeof(double) * no * (size_t)B, "payoffs"))) return rc;
     }
+    if (fixed && !ensure_fixed(*c, x64_digit_bytes(B, N), 8 * (size_t)vstep * N * (size_t)B)) {
+        fixed = false;
+        if ((rc = fp64_conv_log2(conv, N, &logL))) return rc;
+    }
+    if ((rc = upload_tables(*c, plan, st, ts, logL, fixed ? &xt : nullptr))) return rc;
     // device words: kernel error, normals out of range
     if ((rc = ensure(c->acc, 2 * sizeof(unsigned int), "accumulators"))) return rc;
     unsigned int* words = c->acc.as<unsigned int>();

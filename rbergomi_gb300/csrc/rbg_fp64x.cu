@@ -478,9 +478,10 @@ struct PanelSlots {
 // What bounds it: 2304 columns x 128 steps x 16 per chunk, 1152 MMA cycles,
 // against 16 KB of digits and 7.5 KB of panel from L2; the accumulators fill
 // TMEM, so the next block's MMAs wait for the read-out of this one's.
-// FUSE > 0 (sums per path: 2 or 3; 1: two, one group a pass): the read-out warps also do the variance pass on their X, in
-// registers, while the next unit's MMAs run, and write the sums of their 32
-// steps per path and group instead of X: 512 steps, 2^17 paths, one group 1.03 ms
+// FUSE > 0 (sums per path: 2 or 3; 1: two, one group a pass): the read-out warps
+// also do the variance pass on their X, in registers, while the next unit's MMAs
+// run, and write the sums of their 32 steps per path and group instead of X:
+// 512 steps, 2^17 paths, one group 1.03 ms
 // with k_slot_sums, against 0.88 + 0.38 ms with X through memory and
 // k_variance_fixed, and 13.2 ms for the FP64 FFT convolution and exponentials; 100
 // steps, 2^16 paths 0.111 ms, against 0.133 and, for the direct FP64 sum, 1.46 ms.
