@@ -89,6 +89,12 @@ __device__ __forceinline__ uint4 philox_group(uint64_t seed, uint64_t p, uint32_
     return philox_group(philox_keys(seed), p, g, s);
 }
 
+// The warp's index, read from lane 0: the compiler then knows it is the same for
+// the warp and keeps what follows from it in uniform registers (FP64 form: normals of
+// 2^17 x 512 steps 839 -> 832 us, variance pass of 64 groups 1573 -> 1554 with its
+// convolution, convolution with variance of 100 steps 111 -> 109).
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 // A table of BYTES from global to shared memory by THREADS threads, 16 bytes a
 // load, every load in flight at once: store() after what else there is to do.
 template <int THREADS, int BYTES>

@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kNormalThreads, 4) k_normals_fixed(uint64_t se
     const bool vec = (N & 1) == 0;
     const PhiloxKeys keys = philox_keys(seed);
     const int64_t warps = (int64_t)gridDim.x * (kNormalThreads / 32);
-    for (int64_t t = blockIdx.x * (int64_t)(kNormalThreads / 32) + (threadIdx.x >> 5); t < tasks; t += warps) {
+    for (int64_t t = blockIdx.x * (int64_t)(kNormalThreads / 32) + warp_index(); t < tasks; t += warps) {
         const int64_t r = t / segs;
         const int c0 = (int)(t - r * segs) * kSeg, c1 = min(nch, c0 + kSeg);
         const int s = (int)(r % ns);
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(kNormalThreads) k_digits(const double* __restr
     const int64_t tasks = (B + kXPaths - 1) / kXPaths * (kXPaths / 8) * segs;
     const int64_t warps = (int64_t)gridDim.x * (kNormalThreads / 32);
     bool bad = false;
-    for (int64_t t = blockIdx.x * (int64_t)(kNormalThreads / 32) + (threadIdx.x >> 5); t < tasks; t += warps) {
+    for (int64_t t = blockIdx.x * (int64_t)(kNormalThreads / 32) + warp_index(); t < tasks; t += warps) {
         const int64_t r = t / segs, m = r * 8 + pl;
         const int c0 = (int)(t - r * segs) * kSeg, c1 = min(nch, c0 + kSeg);
         const double* z0 = Z + m * ns * (int64_t)N;
@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(kXThreads, 1) k_volterra_exact(const unsigned 
     uint64_t* acce = accf + 1;
     uint64_t* fin = accf + 2;
     uint32_t* holder = (uint32_t*)(accf + 3);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int nb = (N + kXBlock - 1) / kXBlock, nch = (N + kXSteps - 1) / kXSteps;
     const int64_t groups = (B + kXPaths - 1) / kXPaths, per = groups * nv, units = per * nb;
 
@@ -857,7 +857,7 @@ __global__ void __launch_bounds__(var_threads(GB), 2) k_variance_fixed(const X64
     constexpr int kVarThreads = var_threads(GB);
     extern __shared__ uint64_t vsm[];
     uint64_t* E = vsm;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, w = warp_index();
     double* red = reinterpret_cast<double*>(vsm + kExpTable) + (size_t)w * kVarVals * 33;
     for (int i = threadIdx.x; i < kExpTable; i += kVarThreads) E[i] = ft->exp2[i];
     __syncthreads();

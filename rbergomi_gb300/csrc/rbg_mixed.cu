@@ -807,9 +807,7 @@ __global__ void __launch_bounds__(PM > 0 ? kThreads + 32 : kThreads, 1) k_mixed_
     uint64_t* cempty = bars + 17;  // [kCSlots]
     uint64_t* ydone = bars + 20;   // thread 1's far-field of a pass complete
 
-    // (read from lane 0: the compiler then knows it is the same for the warp, and keeps what
-    // follows from it in uniform registers)
-    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int Np = a.Np, nc = a.nc;
     const PassPlan<PM> pp(a);
     const int FB = (PM == 2 || PM == 3) ? L.fstride : kStageFB;  // bytes per stage of the FP32-tile region
@@ -1492,9 +1490,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_mixed_gemm_jobs(const __grid_co
     uint64_t* final_bar = bars + 11;
     uint32_t* tmem_holder = (uint32_t*)(bars + 12);
     uint64_t* strip_free = bars + 13;  // every MMA issued on the old strip has completed
-    // (read from lane 0: the compiler then knows it is the same for the warp, and keeps what
-    // follows from it in uniform registers)
-    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
 
     // this CTA's tiles [t_first, t_last), starting in job jb
     const int64_t T = a.job_tile0[a.n_jobs];
