@@ -183,6 +183,7 @@ struct Ctx {
     // fixed-point FP64 path pass: digits of W1, X, and the Toeplitz panels of the tables in `tabs`
     DevBuf xdig, xbuf, xpan;
     PinBuf pin;
+    cudaEvent_t digits_done = nullptr;  // the caller's normals of a batch are in xdig (payoffs_quadrature)
     bool xpan_ready = false;
     // host images of what `tabs`, `mixed_ws` and `sobol` hold, so that a call
     // with the same tables (a calibration loop, a benchmark) uploads nothing
@@ -943,10 +944,10 @@ static int payoffs_quadrature(const rbg_params* p, const double* Z, double* payo
     TableSet ts;
     int logL = 0;
     // no backend asked for: the exact tensor-core convolution and fixed-point
-    // functions; a batch with normals outside their range takes the direct FP64 sum
+    // functions; a batch with normals outside their range takes the FP64 kernels
     X64Tables xt;
+    if ((rc = fp64_conv_log2(conv, plan.N, &logL))) return rc;
     bool fixed = conv == RBG_CONV_AUTO && x64_prepare(plan, xt, true);
-    if (!fixed && (rc = fp64_conv_log2(conv, plan.N, &logL))) return rc;
     const int no = (int)plan.outs.size(), N = plan.N, ns = mc ? 3 : 2, nv = (int)plan.vols.size();
     const int64_t M = p->M;
     int64_t B = fp64_batch(plan, M, ns);
@@ -960,15 +961,20 @@ static int payoffs_quadrature(const rbg_params* p, const double* Z, double* payo
         if ((rc = ensure(c->z, sizeof(double) * ns * N * (size_t)B, "normals"))) return rc;
         if ((rc = ensure(c->pay, sizeof(double) * no * (size_t)B, "payoffs"))) return rc;
     }
-    if (fixed && !ensure_fixed(*c, x64_digit_bytes(B, N), 8 * (size_t)vstep * N * (size_t)B)) {
-        fixed = false;
-        if ((rc = fp64_conv_log2(conv, N, &logL))) return rc;
-    }
-    if ((rc = upload_tables(*c, plan, st, ts, logL, fixed ? &xt : nullptr))) return rc;
-    // device words: kernel error, normals out of range
+    if (fixed && !ensure_fixed(*c, x64_digit_bytes(B, N), 8 * (size_t)vstep * N * (size_t)B)) fixed = false;
+    // the FP64 kernels' own tables wait for a batch that needs them
+    bool fp64_tables = !fixed;
+    if ((rc = upload_tables(*c, plan, st, ts, fixed ? 0 : logL, fixed ? &xt : nullptr, fp64_tables))) return rc;
+    // device words: kernel error, normals out of range; read through pinned memory
     if ((rc = ensure(c->acc, 2 * sizeof(unsigned int), "accumulators"))) return rc;
     unsigned int* words = c->acc.as<unsigned int>();
-    if (fixed) RBG_CUDA(cudaMemsetAsync(words, 0, 2 * sizeof(unsigned int), st));
+    volatile unsigned int* seen = nullptr;
+    if (fixed) {
+        if (c->pin.ensure(2 * sizeof(unsigned int))) return fail(RBG_ERR_NOMEM, "pinned result buffer");
+        seen = (unsigned int*)c->pin.p;
+        if (!c->digits_done) RBG_CUDA(cudaEventCreateWithFlags(&c->digits_done, cudaEventDisableTiming));
+        RBG_CUDA(cudaMemsetAsync(words, 0, 2 * sizeof(unsigned int), st));
+    }
     for (int64_t m0 = 0; m0 < M; m0 += B) {
         const int64_t b = std::min(B, M - m0);
         const double* Zd;
@@ -985,6 +991,8 @@ static int payoffs_quadrature(const rbg_params* p, const double* Z, double* payo
         if (fixed) {
             if (m0) RBG_CUDA(cudaMemsetAsync(words + 1, 0, sizeof(unsigned int), st));
             launch_digits(Zd, b, N, ns, c->xdig.as<unsigned char>(), words + 1, st);
+            RBG_CUDA(cudaMemcpyAsync((void*)(seen + 1), words + 1, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
+            RBG_CUDA(cudaEventRecord(c->digits_done, st));
             for (int v0 = 0; v0 < nv; v0 += vstep) {
                 const int k = std::min(vstep, nv - v0);
                 if (launch_volterra_exact(c->xdig.as<unsigned char>(),
@@ -995,21 +1003,29 @@ static int payoffs_quadrature(const rbg_params* p, const double* Z, double* payo
                     return fail(RBG_ERR_CUDA, "FP64 path kernels could not be configured");
             }
         }
-        launch_path_fp64(ts.t, Zd, b, c->ivb.as<double>(), st, ivp, nullptr, fixed ? words + 1 : nullptr);
+        // whether the batch's normals were in range is known once the digits are, while
+        // the kernels queued behind them run
+        bool out_of_range = false;
+        if (fixed) {
+            RBG_CUDA(cudaEventSynchronize(c->digits_done));
+            out_of_range = seen[1] != 0;
+        }
+        if (out_of_range && !fp64_tables) {
+            if ((rc = upload_tables(*c, plan, st, ts, logL, &xt, true))) return rc;
+            fp64_tables = true;
+        }
+        if (!fixed || out_of_range) launch_path_fp64(ts.t, Zd, b, c->ivb.as<double>(), st, ivp);
         if (launch_payoff_store(ts.t, c->ivb.as<double>(), b, b, Pd, st, ivp))
             return fail(RBG_ERR_CUDA, "FP64 payoff kernel could not be configured");
         RBG_CUDA(cudaGetLastError());
         if (!device_ptrs)
             RBG_CUDA(cudaMemcpyAsync(payoff + m0 * no, Pd, sizeof(double) * no * b, cudaMemcpyDeviceToHost, st));
     }
-    if (fixed) {
-        if (c->pin.ensure(sizeof(unsigned int))) return fail(RBG_ERR_NOMEM, "pinned result buffer");
-        RBG_CUDA(cudaMemcpyAsync(c->pin.p, words, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
-    }
+    if (fixed) RBG_CUDA(cudaMemcpyAsync((void*)seen, words, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
     RBG_CUDA(cudaStreamSynchronize(st));
-    if (fixed && *(unsigned int*)c->pin.p)
-        return fail(RBG_ERR_TIMEOUT, "FP64 convolution: a bounded pipeline wait expired (site " +
-                                         std::to_string(*(unsigned int*)c->pin.p) + ")");
+    if (fixed && seen[0])
+        return fail(RBG_ERR_TIMEOUT,
+                    "FP64 convolution: a bounded pipeline wait expired (site " + std::to_string(seen[0]) + ")");
     return RBG_OK;
 }
 

@@ -40,9 +40,8 @@ namespace rbg {
 // (Ivdt, IsvdW).
 template <int NS, bool ANTI>
 __global__ void k_path_fp64(Fp64Tables t, const double* __restrict__ Z, int64_t B, double2* __restrict__ ivb,
-                            double* __restrict__ ivp, double2* __restrict__ ivn, const unsigned int* only_if)
+                            double* __restrict__ ivp, double2* __restrict__ ivn)
 {
-    if (only_if && *only_if == 0u) return;
     extern __shared__ double sm[];
     const int N = t.N;
     const int warps = blockDim.x >> 5;
@@ -334,7 +333,7 @@ int path_fp64_warps(int N)
 size_t path_fp64_smem(int N, int warps) { return 8 * (size_t)N + (size_t)warps * 16 * N; }
 
 void launch_path_fp64(const Fp64Tables& t, const double* Z, int64_t B, double* ivb, void* stream, double* ivp,
-                      double* ivn, const unsigned int* only_if)
+                      double* ivn)
 {
     const int warps = path_fp64_warps(t.N);
     const size_t smem = path_fp64_smem(t.N, warps);
@@ -360,11 +359,11 @@ void launch_path_fp64(const Fp64Tables& t, const double* Z, int64_t B, double* i
     const int64_t blocks = (B + warps - 1) / warps;
     if (ivn)
         k_path_fp64<2, true><<<(unsigned)blocks, warps * 32, smem, st>>>(t, Z, B, (double2*)ivb, nullptr,
-                                                                         (double2*)ivn, only_if);
+                                                                         (double2*)ivn);
     else if (ivp)
-        k_path_fp64<3, false><<<(unsigned)blocks, warps * 32, smem, st>>>(t, Z, B, (double2*)ivb, ivp, nullptr, only_if);
+        k_path_fp64<3, false><<<(unsigned)blocks, warps * 32, smem, st>>>(t, Z, B, (double2*)ivb, ivp, nullptr);
     else
-        k_path_fp64<2, false><<<(unsigned)blocks, warps * 32, smem, st>>>(t, Z, B, (double2*)ivb, nullptr, nullptr, only_if);
+        k_path_fp64<2, false><<<(unsigned)blocks, warps * 32, smem, st>>>(t, Z, B, (double2*)ivb, nullptr, nullptr);
     count_launch();
 }
 

@@ -123,10 +123,9 @@ int launch_sobol_normals(const unsigned long long* Vt, int N, uint64_t s0, int64
                          double* Z, void* stream, int f32 = 0);
 int path_fp64_warps(int N);
 size_t path_fp64_smem(int N, int warps);
-// ivp non-null: Z has three streams per path (plain MC) and ivp[g][B] gets IsvdWp;
-// only_if (t.logL = 0): nothing is done where the device word is zero
+// ivp non-null: Z has three streams per path (plain MC) and ivp[g][B] gets IsvdWp
 void launch_path_fp64(const Fp64Tables& t, const double* Z, int64_t B, double* ivb, void* stream,
-                      double* ivp = nullptr, double* ivn = nullptr, const unsigned int* only_if = nullptr);
+                      double* ivp = nullptr, double* ivn = nullptr);
 // control-variate form (ML_console_ST): pilot statistics per output -- Q = max
 // 2 Ivdt over the pilot, alpha = -cov(X, Y) / var(Y) -- from the pilot's
 // (Ivdt, IsvdW) [group][Mc]; xy scratch holds 2 Mc doubles per output

@@ -120,6 +120,20 @@ def test_caller_normals_out_of_range_take_the_fp64_kernels(R, bad, stream):
     assert np.array_equal(p, q, equal_nan=True)
 
 
+@pytest.mark.parametrize("N,fft", [(199, False), (200, True), (300, True), (2048, True), (2049, False)])
+def test_caller_normals_out_of_range_take_the_backend_of_their_length(R, N, fft):
+    """The FP64 kernels' own choice for N steps (FFT from 200 to 2048 steps, else the
+    direct sum), bit for bit, and the call after it is in range again."""
+    conv = R.CONV_FFT if fft else R.CONV_DIRECT
+    Z = np.random.default_rng(1).standard_normal((33, 2, N))
+    args = (XI, [0.1, 0.3], [0.5, 1.0], [-0.7, 0.2], [1.0], [1.0])
+    want = R.payoffs_rt(*args, Z)
+    Zb = Z.copy()
+    Zb[7, 1, N // 2] = 16.0
+    assert np.array_equal(R.payoffs_rt(*args, Zb), R.payoffs_rt(*args, Zb, conv=conv))
+    assert np.array_equal(R.payoffs_rt(*args, Z), want)
+
+
 def test_caller_normals_plain_mc(R):
     Z = np.random.default_rng(3).standard_normal((130, 3, 150))
     Z[5, 2, 7] = 1e3  # Wperp only meets FP64 sums: no range
