@@ -929,6 +929,23 @@ static int price_cv_any(const rbg_cv_params* p, const rbg_options* o, const doub
     return price_cv(*c, plan, *p, *o, Zc, Z, st, res.data());
 }
 
+// Whether a quadrature call of M paths is large enough for the digit convolution.
+// Its kernels fill a path block of 128 steps and start one after the other, about
+// 35 us and 0.04 us a step and pass more than the FP64 path kernel's single launch while
+// that one's paths fit the chip at once; from there the FP64 pipe (two operations a clock and
+// SM, 6e11 a second) decides.  Per path and step the FP64 kernel takes half the
+// steps (direct, both rounded to 32) or 74 (FFT of L points, L / 2 steps) operations a pass and
+// about 44 (plain MC 60) a variance group.  The call on device pointers, digits against FP64
+// kernels: 64 steps, 2000 paths 84 / 64 us, 8000 paths 87 / 120; 100 steps, 1000
+// paths 98 / 68, 4000 paths 101 / 151; 512 steps, 256 paths 203 / 146, 1000
+// paths 202 / 239; 3 passes of 512 steps, 256 paths 366 / 320, 1000 paths 380 / 533.
+static bool quadrature_by_digits(const Plan& plan, int64_t M, int ns, int logL)
+{
+    const double nv = (double)plan.vols.size(), ng = (double)plan.vgs.size(), up = (plan.N + 31) / 32 * 32;
+    const double steps = logL > 0 ? (double)(1 << (logL - 1)) : up, conv = logL > 0 ? 74.0 : 0.5 * up + 16.0;
+    return (double)M * steps * (nv * conv + ng * (ns == 3 ? 60.0 : 44.0)) >= 2.4e7 + 4.9e4 * plan.N * nv;
+}
+
 static int payoffs_quadrature(const rbg_params* p, const double* Z, double* payoff, int device_ptrs,
                               cudaStream_t user_stream, bool mc = false, int conv = RBG_CONV_AUTO)
 {
@@ -943,13 +960,13 @@ static int payoffs_quadrature(const rbg_params* p, const double* Z, double* payo
     cudaStream_t st = user_stream ? user_stream : c->stream;
     TableSet ts;
     int logL = 0;
-    // no backend asked for: the exact tensor-core convolution and fixed-point
-    // functions; a batch with normals outside their range takes the FP64 kernels
+    // no backend asked for, and paths enough: the exact tensor-core convolution and
+    // fixed-point functions; a batch with normals outside their range takes the FP64 kernels
     X64Tables xt;
     if ((rc = fp64_conv_log2(conv, plan.N, &logL))) return rc;
-    bool fixed = conv == RBG_CONV_AUTO && x64_prepare(plan, xt, true);
     const int no = (int)plan.outs.size(), N = plan.N, ns = mc ? 3 : 2, nv = (int)plan.vols.size();
     const int64_t M = p->M;
+    bool fixed = conv == RBG_CONV_AUTO && quadrature_by_digits(plan, M, ns, logL) && x64_prepare(plan, xt, true);
     int64_t B = fp64_batch(plan, M, ns);
     // payoffs of a batch within 1 GiB too
     B = std::min<int64_t>(B, std::max<int64_t>(256, ((int64_t)1 << 30) / (8 * (int64_t)no)));

@@ -120,18 +120,58 @@ def test_caller_normals_out_of_range_take_the_fp64_kernels(R, bad, stream):
     assert np.array_equal(p, q, equal_nan=True)
 
 
-@pytest.mark.parametrize("N,fft", [(199, False), (200, True), (300, True), (2048, True), (2049, False)])
-def test_caller_normals_out_of_range_take_the_backend_of_their_length(R, N, fft):
-    """The FP64 kernels' own choice for N steps (FFT from 200 to 2048 steps, else the
-    direct sum), bit for bit, and the call after it is in range again."""
-    conv = R.CONV_FFT if fft else R.CONV_DIRECT
-    Z = np.random.default_rng(1).standard_normal((33, 2, N))
-    args = (XI, [0.1, 0.3], [0.5, 1.0], [-0.7, 0.2], [1.0], [1.0])
+# calls large enough for the digit convolution, at the edges of its tiles
+LARGE = [(2, 12001), (17, 12002), (128, 3009), (129, 3007), (300, 1030), (1030, 641)]
+
+
+def large_inputs(kind, N, M, ns):
+    g = np.random.default_rng(N + M)
+    if kind == "normal":
+        return g.standard_normal((M, ns, N)), 1.9
+    if kind == "constant":
+        return np.broadcast_to(g.uniform(-1, 1, (M, ns, 1)), (M, ns, N)).copy(), 1.9 / np.sqrt(N)
+    # every lower digit of W1 at an end of its range
+    return np.where(g.random((M, ns, 1)) < 0.5, -1, 1) * np.full((M, ns, N), 0x7f7f7f7f7f7f7 / 2.0 ** 51), 1.9 / np.sqrt(N)
+
+
+@pytest.mark.parametrize("kind", ["normal", "constant", "extreme digits"])
+@pytest.mark.parametrize("mc", [False, True])
+@pytest.mark.parametrize("N,M", LARGE)
+def test_caller_normals_large_calls(R, N, M, mc, kind):
+    """As test_caller_normals, where the call takes the digit convolution (its
+    results are not the direct sum's bit for bit)."""
+    Z, eta = large_inputs(kind, N, M, 3 if mc else 2)
+    args = (XI, [0.07, 0.4], [eta, eta], [-0.9, 0.3], [1.0, 0.5], [0.9, 1.1], Z)
+    pay = R.payoffs_mc if mc else R.payoffs_rt
+    p, q = pay(*args), pay(*args, conv=R.CONV_DIRECT)
+    assert np.all(np.abs(p - q) <= 2e-13 * np.maximum(np.abs(q), 1.0)), np.max(np.abs(p - q))
+    assert kind != "normal" or not np.array_equal(p, q)
+
+
+@pytest.mark.parametrize("bad", [15.5, -np.inf, np.nan])
+@pytest.mark.parametrize("N,fft", [(16, False), (199, False), (200, True), (300, True), (2048, True), (2049, False)])
+def test_caller_normals_out_of_range_take_the_backend_of_their_length(R, N, fft, bad):
+    """Large calls with a normal past the digits' range: the FP64 kernels' own choice
+    for N steps (FFT from 200 to 2048 steps, else the direct sum), bit for bit, and
+    the call after it is in range again."""
+    conv, M = R.CONV_FFT if fft else R.CONV_DIRECT, 12001 if N < 100 else 2003 if N < 1000 else 901
+    Z = np.random.default_rng(1).standard_normal((M, 2, N))
+    args = (XI, [0.1], [0.5], [-0.7], [1.0], [1.0])
     want = R.payoffs_rt(*args, Z)
+    assert not np.array_equal(want, R.payoffs_rt(*args, Z, conv=conv))
     Zb = Z.copy()
-    Zb[7, 1, N // 2] = 16.0
-    assert np.array_equal(R.payoffs_rt(*args, Zb), R.payoffs_rt(*args, Zb, conv=conv))
+    Zb[7, 1, N // 2] = bad
+    assert np.array_equal(R.payoffs_rt(*args, Zb), R.payoffs_rt(*args, Zb, conv=conv), equal_nan=True)
     assert np.array_equal(R.payoffs_rt(*args, Z), want)
+
+
+def test_small_quadrature_calls_take_the_fp64_kernels(R):
+    """Few paths: the FP64 path kernel's one launch, its results bit for bit."""
+    for N, M, conv in ((2, 500, R.CONV_DIRECT), (64, 1000, R.CONV_DIRECT), (199, 100, R.CONV_DIRECT),
+                       (200, 400, R.CONV_FFT), (512, 130, R.CONV_FFT)):
+        Z = np.random.default_rng(N).standard_normal((M, 2, N))
+        args = (XI, [0.1], [1.5], [-0.7], [1.0], [1.0], Z)
+        assert np.array_equal(R.payoffs_rt(*args), R.payoffs_rt(*args, conv=conv))
 
 
 def test_caller_normals_plain_mc(R):
