@@ -1,12 +1,14 @@
 """Builds librbergomi_gb300.so in-tree with nvcc for sm_103a.
 
-Each translation unit compiles in parallel into rbergomi_gb300/_build/, then
-one nvcc link produces rbergomi_gb300/librbergomi_gb300.so.  No cmake, no
+A small host program prints the fixed-point tables that one unit includes.  Each
+translation unit compiles in parallel into rbergomi_gb300/_build/, then one nvcc
+link produces rbergomi_gb300/librbergomi_gb300.so.  No cmake, no
 torch extension machinery: the library is a plain C-ABI shared object.
 """
 from __future__ import annotations
 
 import os
+import platform
 import shutil
 import subprocess
 import sys
@@ -19,7 +21,10 @@ OUT_DIR = os.path.join(PKG, "_build")
 LIB = os.path.join(PKG, "librbergomi_gb300.so")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-I" + os.path.join(ROOT, "include"), "-I" + CSRC]
+COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-I" + os.path.join(ROOT, "include"), "-I" + CSRC,
+          "-I" + os.path.join(OUT_DIR, platform.machine())]
+# by machine: the host's extended precision rounds the tables' last bit
+TABLES = os.path.join(OUT_DIR, platform.machine(), "rbg_fixed_tables.inc")
 
 SOURCES = ["rbg_plan.cpp", "rbg_api.cpp", "rbg_fp64.cu", "rbg_fp64x.cu", "rbg_mixed.cu", "rbg_fft.cu", "rbg_static.cu", "rbg_qmc.cu",
            "rbg_server.cpp", "rbg_cxx.cpp"]
@@ -32,12 +37,31 @@ def nvcc() -> str:
     raise RuntimeError("nvcc not found")
 
 
+def _stale(out: str, deps: list) -> bool:
+    return not os.path.exists(out) or any(os.path.getmtime(out) < os.path.getmtime(d) for d in deps)
+
+
+def _tables() -> None:
+    """rbg_fixed_tables.inc, printed by rbg_tables_gen.cpp."""
+    src, head = (os.path.join(CSRC, f) for f in ("rbg_tables_gen.cpp", "rbg_fixed.cuh"))
+    if not _stale(TABLES, [src, head]):
+        return
+    os.makedirs(os.path.dirname(TABLES), exist_ok=True)
+    exe = os.path.join(os.path.dirname(TABLES), "rbg_tables_gen")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-I" + CSRC, src, "-o", exe], check=True)
+    text = subprocess.run([exe], check=True, capture_output=True, text=True).stdout
+    with open(TABLES + ".tmp", "w") as f:
+        f.write(text)
+    os.replace(TABLES + ".tmp", TABLES)
+
+
 def _compile(src: str) -> str:
     obj = os.path.join(OUT_DIR, os.path.splitext(src)[0] + ".o")
     path = os.path.join(CSRC, src)
     deps = [path] + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".hpp", ".cuh"))]
     deps += [os.path.join(ROOT, "include", h) for h in ("rbergomi_gb300.h", "rbergomi_gb300.hpp")]
-    if os.path.exists(obj) and all(os.path.getmtime(obj) >= os.path.getmtime(d) for d in deps):
+    deps += [TABLES] if src == "rbg_fp64x.cu" else []
+    if not _stale(obj, deps):
         return obj
     cmd = [nvcc()] + ARCH + COMMON + ["-c", path, "-o", obj]
     if src.endswith(".cu"):
@@ -53,9 +77,10 @@ def _compile(src: str) -> str:
 
 def build(verbose: bool = False) -> str:
     os.makedirs(OUT_DIR, exist_ok=True)
+    _tables()
     with ThreadPoolExecutor(max_workers=len(SOURCES)) as ex:
         objs = list(ex.map(_compile, SOURCES))
-    if not os.path.exists(LIB) or any(os.path.getmtime(o) > os.path.getmtime(LIB) for o in objs):
+    if _stale(LIB, objs):
         cmd = [nvcc()] + ARCH + ["-shared", "-o", LIB] + objs + ["-lcudart"]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:

@@ -501,7 +501,7 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
             } else if (launch_normals_fixed(o.seed, o.path_offset + m0, b, N, o.normals == RBG_NORMALS_F32,
                                             c.z.as<double>(), fixed ? c.xdig.as<unsigned char>() : nullptr,
                                             !fixed ? 0 : (fused ? kFixAll : kFixW1perp), ns, st)) {
-                return fail(RBG_ERR_CUDA, "normal tables could not be set up");
+                return fail(RBG_ERR_CUDA, "fixed-point tables not found on the device");
             }
         }
         {
@@ -535,7 +535,7 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
             ProfScope ps(kStageReduce, st);
             if (launch_merge(c.part.as<double>(), nchunks, no, c.acc.as<double>(), m0 == 0, st,
                              m0 + B >= M ? &fin : nullptr))
-                return fail(RBG_ERR_CUDA, "merge tables could not be set up");
+                return fail(RBG_ERR_CUDA, "fixed-point tables not found on the device");
         }
         RBG_CUDA(cudaGetLastError());
     }
@@ -602,7 +602,7 @@ static int mixed_run(Ctx& c, const Plan& plan, const TableSet& ts, const MixedJo
     const MergeFinal fin{ts.t.outs, ts.Tvals, c.res.as<double>(), M, o.compute_iv};
     auto merge = [&](int rows, int64_t m0) {
         return launch_merge(c.part.as<double>(), rows, no, c.acc.as<double>(), m0 == 0, st, m0 + B >= M ? &fin : nullptr)
-                   ? fail(RBG_ERR_CUDA, "merge tables could not be set up")
+                   ? fail(RBG_ERR_CUDA, "fixed-point tables not found on the device")
                    : RBG_OK;
     };
     for (int64_t m0 = 0; m0 < M; m0 += B) {
@@ -782,7 +782,7 @@ static int price_cv(Ctx& c, const Plan& plan, const rbg_cv_params& p, const rbg_
     } else {
         if (launch_normals_fixed(o.seed, kCvPilotPath0 + o.path_offset, Mc, N, o.normals == RBG_NORMALS_F32,
                                  c.z.as<double>(), nullptr, 0, 2, st))
-            return fail(RBG_ERR_CUDA, "normal tables could not be set up");
+            return fail(RBG_ERR_CUDA, "fixed-point tables not found on the device");
     }
     launch_path_fp64(ts.t, c.z.as<double>(), Mc, c.ivb.as<double>(), st);
     launch_cv_pilot(ts.t, c.ivb.as<double>(), Mc, xy, alpha, Q, st);
@@ -796,19 +796,19 @@ static int price_cv(Ctx& c, const Plan& plan, const rbg_cv_params& p, const rbg_
         } else {
             if (launch_normals_fixed(o.seed, o.path_offset + m0, b, N, o.normals == RBG_NORMALS_F32, c.z.as<double>(),
                                      nullptr, 0, 2, st))
-                return fail(RBG_ERR_CUDA, "normal tables could not be set up");
+                return fail(RBG_ERR_CUDA, "fixed-point tables not found on the device");
         }
         launch_path_fp64(ts.t, c.z.as<double>(), b, c.ivb.as<double>(), st, nullptr, c.ivp.as<double>());
         const int nchunks = (int)((b + 256 * (int64_t)G - 1) / (256 * (int64_t)G));
         launch_payoff_sums_cv(ts.t, c.ivb.as<double>(), c.ivp.as<double>(), b, alpha, Q, p.Q_max, G,
                               c.part.as<double>(), count, nchunks, st);
         if (launch_merge(c.part.as<double>(), nchunks, no, c.acc.as<double>(), m0 == 0, st))
-            return fail(RBG_ERR_CUDA, "merge tables could not be set up");
+            return fail(RBG_ERR_CUDA, "fixed-point tables not found on the device");
         RBG_CUDA(cudaGetLastError());
     }
     if (launch_finalize_cv(c.acc.as<double>(), no, M, ts.t.outs, ts.Tvals, alpha, Q, count, p.Q_max, o.compute_iv,
                            c.res.as<double>(), st))
-        return fail(RBG_ERR_CUDA, "merge tables could not be set up");
+        return fail(RBG_ERR_CUDA, "fixed-point tables not found on the device");
     RBG_CUDA(cudaGetLastError());
     RBG_CUDA(cudaMemcpyAsync(host_res, c.res.p, sizeof(double) * 5 * no, cudaMemcpyDeviceToHost, st));
     RBG_CUDA(cudaStreamSynchronize(st));
@@ -854,7 +854,7 @@ static int price_cv_mixed(Ctx& c, const Plan& plan, const rbg_cv_params& p, cons
     double* xy = (double*)(count + no);
     // pilot: one FP64 batch of Mc paths on FP32 normals
     if (launch_normals_fixed(o.seed, kCvPilotPath0 + o.path_offset, Mc, N, 1, c.z.as<double>(), nullptr, 0, 2, st))
-        return fail(RBG_ERR_CUDA, "normal tables could not be set up");
+        return fail(RBG_ERR_CUDA, "fixed-point tables not found on the device");
     launch_path_fp64(ts.t, c.z.as<double>(), Mc, c.ivp.as<double>(), st);
     launch_cv_pilot(ts.t, c.ivp.as<double>(), Mc, xy, alpha, Q, st);
     RBG_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned long long) * no, st));
@@ -889,13 +889,13 @@ static int price_cv_mixed(Ctx& c, const Plan& plan, const rbg_cv_params& p, cons
         {
             ProfScope ps(kStageReduce, st);
             if (launch_merge(c.part.as<double>(), nchunks, no, c.acc.as<double>(), m0 == 0, st))
-                return fail(RBG_ERR_CUDA, "merge tables could not be set up");
+                return fail(RBG_ERR_CUDA, "fixed-point tables not found on the device");
         }
         RBG_CUDA(cudaGetLastError());
     }
     if (launch_finalize_cv(c.acc.as<double>(), no, M, ts.t.outs, ts.Tvals, alpha, Q, count, p.Q_max, o.compute_iv,
                            c.res.as<double>(), st))
-        return fail(RBG_ERR_CUDA, "merge tables could not be set up");
+        return fail(RBG_ERR_CUDA, "fixed-point tables not found on the device");
     RBG_CUDA(cudaGetLastError());
     if ((rc = mixed_check(job, c.mixed_ws.p, st, g_err))) return rc;
     RBG_CUDA(cudaMemcpyAsync(host_res, c.res.p, sizeof(double) * 5 * no, cudaMemcpyDeviceToHost, st));
@@ -1253,7 +1253,7 @@ int rbg_generate_normals_streams(uint64_t seed, int64_t path_offset, int64_t M, 
         const int64_t b = std::min(B, M - m0);
         if (launch_normals_fixed(seed, path_offset + m0, b, N, precision == RBG_MIXED, c->z.as<double>(), nullptr, 0, ns,
                                  c->stream))
-            return fail(RBG_ERR_CUDA, "normal tables could not be set up");
+            return fail(RBG_ERR_CUDA, "fixed-point tables not found on the device");
         RBG_CUDA(cudaGetLastError());
         RBG_CUDA(cudaMemcpyAsync(Z + m0 * ns * N, c->z.p, sizeof(double) * ns * N * b, cudaMemcpyDeviceToHost,
                                  c->stream));
@@ -1439,7 +1439,7 @@ int rbg_implied_vol(int n, const double* price, const double* K, const double* T
     RBG_CUDA(cudaMemcpyAsync(d + n, K, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
     RBG_CUDA(cudaMemcpyAsync(d + 2 * n, T, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
     if (launch_implied_vol(n, d, d + n, d + 2 * n, d + 3 * n, c->stream))
-        return fail(RBG_ERR_CUDA, "implied-vol tables could not be set up");
+        return fail(RBG_ERR_CUDA, "fixed-point tables not found on the device");
     RBG_CUDA(cudaGetLastError());
     RBG_CUDA(cudaMemcpyAsync(iv, d + 3 * n, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
     RBG_CUDA(cudaStreamSynchronize(c->stream));

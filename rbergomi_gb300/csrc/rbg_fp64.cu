@@ -991,8 +991,8 @@ int launch_merge_jobs(const AccJob* jobs, const FinJob* fins, int n_jobs, int64_
     return 0;
 }
 
-// Loads the merge kernels and their tables (a serving loop's first request
-// must not meet either).
+// Loads the merge kernels and looks up their tables (a serving loop's first
+// request must not meet either).
 void reduce_preload()
 {
     cudaFuncAttributes fa;

@@ -44,9 +44,12 @@
 namespace rbg {
 
 // ------------------------------------------------------------------ tables
-__device__ FixedTables g_fixed_tables;
+// Printed by rbg_tables_gen.cpp when the library is built.
+__device__ const FixedTables g_fixed_tables = {
+#include "rbg_fixed_tables.inc"
+};
 
-// The device's tables, filled on first use; null where that fails.
+// The tables' address on the current device, looked up once; null where that fails.
 const FixedTables* fixed_tables()
 {
     static std::mutex mu;
@@ -58,12 +61,8 @@ const FixedTables* fixed_tables()
     }
     std::lock_guard<std::mutex> lk(mu);
     if (!at[dev]) {
-        static FixedTables T;
         void* p = nullptr;
-        fill_fixed_tables(T);
-        if (cudaGetSymbolAddress(&p, g_fixed_tables) != cudaSuccess ||
-            cudaMemcpy(p, &T, sizeof T, cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaDeviceSynchronize() != cudaSuccess) {
+        if (cudaGetSymbolAddress(&p, g_fixed_tables) != cudaSuccess) {
             cudaGetLastError();
             return nullptr;
         }

@@ -46,8 +46,8 @@ int x64_blocks(int N);
 size_t x64_panel_bytes(int N);  // per Volterra pass
 size_t x64_digit_bytes(int64_t B, int N);
 
-// The fixed-point and tail tables of the current device (rbg_fixed.cuh), null
-// where they could not be set up.
+// The fixed-point and tail tables on the current device (rbg_fixed.cuh), part of
+// the module; null where their address could not be had.
 struct FixedTables;
 const FixedTables* fixed_tables();
 

@@ -183,7 +183,7 @@ struct FinJob {  // then its price, stat, implied vol; invM = 1 / M, isqM = 1 / 
     int compute_iv, pad;
 };
 int launch_merge_jobs(const AccJob* jobs, const FinJob* fins, int n_jobs, int64_t blocks, void* stream);
-// Loads the merge kernels and their tables (modules load lazily, on first use).
+// Loads the merge kernels (modules load lazily, on first use).
 void reduce_preload();
 
 // Kernel-launch counter shared by all launchers.

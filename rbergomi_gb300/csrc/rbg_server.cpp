@@ -336,15 +336,17 @@ int Server::launch(Slot& s, Req& r, std::string& err)
             cudaMemsetAsync(s.part.p, 0, sizeof(double) * 4 * no * (size_t)nr, st);
             rc = mixed_launch(job, s.ws.p, r.opt.seed, r.opt.path_offset + m0, b, nullptr, st, kerr, nullptr,
                               nullptr, (double*)s.part.p);
-            if (rc == RBG_OK && launch_merge((const double*)s.part.p, nr, no, (double*)s.acc.p, m0 == 0, st, last))
+            if (rc == RBG_OK && launch_merge((const double*)s.part.p, nr, no, (double*)s.acc.p, m0 == 0, st, last)) {
+                kerr = "fixed-point tables not found on the device";
                 rc = RBG_ERR_CUDA;
+            }
         } else {
             rc = mixed_launch(job, s.ws.p, r.opt.seed, r.opt.path_offset + m0, b, s.ivb.p, st, kerr);
             const int nchunks = (int)((b + 256 * (int64_t)G - 1) / (256 * (int64_t)G));
             if (rc == RBG_OK) {
                 launch_payoff_sums_f32(d_outs, no, s.ivb.p, b, G, (double*)s.part.p, nchunks, st);
                 if (launch_merge((const double*)s.part.p, nchunks, no, (double*)s.acc.p, m0 == 0, st, last)) {
-                    kerr = "merge tables could not be set up";
+                    kerr = "fixed-point tables not found on the device";
                     rc = RBG_ERR_CUDA;
                 }
             }
@@ -584,7 +586,7 @@ int Server::launch_batch(BatchSlot& b, std::vector<Req*>& rs, std::string& err)
     if (rc == RBG_OK) {
         launch_payoff_sums_f32_jobs((const PayoffJob*)(din + off_pj), n, pblocks, st);
         if (launch_merge_jobs((const AccJob*)(din + off_aj), (const FinJob*)(din + off_fj), n, ablocks, st)) {
-            err = "merge tables could not be set up";
+            err = "fixed-point tables not found on the device";
             rc = RBG_ERR_CUDA;
         }
         cudaMemcpyAsync(b.pin, din, 4, cudaMemcpyDeviceToHost, st);

@@ -176,7 +176,7 @@ int rbg_price_rt_static(const rbg_params* p, const rbg_options* o, double* price
             rc = mixed_launch(job, s + off_ws, o->seed, o->path_offset + m0, b, nullptr, st, err, nullptr, nullptr,
                               (double*)(s + off_part));
             if (rc) return fail_queued(rc, err);
-            if (merge(rows, m0)) return fail_queued(RBG_ERR_CUDA, "merge tables could not be set up");
+            if (merge(rows, m0)) return fail_queued(RBG_ERR_CUDA, "fixed-point tables not found on the device");
             continue;
         }
         rc = mixed_launch(job, s + off_ws, o->seed, o->path_offset + m0, b, s + off_ivb, st, err);
@@ -184,7 +184,7 @@ int rbg_price_rt_static(const rbg_params* p, const rbg_options* o, double* price
         const int nchunks = (int)((b + chunk - 1) / chunk);
         launch_payoff_sums_f32((const OutDev*)(s + off_outs), n_out, s + off_ivb, b, G, (double*)(s + off_part),
                                nchunks, st);
-        if (merge(nchunks, m0)) return fail_queued(RBG_ERR_CUDA, "merge tables could not be set up");
+        if (merge(nchunks, m0)) return fail_queued(RBG_ERR_CUDA, "fixed-point tables not found on the device");
     }
     // the error word after the finalize is queued: one wait for the whole call
     if ((rc = mixed_check(job, s + off_ws, st, err))) return fail_queued(rc, err);
