@@ -377,6 +377,7 @@ void launch_path_fp64(const Fp64Tables& t, const double* Z, int64_t B, double* i
 // ms; 8192 paths x 2112 outputs: 7.06 -> 0.49 ms.
 constexpr int kOPB = 8;  // outputs per task
 constexpr int kPayThreads = 256;
+constexpr int kPlainPaths = 8;  // paths a thread adds up in one FP64 sum
 
 struct OutF64 {
     double rho, K, lnK, om, hr;  // om = 1 - rho^2 (plain MC: its root), hr = -rho^2 / 2
@@ -389,6 +390,7 @@ struct PayoffSmem {
     MillsTable T;
     OutF64 out[kOPB];
     double red[kPayThreads / 32][2 * kOPB];
+    double sum[2 * kOPB], comp[2 * kOPB];  // of a task's rounds so far
 };
 
 // Outputs o0 .. o0 + 7 of the task, by the first threads of the block.
@@ -475,11 +477,57 @@ __device__ __forceinline__ double warp_sums16_f64(double (&v)[2 * kOPB])
     return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
+// s + e = a + b exactly, s the rounded sum (the larger of the two is found by integers).
+__device__ __forceinline__ void two_sum(double a, double b, double& s, double& e)
+{
+    const bool swap = (double_bits(a) << 1) < (double_bits(b) << 1);
+    const double hi = swap ? b : a, lo = swap ? a : b;
+    s = hi + lo;
+    e = lo - (s - hi);
+}
+
+// One round's sums of the block's eight warps into the task's, by one warp: lanes 0-15
+// take four warps' sums, lanes 16-31 the other four's; after the last round the
+// chunk's (sum, comp, sum2, comp2) of n outputs go to p.
+template <int MC>
+__device__ __forceinline__ void merge_round(PayoffSmem<MC>& sm, bool first, bool last, double* __restrict__ p, int n)
+{
+    const int lane = threadIdx.x & 31, k = lane & 15;
+    const double(*a)[2 * kOPB] = sm.red + 4 * (lane >> 4);
+    double s01, s23, s, e01, e23, e03, e;
+    two_sum(a[0][k], a[1][k], s01, e01);
+    two_sum(a[2][k], a[3][k], s23, e23);
+    two_sum(s01, s23, s, e03);
+    e = e01 + e23 + e03;
+    two_sum(s, __shfl_xor_sync(0xffffffffu, s, 16), s, e03);
+    e += __shfl_xor_sync(0xffffffffu, e, 16) + e03;
+    if (!first) {
+        two_sum(sm.sum[k], s, s, e03);
+        e += sm.comp[k] + e03;
+    }
+    if (!last) {
+        __syncwarp();
+        sm.sum[k] = s;
+        sm.comp[k] = e;
+    } else if (lane < 2 * kOPB && (lane & (kOPB - 1)) < n) {
+        p += 4 * (lane & (kOPB - 1)) + 2 * (lane / kOPB);
+        p[0] = s;
+        p[1] = e;
+    }
+}
+
 // chunk c covers paths [c G 256, (c+1) G 256) of the batch, G per thread;
-// part[(c * n_out + i) * 4 + {0,1,2,3}] = (sum, comp, sum2, comp2).
+// part[(c * n_out + i) * 4 + {0,1,2,3}] = (sum, comp, sum2, comp2).  A thread adds
+// up at most kPlainPaths paths in one FP64 sum; from the warps' sums on, every
+// rounding error is kept in the compensation.  (An FP64 warp instruction holds
+// its pipe for 64 cycles: the warps' sums are merged pairwise by one warp, another
+// one each task, in 16 of them, where plain additions in a row by the first warp were 8.
+// Three blocks an SM as the launcher asks for: left to itself the compiler takes 118
+// registers and two blocks, 2.66 ms for the grid of 8192 paths x 2112 outputs instead
+// of 2.48.)
 // MC = 1: plain Monte Carlo payoff from (Ivdt, IsvdW) and ivp = IsvdWp.
 template <int MC>
-__global__ void __launch_bounds__(kPayThreads) k_payoff_sums(Fp64Tables t, const double2* __restrict__ ivb, int64_t B,
+__global__ void __launch_bounds__(kPayThreads, 3) k_payoff_sums(Fp64Tables t, const double2* __restrict__ ivb, int64_t B,
                                                      int64_t stride, int G, double* __restrict__ part, int nchunks,
                                                      const double* __restrict__ ivp, const FixedTables* __restrict__ ft)
 {
@@ -488,17 +536,19 @@ __global__ void __launch_bounds__(kPayThreads) k_payoff_sums(Fp64Tables t, const
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t tasks = (int64_t)nchunks * ((t.n_out + kOPB - 1) / kOPB);
     payoff_start<MC>(sm, t, (int)(blockIdx.x / nchunks) * kOPB, ft);
-    for (int64_t task = blockIdx.x; task < tasks; task += gridDim.x) {
+    int sub0 = 0;  // the round of at most kPlainPaths paths a thread
+    for (int64_t task = blockIdx.x; task < tasks;) {
         const int c = (int)(task % nchunks), o0 = (int)(task / nchunks) * kOPB;
-        if (task != blockIdx.x) {
-            __syncthreads();  // the previous task's readers
-            payoff_outs<MC>(sm, t, o0);
+        if (task != blockIdx.x || sub0) {
+            __syncthreads();  // the previous round's readers
+            if (!sub0) payoff_outs<MC>(sm, t, o0);
             __syncthreads();
         }
         double s[2 * kOPB];  // sums of x, then of x^2
 #pragma unroll
         for (int q = 0; q < 2 * kOPB; ++q) s[q] = 0.0;
-        for (int sub = 0; sub < G; ++sub) {
+        const int sub1 = min(sub0 + kPlainPaths, G);
+        for (int sub = sub0; sub < sub1; ++sub) {
             const int64_t m = ((int64_t)c * G + sub) * 256 + threadIdx.x;
             if (m >= B) break;
             RtState r;
@@ -517,13 +567,13 @@ __global__ void __launch_bounds__(kPayThreads) k_payoff_sums(Fp64Tables t, const
         const double v = warp_sums16_f64(s);
         if (!(lane & 1)) sm.red[w][lane >> 1] = v;
         __syncthreads();
-        if (threadIdx.x < 2 * kOPB && o0 + (int)(threadIdx.x & (kOPB - 1)) < t.n_out) {
-            const int q = threadIdx.x & (kOPB - 1), z = threadIdx.x / kOPB;
-            double S = 0;
-            for (int k = 0; k < kPayThreads / 32; ++k) S += sm.red[k][threadIdx.x];
-            double* p = part + ((size_t)c * t.n_out + o0 + q) * 4 + 2 * z;
-            p[0] = S;
-            p[1] = 0.0;
+        if (w == (int)(task & (kPayThreads / 32 - 1)))
+            merge_round<MC>(sm, sub0 == 0, sub1 == G, part + ((size_t)c * t.n_out + o0) * 4, t.n_out - o0);
+        if (sub1 < G) {
+            sub0 = sub1;
+        } else {
+            sub0 = 0;
+            task += gridDim.x;
         }
     }
 }
