@@ -173,6 +173,7 @@ struct TableSet {
     const X64Vol* xvols = nullptr;  // fixed-point path pass only
     const X64Group* xgrps = nullptr;
     const uint64_t* xcomp = nullptr;
+    const int64_t* xgam = nullptr;
 };
 
 struct Ctx {
@@ -245,19 +246,31 @@ static int device_ctxs(std::vector<Ctx*>& out)
     return RBG_OK;
 }
 
-static int ensure(DevBuf& b, size_t bytes, const char* what)
+// The buffers only the digit convolution uses.  (cudaFree waits for work in flight.)
+static void release_fixed(Ctx& c)
 {
+    for (DevBuf* b : {&c.xdig, &c.xbuf, &c.xpan}) b->release();
+    c.xpan_ready = false;
+}
+
+// Grows one of the context's buffers.  The digit convolution's buffers, which an
+// earlier call on the stream may have left, make room where there is none; a call
+// therefore asks for what it cannot do without before it asks for those.
+static int ensure(Ctx& c, DevBuf& b, size_t bytes, const char* what)
+{
+    if (!b.ensure(bytes)) return RBG_OK;
+    release_fixed(c);
     if (b.ensure(bytes)) return fail(RBG_ERR_NOMEM, std::string("device allocation failed: ") + what);
     return RBG_OK;
 }
 
-// The FP64 form's digit and X (or sum) buffers.  Without room for them the call
-// goes on with the FP64 kernels, which need neither.
-static bool ensure_fixed(Ctx& c, size_t digits, size_t paths)
+// The digit convolution's buffers: digits, X (or sums), panels.  Without room for
+// them the call goes on with the FP64 kernels, which need none of them.
+static bool ensure_fixed(Ctx& c, size_t digits, size_t paths, size_t panels)
 {
-    if (!c.xdig.ensure(digits) && !c.xbuf.ensure(paths)) return true;
-    c.xdig.release();
-    c.xbuf.release();
+    if (c.xpan.n < panels) c.xpan_ready = false;
+    if (!c.xdig.ensure(digits) && !c.xbuf.ensure(paths) && !c.xpan.ensure(panels)) return true;
+    release_fixed(c);
     return false;
 }
 
@@ -282,8 +295,8 @@ static int fp64_conv_log2(int conv, int N, int* logL)
 }
 
 // logL > 0: also the FP64 FFT convolution's spectra (one per distinct H) and
-// twiddles; xt: also the fixed-point path pass's tables, and its Toeplitz
-// panels (built on the device, kept with the tables)
+// twiddles; xt: also the fixed-point path pass's tables (fixed_panels builds their
+// Toeplitz panels)
 // fp64: the FP64 path kernels' Gamma and compensators too (the other path
 // passes bring their own).
 static int upload_tables(Ctx& c, const Plan& plan, cudaStream_t st, TableSet& ts, int logL = 0,
@@ -339,7 +352,7 @@ static int upload_tables(Ctx& c, const Plan& plan, cudaStream_t st, TableSet& ts
         c.tabs_img.clear();
         c.xpan_ready = false;
         ++c.img_gen;
-        int rc = ensure(c.tabs, total, "tables");
+        int rc = ensure(c, c.tabs, total, "tables");
         if (rc) return rc;
         // a pageable source is staged before the call returns, so `host` may die
         RBG_CUDA(cudaMemcpyAsync(c.tabs.p, host.data(), total, cudaMemcpyHostToDevice, st));
@@ -365,15 +378,46 @@ static int upload_tables(Ctx& c, const Plan& plan, cudaStream_t st, TableSet& ts
         ts.xvols = (const X64Vol*)(base + off_xvols);
         ts.xgrps = (const X64Group*)(base + off_xgrps);
         ts.xcomp = (const uint64_t*)(base + off_xcomp);
-        if (!c.xpan_ready) {
-            int rc = ensure(c.xpan, x64_panel_bytes(N) * (size_t)nv, "convolution panels");
-            if (rc) return rc;
-            launch_panels((const int64_t*)(base + off_xgam), nv, N, (unsigned char*)c.xpan.p, st);
-            RBG_CUDA(cudaGetLastError());
-            c.xpan_ready = true;
-        }
+        ts.xgam = (const int64_t*)(base + off_xgam);
     }
     return RBG_OK;
+}
+
+// What the digit convolution holds beside the FP64 kernels' buffers: digits of a batch
+// (16 bytes a path-step, within 2 GiB by the batch's size), X or the fused sums of vstep
+// passes and their panels, each within 2 GiB.
+constexpr int64_t kFixedBytes = (int64_t)1 << 31;
+struct FixedPlan {
+    int vstep = 1;       // passes a convolution launch
+    size_t paths = 0;    // bytes of X or sums of vstep passes
+    size_t panels = 0;   // bytes of panels: of every pass where that fits, else of vstep
+    bool keep = false;   // every pass's panels, kept with the tables
+};
+// per: bytes of X or sums of one pass
+static FixedPlan fixed_plan(int nv, int N, size_t per)
+{
+    const int64_t pan = (int64_t)x64_panel_bytes(N);
+    FixedPlan f;
+    f.keep = pan * nv <= kFixedBytes;
+    f.vstep = (int)std::max<int64_t>(1, std::min({(int64_t)nv, kFixedBytes / (int64_t)per, kFixedBytes / pan}));
+    f.paths = (size_t)f.vstep * per;
+    f.panels = (size_t)(pan * (f.keep ? nv : f.vstep));
+    return f;
+}
+
+// Panels of the passes v0 .. v0 + k - 1 of the tables in c.tabs, in c.xpan.
+static const unsigned char* fixed_panels(Ctx& c, const TableSet& ts, const FixedPlan& f, int v0, int k, cudaStream_t st)
+{
+    unsigned char* at = c.xpan.as<unsigned char>();
+    const int N = ts.t.N;
+    if (!f.keep) {
+        c.xpan_ready = false;
+        launch_panels(ts.xgam + (size_t)v0 * N, k, N, at, st);
+        return at;
+    }
+    if (!c.xpan_ready) launch_panels(ts.xgam, ts.t.n_vol, N, at, st);
+    c.xpan_ready = true;
+    return at + (size_t)v0 * x64_panel_bytes(N);
 }
 
 // ------------------------------------------------------------ FP64 form
@@ -465,29 +509,34 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
     if (rc) return rc;
     const int no = (int)plan.outs.size(), N = plan.N, ns = mc ? 3 : 2, nv = (int)plan.vols.size();
     const int64_t B = fp64_batch(plan, M, ns);
-    if ((rc = ensure(c.z, sizeof(double) * ns * N * (size_t)B, "normals"))) return rc;
-    if ((rc = ensure(c.ivb, sizeof(double) * 2 * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
-    if (mc && (rc = ensure(c.ivp, sizeof(double) * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
+    if ((rc = ensure(c, c.z, sizeof(double) * ns * N * (size_t)B, "normals"))) return rc;
+    if ((rc = ensure(c, c.ivb, sizeof(double) * 2 * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
+    if (mc && (rc = ensure(c, c.ivp, sizeof(double) * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
     double* ivp = mc ? c.ivp.as<double>() : nullptr;
     // The variance pass inside the convolution's read-out for up to x64_fuse_groups
     // variance groups a pass, where its sums (one value per group, path and 32 steps)
     // stay within X's limit of 2 GiB for one pass.
     const size_t sums = (size_t)std::max(xt.max_groups, 1) * x64_slot_bytes(B, N, ns);
     const bool fused = xt.u53 && xt.max_groups <= x64_fuse_groups(ns) && sums <= ((size_t)1 << 31);
-    const size_t per = fused ? sums : 8 * (size_t)N * (size_t)B;
-    // passes per convolution launch: X or the sums within 2 GiB
-    const int vstep = (int)std::max<int64_t>(1, std::min<int64_t>(nv, ((int64_t)1 << 31) / (int64_t)per));
-    if (fixed && !ensure_fixed(c, x64_digit_bytes(B, N), (size_t)vstep * per)) {
-        fixed = false;
-        if ((rc = fp64_conv_log2(o.conv, N, &logL))) return rc;
-    }
-    if ((rc = upload_tables(c, plan, st, ts, logL, fixed ? &xt : nullptr, !fixed))) return rc;
+    const FixedPlan fp = fixed_plan(nv, N, fused ? sums : 8 * (size_t)N * (size_t)B);
+    const int vstep = fp.vstep;
     const int G = payoff_paths_per_thread(B, device_sms());
     const int64_t max_chunks = (B + 256 * (int64_t)G - 1) / (256 * (int64_t)G);
-    if ((rc = ensure(c.part, sizeof(double) * 4 * no * (size_t)max_chunks, "partials"))) return rc;
+    if ((rc = ensure(c, c.part, sizeof(double) * 4 * no * (size_t)max_chunks, "partials"))) return rc;
     // the kernel error word follows the accumulators
-    if ((rc = ensure(c.acc, sizeof(double) * (4 * no + 1), "accumulators"))) return rc;
-    if ((rc = ensure(c.res, sizeof(double) * 5 * no, "results"))) return rc;
+    if ((rc = ensure(c, c.acc, sizeof(double) * (4 * no + 1), "accumulators"))) return rc;
+    if ((rc = ensure(c, c.res, sizeof(double) * 5 * no, "results"))) return rc;
+    // what both forms need is there; without room for the rest of the digit
+    // convolution's the FP64 kernels take the call
+    if (fixed) {
+        rc = upload_tables(c, plan, st, ts, 0, &xt, false);
+        if (rc && rc != RBG_ERR_NOMEM) return rc;
+        fixed = !rc && ensure_fixed(c, x64_digit_bytes(B, N), fp.paths, fp.panels);
+    }
+    if (!fixed) {
+        if ((rc = fp64_conv_log2(o.conv, N, &logL))) return rc;
+        if ((rc = upload_tables(c, plan, st, ts, logL))) return rc;
+    }
     unsigned int* err = (unsigned int*)(c.acc.as<double>() + 4 * no);
     if (fixed) RBG_CUDA(cudaMemsetAsync(err, 0, sizeof(unsigned int), st));
     const MergeFinal fin{ts.t.outs, ts.Tvals, c.res.as<double>(), M, o.compute_iv};
@@ -509,7 +558,7 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
             if (!fixed) launch_path_fp64(ts.t, c.z.as<double>(), b, c.ivb.as<double>(), st, ivp);
             for (int v0 = 0; fixed && v0 < nv; v0 += vstep) {
                 const int k = std::min(vstep, nv - v0);
-                const unsigned char* pan = c.xpan.as<unsigned char>() + (size_t)v0 * x64_panel_bytes(N);
+                const unsigned char* pan = fixed_panels(c, ts, fp, v0, k, st);
                 if (fused) {
                     const int g0 = plan.vols[v0].vg_begin, ng = plan.vols[v0 + k - 1].vg_end - g0;
                     if (launch_volterra_variance(c.xdig.as<unsigned char>(), pan, ts.xvols + v0, ts.xgrps, ts.xcomp,
@@ -568,16 +617,16 @@ static int mixed_setup(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M
     if (sob && (job.backend != RBG_CONV_GEMM || plan.N > 1024))
         return fail(RBG_ERR_UNSUPPORTED, "Sobol' normals in the mixed form need the GEMM backend and N <= 1024");
     const int64_t B = job.batch;
-    if (sz && (rc = ensure(c.z, sizeof(double) * 2 * plan.N * (size_t)B, "normals"))) return rc;
-    if ((rc = ensure(c.mixed_ws, job.workspace_bytes, "mixed workspace"))) return rc;
+    if (sz && (rc = ensure(c, c.z, sizeof(double) * 2 * plan.N * (size_t)B, "normals"))) return rc;
+    if ((rc = ensure(c, c.mixed_ws, job.workspace_bytes, "mixed workspace"))) return rc;
     const int G = payoff_paths_per_thread(B, job.sms);
     const int64_t max_chunks = job.fused ? mixed_part_rows(job, B) : (B + 256 * (int64_t)G - 1) / (256 * (int64_t)G);
-    if (!job.fused && (rc = ensure(c.ivb, sizeof(float) * 2 * plan.vgs.size() * (size_t)B, "variance sums")))
+    if (!job.fused && (rc = ensure(c, c.ivb, sizeof(float) * 2 * plan.vgs.size() * (size_t)B, "variance sums")))
         return rc;
-    if (mc && (rc = ensure(c.ivp, sizeof(float) * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
-    if ((rc = ensure(c.part, sizeof(double) * 4 * no * (size_t)max_chunks, "partials"))) return rc;
-    if ((rc = ensure(c.acc, sizeof(double) * 4 * no, "accumulators"))) return rc;
-    if ((rc = ensure(c.res, sizeof(double) * 5 * no, "results"))) return rc;
+    if (mc && (rc = ensure(c, c.ivp, sizeof(float) * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
+    if ((rc = ensure(c, c.part, sizeof(double) * 4 * no * (size_t)max_chunks, "partials"))) return rc;
+    if ((rc = ensure(c, c.acc, sizeof(double) * 4 * no, "accumulators"))) return rc;
+    if ((rc = ensure(c, c.res, sizeof(double) * 5 * no, "results"))) return rc;
     if (c.mixed_img != job.host_ws) {
         c.mixed_img.clear();
         ++c.img_gen;
@@ -762,20 +811,20 @@ static int price_cv(Ctx& c, const Plan& plan, const rbg_cv_params& p, const rbg_
     const int64_t B = fp64_batch(plan, M, 4);  // normals plus two (Ivdt, IsvdW) sets per path
     if (Mc > fp64_batch(plan, Mc, 2)) return fail(RBG_ERR_ARG, "M_control too large for one pilot batch");
     const int64_t zpaths = std::max(B, Mc);
-    if ((rc = ensure(c.z, sizeof(double) * 2 * N * (size_t)zpaths, "normals"))) return rc;
-    if ((rc = ensure(c.ivb, sizeof(double) * 2 * ng * (size_t)zpaths, "variance sums"))) return rc;
-    if ((rc = ensure(c.ivp, sizeof(double) * 2 * ng * (size_t)B, "antithetic sums"))) return rc;
+    if ((rc = ensure(c, c.z, sizeof(double) * 2 * N * (size_t)zpaths, "normals"))) return rc;
+    if ((rc = ensure(c, c.ivb, sizeof(double) * 2 * ng * (size_t)zpaths, "variance sums"))) return rc;
+    if ((rc = ensure(c, c.ivp, sizeof(double) * 2 * ng * (size_t)B, "antithetic sums"))) return rc;
     const size_t cv_bytes = sizeof(double) * (size_t)no * (2 * (size_t)Mc + 2) + sizeof(unsigned long long) * no;
-    if ((rc = ensure(c.cv, cv_bytes, "control-variate scratch"))) return rc;
+    if ((rc = ensure(c, c.cv, cv_bytes, "control-variate scratch"))) return rc;
     double* alpha = c.cv.as<double>();
     double* Q = alpha + no;
     unsigned long long* count = (unsigned long long*)(Q + no);
     double* xy = (double*)(count + no);
     const int G = payoff_paths_per_thread(B, device_sms());
     const int64_t max_chunks = (B + 256 * (int64_t)G - 1) / (256 * (int64_t)G);
-    if ((rc = ensure(c.part, sizeof(double) * 4 * no * (size_t)max_chunks, "partials"))) return rc;
-    if ((rc = ensure(c.acc, sizeof(double) * 4 * no, "accumulators"))) return rc;
-    if ((rc = ensure(c.res, sizeof(double) * 5 * no, "results"))) return rc;
+    if ((rc = ensure(c, c.part, sizeof(double) * 4 * no * (size_t)max_chunks, "partials"))) return rc;
+    if ((rc = ensure(c, c.acc, sizeof(double) * 4 * no, "accumulators"))) return rc;
+    if ((rc = ensure(c, c.res, sizeof(double) * 5 * no, "results"))) return rc;
     // pilot: one batch of Mc paths
     if (Zc) {
         RBG_CUDA(cudaMemcpyAsync(c.z.p, Zc, sizeof(double) * 2 * N * Mc, cudaMemcpyHostToDevice, st));
@@ -839,15 +888,15 @@ static int price_cv_mixed(Ctx& c, const Plan& plan, const rbg_cv_params& p, cons
     const int64_t B = job.batch;
     const int G = payoff_paths_per_thread(B, job.sms);
     const int64_t max_chunks = (B + 256 * (int64_t)G - 1) / (256 * (int64_t)G);
-    if ((rc = ensure(c.z, sizeof(double) * 2 * N * (size_t)Mc, "pilot normals"))) return rc;
-    if ((rc = ensure(c.ivp, sizeof(double) * 2 * ng * (size_t)Mc, "pilot sums"))) return rc;
-    if ((rc = ensure(c.ivb, sizeof(float) * 4 * ng * (size_t)B, "variance sums"))) return rc;
+    if ((rc = ensure(c, c.z, sizeof(double) * 2 * N * (size_t)Mc, "pilot normals"))) return rc;
+    if ((rc = ensure(c, c.ivp, sizeof(double) * 2 * ng * (size_t)Mc, "pilot sums"))) return rc;
+    if ((rc = ensure(c, c.ivb, sizeof(float) * 4 * ng * (size_t)B, "variance sums"))) return rc;
     const size_t cv_bytes = sizeof(double) * (size_t)no * (2 * (size_t)Mc + 2) + sizeof(unsigned long long) * no;
-    if ((rc = ensure(c.cv, cv_bytes, "control-variate scratch"))) return rc;
-    if ((rc = ensure(c.mixed_ws, job.workspace_bytes, "mixed workspace"))) return rc;
-    if ((rc = ensure(c.part, sizeof(double) * 4 * no * (size_t)max_chunks, "partials"))) return rc;
-    if ((rc = ensure(c.acc, sizeof(double) * 4 * no, "accumulators"))) return rc;
-    if ((rc = ensure(c.res, sizeof(double) * 5 * no, "results"))) return rc;
+    if ((rc = ensure(c, c.cv, cv_bytes, "control-variate scratch"))) return rc;
+    if ((rc = ensure(c, c.mixed_ws, job.workspace_bytes, "mixed workspace"))) return rc;
+    if ((rc = ensure(c, c.part, sizeof(double) * 4 * no * (size_t)max_chunks, "partials"))) return rc;
+    if ((rc = ensure(c, c.acc, sizeof(double) * 4 * no, "accumulators"))) return rc;
+    if ((rc = ensure(c, c.res, sizeof(double) * 5 * no, "results"))) return rc;
     double* alpha = c.cv.as<double>();
     double* Q = alpha + no;
     unsigned long long* count = (unsigned long long*)(Q + no);
@@ -970,20 +1019,26 @@ static int payoffs_quadrature(const rbg_params* p, const double* Z, double* payo
     int64_t B = fp64_batch(plan, M, ns);
     // payoffs of a batch within 1 GiB too
     B = std::min<int64_t>(B, std::max<int64_t>(256, ((int64_t)1 << 30) / (8 * (int64_t)no)));
-    const int vstep = (int)std::max<int64_t>(1, std::min<int64_t>(nv, ((int64_t)1 << 31) / (8 * (int64_t)N * B)));
-    if ((rc = ensure(c->ivb, sizeof(double) * 2 * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
-    if (mc && (rc = ensure(c->ivp, sizeof(double) * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
+    const FixedPlan fp = fixed_plan(nv, N, 8 * (size_t)N * (size_t)B);
+    const int vstep = fp.vstep;
+    if ((rc = ensure(*c, c->ivb, sizeof(double) * 2 * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
+    if (mc && (rc = ensure(*c, c->ivp, sizeof(double) * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
     double* ivp = mc ? c->ivp.as<double>() : nullptr;
     if (!device_ptrs) {
-        if ((rc = ensure(c->z, sizeof(double) * ns * N * (size_t)B, "normals"))) return rc;
-        if ((rc = ensure(c->pay, sizeof(double) * no * (size_t)B, "payoffs"))) return rc;
+        if ((rc = ensure(*c, c->z, sizeof(double) * ns * N * (size_t)B, "normals"))) return rc;
+        if ((rc = ensure(*c, c->pay, sizeof(double) * no * (size_t)B, "payoffs"))) return rc;
     }
-    if (fixed && !ensure_fixed(*c, x64_digit_bytes(B, N), 8 * (size_t)vstep * N * (size_t)B)) fixed = false;
-    // the FP64 kernels' own tables wait for a batch that needs them
-    bool fp64_tables = !fixed;
-    if ((rc = upload_tables(*c, plan, st, ts, fixed ? 0 : logL, fixed ? &xt : nullptr, fp64_tables))) return rc;
     // device words: kernel error, normals out of range; read through pinned memory
-    if ((rc = ensure(c->acc, 2 * sizeof(unsigned int), "accumulators"))) return rc;
+    if ((rc = ensure(*c, c->acc, 2 * sizeof(unsigned int), "accumulators"))) return rc;
+    // without room for the digit convolution's buffers the FP64 kernels take the call;
+    // beside it their own tables wait for a batch that needs them
+    if (fixed) {
+        rc = upload_tables(*c, plan, st, ts, 0, &xt, false);
+        if (rc && rc != RBG_ERR_NOMEM) return rc;
+        fixed = !rc && ensure_fixed(*c, x64_digit_bytes(B, N), fp.paths, fp.panels);
+    }
+    if (!fixed && (rc = upload_tables(*c, plan, st, ts, logL))) return rc;
+    bool fp64_tables = !fixed;
     unsigned int* words = c->acc.as<unsigned int>();
     volatile unsigned int* seen = nullptr;
     if (fixed) {
@@ -1012,9 +1067,8 @@ static int payoffs_quadrature(const rbg_params* p, const double* Z, double* payo
             RBG_CUDA(cudaEventRecord(c->digits_done, st));
             for (int v0 = 0; v0 < nv; v0 += vstep) {
                 const int k = std::min(vstep, nv - v0);
-                if (launch_volterra_exact(c->xdig.as<unsigned char>(),
-                                          c->xpan.as<unsigned char>() + (size_t)v0 * x64_panel_bytes(N), ts.xvols + v0, k, N,
-                                          b, true, c->xbuf.as<uint64_t>(), words, st) ||
+                if (launch_volterra_exact(c->xdig.as<unsigned char>(), fixed_panels(*c, ts, fp, v0, k, st), ts.xvols + v0, k,
+                                          N, b, true, c->xbuf.as<uint64_t>(), words, st) ||
                     launch_variance_fixed(ts.xvols + v0, ts.xgrps, ts.xcomp, Zd, c->xbuf.as<uint64_t>(), k, xt.max_groups,
                                           xt.u53, true, ns, N, b, c->ivb.as<double>(), ivp, st))
                     return fail(RBG_ERR_CUDA, "FP64 path kernels could not be configured");
@@ -1028,8 +1082,10 @@ static int payoffs_quadrature(const rbg_params* p, const double* Z, double* payo
             out_of_range = seen[1] != 0;
         }
         if (out_of_range && !fp64_tables) {
+            // (growing the tables may have taken the digit convolution's buffers)
             if ((rc = upload_tables(*c, plan, st, ts, logL, &xt, true))) return rc;
             fp64_tables = true;
+            fixed = c->xdig.p && c->xbuf.p && c->xpan.p;
         }
         if (!fixed || out_of_range) launch_path_fp64(ts.t, Zd, b, c->ivb.as<double>(), st, ivp);
         if (launch_payoff_store(ts.t, c->ivb.as<double>(), b, b, Pd, st, ivp))
@@ -1038,9 +1094,9 @@ static int payoffs_quadrature(const rbg_params* p, const double* Z, double* payo
         if (!device_ptrs)
             RBG_CUDA(cudaMemcpyAsync(payoff + m0 * no, Pd, sizeof(double) * no * b, cudaMemcpyDeviceToHost, st));
     }
-    if (fixed) RBG_CUDA(cudaMemcpyAsync((void*)seen, words, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
+    if (seen) RBG_CUDA(cudaMemcpyAsync((void*)seen, words, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
     RBG_CUDA(cudaStreamSynchronize(st));
-    if (fixed && seen[0])
+    if (seen && seen[0])
         return fail(RBG_ERR_TIMEOUT,
                     "FP64 convolution: a bounded pipeline wait expired (site " + std::to_string(seen[0]) + ")");
     return RBG_OK;
@@ -1071,13 +1127,13 @@ static int payoffs_quadrature_mixed(const rbg_params* p, const rbg_options& o, c
     B = std::min<int64_t>(B, std::max<int64_t>(256, ((int64_t)1 << 30) / (8 * (int64_t)no)));  // payoffs <= 1 GiB
     if (!device_ptrs)  // staged normals <= 2 GiB
         B = std::min<int64_t>(B, std::max<int64_t>(256, ((int64_t)1 << 31) / (8 * (int64_t)ns * N)));
-    if ((rc = ensure(c->mixed_ws, job.workspace_bytes, "mixed workspace"))) return rc;
-    if ((rc = ensure(c->ivb, sizeof(float) * 2 * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
-    if (mc && (rc = ensure(c->ivp, sizeof(float) * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
+    if ((rc = ensure(*c, c->mixed_ws, job.workspace_bytes, "mixed workspace"))) return rc;
+    if ((rc = ensure(*c, c->ivb, sizeof(float) * 2 * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
+    if (mc && (rc = ensure(*c, c->ivp, sizeof(float) * plan.vgs.size() * (size_t)B, "variance sums"))) return rc;
     float* ivq = mc ? c->ivp.as<float>() : nullptr;
     if (!device_ptrs) {
-        if ((rc = ensure(c->z, sizeof(double) * ns * N * (size_t)B, "normals"))) return rc;
-        if ((rc = ensure(c->pay, sizeof(double) * no * (size_t)B, "payoffs"))) return rc;
+        if ((rc = ensure(*c, c->z, sizeof(double) * ns * N * (size_t)B, "normals"))) return rc;
+        if ((rc = ensure(*c, c->pay, sizeof(double) * no * (size_t)B, "payoffs"))) return rc;
     }
     if (c->mixed_img != job.host_ws) {
         c->mixed_img.clear();
@@ -1248,7 +1304,7 @@ int rbg_generate_normals_streams(uint64_t seed, int64_t path_offset, int64_t M, 
     std::lock_guard<std::mutex> lk(c->mu);
     const int ns = streams;
     const int64_t B = std::max<int64_t>(1, std::min<int64_t>(M, ((int64_t)1 << 30) / (8 * ns * (int64_t)N)));
-    if ((rc = ensure(c->z, sizeof(double) * ns * N * (size_t)B, "normals"))) return rc;
+    if ((rc = ensure(*c, c->z, sizeof(double) * ns * N * (size_t)B, "normals"))) return rc;
     for (int64_t m0 = 0; m0 < M; m0 += B) {
         const int64_t b = std::min(B, M - m0);
         if (launch_normals_fixed(seed, path_offset + m0, b, N, precision == RBG_MIXED, c->z.as<double>(), nullptr, 0, ns,
@@ -1294,7 +1350,7 @@ static int sobol_setup(Ctx& c, const uint64_t* dirs, int dims, int N, int bridge
     for (int k = 0; k < kSobolBits; ++k)
         for (int d = 0; d < D; ++d) img[(size_t)k * D + d] = dirs[(size_t)d * kSobolBits + k];
     if (img != c.sobol_img) {
-        int rc = ensure(c.sobol, sizeof(unsigned long long) * img.size(), "Sobol' table");
+        int rc = ensure(c, c.sobol, sizeof(unsigned long long) * img.size(), "Sobol' table");
         if (rc) return rc;
         c.sobol_img.clear();
         RBG_CUDA(cudaMemcpyAsync(c.sobol.p, img.data(), sizeof(unsigned long long) * img.size(),
@@ -1322,7 +1378,7 @@ int rbg_sobol_normals(const uint64_t* directions, int dims, int N, int64_t M, in
     SobolBridge br{};
     if ((rc = sobol_setup(*c, directions, dims, N, bridge, path_offset, M, c->stream, br))) return rc;
     const int64_t B = std::max<int64_t>(1, std::min<int64_t>(M, ((int64_t)1 << 30) / (16 * (int64_t)N)));
-    if ((rc = ensure(c->z, sizeof(double) * 2 * N * (size_t)B, "normals"))) return rc;
+    if ((rc = ensure(*c, c->z, sizeof(double) * 2 * N * (size_t)B, "normals"))) return rc;
     for (int64_t m0 = 0; m0 < M; m0 += B) {
         const int64_t b = std::min(B, M - m0);
         if (launch_sobol_normals(c->sobol.as<unsigned long long>(), N, (uint64_t)(path_offset + m0 + 1), b,
@@ -1351,7 +1407,7 @@ static int sobol32_setup(Ctx& c, const uint64_t* dirs, int dims, int N, int64_t 
     for (int k = 0; k < 32; ++k)
         for (int d = 0; d < D; ++d) img[(size_t)k * D + d] = (unsigned int)(dirs[(size_t)d * kSobolBits + k] >> 30);
     if (img != c.sobol32_img) {
-        int rc = ensure(c.sobol32, sizeof(unsigned int) * img.size(), "Sobol' table");
+        int rc = ensure(c, c.sobol32, sizeof(unsigned int) * img.size(), "Sobol' table");
         if (rc) return rc;
         c.sobol32_img.clear();
         RBG_CUDA(cudaMemcpyAsync(c.sobol32.p, img.data(), sizeof(unsigned int) * img.size(), cudaMemcpyHostToDevice,
@@ -1433,7 +1489,7 @@ int rbg_implied_vol(int n, const double* price, const double* K, const double* T
     int rc = get_ctx(&c);
     if (rc) return rc;
     std::lock_guard<std::mutex> lk(c->mu);
-    if ((rc = ensure(c->res, sizeof(double) * 4 * (size_t)n, "iv buffers"))) return rc;
+    if ((rc = ensure(*c, c->res, sizeof(double) * 4 * (size_t)n, "iv buffers"))) return rc;
     double* d = c->res.as<double>();
     RBG_CUDA(cudaMemcpyAsync(d, price, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
     RBG_CUDA(cudaMemcpyAsync(d + n, K, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
@@ -1498,7 +1554,7 @@ int rbg_debug_mixed_paths(const rbg_params* p, const rbg_options* o, float* norm
     if (job.batch < p->M) return fail(RBG_ERR_ARG, "diagnostic run does not fit one batch");
     const int Np = (plan.N + 31) / 32 * 32;
     const size_t M = (size_t)p->M, nvg = plan.vgs.size();
-    if ((rc = ensure(c->mixed_ws, job.workspace_bytes, "mixed workspace"))) return rc;
+    if ((rc = ensure(*c, c->mixed_ws, job.workspace_bytes, "mixed workspace"))) return rc;
     DevBuf dbg;
     if (dbg.ensure(sizeof(float) * (M * 2 * Np + M * Np + 2 * nvg * M))) return fail(RBG_ERR_NOMEM, "debug buffers");
     float* dw = dbg.as<float>();
@@ -1587,7 +1643,7 @@ int rbg_debug_mixed_profile(const rbg_params* p, const rbg_options* o, uint64_t*
     if ((rc = mixed_prepare(plan, *o, p->M, job, g_err))) return rc;
     if (job.batch < p->M) return fail(RBG_ERR_ARG, "diagnostic run does not fit one batch");
     const int no = (int)plan.outs.size();
-    if ((rc = ensure(c->mixed_ws, job.workspace_bytes, "mixed workspace"))) return rc;
+    if ((rc = ensure(*c, c->mixed_ws, job.workspace_bytes, "mixed workspace"))) return rc;
     DevBuf dbg;
     const size_t ivb_bytes = job.fused ? 0 : sizeof(float) * 2 * plan.vgs.size() * (size_t)p->M;
     const size_t part_bytes = sizeof(double) * 4 * no * (size_t)std::max(1, mixed_part_rows(job, p->M));
