@@ -311,6 +311,21 @@ RBG_HD double exp2_fixed53(int64_t x, const uint64_t* E)
     return bits_double(e < -1022 ? 0ull : b);                 // e <= 1023: x 2^-53 < 1024
 }
 
+// ------------------------------------------------------- sums of 32 steps
+// Terms of the sums of 2^(2 t) and 2^t W over the 32 steps of a warp (the variance
+// pass in the convolution's read-out), m = 2^t in units of 2^-61 of the steps'
+// largest power of two: m^2 2^-64, and m (w 2^-64) for half = (2^63 + w) >> 1, the
+// normal w in units of 2^-59.
+RBG_HD int64_t slot_square(uint64_t m)
+{
+    return (int64_t)(mul32(hi32(m), hi32(m)) + (mul32(hi32(m), lo32(m)) >> 31));
+}
+RBG_HD int64_t slot_product(uint64_t m, uint64_t half) { return (int64_t)(mulhi64(m, half) - (m >> 2)); }
+// What a sum of `live` terms loses to truncation on average, shifting 2^t to m
+// included: seven eighths of a unit a term (square 0.75 and m 2^-64, product
+// 0.9); steps past the last one lose nothing.
+RBG_HD int64_t slot_back(int live) { return (7 * live + 4) >> 3; }
+
 // ---------------------------------------------------------- normal tail
 // Mills' ratio M(x) = (1 - Phi(x)) / phi(x), x >= 0, on 64 intervals per octave
 // of y = 1 + x, y < 64: with f the position inside the interval (0 .. 1),

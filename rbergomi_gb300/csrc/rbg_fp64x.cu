@@ -379,7 +379,8 @@ struct FuseArgs {
 // warp's sums of 2^(2 t) and 2^t W over its 32 steps, v = xi 2^(2 t) (k_variance_fixed).
 // The sums are taken in integers: with 2^t = m 2^(e - 63), E the largest e of the
 // 32 steps and m' = m >> (E - e + 3), 32 terms m'^2 and m' W / 2 fit 64 bits, and
-// half a unit a term goes back for the truncation.  The square's unit is 2^-54 of
+// what truncation takes of the live terms on average goes back (slot_square,
+// slot_product, slot_back).  The square's unit is 2^-54 of
 // the largest term or less, the product's 2^-54 2^E; an FP64 sum rounds every product
 // to 2^-53 of itself and every partial sum likewise.  The same in FP64 (two
 // products, the lanes' additions) holds the FP64 pipe: 30011 paths of 250 steps, two
@@ -398,6 +399,7 @@ __device__ __forceinline__ void fused_variance(uint64_t (&x)[2][8], const X64Vol
     const int jc = min(j, N - 2), left = (int)min(B - m0, (int64_t)16);  // paths of the warp's 16
     const bool whole = left == 16 && __all_sync(0xffffffffu, in);
     if (left <= 0) return;
+    const int64_t back = slot_back(max(0, min(32, N - 1 - 32 * slot)));
     const uint64_t* z0 = fa.Z + m0 * NS * (int64_t)N + jc;
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
@@ -426,11 +428,11 @@ __device__ __forceinline__ void fused_variance(uint64_t (&x)[2][8], const X64Vol
                 }
                 top[p] = __reduce_max_sync(0xffffffffu, e);
                 mt >>= min(top[p] - e + 3, 63);
-                s[2 * p] = (int64_t)(mul32(hi32(mt), hi32(mt)) + (mul32(hi32(mt), lo32(mt)) >> 31));  // m'^2 2^-64
-                s[2 * p + 1] = (int64_t)(mulhi64(mt, w1[p]) - (mt >> 2));
-                if (NS == 3) sq[p] = (int64_t)(mulhi64(mt, wq[p]) - (mt >> 2));
+                s[2 * p] = slot_square(mt);
+                s[2 * p + 1] = slot_product(mt, w1[p]);
+                if (NS == 3) sq[p] = slot_product(mt, wq[p]);
             }
-            const int64_t i0 = warp_sums_i64<8>(s) + 16;  // value lane / 4 = 2 path + sum
+            const int64_t i0 = warp_sums_i64<8>(s) + back;  // value lane / 4 = 2 path + sum
             const int pa = lane >> 3, c = (lane >> 2) & 1;
             const int tp = pa & 2 ? (pa & 1 ? top[3] : top[2]) : (pa & 1 ? top[1] : top[0]);
             const double sc = bits_double((uint64_t)(uint32_t)(tp + 1023) << 52);
@@ -438,7 +440,7 @@ __device__ __forceinline__ void fused_variance(uint64_t (&x)[2][8], const X64Vol
             const double r = (c ? (double)i0 * 0x1p-54 : (double)i0 * 0x1p-56 * sc) * sc;
             if (!(lane & 3) && 4 * h + pa < left) out[c] = r;
             if constexpr (NS == 3) {
-                const int64_t i2 = warp_sums_i64<4>(sq) + 16;
+                const int64_t i2 = warp_sums_i64<4>(sq) + back;
                 if (!(lane & 7) && 4 * h + pa < left) out[2] = (double)i2 * 0x1p-54 * sc;
             }
         }
