@@ -539,6 +539,7 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
     }
     unsigned int* err = (unsigned int*)(c.acc.as<double>() + 4 * no);
     if (fixed) RBG_CUDA(cudaMemsetAsync(err, 0, sizeof(unsigned int), st));
+    bool wide = true;
     const MergeFinal fin{ts.t.outs, ts.Tvals, c.res.as<double>(), M, o.compute_iv};
     for (int64_t m0 = 0; m0 < M; m0 += B) {
         const int64_t b = std::min(B, M - m0);
@@ -553,6 +554,7 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
                 return fail(RBG_ERR_CUDA, "fixed-point tables not found on the device");
             }
         }
+        if (fixed && m0 == 0) wide = x64_wide(xt, N);
         {
             ProfScope ps(kStagePathFp64, st, fixed ? 2 * ((nv + vstep - 1) / vstep) : 1);
             if (!fixed) launch_path_fp64(ts.t, c.z.as<double>(), b, c.ivb.as<double>(), st, ivp);
@@ -562,10 +564,10 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
                 if (fused) {
                     const int g0 = plan.vols[v0].vg_begin, ng = plan.vols[v0 + k - 1].vg_end - g0;
                     if (launch_volterra_variance(c.xdig.as<unsigned char>(), pan, ts.xvols + v0, ts.xgrps, ts.xcomp,
-                                                 c.z.as<double>(), k, g0, ng, ns, N, b, c.xbuf.as<double>(),
+                                                 c.z.as<double>(), k, g0, ng, ns, wide, N, b, c.xbuf.as<double>(),
                                                  c.ivb.as<double>(), ivp, err, st))
                         return fail(RBG_ERR_CUDA, "FP64 path kernels could not be configured");
-                } else if (launch_volterra_exact(c.xdig.as<unsigned char>(), pan, ts.xvols + v0, k, N, b, false,
+                } else if (launch_volterra_exact(c.xdig.as<unsigned char>(), pan, ts.xvols + v0, k, N, b, false, wide,
                                                  c.xbuf.as<uint64_t>(), err, st) ||
                            launch_variance_fixed(ts.xvols + v0, ts.xgrps, ts.xcomp, c.z.as<double>(),
                                                  c.xbuf.as<uint64_t>(), k, xt.max_groups, xt.u53, false, ns, N, b,
@@ -1068,7 +1070,7 @@ static int payoffs_quadrature(const rbg_params* p, const double* Z, double* payo
             for (int v0 = 0; v0 < nv; v0 += vstep) {
                 const int k = std::min(vstep, nv - v0);
                 if (launch_volterra_exact(c->xdig.as<unsigned char>(), fixed_panels(*c, ts, fp, v0, k, st), ts.xvols + v0, k,
-                                          N, b, true, c->xbuf.as<uint64_t>(), words, st) ||
+                                          N, b, true, true, c->xbuf.as<uint64_t>(), words, st) ||
                     launch_variance_fixed(ts.xvols + v0, ts.xgrps, ts.xcomp, Zd, c->xbuf.as<uint64_t>(), k, xt.max_groups,
                                           xt.u53, true, ns, N, b, c->ivb.as<double>(), ivp, st))
                     return fail(RBG_ERR_CUDA, "FP64 path kernels could not be configured");

@@ -20,11 +20,16 @@
 //
 // Exactness of the convolution.  A digit is an integer in [-128, 127], exact in
 // FP16; a product has 14 bits, and an FP32 accumulator holds integers up to
-// 2^24 exactly.  The digits of W1 below the first are uniform over their range
-// and independent between steps (the first is round(8 W1), below 55), so a
-// diagonal of (d + 1) K products has a standard deviation below 74^2 sqrt((d +
-// 1) K): 7.1e5 = 2^19.4 at d = 7 and K = 2048, 24 standard deviations from 2^24
-// (17 at K = 4096).  Left out are the products with d >= 8, below 2^-60 of the
+// 2^24 exactly.  The digits of W1 below the first are uniform over [-128, 127] (mean
+// -1/2, root mean square 73.9) and independent between steps; the first is round(8 W1), below
+// 55 and of root mean square 8.  Gamma's digits are what they are: a diagonal's mean and
+// standard deviation follow from the sums of them and of their squares, which
+// digit_margin adds up for the plan's own Gamma.  The read-out by 1.5 2^23 is taken up
+// to 1024 steps where every partial sum is 9 standard deviations or more from that one's
+// limit of 2^22 (2e-19 a sum; x64_wide), else the conversion, and x64_prepare leaves to the FP64
+// kernels a plan that comes closer than that to 2^24.  The least over H = 0.01 .. 0.99: 18.4 standard
+// deviations from 2^22 at 256 steps, 13.0 at 512, 9.1 at 1024 (H = 0.6), and from 2^24 26 at
+// 2048, 18 at 4096.  Left out are the products with d >= 8, below 2^-60 of the
 // operands' product each: the sums are within about 2^-54 of the exact ones,
 // against 2^-45 for an FP64 FFT of 1024 points and 2^-50 for the direct FP64
 // sum of 100 steps.
@@ -472,8 +477,8 @@ struct PanelSlots {
 
 // One (block b, pass v, group of 64 paths) at a time, the longest blocks
 // first.  Warps 0-15 read the accumulators, warp 16 loads, warps 17 and 18 issue
-// the MMAs.  WIDE: accumulators may pass 2^22 (N > 1024): converted by F2I, else by
-// adding 1.5 2^23.  SEG: the caller's normals, whose digits may add up: the
+// the MMAs.  WIDE: accumulators may pass 2^22 (above 1024 steps, and where
+// x64_wide finds it of Gamma's digits, which it does not for H below 1): converted by F2I, else by adding 1.5 2^23.  SEG: the caller's normals, whose digits may add up: the
 // accumulators are read out every 128 steps and X summed in integers, which is
 // exact for any digits.
 // What bounds it: 2304 columns x 128 steps x 16 per chunk, 1152 MMA cycles,
@@ -801,11 +806,11 @@ static int volterra_grid(int64_t B, int N, int nv)
 
 int launch_volterra_variance(const unsigned char* dig, const unsigned char* panels, const X64Vol* vols,
                              const X64Group* grps, const uint64_t* comp, const double* Z, int nv, int grp0, int ng, int ns,
-                             int N, int64_t B, double* part, double* ivb, double* ivp, unsigned int* err, cudaStream_t st)
+                             bool wide, int N, int64_t B, double* part, double* ivb, double* ivp, unsigned int* err,
+                             cudaStream_t st)
 {
     const FixedTables* ft = fixed_tables();
     if (!ft) return -1;
-    const bool wide = N > 1024;
     const bool one = ng == nv;  // every pass has at least one group
     auto* kern = ns == 3 ? (wide ? k_volterra_exact<true, false, 3> : k_volterra_exact<false, false, 3>)
                  : one   ? (wide ? k_volterra_exact<true, false, 1> : k_volterra_exact<false, false, 1>)
@@ -822,11 +827,11 @@ int launch_volterra_variance(const unsigned char* dig, const unsigned char* pane
 }
 
 int launch_volterra_exact(const unsigned char* dig, const unsigned char* panels, const X64Vol* vols, int nv, int N,
-                          int64_t B, bool any, uint64_t* X, unsigned int* err, cudaStream_t st)
+                          int64_t B, bool any, bool wide, uint64_t* X, unsigned int* err, cudaStream_t st)
 {
     // any digits: sums of at most 128 steps, whose diagonals stay within 2^24 whatever the digits are
     auto* kern = any ? k_volterra_exact<true, true, 0>
-                     : (N > 1024 ? k_volterra_exact<true, false, 0> : k_volterra_exact<false, false, 0>);
+                     : (wide ? k_volterra_exact<true, false, 0> : k_volterra_exact<false, false, 0>);
     if (!allow_smem((const void*)kern, kXSmemPlain)) return -1;
     kern<<<volterra_grid(B, N, nv), kXThreads, kXSmemPlain, st>>>(dig, panels, vols, nv, N, B, X, err, FuseArgs{});
     count_launch();
@@ -996,6 +1001,53 @@ int launch_variance_fixed(const X64Vol* vols, const X64Group* grps, const uint64
 }
 
 // -------------------------------------------------------------------- host
+double digit_margin(const int64_t* gam, int N, double limit)
+{
+    // sums of every digit and of its square; the largest partial sum is found every 16 steps
+    double most[8] = {}, square[8] = {}, total[8] = {};
+    for (int k0 = 0; k0 < N; k0 += 16) {
+        int s[8] = {}, q[8] = {};
+        for (int k = k0; k < std::min(N, k0 + 16); ++k) {
+            const uint64_t u = (uint64_t)gam[k] + 0x8080808080808080ull;
+            unsigned char byte[8];
+            std::memcpy(byte, &u, 8);
+            for (int b = 0; b < 8; ++b) {
+                const int x = byte[b] - 128;
+                s[b] += x;
+                q[b] += x * x;
+            }
+        }
+        for (int b = 0; b < 8; ++b) {
+            total[b] += s[b];
+            square[b] += q[b];
+            most[b] = std::max(most[b], std::fabs(total[b]));
+        }
+    }
+    // the digits of W1: root mean square squared, size of the mean (FP32 normals: the
+    // last bits of the fourth are zero, mean -4.5)
+    const double sq[8] = {64.0, 5461.5, 5461.5, 5461.5, 5461.5, 5461.5, 5461.5, 5461.5};
+    const double mean[8] = {0.0, 0.5, 0.5, 5.0, 0.5, 0.5, 0.5, 0.5};
+    double margin = HUGE_VAL;
+    for (int d = 0; d < kXDigits; ++d) {
+        double v = 0.0, m = 0.0;
+        for (int j = 0; j <= d; ++j) {
+            v += square[7 - j] * sq[d - j];
+            m += (most[7 - j] + 16.0 * 128.0) * mean[d - j];
+        }
+        if (v > 0.0) margin = std::min(margin, (limit - m) / std::sqrt(v));
+    }
+    return margin;
+}
+
+bool x64_wide(const X64Tables& t, int N)
+{
+    if (N > 1024) return true;
+    if (N <= 256) return false;  // the margin is 9 whatever Gamma's digits are
+    for (size_t v = 0; v < t.vols.size(); ++v)
+        if (digit_margin(t.gam.data() + v * N, N, 0x1p22) < kXMargin) return true;
+    return false;
+}
+
 bool x64_prepare(const Plan& plan, X64Tables& out, bool ext)
 {
     const int N = plan.N, nv = (int)plan.vols.size(), ng = (int)plan.vgs.size();
@@ -1040,6 +1092,9 @@ bool x64_prepare(const Plan& plan, X64Tables& out, bool ext)
         q[0] = (int64_t)(V.a1 * unit);  // whole units from 2^(e - 10) up, truncated below
         for (int d = 1; d < N; ++d) q[d] = (int64_t)(G[d] * unit);
         out.max_groups = std::max(out.max_groups, V.vg_end - V.vg_begin);
+        // (up to 2048 steps the margin is larger whatever Gamma's digits are; the caller's normals are summed
+        // in parts that no digits can take past 2^24)
+        if (!ext && N > 2048 && digit_margin(q, N, 0x1p24) < kXMargin) return false;
     }
     const double l2 = 1.4426950408889634074, l2lo = 2.0355273740931033e-17;  // log2 e
     for (int g = 0; g < ng; ++g) {

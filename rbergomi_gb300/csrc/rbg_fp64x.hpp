@@ -38,6 +38,14 @@ struct X64Tables {
 };
 // Size that the caller's normals (ext) stay below: 15.5.
 constexpr double kExtMax = 15.5;
+// Standard deviations the convolution's accumulators keep from their limits.
+constexpr double kXMargin = 9.0;
+// How many standard deviations every partial sum of W1's digits times those of Gamma' (gam, N
+// steps) stays from `limit`, at least.
+double digit_margin(const int64_t* gam, int N, double limit);
+// Whether the convolution's accumulators may pass 2^22 (4 us a pass of 512 steps on the
+// host: callers ask while the normals are drawn).
+bool x64_wide(const X64Tables& t, int N);
 // False where the plan's numbers do not fit the fixed-point ranges; ext: for the
 // caller's normals.
 bool x64_prepare(const Plan& plan, X64Tables& out, bool ext = false);
@@ -67,7 +75,7 @@ void launch_digits(const double* Z, int64_t B, int N, int ns, unsigned char* dig
 // X[v][m][j] + 2^63; any: exact for any digits, not only for those of independent
 // normals
 int launch_volterra_exact(const unsigned char* dig, const unsigned char* panels, const X64Vol* vols, int nv, int N,
-                          int64_t B, bool any, uint64_t* X, unsigned int* err, cudaStream_t st);
+                          int64_t B, bool any, bool wide, uint64_t* X, unsigned int* err, cudaStream_t st);
 // Both passes in one kernel, for groups with 53 fraction bits; the passes'
 // groups are grp0 .. grp0 + ng - 1, part holds x64_slot_bytes per group.
 // Worth it up to x64_fuse_groups groups a pass (path pass in microseconds, fused
@@ -78,7 +86,7 @@ constexpr int x64_fuse_groups(int ns) { return ns == 3 ? 6 : 3; }
 size_t x64_slot_bytes(int64_t B, int N, int ns);
 int launch_volterra_variance(const unsigned char* dig, const unsigned char* panels, const X64Vol* vols,
                              const X64Group* grps, const uint64_t* comp, const double* Z, int nv, int grp0, int ng, int ns,
-                             int N, int64_t B, double* part, double* ivb, double* ivp, unsigned int* err, cudaStream_t st);
+                             bool wide, int N, int64_t B, double* part, double* ivb, double* ivp, unsigned int* err, cudaStream_t st);
 // ivb[g][B] (Ivdt, IsvdW); ns = 3: ivp[g][B] IsvdWp too; ext: Z holds doubles
 // throughout
 int launch_variance_fixed(const X64Vol* vols, const X64Group* grps, const uint64_t* comp, const double* Z,
