@@ -694,19 +694,14 @@ struct MergeSmem {
 };
 
 // Output i: acc (S, C, S2, C2) plus every chunk's, or just these where `fresh`;
-// stored to acc and, on every thread, in v.  A sum with a NaN or infinity in
+// stored to acc and sm.out.  By the first kMergeThreads threads of the block, which
+// wait for one another only.  A sum with a NaN or infinity in
 // it is added up in FP64 by one thread.
-__device__ void merge_block(const double* __restrict__ part, int nchunks, int n_out, double* __restrict__ acc, int i,
-                            bool fresh, MergeSmem& sm, double (&v)[4])
+__device__ __forceinline__ void merge_add(const double* __restrict__ part, int nchunks, int n_out,
+                                          double* __restrict__ acc, int i, bool fresh, MergeSmem& sm)
 {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (w >= kMergeThreads / 32) {  // waits for the sums with the others
-#pragma unroll
-        for (int k = 0; k < 3; ++k) __syncthreads();
-#pragma unroll
-        for (int k = 0; k < 4; ++k) v[k] = sm.out[k];
-        return;
-    }
+    auto adders = [] { asm volatile("barrier.sync 1, %0;" ::"n"(kMergeThreads) : "memory"); };
     // the largest exponent of either sum
     int em[2] = {0, 0};
     for (int c = threadIdx.x; c < nchunks; c += kMergeThreads) {
@@ -722,7 +717,7 @@ __device__ void merge_block(const double* __restrict__ part, int nchunks, int n_
         em[z] = __reduce_max_sync(0xffffffffu, em[z]);
         if (lane == 0) sm.emax[w][z] = em[z];
     }
-    __syncthreads();
+    adders();
 #pragma unroll
     for (int z = 0; z < 2; ++z)
 #pragma unroll
@@ -749,7 +744,7 @@ __device__ void merge_block(const double* __restrict__ part, int nchunks, int n_
             fix_add(s[z], __shfl_xor_sync(0xffffffffu, s[z].lo, o), __shfl_xor_sync(0xffffffffu, s[z].hi, o));
         if (lane == 0) sm.s[w][z] = s[z];
     }
-    __syncthreads();
+    adders();
     if (threadIdx.x < 2) {
         const int z = threadIdx.x;
         double S, C;
@@ -765,6 +760,13 @@ __device__ void merge_block(const double* __restrict__ part, int nchunks, int n_
         acc[i * 4 + 2 * z] = sm.out[2 * z] = S;
         acc[i * 4 + 2 * z + 1] = sm.out[2 * z + 1] = C;
     }
+}
+
+// The same on every thread of the block, in v; the last warp only waits.
+__device__ void merge_block(const double* __restrict__ part, int nchunks, int n_out, double* __restrict__ acc, int i,
+                            bool fresh, MergeSmem& sm, double (&v)[4])
+{
+    if (threadIdx.x < kMergeThreads) merge_add(part, nchunks, n_out, acc, i, fresh, sm);
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 4; ++k) v[k] = sm.out[k];
