@@ -188,11 +188,10 @@ RBG_HD uint64_t sqrt_fixed(uint64_t w)
 // with the residual of w y^2, four rotation products and every series term to
 // 2^-60 (1.40 units): 0.91 -> 0.84 ms for k_normals_fixed's stated draw.  A second
 // table for the next nine bits of the angle saves four more and is slower (0.85).
-RBG_HD void box_muller_fixed(uint32_t a, uint32_t b, const NormalTables& T, int64_t& z0, int64_t& z1)
+//
+// -2 ln u0 = w 2^-64 2^ex, w in [2^62, 2^64), ex even.
+RBG_HD void box_muller_log(uint32_t a, const NormalTables& T, uint64_t& w, int& ex)
 {
-    // -2 ln u0 = w 2^-64 2^ex, w in [2^62, 2^64), ex even
-    uint64_t w;
-    int ex;
     if (a - 1u >= 0xFFEFFFFFu) {
         if (a == 0u) {
             w = 0xB6FDA8B7905DF579ull;  // 66 ln 2 / 64
@@ -237,8 +236,11 @@ RBG_HD void box_muller_fixed(uint32_t a, uint32_t b, const NormalTables& T, int6
         w = shl(L, k);
         ex = c0 - k;
     }
-    const uint64_t r = shr(sqrt_fixed(w), 3 - (ex >> 1));  // sqrt(-2 ln u0), unit 2^-60
+}
 
+// Cosine and sine of 2 pi u1 less its quadrant, units 2^-63.
+RBG_HD void box_muller_angle(uint32_t b, const NormalTables& T, uint64_t& c, uint64_t& sn)
+{
     // 2 pi u1 = (quadrant) pi / 2 + pi k / 1024 + d, d = p pi 2^-32 with p = 2 (b mod 2^21) + 1
     const uint32_t p = 2u * (b & 0x1FFFFFu) + 1u;
     const FixedPair cs = T.trig[(b >> 21) & (kTrigTable - 1)];
@@ -254,8 +256,17 @@ RBG_HD void box_muller_fixed(uint32_t a, uint32_t b, const NormalTables& T, int6
     // (cos, sin)(a + d) = (x - x nc - y sd, y - y nc + x sd) in three products: with p = (x + y)(sd - nc) the
     // sine is y + p + x nc - y sd
     const uint64_t xn = mulhi64(cs.x, nc) >> 17, ys = mulhi64(cs.y, sd) >> 8;
-    const uint64_t c = cs.x - xn - ys;  // unit 2^-63
-    const uint64_t sn = cs.y + (mulhi64((cs.x >> 1) + (cs.y >> 1), sd - (nc >> 9)) >> 7) + xn - ys;
+    c = cs.x - xn - ys;
+    sn = cs.y + (mulhi64((cs.x >> 1) + (cs.y >> 1), sd - (nc >> 9)) >> 7) + xn - ys;
+}
+
+RBG_HD void box_muller_fixed(uint32_t a, uint32_t b, const NormalTables& T, int64_t& z0, int64_t& z1)
+{
+    uint64_t w, c, sn;
+    int ex;
+    box_muller_log(a, T, w, ex);
+    const uint64_t r = shr(sqrt_fixed(w), 3 - (ex >> 1));  // sqrt(-2 ln u0), unit 2^-60
+    box_muller_angle(b, T, c, sn);
     // quadrant q: (c, s), (-s, c), (-c, -s), (s, -c)
     const bool odd = (b & 0x40000000u) != 0u;
     const uint64_t m0 = mulhi64(r, odd ? sn : c), m1 = mulhi64(r, odd ? c : sn);  // unit 2^-59
@@ -263,6 +274,47 @@ RBG_HD void box_muller_fixed(uint32_t a, uint32_t b, const NormalTables& T, int6
     const uint64_t s1 = (uint64_t)(int64_t)((int32_t)b >> 31);               // sine in 2, 3
     z0 = (int64_t)((m0 ^ s0) - s0);
     z1 = (int64_t)((m1 ^ s1) - s1);
+}
+
+// sin(q pi 2^-32), relative accuracy for any 0 < q < 2^31: fixed, unit 2^-63, is it to
+// within 2^-59 (half a unit of 2^-53 of it from 2^-5 up).
+RBG_HD double sine_double(uint32_t q, uint64_t fixed)
+{
+    if (fixed >= 1ull << 58) return (double)fixed * 0x1p-63;  // (one is 2^63)
+    // pi in two parts, and one more rounding for d - d^3 (1/6 - d^2 / 120 + d^4 / 5040)
+    const double p = (double)(int32_t)q, d = fma(p, 0x1.921fb54442d18p+1 * 0x1p-32, p * (0x1.1a62633145c07p-53 * 0x1p-32));
+    const double d2 = d * d;
+    return fma(d * d2, fma(d2, fma(d2, -1.0 / 5040, 1.0 / 120), -1.0 / 6), d);
+}
+
+// The same normals as doubles, within 3 2^-53 of them relatively however small (9 2^-53
+// for 1 - u0 down to 2^-12, 3 again below): from the fixed-point ones down to 1/8,
+// below by their factors' significant bits.
+// (Normals that a caller asks for; a unit of 2^-59 is all the pricing sums need.)
+RBG_HD void box_muller_double(uint32_t a, uint32_t b, const NormalTables& T, double& z0, double& z1)
+{
+    int64_t v0, v1;
+    box_muller_fixed(a, b, T, v0, v1);
+    z0 = fixed_to_double(v0);
+    z1 = fixed_to_double(v1);
+    constexpr int64_t lim = 1ll << (kNormalBits - 3);
+    const bool s0 = v0 < lim && v0 > -lim, s1 = v1 < lim && v1 > -lim;
+    if (!s0 && !s1) return;
+    uint64_t w, c, sn;
+    int ex;
+    box_muller_log(a, T, w, ex);
+    box_muller_angle(b, T, c, sn);
+    // the radius in two parts
+    const int64_t root = (int64_t)sqrt_fixed(w);
+    const double unit = bits_double((uint64_t)(uint32_t)(1023 - 63 + (ex >> 1)) << 52);
+    const double rh = (double)(root & ~0x3FFll) * unit, rl = (double)(root & 0x3FFll) * unit;
+    const uint32_t q = 2u * (b & 0x3FFFFFFFu) + 1u;
+    const double cd = sine_double(0x80000000u - q, c), sd = sine_double(q, sn);
+    const double x = fma(rh, cd, rl * cd), y = fma(rh, sd, rl * sd);
+    const bool odd = (b & 0x40000000u) != 0u;
+    const double m0 = odd ? y : x, m1 = odd ? x : y;
+    if (s0) z0 = (int32_t)(b ^ (b << 1)) < 0 ? -m0 : m0;
+    if (s1) z1 = (int32_t)b < 0 ? -m1 : m1;
 }
 
 // --------------------------------------------------------------- 2^x

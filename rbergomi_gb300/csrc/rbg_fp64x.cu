@@ -121,34 +121,37 @@ __device__ __forceinline__ void store_digits(const int64_t (&v)[4], unsigned cha
 // 2.  dig non-null (the fixed-point path pass follows): also the digits of W1,
 // zero past N and past B.  Streams s with bit s of fix set are stored as 64-bit
 // fixed point (unit 2^-59) in place of doubles.
-// A warp takes up to kSeg chunks of 16 steps of 8 paths' stream, four lanes a
-// path and four steps a lane, so a path's 16 values and each digit's 8 rows are
+// FORM 0: 64-bit integers; 1: FP32 Box-Muller; 2: doubles with all their bits significant
+// however small (box_muller_double), where no digits are asked for.
+// A warp takes up to kSeg chunks of 16 steps (forms 1 and 2 one where that leaves fewer warps
+// than the launch has: 1000 paths of 100 steps in FP32 39 -> 31 us a call) of 8 paths' stream, four lanes a path and four steps a lane, so a path's 16 values and each digit's 8 rows are
 // contiguous.  Integer instructions bound it: 330 a warp and pair of normals, 57
 // of them 32 x 32 -> 64 multiplies (four cycles each): the FMA-heavy pipe is 78 %
 // busy.  2 x 512 steps, 2^17 paths, left in fixed point: 0.84 ms, against 5.40 ms
 // for the same draw in FP64 (table-driven logarithm and sine, about 40 FP64
 // operations a pair).
 constexpr int kNormalThreads = 256, kSeg = 8;
-template <int F32>
-__global__ void __launch_bounds__(kNormalThreads, 4) k_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int ns,
+template <int FORM>
+__global__ void __launch_bounds__(kNormalThreads, FORM == 2 ? 3 : 4) k_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int ns,
                                                                     double* __restrict__ Z,
-                                                                    unsigned char* __restrict__ dig, int fix,
+                                                                    unsigned char* __restrict__ dig, int fix, int short_seg,
                                                                     const FixedTables* __restrict__ ft)
 {
     __shared__ NormalTables T;
-    if (!F32) {
+    if (FORM != 1) {
         TableCopy<kNormalThreads, (int)sizeof(NormalTables)>(&ft->normals).store(&T);
         __syncthreads();
     }
     const int lane = threadIdx.x & 31, g = lane & 3, pl = lane >> 2;
-    const int nch = (N + kXSteps - 1) / kXSteps, segs = (nch + kSeg - 1) / kSeg;
+    const int seg = FORM == 0 ? kSeg : short_seg;
+    const int nch = (N + kXSteps - 1) / kXSteps, segs = (nch + seg - 1) / seg;
     const int64_t tasks = (B + kXPaths - 1) / kXPaths * (kXPaths / 8) * ns * segs;
     const bool vec = (N & 1) == 0;
     const PhiloxKeys keys = philox_keys(seed);
     const int64_t warps = (int64_t)gridDim.x * (kNormalThreads / 32);
     for (int64_t t = blockIdx.x * (int64_t)(kNormalThreads / 32) + warp_index(); t < tasks; t += warps) {
         const int64_t r = t / segs;
-        const int c0 = (int)(t - r * segs) * kSeg, c1 = min(nch, c0 + kSeg);
+        const int c0 = (int)(t - r * segs) * seg, c1 = min(nch, c0 + seg);
         const int s = (int)(r % ns);
         const int64_t m = r / ns * 8 + pl;
         const bool valid = m < B, digits = s == 0 && dig != nullptr;
@@ -164,7 +167,10 @@ __global__ void __launch_bounds__(kNormalThreads, 4) k_normals_fixed(uint64_t se
             if (valid && j0 < N) {
                 const uint4 x = philox_group(keys, (uint64_t)(path0 + m), (uint32_t)(j0 >> 2), (uint32_t)s);
                 double z[4];
-                if (F32) {
+                if constexpr (FORM == 2) {
+                    box_muller_double(x.x, x.y, T, z[0], z[1]);
+                    box_muller_double(x.z, x.w, T, z[2], z[3]);
+                } else if constexpr (FORM == 1) {
                     float f0, f1, f2, f3;
                     box_muller_f32(x.x, x.y, f0, f1);
                     box_muller_f32(x.z, x.w, f2, f3);
@@ -175,10 +181,10 @@ __global__ void __launch_bounds__(kNormalThreads, 4) k_normals_fixed(uint64_t se
                     box_muller_fixed(x.x, x.y, T, v[0], v[1]);
                     box_muller_fixed(x.z, x.w, T, v[2], v[3]);
                 }
-                if ((fix >> s) & 1) {
+                if (FORM != 2 && ((fix >> s) & 1)) {
 #pragma unroll
                     for (int q = 0; q < 4; ++q) z[q] = __longlong_as_double(v[q]);
-                } else if (!F32) {
+                } else if (FORM == 0) {
 #pragma unroll
                     for (int q = 0; q < 4; ++q) z[q] = fixed_to_double(v[q]);
                 }
@@ -209,11 +215,12 @@ int launch_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int f32
     const FixedTables* ft = fixed_tables();
     if (!ft) return -1;
     const int nch = (N + kXSteps - 1) / kXSteps;
-    const int64_t tasks = (B + kXPaths - 1) / kXPaths * (kXPaths / 8) * ns * ((nch + kSeg - 1) / kSeg);
-    const int64_t need = (tasks + kNormalThreads / 32 - 1) / (kNormalThreads / 32);
-    const int64_t blocks = std::min<int64_t>(need, 8 * (int64_t)device_sms());
-    if (f32) k_normals_fixed<1><<<(unsigned)blocks, kNormalThreads, 0, st>>>(seed, path0, B, N, ns, Z, dig, fix, ft);
-    else k_normals_fixed<0><<<(unsigned)blocks, kNormalThreads, 0, st>>>(seed, path0, B, N, ns, Z, dig, fix, ft);
+    const int64_t rows = (B + kXPaths - 1) / kXPaths * (kXPaths / 8) * ns, most = 8 * (int64_t)device_sms();
+    int seg = kSeg;
+    auto need = [&] { return (rows * ((nch + seg - 1) / seg) + kNormalThreads / 32 - 1) / (kNormalThreads / 32); };
+    auto* kern = f32 ? k_normals_fixed<1> : dig ? k_normals_fixed<0> : k_normals_fixed<2>;
+    if ((f32 || !dig) && need() < most) seg = 1;
+    kern<<<(unsigned)std::min<int64_t>(need(), most), kNormalThreads, 0, st>>>(seed, path0, B, N, ns, Z, dig, fix, seg, ft);
     count_launch();
     return 0;
 }
