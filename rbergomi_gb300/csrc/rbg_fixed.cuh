@@ -181,6 +181,13 @@ RBG_HD uint64_t sqrt_fixed(uint64_t w)
     return wy + (mulhi64(c, wy) >> 19);
 }
 
+// The factors of a pair of normals.
+struct BoxMullerFactors {
+    uint64_t root;  // sqrt(-2 ln u0) 2^63 2^-e
+    int e;
+    uint64_t c, s;  // cosine and sine of 2 pi u1 less its quadrant, unit 2^-63
+};
+
 // Box-Muller of two 32-bit words, u0 = (a + 1/2) 2^-32, u1 = (b + 1/2) 2^-32:
 // sqrt(-2 ln u0) (cos, sin)(2 pi u1) in units of 2^-59, within 12.1 units and
 // 1.53 in root mean square (against quadruple precision; a double of that size
@@ -188,10 +195,13 @@ RBG_HD uint64_t sqrt_fixed(uint64_t w)
 // with the residual of w y^2, four rotation products and every series term to
 // 2^-60 (1.40 units): 0.91 -> 0.84 ms for k_normals_fixed's stated draw.  A second
 // table for the next nine bits of the angle saves four more and is slower (0.85).
-//
-// -2 ln u0 = w 2^-64 2^ex, w in [2^62, 2^64), ex even.
-RBG_HD void box_muller_log(uint32_t a, const NormalTables& T, uint64_t& w, int& ex)
+// Their factors are left in f where it is given.
+RBG_HD void box_muller_fixed(uint32_t a, uint32_t b, const NormalTables& T, int64_t& z0, int64_t& z1,
+                             BoxMullerFactors* f = nullptr)
 {
+    // -2 ln u0 = w 2^-64 2^ex, w in [2^62, 2^64), ex even
+    uint64_t w;
+    int ex;
     if (a - 1u >= 0xFFEFFFFFu) {
         if (a == 0u) {
             w = 0xB6FDA8B7905DF579ull;  // 66 ln 2 / 64
@@ -236,11 +246,8 @@ RBG_HD void box_muller_log(uint32_t a, const NormalTables& T, uint64_t& w, int& 
         w = shl(L, k);
         ex = c0 - k;
     }
-}
+    const uint64_t r = shr(sqrt_fixed(w), 3 - (ex >> 1));  // sqrt(-2 ln u0), unit 2^-60
 
-// Cosine and sine of 2 pi u1 less its quadrant, units 2^-63.
-RBG_HD void box_muller_angle(uint32_t b, const NormalTables& T, uint64_t& c, uint64_t& sn)
-{
     // 2 pi u1 = (quadrant) pi / 2 + pi k / 1024 + d, d = p pi 2^-32 with p = 2 (b mod 2^21) + 1
     const uint32_t p = 2u * (b & 0x1FFFFFu) + 1u;
     const FixedPair cs = T.trig[(b >> 21) & (kTrigTable - 1)];
@@ -256,17 +263,8 @@ RBG_HD void box_muller_angle(uint32_t b, const NormalTables& T, uint64_t& c, uin
     // (cos, sin)(a + d) = (x - x nc - y sd, y - y nc + x sd) in three products: with p = (x + y)(sd - nc) the
     // sine is y + p + x nc - y sd
     const uint64_t xn = mulhi64(cs.x, nc) >> 17, ys = mulhi64(cs.y, sd) >> 8;
-    c = cs.x - xn - ys;
-    sn = cs.y + (mulhi64((cs.x >> 1) + (cs.y >> 1), sd - (nc >> 9)) >> 7) + xn - ys;
-}
-
-RBG_HD void box_muller_fixed(uint32_t a, uint32_t b, const NormalTables& T, int64_t& z0, int64_t& z1)
-{
-    uint64_t w, c, sn;
-    int ex;
-    box_muller_log(a, T, w, ex);
-    const uint64_t r = shr(sqrt_fixed(w), 3 - (ex >> 1));  // sqrt(-2 ln u0), unit 2^-60
-    box_muller_angle(b, T, c, sn);
+    const uint64_t c = cs.x - xn - ys;  // unit 2^-63
+    const uint64_t sn = cs.y + (mulhi64((cs.x >> 1) + (cs.y >> 1), sd - (nc >> 9)) >> 7) + xn - ys;
     // quadrant q: (c, s), (-s, c), (-c, -s), (s, -c)
     const bool odd = (b & 0x40000000u) != 0u;
     const uint64_t m0 = mulhi64(r, odd ? sn : c), m1 = mulhi64(r, odd ? c : sn);  // unit 2^-59
@@ -274,6 +272,7 @@ RBG_HD void box_muller_fixed(uint32_t a, uint32_t b, const NormalTables& T, int6
     const uint64_t s1 = (uint64_t)(int64_t)((int32_t)b >> 31);               // sine in 2, 3
     z0 = (int64_t)((m0 ^ s0) - s0);
     z1 = (int64_t)((m1 ^ s1) - s1);
+    if (f) *f = BoxMullerFactors{sqrt_fixed(w), ex >> 1, c, sn};
 }
 
 // sin(q pi 2^-32), relative accuracy for any 0 < q < 2^31: fixed, unit 2^-63, is it to
@@ -294,22 +293,19 @@ RBG_HD double sine_double(uint32_t q, uint64_t fixed)
 RBG_HD void box_muller_double(uint32_t a, uint32_t b, const NormalTables& T, double& z0, double& z1)
 {
     int64_t v0, v1;
-    box_muller_fixed(a, b, T, v0, v1);
+    BoxMullerFactors f;
+    box_muller_fixed(a, b, T, v0, v1, &f);
     z0 = fixed_to_double(v0);
     z1 = fixed_to_double(v1);
     constexpr int64_t lim = 1ll << (kNormalBits - 3);
     const bool s0 = v0 < lim && v0 > -lim, s1 = v1 < lim && v1 > -lim;
     if (!s0 && !s1) return;
-    uint64_t w, c, sn;
-    int ex;
-    box_muller_log(a, T, w, ex);
-    box_muller_angle(b, T, c, sn);
     // the radius in two parts
-    const int64_t root = (int64_t)sqrt_fixed(w);
-    const double unit = bits_double((uint64_t)(uint32_t)(1023 - 63 + (ex >> 1)) << 52);
+    const int64_t root = (int64_t)f.root;
+    const double unit = bits_double((uint64_t)(uint32_t)(1023 - 63 + f.e) << 52);
     const double rh = (double)(root & ~0x3FFll) * unit, rl = (double)(root & 0x3FFll) * unit;
     const uint32_t q = 2u * (b & 0x3FFFFFFFu) + 1u;
-    const double cd = sine_double(0x80000000u - q, c), sd = sine_double(q, sn);
+    const double cd = sine_double(0x80000000u - q, f.c), sd = sine_double(q, f.s);
     const double x = fma(rh, cd, rl * cd), y = fma(rh, sd, rl * sd);
     const bool odd = (b & 0x40000000u) != 0u;
     const double m0 = odd ? y : x, m1 = odd ? x : y;

@@ -517,16 +517,17 @@ __device__ __forceinline__ void merge_round(PayoffSmem<MC>& sm, bool first, bool
 }
 
 // chunk c covers paths [c G 256, (c+1) G 256) of the batch, G per thread;
-// part[(c * n_out + i) * 4 + {0,1,2,3}] = (sum, comp, sum2, comp2).  A thread adds
-// up at most kPlainPaths paths in one FP64 sum; from the warps' sums on, every
-// rounding error is kept in the compensation.  (An FP64 warp instruction holds
-// its pipe for 64 cycles: the warps' sums are merged pairwise by one warp, another
-// one each task, in 16 of them, where plain additions in a row by the first warp were 8.
+// part[(c * n_out + i) * 4 + {0,1,2,3}] = (sum, comp, sum2, comp2).
+// ONE: a path a thread, the warps' sums added up by 16 threads (no comp).  Else a
+// thread adds up at most kPlainPaths paths in one FP64 sum, and from the warps' sums on
+// every rounding error is kept in the compensation.  An FP64 warp instruction holds
+// its pipe for 64 cycles: that merge is 16 of them by one warp, another one each
+// task, where ONE's is 8 and 2 us faster a call (2^16 paths x 5 outputs 22.9 / 24.9 us).
 // Three blocks an SM as the launcher asks for: left to itself the compiler takes 118
 // registers and two blocks, 2.66 ms for the grid of 8192 paths x 2112 outputs instead
-// of 2.48.)
+// of 2.48.
 // MC = 1: plain Monte Carlo payoff from (Ivdt, IsvdW) and ivp = IsvdWp.
-template <int MC>
+template <int MC, bool ONE>
 __global__ void __launch_bounds__(kPayThreads, 3) k_payoff_sums(Fp64Tables t, const double2* __restrict__ ivb, int64_t B,
                                                      int64_t stride, int G, double* __restrict__ part, int nchunks,
                                                      const double* __restrict__ ivp, const FixedTables* __restrict__ ft)
@@ -547,9 +548,9 @@ __global__ void __launch_bounds__(kPayThreads, 3) k_payoff_sums(Fp64Tables t, co
         double s[2 * kOPB];  // sums of x, then of x^2
 #pragma unroll
         for (int q = 0; q < 2 * kOPB; ++q) s[q] = 0.0;
-        const int sub1 = min(sub0 + kPlainPaths, G);
+        const int sub1 = ONE ? 1 : min(sub0 + kPlainPaths, G);
         for (int sub = sub0; sub < sub1; ++sub) {
-            const int64_t m = ((int64_t)c * G + sub) * 256 + threadIdx.x;
+            const int64_t m = ((int64_t)c * (ONE ? 1 : G) + sub) * 256 + threadIdx.x;
             if (m >= B) break;
             RtState r;
 #pragma unroll
@@ -567,9 +568,19 @@ __global__ void __launch_bounds__(kPayThreads, 3) k_payoff_sums(Fp64Tables t, co
         const double v = warp_sums16_f64(s);
         if (!(lane & 1)) sm.red[w][lane >> 1] = v;
         __syncthreads();
-        if (w == (int)(task & (kPayThreads / 32 - 1)))
+        if constexpr (ONE) {
+            const int q = threadIdx.x & (kOPB - 1), z = threadIdx.x / kOPB;
+            if (threadIdx.x < 2 * kOPB && o0 + q < t.n_out) {
+                double S = 0;
+                for (int k = 0; k < kPayThreads / 32; ++k) S += sm.red[k][threadIdx.x];
+                double* p = part + ((size_t)c * t.n_out + o0 + q) * 4 + 2 * z;
+                p[0] = S;
+                p[1] = 0.0;
+            }
+        } else if (w == (int)(task & (kPayThreads / 32 - 1))) {
             merge_round<MC>(sm, sub0 == 0, sub1 == G, part + ((size_t)c * t.n_out + o0) * 4, t.n_out - o0);
-        if (sub1 < G) {
+        }
+        if (!ONE && sub1 < G) {
             sub0 = sub1;
         } else {
             sub0 = 0;
@@ -594,20 +605,16 @@ static bool payoff_smem_ready(F* kern, size_t bytes, bool (&ready)[64])
 int launch_payoff_sums(const Fp64Tables& t, const double* ivb, int64_t B, int64_t stride, int G, double* part,
                        int nchunks, void* stream, const double* ivp)
 {
-    static bool ready[2][64] = {};
+    static bool ready[4][64] = {};
     const FixedTables* ft = fixed_tables();
     if (!ft) return -1;
     const int64_t tasks = (int64_t)nchunks * ((t.n_out + kOPB - 1) / kOPB);
     const unsigned grid = (unsigned)std::min<int64_t>(tasks, 3 * (int64_t)device_sms());
-    if (ivp) {
-        if (!payoff_smem_ready(k_payoff_sums<1>, sizeof(PayoffSmem<1>), ready[1])) return -1;
-        k_payoff_sums<1><<<grid, kPayThreads, sizeof(PayoffSmem<1>), (cudaStream_t)stream>>>(
-            t, (const double2*)ivb, B, stride, G, part, nchunks, ivp, ft);
-    } else {
-        if (!payoff_smem_ready(k_payoff_sums<0>, sizeof(PayoffSmem<0>), ready[0])) return -1;
-        k_payoff_sums<0><<<grid, kPayThreads, sizeof(PayoffSmem<0>), (cudaStream_t)stream>>>(
-            t, (const double2*)ivb, B, stride, G, part, nchunks, ivp, ft);
-    }
+    auto* kern = ivp ? (G == 1 ? k_payoff_sums<1, true> : k_payoff_sums<1, false>)
+                     : (G == 1 ? k_payoff_sums<0, true> : k_payoff_sums<0, false>);
+    const size_t smem = ivp ? sizeof(PayoffSmem<1>) : sizeof(PayoffSmem<0>);
+    if (!payoff_smem_ready(kern, smem, ready[(ivp ? 2 : 0) + (G == 1)])) return -1;
+    kern<<<grid, kPayThreads, smem, (cudaStream_t)stream>>>(t, (const double2*)ivb, B, stride, G, part, nchunks, ivp, ft);
     count_launch();
     return 0;
 }

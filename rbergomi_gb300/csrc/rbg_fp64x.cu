@@ -411,7 +411,6 @@ __device__ __forceinline__ void fused_variance(uint64_t (&x)[2][8], const X64Vol
     const int jc = min(j, N - 2), left = (int)min(B - m0, (int64_t)16);  // paths of the warp's 16
     const bool whole = left == 16 && __all_sync(0xffffffffu, in);
     if (left <= 0) return;
-    const int64_t back = slot_back(max(0, min(32, N - 1 - 32 * slot)));
     const uint64_t* z0 = fa.Z + m0 * NS * (int64_t)N + jc;
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
@@ -444,7 +443,7 @@ __device__ __forceinline__ void fused_variance(uint64_t (&x)[2][8], const X64Vol
                 s[2 * p + 1] = slot_product(mt, w1[p]);
                 if (NS == 3) sq[p] = slot_product(mt, wq[p]);
             }
-            const int64_t i0 = warp_sums_i64<8>(s) + back;  // value lane / 4 = 2 path + sum
+            const int64_t i0 = warp_sums_i64<8>(s) + (int)slot_back(__popc(__ballot_sync(0xffffffffu, in)));  // value lane / 4 = 2 path + sum
             const int pa = lane >> 3, c = (lane >> 2) & 1;
             const int tp = pa & 2 ? (pa & 1 ? top[3] : top[2]) : (pa & 1 ? top[1] : top[0]);
             const double sc = bits_double((uint64_t)(uint32_t)(tp + 1023) << 52);
@@ -452,7 +451,7 @@ __device__ __forceinline__ void fused_variance(uint64_t (&x)[2][8], const X64Vol
             const double r = (c ? (double)i0 * 0x1p-54 : (double)i0 * 0x1p-56 * sc) * sc;
             if (!(lane & 3) && 4 * h + pa < left) out[c] = r;
             if constexpr (NS == 3) {
-                const int64_t i2 = warp_sums_i64<4>(sq) + back;
+                const int64_t i2 = warp_sums_i64<4>(sq) + (int)slot_back(__popc(__ballot_sync(0xffffffffu, in)));
                 if (!(lane & 7) && 4 * h + pa < left) out[2] = (double)i2 * 0x1p-54 * sc;
             }
         }

@@ -5,7 +5,8 @@ is compensated.  In units of 2^-53 a rounding is 0.41 of the sum it ends in, roo
 mean square.  Eight additions in a row come to 0.72 of a thread's sum, 0.05 once
 averaged over 256 threads; the five levels of a warp's tree to 0.57, 0.20 over 8
 warps; both less by the root of the rounds of 8 paths a chunk has.  One FP64 sum of
-the warps' alone would leave 0.7 whatever the chunk."""
+the warps' alone would leave 0.7 whatever the chunk; with one path a thread it is all
+there is, as each 256 paths' sum of a longer chunk was before it was compensated."""
 import os
 import subprocess
 
@@ -27,5 +28,5 @@ def test_chunk_sums_keep_what_plain_sums_lose(tmp_path):
     rows = [line.split() for line in r.stdout.splitlines()]
     assert len(rows) == 8
     for mc, G, rms, most in rows:
-        limit = 0.2 if int(G) > 9 else 0.35
+        limit = 0.2 if int(G) > 9 else 0.35 if int(G) > 1 else 1.0
         assert float(rms) < limit, r.stdout
