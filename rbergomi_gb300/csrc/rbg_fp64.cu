@@ -410,10 +410,16 @@ __device__ __forceinline__ void payoff_outs(PayoffSmem<MC>& sm, const Fp64Tables
 // The tables, and the first task's outputs while they are on their way.  With 8-byte
 // loads a few at a time a block's first task waited 10 us longer: 2^16 paths x 5
 // outputs 32.8 -> 22.5 us.
-template <int MC>
+// DIRECT: the outputs alone, the tables stay where they are.
+template <int MC, bool DIRECT = false>
 __device__ __forceinline__ void payoff_start(PayoffSmem<MC>& sm, const Fp64Tables& t, int o0,
                                              const FixedTables* __restrict__ ft)
 {
+    if (DIRECT) {
+        payoff_outs<MC>(sm, t, o0);
+        __syncthreads();
+        return;
+    }
     const TableCopy<kPayThreads, kExpTable * 8> e(ft->exp2);
     const TableCopy<kPayThreads, MC ? 16 : (int)sizeof(MillsTable)> m(&ft->mills);
     payoff_outs<MC>(sm, t, o0);
@@ -452,11 +458,11 @@ __device__ __forceinline__ double payoff_rt(RtState& r, const OutF64& o, const d
 // log S = sum sqrt(v) sdt Z - dt/2 sum v = rho IsvdW + sqrt(1 - rho^2) IsvdWp
 // - Ivdt / 2, the same sum regrouped by normal stream; the exponential in fixed point.
 __device__ __forceinline__ double payoff_mc(const OutF64& o, const double2* __restrict__ ivb,
-                                            const double* __restrict__ ivp, size_t at, const PayoffSmem<1>& sm)
+                                            const double* __restrict__ ivp, size_t at, const uint64_t* E)
 {
     const double2 iv = ivb[at];
     const double lnS = o.rho * iv.y + o.om * ivp[at] - 0.5 * iv.x;
-    const double d = (fabs(lnS) < 60.0 ? exp2_fixed53(log2e_fixed53(lnS), sm.E) : exp(lnS)) - o.K;
+    const double d = (fabs(lnS) < 60.0 ? exp2_fixed53(log2e_fixed53(lnS), E) : exp(lnS)) - o.K;
     return d > 0.0 ? d : 0.0;
 }
 
@@ -559,7 +565,7 @@ __global__ void __launch_bounds__(kPayThreads, 3) k_payoff_sums(Fp64Tables t, co
                 if (o.vg < 0) continue;
                 const size_t at = (size_t)o.vg * stride + m;
                 double x;
-                if constexpr (MC) x = payoff_mc(o, ivb, ivp, at, sm);
+                if constexpr (MC) x = payoff_mc(o, ivb, ivp, at, sm.E);
                 else x = payoff_rt(r, o, ivb, at, sm);
                 s[q] += x;
                 s[kOPB + q] = fma(x, x, s[kOPB + q]);
@@ -1093,7 +1099,10 @@ int launch_implied_vol(int n, const double* price, const double* K, const double
 
 // ------------------------------------------------------------ quadrature
 // payoff[m * n_out + i]: tasks of 256 paths x nq <= 8 outputs.
-template <int MC>
+// DIRECT (plain Monte Carlo, a task a block): the exponential's table is read from
+// device memory, one entry a payoff; copying it first took longer than the rest (a call
+// of 64 paths of 16 steps x 5 outputs: 66 us with the table copied, 59 so).
+template <int MC, bool DIRECT>
 __global__ void __launch_bounds__(kPayThreads) k_payoff_store(Fp64Tables t, const double2* __restrict__ ivb, int64_t B,
                                int64_t stride, double* __restrict__ payoff, const double* __restrict__ ivp, int nq,
                                const FixedTables* __restrict__ ft)
@@ -1101,7 +1110,8 @@ __global__ void __launch_bounds__(kPayThreads) k_payoff_store(Fp64Tables t, cons
     extern __shared__ uint64_t psm[];
     PayoffSmem<MC>& sm = *reinterpret_cast<PayoffSmem<MC>*>(psm);
     const int64_t tiles = (B + kPayThreads - 1) / kPayThreads, tasks = tiles * ((t.n_out + nq - 1) / nq);
-    payoff_start<MC>(sm, t, (int)(blockIdx.x / tiles) * nq, ft);
+    payoff_start<MC, DIRECT>(sm, t, (int)(blockIdx.x / tiles) * nq, ft);
+    const uint64_t* E = DIRECT ? ft->exp2 : sm.E;
     for (int64_t task = blockIdx.x; task < tasks; task += gridDim.x) {
         const int o0 = (int)(task / tiles) * nq;
         const int64_t m = task % tiles * kPayThreads + threadIdx.x;
@@ -1117,7 +1127,7 @@ __global__ void __launch_bounds__(kPayThreads) k_payoff_store(Fp64Tables t, cons
             if (o.vg < 0) continue;
             const size_t at = (size_t)o.vg * stride + m;
             double x;
-            if constexpr (MC) x = payoff_mc(o, ivb, ivp, at, sm);
+            if constexpr (MC) x = payoff_mc(o, ivb, ivp, at, E);
             else x = payoff_rt(r, o, ivb, at, sm);
             payoff[m * t.n_out + o0 + q] = x;
         }
@@ -1127,23 +1137,20 @@ __global__ void __launch_bounds__(kPayThreads) k_payoff_store(Fp64Tables t, cons
 int launch_payoff_store(const Fp64Tables& t, const double* ivb, int64_t B, int64_t stride, double* payoff,
                         void* stream, const double* ivp)
 {
-    static bool ready[2][64] = {};
+    static bool ready[3][64] = {};
     const FixedTables* ft = fixed_tables();
     if (!ft) return -1;
     // fewer outputs a task where 8 would leave SMs idle
-    const int64_t tiles = (B + kPayThreads - 1) / kPayThreads;
+    const int64_t tiles = (B + kPayThreads - 1) / kPayThreads, most = 3 * (int64_t)device_sms();
     int nq = kOPB;
     while (nq > 1 && tiles * ((t.n_out + nq - 1) / nq) < 2 * (int64_t)device_sms()) nq >>= 1;
-    const unsigned grid = (unsigned)std::min<int64_t>(tiles * ((t.n_out + nq - 1) / nq), 3 * (int64_t)device_sms());
-    if (ivp) {
-        if (!payoff_smem_ready(k_payoff_store<1>, sizeof(PayoffSmem<1>), ready[1])) return -1;
-        k_payoff_store<1><<<grid, kPayThreads, sizeof(PayoffSmem<1>), (cudaStream_t)stream>>>(t, (const double2*)ivb, B,
-                                                                                             stride, payoff, ivp, nq, ft);
-    } else {
-        if (!payoff_smem_ready(k_payoff_store<0>, sizeof(PayoffSmem<0>), ready[0])) return -1;
-        k_payoff_store<0><<<grid, kPayThreads, sizeof(PayoffSmem<0>), (cudaStream_t)stream>>>(t, (const double2*)ivb, B,
-                                                                                             stride, payoff, ivp, nq, ft);
-    }
+    const int64_t tasks = tiles * ((t.n_out + nq - 1) / nq);
+    const bool direct = ivp && tasks <= most;
+    auto* kern = !ivp ? k_payoff_store<0, false> : direct ? k_payoff_store<1, true> : k_payoff_store<1, false>;
+    const size_t smem = ivp ? sizeof(PayoffSmem<1>) : sizeof(PayoffSmem<0>);
+    if (!payoff_smem_ready(kern, smem, ready[!ivp ? 0 : direct ? 2 : 1])) return -1;
+    kern<<<(unsigned)std::min(tasks, most), kPayThreads, smem, (cudaStream_t)stream>>>(t, (const double2*)ivb, B, stride,
+                                                                                     payoff, ivp, nq, ft);
     count_launch();
     return 0;
 }

@@ -182,6 +182,19 @@ def test_caller_normals_plain_mc(R):
     assert np.all(np.abs(p - q) <= 2e-13 * np.maximum(np.abs(q), 1.0))
 
 
+@pytest.mark.parametrize("M,n_out", [(1, 1), (255, 3), (257, 9), (3000, 40), (60000, 17)])
+def test_plain_mc_payoffs_small_and_large_calls(R, M, n_out):
+    """Calls whose payoff blocks read the exponential's table in place (a task a block)
+    and calls whose blocks copy it: the payoff of one output does not depend on the
+    others, nor on how many paths there are."""
+    Z = np.random.default_rng(M).standard_normal((M, 3, 4))
+    par = (XI, [0.1], [1.5], [-0.7])
+    p = R.payoffs_mc(*par, [1.0] * n_out, np.linspace(0.6, 1.4, n_out), Z, conv=R.CONV_DIRECT)
+    for i in (0, n_out - 1):
+        q = R.payoffs_mc(*par, [1.0], [np.linspace(0.6, 1.4, n_out)[i]], Z[:1], conv=R.CONV_DIRECT)
+        assert np.array_equal(p[:1, i], q[:, 0])
+
+
 @pytest.mark.parametrize("mc,n_t", [(False, 2), (False, 3), (True, 6), (True, 7)])  # around the last fused group count
 @pytest.mark.parametrize("N,M", [(2, 65), (31, 129), (33, 64), (161, 700), (1100, 130)])
 def test_variance_in_the_read_out(R, mc, n_t, N, M):
