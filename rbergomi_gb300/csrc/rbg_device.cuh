@@ -95,8 +95,9 @@ __device__ __forceinline__ uint4 philox_group(uint64_t seed, uint64_t p, uint32_
 // convolution, convolution with variance of 100 steps 111 -> 109).
 __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 
-// A table of BYTES from global to shared memory by THREADS threads, 16 bytes a
-// load, every load in flight at once: store() after what else there is to do.
+// A table of BYTES from global to shared memory (both on 16-byte boundaries) by THREADS
+// threads, 16 bytes a load, every load in flight at once: store() after what else
+// there is to do.
 template <int THREADS, int BYTES>
 struct TableCopy {
     static_assert(BYTES % 16 == 0, "whole 16-byte words");

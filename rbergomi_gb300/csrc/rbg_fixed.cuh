@@ -119,7 +119,7 @@ struct FixedPair {
     uint64_t x, y;
 };
 constexpr int kLnTable = 512, kTrigTable = 512, kLn2Table = 34;
-struct NormalTables {
+struct alignas(16) NormalTables {  // copied 16 bytes at a time
     FixedPair ln[kLnTable];
     FixedPair trig[kTrigTable];
     uint64_t ln2[kLn2Table];

@@ -538,7 +538,7 @@ __global__ void __launch_bounds__(kPayThreads, 3) k_payoff_sums(Fp64Tables t, co
                                                      int64_t stride, int G, double* __restrict__ part, int nchunks,
                                                      const double* __restrict__ ivp, const FixedTables* __restrict__ ft)
 {
-    extern __shared__ uint64_t psm[];
+    extern __shared__ __align__(16) uint64_t psm[];
     PayoffSmem<MC>& sm = *reinterpret_cast<PayoffSmem<MC>*>(psm);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t tasks = (int64_t)nchunks * ((t.n_out + kOPB - 1) / kOPB);
@@ -1107,7 +1107,7 @@ __global__ void __launch_bounds__(kPayThreads) k_payoff_store(Fp64Tables t, cons
                                int64_t stride, double* __restrict__ payoff, const double* __restrict__ ivp, int nq,
                                const FixedTables* __restrict__ ft)
 {
-    extern __shared__ uint64_t psm[];
+    extern __shared__ __align__(16) uint64_t psm[];
     PayoffSmem<MC>& sm = *reinterpret_cast<PayoffSmem<MC>*>(psm);
     const int64_t tiles = (B + kPayThreads - 1) / kPayThreads, tasks = tiles * ((t.n_out + nq - 1) / nq);
     payoff_start<MC, DIRECT>(sm, t, (int)(blockIdx.x / tiles) * nq, ft);

@@ -5,12 +5,18 @@
 // u0 takes over at 2^-12.
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <random>
 
 #include "rbg_fixed.cuh"
 
 using namespace rbg;
+
+// the kernels copy every table 16 bytes at a time, the normals' into shared memory of its type
+static_assert(alignof(NormalTables) % 16 == 0 && sizeof(NormalTables) % 16 == 0, "normals");
+static_assert(alignof(MillsTable) % 16 == 0 && offsetof(FixedTables, exp2) % 16 == 0 &&
+                  offsetof(FixedTables, mills) % 16 == 0, "exponential, tails");
 
 static FixedTables F;
 
