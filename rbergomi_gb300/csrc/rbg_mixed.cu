@@ -99,6 +99,7 @@ constexpr int kThreads = (kMmaWarp + 1) * 32;       // 544
 constexpr int kPassCols = 512;                      // TMEM: 128 lanes x 512 FP32 columns per pass
 constexpr int kMaxNp = 2 * kPassCols;               // two passes with the whole narrow strip resident
 constexpr int kMaxNpMulti = 8 * kPassCols;          // up to eight passes with streamed strip windows
+static_assert(kMaxNpMulti == kMixedMaxSteps, "room of a job's Philox entries");
 constexpr int kStripK = 16;                         // narrow strip width: one K = 16 MMA step
 // Pass mode 3 (below): 256-column passes in two TMEM buffers, and slots for
 // the cached A tiles the far-field MMAs read.
@@ -2292,7 +2293,7 @@ static cudaError_t allow_max_smem(void (*kern)(MixedArgs))
 }
 
 int mixed_prepare(const Plan& plan, const rbg_options& o, int64_t M, MixedJob& job, std::string& err,
-                  int64_t max_batch, bool mc, bool tile_cache)
+                  int64_t max_batch, bool mc, bool tile_cache, bool entries)
 {
     DevInfo dv;
     if (!device_info(&dv)) {
@@ -2350,7 +2351,7 @@ int mixed_prepare(const Plan& plan, const rbg_options& o, int64_t M, MixedJob& j
 
     size_t off = 256;  // the error word lives at offset 0
     job.off_err = 0;
-    if (backend == RBG_CONV_GEMM) {
+    if (backend == RBG_CONV_GEMM && entries) {
         job.off_ent = off;
         off += (size_t)2 * ns * (Np / 4) * sizeof(uint4);
         off = (off + 255) / 256 * 256;
@@ -2584,7 +2585,7 @@ int mixed_launch(const MixedJob& job, void* ws, uint64_t seed, int64_t path0, in
         A.sob = job.sob;
         A.ext = ext;
         mixed_set_seed(A, seed);
-        A.ent = (uint4*)(base + job.off_ent);
+        A.ent = job.ent ? job.ent : (uint4*)(base + job.off_ent);
         A.path0 = path0;
         A.B = B;
         int pm = job.backend == RBG_CONV_GEMM ? pass_mode(A.Np) : 0;
@@ -2680,7 +2681,7 @@ int mixed_jobs_prepare(const std::vector<MixedJobRef>& jobs, void* table, unsign
         A.dbg_x = nullptr;
         A.n_o = 0;
         mixed_set_seed(A, r.seed);
-        A.ent = (uint4*)((unsigned char*)r.ws + r.job->off_ent);
+        A.ent = r.job->ent ? r.job->ent : (uint4*)((unsigned char*)r.ws + r.job->off_ent);
         A.path0 = r.path0;
         A.B = r.B;
         A.jobs = nullptr;

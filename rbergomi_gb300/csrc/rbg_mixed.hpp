@@ -102,7 +102,10 @@ struct MixedJob {
     // past the uploaded image)
     int pmode = 0;
     size_t off_acache = 0;
-    size_t off_ent = 0;  // Philox entries, written by the kernel (inside the uploaded image, GEMM backend)
+    // Philox entries, written by the kernel (GEMM backend): inside the uploaded image, or at `ent` where
+    // mixed_prepare left them out (room for kMixedEntries)
+    size_t off_ent = 0;
+    uint4* ent = nullptr;
     std::vector<MixedLaunch> launches;   // one per (Volterra pass, <= 16 groups)
     std::vector<const void*> table_dev;  // optional device copies of each launch's strip / spectrum
     std::vector<unsigned char> host_ws;  // image uploaded by mixed_upload
@@ -110,9 +113,12 @@ struct MixedJob {
 
 // mc: the plain Monte Carlo estimator (a third normal stream; both backends, every pass mode).
 // tile_cache: pass mode 3 may be chosen (its A-tile cache, sms x up to 16 x
-// 16 KB of device memory, is part of workspace_bytes).
+// 16 KB of device memory, is part of workspace_bytes).  entries: the workspace holds
+// the Philox entries; without them the caller sets job.ent.
+constexpr int kMixedMaxSteps = 4096;                             // GEMM backend
+constexpr int kMixedEntries = 2 * 2 * (kMixedMaxSteps / 4);      // of a Romano-Touzi job, at most
 int mixed_prepare(const Plan& plan, const rbg_options& o, int64_t M, MixedJob& job, std::string& err,
-                  int64_t max_batch = 0, bool mc = false, bool tile_cache = true);
+                  int64_t max_batch = 0, bool mc = false, bool tile_cache = true, bool entries = true);
 // Byte range of launch i's strip (GEMM) or spectrum (FFT) inside host_ws, and
 // of the shared FFT twiddle table (empty for the GEMM backend).
 void mixed_table_range(const MixedJob& job, int i, size_t* off, size_t* bytes);

@@ -7,16 +7,17 @@
 // path.  rbg_price_rt_static serves them.  It runs the same mixed-form
 // kernels as rbg_price_rt (fused Philox + Volterra + variance kernel, FP32
 // payoffs, FP64 merges), but all of its scratch lives in one file-scope
-// __device__ array of kStaticScratchBytes (16 MiB), which every GPU that
-// loads this library holds until the process exits.
+// __device__ array of kStaticScratchBytes (16 MiB; and 64 KB for the path kernel's
+// Philox entries), which every GPU that loads this library holds until the process
+// exits.
 //
-// The device address of that array is looked up once per device, with the
+// The device addresses of the arrays are looked up once per device, with the
 // device current, on the first call on that device (cudaGetSymbolAddress).
-// The address stays cached for the life of the process, so a cudaDeviceReset
+// They stay cached for the life of the process, so a cudaDeviceReset
 // between calls is not supported.  Every call synchronises its stream to
 // return the prices, so none can run under stream capture.  All calls share the array and it keeps
-// the last call's contents; what must start at zero (the kernel error word
-// and the running sums) is cleared by every call.  Calls whose work overlaps
+// the last call's contents; what must start at zero (the kernel error
+// word) is cleared by every call, and the first batch overwrites the running sums.  Calls whose work overlaps
 // on the GPU race on the array, so callers serialise them (one stream, or
 // their own ordering).  A call that fails after it has queued work waits for
 // that work before it returns, so the next call never meets it on the array.
@@ -44,9 +45,15 @@ constexpr int kStaticMaxDevices = 64;
 constexpr int kStaticMaxOutputs = 4096;
 
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
+// The path kernel's Philox entries, beside the scratch that the jobs' limit is stated for (64 KB).
+static __device__ uint4 g_static_entries[kMixedEntries];
 
+struct StaticPtrs {
+    void* scratch = nullptr;
+    uint4* entries = nullptr;
+};
 static std::mutex g_static_mu;
-static void* g_static_ptr[kStaticMaxDevices] = {nullptr};
+static StaticPtrs g_static_ptr[kStaticMaxDevices];
 static thread_local std::string g_static_err;
 
 static int static_fail(int code, const std::string& msg)
@@ -55,8 +62,8 @@ static int static_fail(int code, const std::string& msg)
     return code;
 }
 
-// Device address of the scratch array on the current device (set-up once).
-static int static_scratch(void** out)
+// Device addresses of the two arrays on the current device (set-up once).
+static int static_scratch(StaticPtrs* out)
 {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -66,10 +73,11 @@ static int static_scratch(void** out)
     }
     if (dev < 0 || dev >= kStaticMaxDevices) return static_fail(RBG_ERR_UNSUPPORTED, "device ordinal beyond 63");
     std::lock_guard<std::mutex> lk(g_static_mu);
-    if (!g_static_ptr[dev]) {
-        void* ptr = nullptr;
-        e = cudaGetSymbolAddress((void**)&ptr, g_static_scratch);
-        if (e != cudaSuccess || !ptr) {
+    if (!g_static_ptr[dev].scratch) {
+        StaticPtrs ptr;
+        e = cudaGetSymbolAddress(&ptr.scratch, g_static_scratch);
+        if (e == cudaSuccess) e = cudaGetSymbolAddress((void**)&ptr.entries, g_static_entries);
+        if (e != cudaSuccess || !ptr.scratch || !ptr.entries) {
             cudaGetLastError();
             return static_fail(RBG_ERR_CUDA, std::string("cudaGetSymbolAddress(scratch): ") + cudaGetErrorString(e));
         }
@@ -102,8 +110,8 @@ int rbg_price_rt_static(const rbg_params* p, const rbg_options* o, double* price
     if (n_out > kStaticMaxOutputs)
         return static_fail(RBG_ERR_ARG, "par_size * op_size exceeds 4096 outputs of the static scratch");
     MixedJob job;
-    // the two-pass kernel without the A-tile cache, which would not fit the static scratch
-    int rc = mixed_prepare(plan, *o, p->M, job, err, 0, false, false);
+    // the two-pass kernel without the A-tile cache, which would not fit the static scratch; Philox entries outside it
+    int rc = mixed_prepare(plan, *o, p->M, job, err, 0, false, false, false);
     if (rc) return static_fail(rc, err);
 
     // carve the scratch: workspace image, output tables, sums, results,
@@ -134,9 +142,10 @@ int rbg_price_rt_static(const rbg_params* p, const rbg_options* o, double* price
             return static_fail(RBG_ERR_ARG, "variance groups / outputs of this job exceed the static scratch");
         B = std::max<int64_t>(chunk, (B / 2) / chunk * chunk);
     }
-    void* base = nullptr;
-    if ((rc = static_scratch(&base))) return rc;
-    unsigned char* s = (unsigned char*)base;
+    StaticPtrs ptr;
+    if ((rc = static_scratch(&ptr))) return rc;
+    unsigned char* s = (unsigned char*)ptr.scratch;
+    job.ent = ptr.entries;
     // a null stream means the calling thread's per-thread default stream, which
     // does not synchronise with the other streams of the process as the legacy
     // default stream would
