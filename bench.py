@@ -343,9 +343,9 @@ def run_gpu(args, w):
         return
     stage = R.STAGE_MIXED if prec == R.MIXED else R.STAGE_PATH_FP64
     kms, kn = R.profile_read(stage)
-    # the FP64 form's own path pass is two kernels a batch (convolution with the variance pass, its sums)
-    fp64_exact = prec != R.MIXED and args.conv == "auto" and 2 <= w["N"] <= 4096
-    if fp64_exact:
+    # the FP64 form's path pass as it ran: one kernel a launch, or a pair of them
+    fp64_path = R.profile_path()
+    if prec != R.MIXED and " + " in fp64_path:
         kn //= 2
     avg_kernel_ms = kms / max(kn, 1)
     bf16_peak, hbm_peak, peak_src = peaks()
@@ -355,10 +355,8 @@ def run_gpu(args, w):
     nc = Np // 32
     # split products on the tensor pipe: three (16-bit splits) or two (TF32 with one compensation term)
     exec_flops = (4.0 if args.split == 2 else 6.0) * 32 * 32 * nc * (nc + 1) / 2 * w["M"] / max(1, kn // args.steps)
-    fp64_fft = args.conv == "fft" or (args.conv == "auto" and 200 <= w["N"] <= 2048)
     kname = ("k_mixed_fft" if (args.conv == "fft" or (args.conv == "auto" and w["N"] > 1024))
-             else "k_mixed_gemm") if prec == R.MIXED else ("k_volterra_exact + k_slot_sums" if fp64_exact else
-                                                "k_path_fp64_fft" if fp64_fft else "k_path_fp64")
+             else "k_mixed_gemm") if prec == R.MIXED else fp64_path
     roof = {"bound": "tensor", "achieved": achieved_tf, "peak": bf16_peak, "unit": "TFLOP/s",
             "frac": achieved_tf / bf16_peak, "traffic": traffic_per_launch(kname, w),
             "kernel": kname,

@@ -321,6 +321,9 @@ int rbg_plan_info_unordered(const rbg_unordered* u, int* n_vol, int* n_vgroups, 
 void rbg_profile_enable(int on);
 void rbg_profile_reset(void);
 int rbg_profile_read(int stage, double* total_ms, uint64_t* launches);
+/* Kernels of the last profiled FP64 path pass (stage 1), "a + b" where a launch is
+ * a pair of them; empty before the first.  A static string. */
+const char* rbg_profile_path(void);
 
 /* Host<->device bytes copied by this thread's last rbg_price_rt* call. */
 void rbg_last_transfer_bytes(uint64_t* h2d, uint64_t* d2h);

@@ -67,7 +67,7 @@ EXPORTS = [
     "rbg_price_rt_unordered", "computeIV_tensor", "rbg_price_mc", "rbg_payoffs_mc", "rbg_generate_normals_streams",
     "rbg_plan_info_mc", "rbg_plan_info_unordered", "rbg_price_rt_cv", "rbg_price_rt_cv_normals",
     "rbg_price_rt_sobol", "rbg_sobol_normals", "rbg_debug_wait_timeout", "rbg_merge_sums",
-    "rbg_server_wait_timed",
+    "rbg_server_wait_timed", "rbg_profile_path",
 ]
 
 STAGE_NORMALS, STAGE_PATH_FP64, STAGE_MIXED, STAGE_PAYOFF, STAGE_REDUCE = 0, 1, 2, 3, 4
@@ -124,6 +124,7 @@ def lib():
         L.rbg_profile_reset.restype = None
         L.rbg_profile_read.argtypes = [C.c_int, _dp, C.POINTER(C.c_uint64)]
         L.rbg_profile_read.restype = C.c_int
+        L.rbg_profile_path.restype = C.c_char_p
         L.rbg_last_transfer_bytes.argtypes = [C.POINTER(C.c_uint64), C.POINTER(C.c_uint64)]
         L.rbg_last_transfer_bytes.restype = None
         _fp = C.POINTER(C.c_float)
@@ -517,6 +518,11 @@ def profile_read(stage: int):
     ms, n = C.c_double(), C.c_uint64()
     _check(lib().rbg_profile_read(int(stage), C.byref(ms), C.byref(n)))
     return ms.value, int(n.value)
+
+
+def profile_path() -> str:
+    """Kernels of the last profiled FP64 path pass ("a + b": a launch is a pair of them)."""
+    return lib().rbg_profile_path().decode()
 
 
 def last_transfer_bytes():

@@ -41,6 +41,7 @@ struct Prof {
     bool on = false;
     double ms[kStages] = {0};
     uint64_t n[kStages] = {0};
+    const char* path = "";  // kernels of the last profiled FP64 path pass
     std::vector<cudaEvent_t> pool;
     std::vector<std::tuple<int, cudaEvent_t, cudaEvent_t, int>> pending;
 };
@@ -68,6 +69,13 @@ struct ProfScope {
         g_prof.pending.emplace_back(stage, a, b, count);
     }
 };
+
+// Names the kernels of the FP64 form's path pass, while profiling is on.
+static void prof_path(const char* kernels)
+{
+    std::lock_guard<std::mutex> lk(g_prof.mu);
+    if (g_prof.on) g_prof.path = kernels;
+}
 
 // called after the stream that carried the pending events has synchronised
 static void prof_collect()
@@ -537,6 +545,8 @@ static int price_fp64(Ctx& c, const Plan& plan, const rbg_options& o, int64_t M,
         if ((rc = fp64_conv_log2(o.conv, N, &logL))) return rc;
         if ((rc = upload_tables(c, plan, st, ts, logL))) return rc;
     }
+    prof_path(!fixed ? (logL > 0 ? "k_path_fp64_fft" : "k_path_fp64")
+                     : (fused ? "k_volterra_exact + k_slot_sums" : "k_volterra_exact + k_variance_fixed"));
     unsigned int* err = (unsigned int*)(c.acc.as<double>() + 4 * no);
     if (fixed) RBG_CUDA(cudaMemsetAsync(err, 0, sizeof(unsigned int), st));
     bool wide = true;
@@ -1591,6 +1601,12 @@ void rbg_profile_reset(void)
 {
     std::lock_guard<std::mutex> lk(g_prof.mu);
     for (int i = 0; i < kStages; ++i) { g_prof.ms[i] = 0; g_prof.n[i] = 0; }
+}
+
+const char* rbg_profile_path(void)
+{
+    std::lock_guard<std::mutex> lk(g_prof.mu);
+    return g_prof.path;
 }
 
 int rbg_profile_read(int stage, double* total_ms, uint64_t* launches)
