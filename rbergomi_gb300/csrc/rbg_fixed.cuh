@@ -550,9 +550,23 @@ RBG_HD uint64_t half_square_log2(uint64_t d)
     const bool small = hi32(d) < (8u << (kTailBits - 32));
     const uint64_t x = small ? d << 3 : d;
     const uint64_t q = mulhi64(mulhi64(x, x), 0xB8AA3B295C17F0BCull);  // log2(e) / 2
-    return small ? (q + 6) >> 3 : (q < (900ull << 50) ? q << 3 : 900ull << 53);  // 900: phi below 2^-900
+    return small ? (q + 6) >> 3 : (q < (1023ull << 50) ? q << 3 : 1023ull << 53);  // at most 1023
 }
 constexpr int64_t kLog2Sqrt2Pi53 = 0x002A6C873498DDF7ll;  // log2(2 pi) / 2, unit 2^-53
+
+// S phi(d) for e = log2(S / sqrt(2 pi)): zero from half_square_log2(d) = lim on, where
+// it leaves the doubles' normal range (S phi below 2^-1022, or phi).
+constexpr RBG_HD uint64_t density_limit(int64_t e)
+{
+    constexpr int64_t top = (int64_t)1022 << 53;
+    return (uint64_t)(e < 0 ? top + e : top);
+}
+RBG_HD double density_fixed(int64_t e, uint64_t hs, uint64_t lim, const uint64_t* E)
+{
+    const bool in = hs < lim;
+    const double f = exp2_fixed53(e - (int64_t)(in ? hs : 0ull), E);
+    return in ? f : 0.0;
+}
 
 // The strike-independent parts of a conditional Black-Scholes call (tau = 1, r
 // = 0): spot and its logarithm, volatility and its reciprocal, and in fixed
@@ -560,6 +574,7 @@ constexpr int64_t kLog2Sqrt2Pi53 = 0x002A6C873498DDF7ll;  // log2(2 pi) / 2, uni
 struct SpotFixed {
     double S, lnS, vol, rv;
     int64_t volf, e;
+    uint64_t lim;  // density_limit(e)
 };
 
 // False where the numbers leave the ranges of the fixed-point form.
@@ -574,6 +589,7 @@ RBG_HD bool spot_fixed(double v2, double lnS, const uint64_t* E, SpotFixed& r)
     const int64_t l = log2e_fixed53(lnS);
     r.S = exp2_fixed53(l, E);
     r.e = l - kLog2Sqrt2Pi53;
+    r.lim = density_limit(r.e);
     return true;
 }
 
@@ -590,8 +606,7 @@ RBG_HD double call_fixed(const SpotFixed& r, double K, double lnK, const MillsTa
     const int64_t d2 = (n1 ? -(int64_t)x1 : (int64_t)x1) - r.volf;
     const bool n2 = d2 < 0;
     const uint64_t x2 = (uint64_t)(n2 ? -d2 : d2);
-    const int64_t e = r.e - (int64_t)half_square_log2(x1);
-    const double f = exp2_fixed53(e, E);
+    const double f = density_fixed(r.e, half_square_log2(x1), r.lim, E);
     const int64_t m1 = (int64_t)mills_fixed(x1, T), m2 = (int64_t)mills_fixed(x2, T);
     const double m = tail_to_double((n1 ? m1 : -m1) + (n2 ? -m2 : m2));
     return fma(f, m, (n1 ? 0.0 : r.S) - (n2 ? 0.0 : K));

@@ -794,6 +794,13 @@ struct OtmPrice {
     float d1d2;
 };
 
+// The price for |d1| above 37.6: below the doubles' normal range, which erfc still has.
+// (Not inlined: four copies of two erfc made the merge kernel 2 us longer.)
+__device__ __noinline__ double otm_far(double K, double d1, double v, bool put)
+{
+    return put ? fma(K, phi_cdf(v - d1), -phi_cdf(-d1)) : fma(-K, phi_cdf(d1 - v), phi_cdf(d1));
+}
+
 __device__ __forceinline__ OtmPrice otm_price(double K, double lnK, double v, bool put, const FixedTables* __restrict__ ft)
 {
     const double d1 = fma(-lnK, 1.0 / v, 0.5 * v);
@@ -803,11 +810,14 @@ __device__ __forceinline__ OtmPrice otm_price(double K, double lnK, double v, bo
     const bool n2 = d2 < 0;
     OtmPrice r;
     r.d1d2 = (float)d1 * ((float)d1 - (float)v);
-    r.f = exp2_fixed53(-kLog2Sqrt2Pi53 - (int64_t)half_square_log2(x1), ft->exp2);
+    const uint64_t hs = half_square_log2(x1);
+    constexpr uint64_t lim = density_limit(-kLog2Sqrt2Pi53);
+    r.f = density_fixed(-kLog2Sqrt2Pi53, hs, lim, ft->exp2);
     const int64_t m1 = (int64_t)mills_fixed(x1, ft->mills), m2 = (int64_t)mills_fixed((uint64_t)(n2 ? -d2 : d2), ft->mills);
     // call: [d1 >= 0] - K [d2 >= 0] + f (-+ M1 +- M2); put: less 1 - K, which only leaves K [d2 < 0]
     const double base = put ? (n2 ? K : 0.0) : (n1 ? 0.0 : 1.0);
     r.p = fma(r.f, tail_to_double((n1 ? m1 : -m1) + (n2 ? -m2 : m2)), base);
+    if (hs >= lim) r.p = otm_far(K, d1, v, put);
     return r;
 }
 
