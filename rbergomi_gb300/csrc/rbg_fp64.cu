@@ -807,7 +807,7 @@ __device__ __forceinline__ OtmPrice otm_price(double K, double lnK, double v, bo
     const bool n1 = d1 < 0.0;
     const uint64_t x1 = tail_fixed(d1);
     const int64_t d2 = (n1 ? -(int64_t)x1 : (int64_t)x1) - (int64_t)tail_fixed(v);
-    const bool n2 = d2 < 0;
+    const bool n2 = !put || d2 < 0;  // out of the money a call's d2 is negative, if only just
     OtmPrice r;
     r.d1d2 = (float)d1 * ((float)d1 - (float)v);
     const uint64_t hs = half_square_log2(x1);
@@ -889,7 +889,9 @@ __device__ double implied_vol_warp(double price, double K, double T, const IvSta
     const double target = put ? price - 1.0 + K : price;
     const double upper = put ? K : 1.0;
     const double nan = __longlong_as_double(0x7ff8000000000000ll);
-    if (!(target > 0.0) || !(target < upper) || !(T > 0.0)) return nan;
+    // (strikes and maturities that are NaN or infinite included)
+    constexpr double most = 1.7976931348623157e308;
+    if (!(target > 0.0) || !(target < upper) || !(T > 0.0) || !(T <= most) || !(K <= most)) return nan;
     const double lnK = st.lnK, sqT = st.sqT;
     const float lnK1 = st.lnK1, sqT32 = st.sqT32, K32 = (float)K, t32 = (float)target;
     double lo = 0.0, hi = 0.0, s = 0.0;

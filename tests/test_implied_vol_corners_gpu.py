@@ -49,3 +49,17 @@ def test_prices_below_the_normal_doubles(R):
     assert ok.sum() >= 10
     p = np.exp(log_price[ok])
     np.testing.assert_allclose(R.implied_vol(p, np.full(len(p), K), np.full(len(p), T)), s[ok], rtol=1e-8)
+
+
+def test_no_volatility_for_strikes_and_maturities_that_are_no_numbers(R):
+    nan, inf = np.nan, np.inf
+    P, K, T = (a.ravel() for a in np.meshgrid([1e-300, 1e-10, 0.3, 0.9999], [nan, inf, 1.5], [nan, inf, 1.0], indexing="ij"))
+    iv = R.implied_vol(P, K, T)
+    ok = (K == 1.5) & (T == 1.0)
+    assert np.all(np.isnan(iv[~ok]))
+    assert np.all(np.isfinite(iv[ok]))
+
+
+def test_at_the_money_with_a_vanishing_maturity(R):
+    """No volatility of the search's range reaches a price above 1e-15 in 1e-300 years."""
+    assert np.all(np.isnan(R.implied_vol([1e-15, 1e-10, 0.3, 0.9999], np.ones(4), np.full(4, 1e-300))))
