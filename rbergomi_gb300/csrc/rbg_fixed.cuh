@@ -596,7 +596,7 @@ RBG_HD bool spot_fixed(double v2, double lnS, const uint64_t* E, SpotFixed& r)
 // The call at strike K.  With S phi(d1) = K phi(d2) and 1 - Phi(x) = phi(x) M(x)
 // it is
 //   [d1 >= 0] S - [d2 >= 0] K + S phi(d1) (-+ M(|d1|) +- M(|d2|)):
-// one exponential, tails that keep their relative accuracy, and eight FP64
+// one exponential, tails that keep their relative accuracy, and nine FP64
 // operations with the caller's two sums.
 RBG_HD double call_fixed(const SpotFixed& r, double K, double lnK, const MillsTable& T, const uint64_t* E)
 {

@@ -369,11 +369,12 @@ void launch_path_fp64(const Fp64Tables& t, const double* Z, int64_t B, double* i
 
 // ------------------------------------------------------------ payoff sums
 // The conditional Black-Scholes call by Mills' ratio, the exponential and the
-// square root in fixed point (rbg_fixed.cuh): eight FP64 operations an output
-// and path, the strike-independent parts shared, against about 250 for library
+// square root in fixed point (rbg_fixed.cuh): 14 FP64 instructions an output and
+// path with the sums (counted; the FP64 pipe is 82 % busy), the strike-independent
+// parts shared, against about 250 for library
 // log, exp, sqrt and two erfc each time (FP64 pipe: 64 cycles a warp
 // operation).  Blocks keep both tables in shared memory (50 KB) and walk over
-// (chunk, run of 8 outputs) tasks.  2^17 paths x 21 outputs: 1.17 -> 0.095
+// (chunk, run of 8 outputs) tasks.  2^17 paths x 21 outputs: 1.17 -> 0.094
 // ms; 8192 paths x 2112 outputs: 7.06 -> 0.49 ms.
 constexpr int kOPB = 8;  // outputs per task
 constexpr int kPayThreads = 256;
