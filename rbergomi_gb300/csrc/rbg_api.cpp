@@ -990,21 +990,36 @@ static int price_cv_any(const rbg_cv_params* p, const rbg_options* o, const doub
     return price_cv(*c, plan, *p, *o, Zc, Z, st, res.data());
 }
 
-// Whether a quadrature call of M paths is large enough for the digit convolution.
-// Its kernels fill a path block of 128 steps and start one after the other, about
-// 35 us and 0.04 us a step and pass more than the FP64 path kernel's single launch while
-// that one's paths fit the chip at once; from there the FP64 pipe (two operations a clock and
-// SM, 6e11 a second) decides.  Per path and step the FP64 kernel takes half the
-// steps (direct, both rounded to 32) or 74 (FFT of L points, L / 2 steps) operations a pass and
-// about 44 (plain MC 60) a variance group.  The call on device pointers, digits against FP64
-// kernels: 64 steps, 2000 paths 84 / 64 us, 8000 paths 87 / 120; 100 steps, 1000
-// paths 98 / 68, 4000 paths 101 / 151; 512 steps, 256 paths 203 / 146, 1000
-// paths 202 / 239; 3 passes of 512 steps, 256 paths 366 / 320, 1000 paths 380 / 533.
+// Whether a quadrature call of M paths goes through the digit convolution, by the two
+// forms' times in microseconds beyond what they share, fitted to 478 calls on device
+// pointers (1 to 4096 steps, 1 to 16000 paths, 1 to 1000 H, 1 to 8 groups each; the choice costs
+// 0.4 % of the better form on average, at most 20 %).
+// FP64 kernel: one launch.  The paths the chip holds at once take the time of one, half the
+// steps (direct sum, steps rounded to 32) or a transform (FFT of L points, L / 2 steps) a
+// pass and step; the FP64 pipe, 6.1e11 operations a second, takes the rest.
+// Digits: four launches, then for each pass the blocks of 128 steps of a path group
+// one after the other, with 64 and with 256 paths at full weight.
+// Digits against FP64 kernel: 64 steps, 2000 paths 84 / 64 us, 8000 paths 87 / 120; 100
+// steps, 1000 paths 98 / 68, 4000 paths 101 / 151; 512 steps, 256 paths 203 / 146, 1000 paths
+// 202 / 239; 2048 steps, 1 path 301 / 508; 4096 steps, 1 path 530 / 10900; 100 H of
+// 100 steps, 64 paths 1670 / 3070.
 static bool quadrature_by_digits(const Plan& plan, int64_t M, int ns, int logL)
 {
-    const double nv = (double)plan.vols.size(), ng = (double)plan.vgs.size(), up = (plan.N + 31) / 32 * 32;
-    const double steps = logL > 0 ? (double)(1 << (logL - 1)) : up, conv = logL > 0 ? 74.0 : 0.5 * up + 16.0;
-    return (double)M * steps * (nv * conv + ng * (ns == 3 ? 60.0 : 44.0)) >= 2.4e7 + 4.9e4 * plan.N * nv;
+    const double N = plan.N, nv = (double)plan.vols.size(), ng = (double)plan.vgs.size(), m = (double)M;
+    const double up = (plan.N + 31) / 32 * 32, group = ns == 3 ? 60.0 : 44.0;
+    double one, rest;
+    if (logL > 0) {
+        const double s = (double)(1 << (logL - 1));
+        one = s * (0.05 + 0.15 * nv + 0.02 * ng);
+        rest = std::max(0.0, m - 200.0) * s * (24.0 + 50.0 * nv + group * ng);
+    } else {
+        one = nv * (2.0 + 0.0011 * up * up) + 0.075 * ng * up;
+        rest = std::max(0.0, m - 1216.0) * up * (nv * (0.5 * N + 32.0) + group * ng);
+    }
+    const double a = std::min(1.0, m / 64.0), b = std::min(1.0, m / 256.0);
+    const double digits = 34.0 + N * (0.05 + 0.03 * a) + nv * (2.0 + 3.0 * a + N * (0.04 + 0.09 * a + 0.05 * b)) + (ng - nv) +
+                          m * N * (2.3e-5 * nv + 4e-6 * ng);
+    return digits < one + rest / 6.1e5;
 }
 
 static int payoffs_quadrature(const rbg_params* p, const double* Z, double* payoff, int device_ptrs,

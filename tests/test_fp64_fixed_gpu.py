@@ -166,12 +166,18 @@ def test_caller_normals_out_of_range_take_the_backend_of_their_length(R, N, fft,
 
 
 def test_small_quadrature_calls_take_the_fp64_kernels(R):
-    """Few paths: the FP64 path kernel's one launch, its results bit for bit."""
+    """Few paths of few steps: the FP64 path kernel's one launch, its results bit for bit."""
     for N, M, conv in ((2, 500, R.CONV_DIRECT), (64, 1000, R.CONV_DIRECT), (199, 100, R.CONV_DIRECT),
                        (200, 400, R.CONV_FFT), (512, 130, R.CONV_FFT)):
         Z = np.random.default_rng(N).standard_normal((M, 2, N))
         args = (XI, [0.1], [1.5], [-0.7], [1.0], [1.0], Z)
         assert np.array_equal(R.payoffs_rt(*args), R.payoffs_rt(*args, conv=conv))
+    # and not where a path alone takes long: one path of 4096 steps 0.5 ms by digits, 10.9 in FP64
+    for N, M, conv in ((700, 1, R.CONV_FFT), (2048, 1, R.CONV_FFT), (2049, 1, R.CONV_DIRECT), (4096, 5, R.CONV_DIRECT)):
+        Z = np.random.default_rng(N).standard_normal((M, 2, N))
+        args = (XI, [0.1, 0.2], [1.5, 1.0], [-0.7, -0.5], [1.0, 1.0], [0.8, 1.0], Z)
+        p, q = R.payoffs_rt(*args), R.payoffs_rt(*args, conv=conv)
+        assert not np.array_equal(p, q) and np.all(np.abs(p - q) <= 1e-12)
 
 
 def test_caller_normals_plain_mc(R):

@@ -101,7 +101,7 @@ def test_more_passes_than_kept_panels(R, ext):
     n = 35000
     par = (0.04, np.linspace(0.05, 0.45, n), np.full(n, 1.5), np.full(n, -0.7), [1.0], [1.0])
     if ext:
-        Z = np.random.default_rng(3).standard_normal((512, 2, 16))  # paths enough for the digits
+        Z = np.random.default_rng(3).standard_normal((64, 2, 100))  # steps enough for the digits
         p, q = R.payoffs_rt(*par, Z), R.payoffs_rt(*par, Z, conv=R.CONV_DIRECT)
         assert np.all(np.abs(p - q) <= 2e-13 * np.maximum(np.abs(q), 1.0))
     else:
