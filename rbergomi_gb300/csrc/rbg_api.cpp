@@ -1335,7 +1335,7 @@ int rbg_generate_normals_streams(uint64_t seed, int64_t path_offset, int64_t M, 
     for (int64_t m0 = 0; m0 < M; m0 += B) {
         const int64_t b = std::min(B, M - m0);
         if (launch_normals_fixed(seed, path_offset + m0, b, N, precision == RBG_MIXED, c->z.as<double>(), nullptr, 0, ns,
-                                 c->stream))
+                                 c->stream, true))
             return fail(RBG_ERR_CUDA, "fixed-point tables not found on the device");
         RBG_CUDA(cudaGetLastError());
         RBG_CUDA(cudaMemcpyAsync(Z + m0 * ns * N, c->z.p, sizeof(double) * ns * N * b, cudaMemcpyDeviceToHost,

@@ -122,7 +122,7 @@ __device__ __forceinline__ void store_digits(const int64_t (&v)[4], unsigned cha
 // zero past N and past B.  Streams s with bit s of fix set are stored as 64-bit
 // fixed point (unit 2^-59) in place of doubles.
 // FORM 0: 64-bit integers; 1: FP32 Box-Muller; 2: doubles with all their bits significant
-// however small (box_muller_double), where no digits are asked for.
+// however small (box_muller_double; a draw takes 1.8 times as long).
 // A warp takes up to kSeg chunks of 16 steps (forms 1 and 2 one where that leaves fewer warps
 // than the launch has: 1000 paths of 100 steps in FP32 39 -> 31 us a call) of 8 paths' stream, four lanes a path and four steps a lane, so a path's 16 values and each digit's 8 rows are
 // contiguous.  Integer instructions bound it: 330 a warp and pair of normals, 57
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(kNormalThreads, FORM == 2 ? 3 : 4) k_normals_f
 }
 
 int launch_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int f32, double* Z, unsigned char* dig, int fix,
-                         int ns, cudaStream_t st)
+                         int ns, cudaStream_t st, bool exact)
 {
     const FixedTables* ft = fixed_tables();
     if (!ft) return -1;
@@ -218,8 +218,8 @@ int launch_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int f32
     const int64_t rows = (B + kXPaths - 1) / kXPaths * (kXPaths / 8) * ns, most = 8 * (int64_t)device_sms();
     int seg = kSeg;
     auto need = [&] { return (rows * ((nch + seg - 1) / seg) + kNormalThreads / 32 - 1) / (kNormalThreads / 32); };
-    auto* kern = f32 ? k_normals_fixed<1> : dig ? k_normals_fixed<0> : k_normals_fixed<2>;
-    if ((f32 || !dig) && need() < most) seg = 1;
+    auto* kern = f32 ? k_normals_fixed<1> : exact ? k_normals_fixed<2> : k_normals_fixed<0>;
+    if ((f32 || exact) && need() < most) seg = 1;
     kern<<<(unsigned)std::min<int64_t>(need(), most), kNormalThreads, 0, st>>>(seed, path0, B, N, ns, Z, dig, fix, seg, ft);
     count_launch();
     return 0;

@@ -66,8 +66,10 @@ const FixedTables* fixed_tables();
 // fixed point, unit 2^-59, in place of doubles: kFixAll for the fused pass, kFixW1perp
 // for the separate one, whose FP64 sums take the doubles.
 constexpr int kFixAll = 7, kFixW1perp = 2;
+// exact: doubles with all their bits significant however small (f32 = 0, no digits), for
+// normals that leave the library; a unit of 2^-59 is all the pricing sums need.
 int launch_normals_fixed(uint64_t seed, int64_t path0, int64_t B, int N, int f32, double* Z, unsigned char* dig, int fix,
-                         int ns, cudaStream_t st);
+                         int ns, cudaStream_t st, bool exact = false);
 void launch_panels(const int64_t* gam, int nv, int N, unsigned char* panels, cudaStream_t st);
 // Digits of the caller's W1; *flag |= 1 where W1 or W1perp is kExtMax or more in
 // size, or NaN.
