@@ -411,6 +411,10 @@ __device__ __forceinline__ void fused_variance(uint64_t (&x)[2][8], const X64Vol
     const int jc = min(j, N - 2), left = (int)min(B - m0, (int64_t)16);  // paths of the warp's 16
     const bool whole = left == 16 && __all_sync(0xffffffffu, in);
     if (left <= 0) return;
+    // what the live steps lose goes back (28 of 32); counted where it is used, as a register
+    // held over the loops costs spills, and with several groups or sums only where the slot is partial
+    // (2 groups a pass, 16 steps, 3 passes 2.78 -> 2.73 ms; with one group it is 1.15 times slower)
+    auto back = [&] { return !ONE && whole ? 28 : (int)slot_back(__popc(__ballot_sync(0xffffffffu, in))); };
     const uint64_t* z0 = fa.Z + m0 * NS * (int64_t)N + jc;
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
@@ -443,7 +447,7 @@ __device__ __forceinline__ void fused_variance(uint64_t (&x)[2][8], const X64Vol
                 s[2 * p + 1] = slot_product(mt, w1[p]);
                 if (NS == 3) sq[p] = slot_product(mt, wq[p]);
             }
-            const int64_t i0 = warp_sums_i64<8>(s) + (int)slot_back(__popc(__ballot_sync(0xffffffffu, in)));  // value lane / 4 = 2 path + sum
+            const int64_t i0 = warp_sums_i64<8>(s) + back();  // value lane / 4 = 2 path + sum
             const int pa = lane >> 3, c = (lane >> 2) & 1;
             const int tp = pa & 2 ? (pa & 1 ? top[3] : top[2]) : (pa & 1 ? top[1] : top[0]);
             const double sc = bits_double((uint64_t)(uint32_t)(tp + 1023) << 52);
@@ -451,7 +455,7 @@ __device__ __forceinline__ void fused_variance(uint64_t (&x)[2][8], const X64Vol
             const double r = (c ? (double)i0 * 0x1p-54 : (double)i0 * 0x1p-56 * sc) * sc;
             if (!(lane & 3) && 4 * h + pa < left) out[c] = r;
             if constexpr (NS == 3) {
-                const int64_t i2 = warp_sums_i64<4>(sq) + (int)slot_back(__popc(__ballot_sync(0xffffffffu, in)));
+                const int64_t i2 = warp_sums_i64<4>(sq) + back();
                 if (!(lane & 7) && 4 * h + pa < left) out[2] = (double)i2 * 0x1p-54 * sc;
             }
         }
